@@ -19,7 +19,7 @@ LIB_PATH = os.path.join(PKG_DIR, "libfastlstm_b200.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
-    "-Xcompiler", "-fPIC", "-shared",
+    "-Xcompiler", "-fPIC", "-shared", "--threads", "0",     # one compiler process per source file
 ]
 
 

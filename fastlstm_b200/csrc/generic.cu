@@ -11,6 +11,7 @@
 // hand h[t] (or d_ifgo[t]) to their peers through global memory, one int32
 // arrival counter per (step, batch tile), every wait bounded.
 #include "generic.cuh"
+#include "sm100.cuh"
 
 namespace blstm {
 
@@ -566,7 +567,10 @@ fused_fwd_kernel(int Tn, int B, int I, int H, int inference, const T* __restrict
 bool generic_fused_fwd_supported(const blstm_desc& d) {
   if (d.flags & BLSTM_FLAG_NO_FUSED) return false;
   const int size = d.hidden_size > d.input_size ? d.hidden_size : d.input_size;
-  return size <= (d.dtype == BLSTM_F32 ? 32 : 64);
+  if (d.dtype == BLSTM_F32) return size <= 32;
+  // 16-bit: a step takes 3.2 us here against 0.5 us in the small-batch recurrence (H = 64), whose projection and second
+  // launch cost some 10 us: a few steps, and sizes the tcgen05 projection does not take.
+  return size <= 64 && (d.seq_len <= 12 || !sm100_gemm_supported(d));
 }
 
 template <typename T>

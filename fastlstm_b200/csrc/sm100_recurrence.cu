@@ -29,6 +29,7 @@
 #include "sm100.cuh"
 #include "sm100_common.cuh"
 #include "sm100_rec_util.cuh"
+#include "sm100_small.cuh"
 
 namespace blstm {
 namespace sm100 {
@@ -1758,13 +1759,18 @@ static int launch_bwd_t(const BwdPlan& pl, const CUtensorMap& tw, const CUtensor
 using namespace sm100;
 
 bool sm100_recurrence_supported(const blstm_desc& d, int phase) {
+  if (small_plan(d, phase).ok) return true;
   return phase == BLSTM_PHASE_BWD ? make_bwd_plan(d).ok : make_plan(d, phase).ok;
 }
 size_t sm100_recurrence_workspace(const blstm_desc& d, int phase) {
+  const SmallPlan sp = small_plan(d, phase);
+  if (sp.ok) return small_workspace(d, sp, phase);
   return phase == BLSTM_PHASE_BWD ? make_bwd_plan(d).ws_bytes : make_plan(d, phase).ws_bytes;
 }
 
 int sm100_plan_detail(const blstm_desc& d, int phase, char* buf, size_t n) {
+  const SmallPlan sp = small_plan(d, phase);
+  if (sp.ok) return small_plan_detail(d, sp, phase, buf, n);
   if (phase == BLSTM_PHASE_BWD) {
     const BwdPlan p = make_bwd_plan(d);
     if (!p.ok) return 0;
@@ -1777,9 +1783,6 @@ int sm100_plan_detail(const blstm_desc& d, int phase, char* buf, size_t n) {
   }
   const RecPlan p = make_plan(d, phase);
   if (!p.ok) return 0;
-  if (sm100_fwd_cluster_shape(d))
-    return snprintf(buf, n, "sm100 fwd cluster=%d (one per batch tile, h handed over in shared memory) UH=16 TI=1 grid=%d "
-                    "threads=288 wh=resident", d.hidden_size / 16, d.hidden_size / 16 * p.nbt);
   char wh[48];
   if (p.ws) snprintf(wh, sizeof(wh), "%d/%d chunks resident, rest streamed", p.kr, d.hidden_size / RK);
   else snprintf(wh, sizeof(wh), "resident");
@@ -1789,6 +1792,8 @@ int sm100_plan_detail(const blstm_desc& d, int phase, char* buf, size_t n) {
 
 int sm100_fwd_recurrence(const blstm_desc& d, void* ifgo, const void* Wh, void* out, void* cell, void* ws,
                          size_t ws_bytes, cudaStream_t st) {
+  const SmallPlan sp = small_plan(d, BLSTM_PHASE_FWD);
+  if (sp.ok) return small_fwd_recurrence(d, sp, ifgo, Wh, out, cell, ws, st);
   const RecPlan pl = make_plan(d, BLSTM_PHASE_FWD);
   if (!pl.ok) return BLSTM_E_UNSUPPORTED;
   if (ws_bytes < pl.ws_bytes) return BLSTM_E_WORKSPACE;
@@ -1825,11 +1830,6 @@ int sm100_fwd_recurrence(const blstm_desc& d, void* ifgo, const void* Wh, void* 
     }
   }
   BLSTM_CUDA_OK(cudaMemsetAsync(ws, 0, pl.ws_bytes, st));
-  {  // small hidden sizes with few batch tiles: hand-off inside one cluster per tile
-    bool taken = false;
-    rc = sm100_fwd_cluster(d, ifgo, Wh, out, cell, ws, st, &taken);
-    if (rc || taken) return rc;
-  }
   FwdParams p;
   p.npb = pl.npb;
   p.ep_bytes = (int)pl.ep_bytes;
@@ -1873,6 +1873,8 @@ int sm100_fwd_recurrence(const blstm_desc& d, void* ifgo, const void* Wh, void* 
 int sm100_bwd_recurrence(const blstm_desc& d, const void* dout, const void* dh_n, const void* dc_n,
                          const void* ifgo, const void* cell, const void* Wh, void* d_ifgo, void* dh0, void* dc0,
                          float* db, void* ws, size_t ws_bytes, cudaStream_t st) {
+  const SmallPlan sp = small_plan(d, BLSTM_PHASE_BWD);
+  if (sp.ok) return small_bwd_recurrence(d, sp, dout, dh_n, dc_n, ifgo, cell, Wh, d_ifgo, dh0, dc0, db, ws, st);
   const BwdPlan pl = make_bwd_plan(d);
   if (!pl.ok) return BLSTM_E_UNSUPPORTED;
   if (ws_bytes < pl.ws_bytes) return BLSTM_E_WORKSPACE;

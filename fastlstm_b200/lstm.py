@@ -247,18 +247,21 @@ def Wgrad(d_ifgo, x, h):
 
 # ---------------------------------------------------------------------------
 # Ragged 16-bit shapes on the tensor-core kernels: TMA wants 16-byte row pitches (I % 8 == 0) and the
-# tcgen05 recurrences hidden sizes in multiples of 64.  Other shapes are zero-padded on the host: a padded
+# tcgen05 recurrences hidden sizes in multiples of 64 (small batches: of 8).  Other shapes are zero-padded on the host: a padded
 # hidden unit has zero weights, bias and state, so its pre-activations are 0, its cell and output stay
 # exactly 0 and it feeds nothing into the real units; padded input columns meet zero weights.  The
 # padded copies cost a few small kernels per call - far less than the CUDA-core kernels they replace.
 # ---------------------------------------------------------------------------
-def _padded_sizes(dtype, I, H):
-    """(Ip, Hp) when the layer should run zero-padded on the tensor-core kernels, else None."""
+def _padded_sizes(dtype, I, H, T=1, B=None):
+    """(Ip, Hp) when the layer should run zero-padded on the tensor-core kernels, else None.  With a
+    batch size: hidden sizes in multiples of 8 where the small-batch recurrences take them."""
     if dtype not in (torch.float16, torch.bfloat16) or _FORCE_GENERIC:
         return None
-    if max(I, H) <= 64:                       # tiny sizes have the fused kernel
+    if max(I, H) <= 64 and T <= 12:           # tiny sizes have the fused kernel
         return None
-    Ip, Hp = -(-I // 8) * 8, -(-H // 64) * 64
+    Ip, Hp = -(-I // 8) * 8, -(-H // 8) * 8
+    if B is None or any(plan_name(dtype, T, B, Ip, Hp, phase) != "sm100" for phase in ("fwd", "bwd")):
+        Hp = -(-H // 64) * 64
     if (Ip, Hp) == (I, H) or Hp > 2048:
         return None
     return Ip, Hp
@@ -304,7 +307,7 @@ class PersistentLSTMfn(torch.autograd.Function):
             c_0 = None if c_0 is None else c_0.to(target)
         x = x.contiguous()
         I, H = x.shape[-1], Wh.shape[1]
-        ctx.pad = _padded_sizes(x.dtype, I, H)
+        ctx.pad = _padded_sizes(x.dtype, I, H, x.shape[0], x.shape[1])
         ctx.sizes = (I, H)
         if ctx.pad is not None:
             Ip, Hp = ctx.pad

@@ -58,13 +58,13 @@ enum {
                                    out[1..T] and cell[T] are still produced.  Halves the bytes a
                                    step moves (5*B*H*e instead of 10*B*H*e). */
   BLSTM_FLAG_NO_FUSED = 32,     /* blstm_fwd: do not use the single-kernel forward (projection inside the
-                                   time loop) that tiny sizes (max(H, I) <= 32 in fp32, <= 64 in 16 bit)
-                                   otherwise get; for comparisons and tests */
+                                   time loop) that tiny sizes (max(H, I) <= 32 in fp32; <= 64 in 16 bit
+                                   with at most a dozen steps) otherwise get; for comparisons and tests */
   BLSTM_FLAG_HALF_DEVICE = 128, /* recurrences: plan for half of the SMs, so that two persistent kernels (two
                                    layers of a stack working on neighbouring time chunks) fit side by side */
-  BLSTM_FLAG_NO_CLUSTER = 16,   /* forward: do not use the cluster hand-off kernel that small hidden
-                                   sizes (H = 64, 128, 256 with at most 7 batch tiles) otherwise get;
-                                   for comparisons and tests */
+  BLSTM_FLAG_NO_CLUSTER = 16,   /* recurrences: do not use the small-batch kernels (weights and hand-off
+                                   inside one cluster) that 16-bit problems with few rows per cluster
+                                   otherwise get; for comparisons and tests */
   BLSTM_FLAG_TEST_NO_ARRIVE = 4 /* test hook: CTAs never signal step completion, so every
                                    cross-CTA wait runs into wait_limit_us and the launch ends
                                    with BLSTM_E_WAIT_TIMEOUT in the control block (no fault) */

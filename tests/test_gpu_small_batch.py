@@ -1,0 +1,81 @@
+"""Small-batch recurrences (weights and the step hand-off inside one cluster of 1 to 16 CTAs) at the edges of their
+tiles: against fp32 step-by-step maths and bit for bit over repeats and batch shards."""
+import ctypes
+
+import pytest
+import torch
+
+from fastlstm_b200 import _lib
+from test_gpu_recurrence import TD, _bwd, _cmp, _desc, _fwd, _torch_bwd, _torch_fwd
+
+pytestmark = pytest.mark.gpu
+
+# (T, B, H): one CTA with 1, 3 and 8 unit groups; several chunks; clusters of 3, 4, 6, 8 with whole and partial last
+# CTAs; K split over two warps (11 to 16 CTAs, K steps in odd halves); weights partly in shared memory; batches of
+# one row, one row past a chunk, chunks shared by replicas
+SHAPES = [(5, 3, 8), (4, 9, 24), (9, 1300, 64), (3, 1, 64), (5, 33, 72), (6, 270, 128), (4, 17, 136), (7, 120, 200),
+          (5, 400, 256), (1, 9, 256), (6, 8, 264), (4, 57, 288), (5, 130, 384), (3, 40, 448), (6, 250, 512), (2, 1, 512),
+          (4, 15, 520), (3, 50, 640), (4, 9, 768)]
+
+
+def _plan(d, phase):
+    buf = ctypes.create_string_buffer(512)
+    assert _lib.load().blstm_plan_detail(d, phase, buf, 512) == 0
+    return buf.value.decode()
+
+
+@pytest.mark.parametrize("dtype", ["fp16", "bf16"])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_small_batch_recurrences_against_fp32_maths(dtype, shape):
+    lib, (T, B, H), dt = _lib.load(), shape, TD[dtype]
+    g = torch.Generator(device="cuda").manual_seed(B * 31 + H)
+    r = lambda *s, std=1.0: (torch.randn(*s, generator=g, device="cuda") * std).to(dt)
+    pre, h0, c0 = r(T, B, 4 * H), r(B, H, std=0.3), r(B, H, std=0.3)
+    dout, dh_n, dc_n = r(T, B, H), r(B, H), r(B, H)
+    Wh = ((torch.rand(4 * H, H, generator=g, device="cuda") * 2 - 1) / H ** 0.5).to(dt)
+    d = _desc(dtype, T, B, H)
+    assert "small-batch" in _plan(d, 0)
+    ifgo, out, cell = _fwd(lib, d, pre, Wh, h0, c0)
+    rg, ro, rc = _torch_fwd(pre, Wh, h0, c0)
+    tol = 4e-3 if dtype == "fp16" else 3e-2
+    _cmp("ifgo", ifgo, rg, tol * 4)
+    _cmp("out", out[1:], ro, tol)
+    _cmp("cell", cell[1:], rc, tol * 2)
+    infer = _fwd(lib, _desc(dtype, T, B, H, _lib.FLAG_INFERENCE), pre, Wh, h0, c0)
+    assert torch.equal(infer[1], out) and torch.equal(infer[2][T], cell[T]) and torch.equal(infer[0], pre)
+    n = (B + 1) // 2                                   # a shard of the rows sums in the same order
+    part = _fwd(lib, _desc(dtype, T, n, H), pre[:, :n].contiguous(), Wh, h0[:n].contiguous(), c0[:n].contiguous())
+    assert torch.equal(part[1], out[:, :n]) and torch.equal(part[2][1:], cell[1:, :n])
+    if H > 640:
+        return
+    assert "small-batch" in _plan(d, 1)
+    got = _bwd(lib, d, dout, dh_n, dc_n, ifgo, cell, Wh)
+    wg, wh, wc = _torch_bwd(dout, dh_n, dc_n, ifgo, cell, Wh)
+    tol = 6e-3 if dtype == "fp16" else 4e-2
+    for name, a, b in (("d_ifgo", got[0], wg), ("dh0", got[1][None], wh[None]), ("dc0", got[2][None], wc[None])):
+        _cmp(name, a, b, tol * max(float(b.float().abs().max()), 1.0))
+    assert torch.allclose(got[3], got[0].float().sum(dim=(0, 1)), rtol=1e-4, atol=1e-3 * T * B ** 0.5)
+    again = _bwd(lib, d, dout, dh_n, dc_n, ifgo, cell, Wh)
+    assert all(torch.equal(a, b) for a, b in zip(got, again))
+
+
+@pytest.mark.parametrize("phase", ["fwd", "bwd"])
+@pytest.mark.parametrize("shape", [(5, 9, 256), (5, 40, 512)])
+def test_small_batch_recurrences_give_up_with_a_status_when_nothing_arrives(phase, shape):
+    """With the arrivals suppressed every wait runs out (20 ms), the blocks leave together and the next launch works."""
+    lib, (T, B, H) = _lib.load(), shape
+    z = lambda *s: torch.zeros(*s, device="cuda", dtype=torch.bfloat16)
+    s = torch.cuda.current_stream().cuda_stream
+    ph = _lib.PHASE_FWD if phase == "fwd" else _lib.PHASE_BWD
+    ifgo, out, cell, Wh, dg, dh0, dc0 = (z(T, B, 4 * H), z(T + 1, B, H), z(T + 1, B, H), z(4 * H, H), z(T, B, 4 * H), z(B, H), z(B, H))
+    for flags, want in ((_lib.FLAG_TEST_NO_ARRIVE, _lib.E_WAIT_TIMEOUT), (0, 0)):
+        d = _lib.Desc(_lib.BF16, T, B, H, H, flags, 20000, 0)
+        assert "small-batch" in _plan(d, ph)
+        n = lib.blstm_workspace_bytes(d, ph)
+        ws = torch.zeros(n, dtype=torch.uint8, device="cuda")
+        if phase == "fwd":
+            rc = lib.blstm_fwd_recurrence(d, ifgo.data_ptr(), Wh.data_ptr(), out.data_ptr(), cell.data_ptr(), ws.data_ptr(), n, s)
+        else:
+            rc = lib.blstm_bwd_recurrence(d, out.data_ptr(), None, None, ifgo.data_ptr(), cell.data_ptr(), Wh.data_ptr(),
+                                          dg.data_ptr(), dh0.data_ptr(), dc0.data_ptr(), None, ws.data_ptr(), n, s)
+        assert rc == 0 and lib.blstm_read_status(ws.data_ptr(), None, s) == want
