@@ -1,12 +1,14 @@
 // extern "C" entry points (declared in include/fastlstm_b200.h): argument
 // validation, kernel-family choice, workspace carving.  No allocation, no
 // host synchronisation except blstm_read_status.
+#include <algorithm>
 #include <atomic>
 #include <mutex>
 #include <stdio.h>
 #include <string.h>
 
 #include "common.cuh"
+#include "f32_gemm.cuh"
 #include "generic.cuh"
 #include "sm100.cuh"
 
@@ -92,6 +94,12 @@ static BwdLayout bwd_layout(const blstm_desc& d) {
   }
   L.gemm_off = round_up(L.rec_bytes, 256);
   L.gemm_bytes = sm100_gemm_supported(d) ? sm100_bwd_gemm_workspace(d) : 0;
+  if (d.dtype == BLSTM_F32) {
+    const int G = 4 * d.hidden_size, TB = d.seq_len * d.batch, I = d.input_size, H = d.hidden_size;
+    const int sx = f32_gemm_splits(G, I, TB, plan_sm_count()), sh = f32_gemm_splits(G, H, TB, plan_sm_count());
+    const int sd = f32_gemm_splits(TB, I, G, plan_sm_count());
+    L.gemm_bytes = 4 * std::max({sx > 1 ? (size_t)sx * G * I : 0, sh > 1 ? (size_t)sh * G * H : 0, sd > 1 ? (size_t)sd * TB * I : 0});
+  }
   L.total = round_up(L.gemm_off + L.gemm_bytes, 256);
   return L;
 }
@@ -188,6 +196,9 @@ int blstm_input_projection(const blstm_desc* d, const void* x, const void* Wx, c
   cudaStream_t st = (cudaStream_t)stream;
   const int M = d->seq_len * d->batch, N = 4 * d->hidden_size, K = d->input_size;
   if (sm100_gemm_supported(*d)) return sm100_input_projection(*d, x, Wx, bx, bh, ifgo, st);
+  if (d->dtype == BLSTM_F32)
+    return f32_gemm(M, N, K, (const float*)x, K, true, (const float*)Wx, K, true, (float*)ifgo, (const float*)bx, (const float*)bh,
+                    1, nullptr, st);
   return generic_gemm(d->dtype, false, M, N, K, x, K, 1, Wx, 1, K, ifgo, N, bx, bh, st);
 }
 
@@ -261,6 +272,12 @@ int blstm_dgrad_input(const blstm_desc* d, const void* d_ifgo, const void* Wx, v
     if (!ws_ok(workspace, workspace_bytes, L.total)) return BLSTM_E_WORKSPACE;
     return sm100_dgrad_input(*d, d_ifgo, Wx, dx, static_cast<char*>(workspace) + L.gemm_off, L.gemm_bytes, st);
   }
+  if (d->dtype == BLSTM_F32) {
+    const BwdLayout L = bwd_layout(*d);
+    if (!ws_ok(workspace, workspace_bytes, L.total)) return BLSTM_E_WORKSPACE;
+    return f32_gemm(M, N, K, (const float*)d_ifgo, K, true, (const float*)Wx, N, false, (float*)dx, nullptr, nullptr,
+                    f32_gemm_splits(M, N, K, plan_sm_count()), reinterpret_cast<float*>(static_cast<char*>(workspace) + L.gemm_off), st);
+  }
   return generic_gemm(d->dtype, false, M, N, K, d_ifgo, K, 1, Wx, N, 1, dx, N, nullptr, nullptr, st);
 }
 
@@ -276,6 +293,16 @@ int blstm_wgrad(const blstm_desc* d, const void* d_ifgo, const void* x, const vo
     const BwdLayout L = bwd_layout(*d);
     if (!ws_ok(workspace, workspace_bytes, L.total)) return BLSTM_E_WORKSPACE;
     return sm100_wgrad(*d, d_ifgo, x, out, dWx, dWh, static_cast<char*>(workspace) + L.gemm_off, L.gemm_bytes, st);
+  }
+  if (d->dtype == BLSTM_F32) {
+    const BwdLayout L = bwd_layout(*d);
+    if (!ws_ok(workspace, workspace_bytes, L.total)) return BLSTM_E_WORKSPACE;
+    float* part = reinterpret_cast<float*>(static_cast<char*>(workspace) + L.gemm_off);
+    const float* g = (const float*)d_ifgo;
+    const int sms = plan_sm_count();
+    rc = f32_gemm(G, I, TB, g, G, false, (const float*)x, I, false, dWx, nullptr, nullptr, f32_gemm_splits(G, I, TB, sms), part, st);
+    if (rc) return rc;
+    return f32_gemm(G, H, TB, g, G, false, (const float*)out, H, false, dWh, nullptr, nullptr, f32_gemm_splits(G, H, TB, sms), part, st);
   }
   rc = generic_gemm(d->dtype, true, G, I, TB, d_ifgo, 1, G, x, I, 1, dWx, I, nullptr, nullptr, st);
   if (rc) return rc;

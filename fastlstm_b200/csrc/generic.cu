@@ -1,7 +1,7 @@
 // CUDA-core (FFMA) kernels: the fp32 path (tolerance 1e-5 forbids TF32) and the
 // path for shapes the tcgen05 kernels do not cover (ragged H/I/B).
 //
-//   gemm_generic_kernel   C = A*B (+bias), fp32 accumulate, arbitrary strides
+//   gemm_generic_kernel   C = A*B (+bias), 16-bit operands, fp32 accumulate, arbitrary strides (fp32: f32_gemm.cu)
 //   gen_fwd_kernel        persistent forward recurrence   (reference: fastlstm/kernels.py:414-663)
 //   gen_bwd_kernel        persistent reverse recurrence   (reference: fastlstm/kernels.py:1201-1409)
 //   reduce_db_kernel      db = sum of per-batch-tile partial bias gradients
@@ -10,7 +10,10 @@
 // hidden tile), carry c / dc / dh in fp32 registers over the time loop and
 // hand h[t] (or d_ifgo[t]) to their peers through global memory, one int32
 // arrival counter per (step, batch tile), every wait bounded.
+#include <algorithm>
+
 #include "generic.cuh"
+#include "f32_cluster.cuh"
 #include "sm100.cuh"
 
 namespace blstm {
@@ -93,8 +96,6 @@ int generic_gemm(int dtype, bool out_f32, int M, int N, int K, const void* A, lo
                  const void* bias0, const void* bias1, cudaStream_t st) {
   if (M <= 0 || N <= 0) return BLSTM_OK;
   switch (dtype) {
-    case BLSTM_F32:
-      return launch_gemm<float, float, float, float>(M, N, K, A, sam, sak, B, sbk, sbn, C, ldc, bias0, bias1, st);
     case BLSTM_F16:
       return out_f32 ? launch_gemm<__half, __half, float, __half>(M, N, K, A, sam, sak, B, sbk, sbn, C, ldc, bias0, bias1, st)
                      : launch_gemm<__half, __half, __half, __half>(M, N, K, A, sam, sak, B, sbk, sbn, C, ldc, bias0, bias1, st);
@@ -373,6 +374,8 @@ void GenericPlan::make(const blstm_desc& d, int phase) {
   off_flags = sizeof(Control);
   off_db = off_flags + round_up(n_flags * sizeof(int), 256);
   ws_bytes = off_db + (phase == BLSTM_PHASE_BWD ? round_up((size_t)nbt * 4 * H * sizeof(float), 256) : 0);
+  const sm100::F32Plan fp = sm100::f32_plan(d, phase);
+  if (fp.ok) ws_bytes = std::max(ws_bytes, f32_workspace(d, fp, phase));
 }
 
 template <typename Kern>
@@ -425,6 +428,8 @@ int generic_fwd_recurrence(const blstm_desc& d, void* ifgo, const void* Wh, void
   GenericPlan pl;
   pl.make(d, BLSTM_PHASE_FWD);
   if (ws_bytes < pl.ws_bytes) return BLSTM_E_WORKSPACE;
+  const sm100::F32Plan fp = sm100::f32_plan(d, BLSTM_PHASE_FWD);
+  if (fp.ok) return f32_fwd_recurrence(d, fp, ifgo, Wh, out, cell, ws, st);
   BLSTM_CUDA_OK(cudaMemsetAsync(ws, 0, pl.off_db, st));
   switch (d.dtype) {
     case BLSTM_F32: return launch_fwd<float>(d, pl, ifgo, Wh, out, cell, ws, st);
@@ -458,6 +463,8 @@ int generic_bwd_recurrence(const blstm_desc& d, const void* dout, const void* dh
   GenericPlan pl;
   pl.make(d, BLSTM_PHASE_BWD);
   if (ws_bytes < pl.ws_bytes) return BLSTM_E_WORKSPACE;
+  const sm100::F32Plan fp = sm100::f32_plan(d, BLSTM_PHASE_BWD);
+  if (fp.ok) return f32_bwd_recurrence(d, fp, dout, dh_n, dc_n, ifgo, cell, Wh, d_ifgo, dh0, dc0, db, ws, st);
   BLSTM_CUDA_OK(cudaMemsetAsync(ws, 0, pl.off_db, st));
   int rc = BLSTM_E_INVALID_ARG;
   switch (d.dtype) {
@@ -567,9 +574,9 @@ fused_fwd_kernel(int Tn, int B, int I, int H, int inference, const T* __restrict
 bool generic_fused_fwd_supported(const blstm_desc& d) {
   if (d.flags & BLSTM_FLAG_NO_FUSED) return false;
   const int size = d.hidden_size > d.input_size ? d.hidden_size : d.input_size;
-  if (d.dtype == BLSTM_F32) return size <= 32;
-  // 16-bit: a step takes 3.2 us here against 0.5 us in the small-batch recurrence (H = 64), whose projection and second
-  // launch cost some 10 us: a few steps, and sizes the tcgen05 projection does not take.
+  // A step takes 1.5 to 3.2 us here against 0.5 to 0.7 us in the recurrences inside one cluster (fp32 H = 32, 16-bit H = 64),
+  // whose projection and second launch cost some 10 us: for a few steps, and sizes the tcgen05 projection does not take.
+  if (d.dtype == BLSTM_F32) return size <= 32 && (d.seq_len <= 12 || !sm100::f32_plan(d, BLSTM_PHASE_FWD).ok);
   return size <= 64 && (d.seq_len <= 12 || !sm100_gemm_supported(d));
 }
 

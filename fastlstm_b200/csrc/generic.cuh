@@ -18,7 +18,7 @@ struct GenericPlan {
 };
 
 // C[M,N] = A*B (+bias0+bias1); A(m,k) = A[m*sam + k*sak], B(k,n) = B[k*sbk + n*sbn].
-// dtype selects the element type of A, B and the biases; C is fp32 when out_f32.
+// dtype (16-bit) selects the element type of A, B and the biases; C is fp32 when out_f32.
 int generic_gemm(int dtype, bool out_f32, int M, int N, int K, const void* A, long long sam,
                  long long sak, const void* B, long long sbk, long long sbn, void* C, long long ldc,
                  const void* bias0, const void* bias1, cudaStream_t st);

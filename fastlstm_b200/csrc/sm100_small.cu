@@ -24,15 +24,13 @@
 
 #include "sm100.cuh"
 #include "sm100_common.cuh"
+#include "cluster_util.cuh"
 #include "sm100_rec_util.cuh"
 #include "generic.cuh"
 #include "sm100_small.cuh"
 
 namespace blstm {
 namespace sm100 {
-
-constexpr int SB_MAX_CHUNKS = 16;
-constexpr int SB_MAX_SLOTS = 32;
 
 // ---------------------------------------------------------------- primitives
 template <typename T16>
@@ -60,35 +58,6 @@ __device__ __forceinline__ uint32_t transpose8x8(uint32_t v) {
   asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(v));
   return r;
 }
-__device__ __forceinline__ void st_async16(uint32_t addr, uint4 v, uint32_t bar) {
-  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1,%2,%3,%4}, [%5];"
-               ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "r"(bar) : "memory");
-}
-__device__ __forceinline__ void st_shared16(uint32_t addr, uint4 v) {
-  asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
-}
-// Bounded mbarrier wait, inlined on purpose: a call would spill the weight fragments around it.
-__device__ __forceinline__ bool wait_inline(uint64_t* bar, uint32_t parity, volatile int* dead, Control* ctl,
-                                            unsigned long long limit_ns, int d0, int d1) {
-  if (mbar_try_wait_cluster(bar, parity)) return true;
-  unsigned spins = 0;
-  unsigned long long t0 = 0;
-  while (!mbar_try_wait_cluster(bar, parity)) {
-    if ((++spins & 63u) != 0u) continue;
-    if (*dead || ld_relaxed_gpu(&ctl->abort) != 0) { *dead = 1; return false; }
-    const unsigned long long now = globaltimer_ns();
-    if (t0 == 0) t0 = now;
-    if (now - t0 > limit_ns) {
-      *dead = 1;
-      if (atomicCAS(&ctl->status, 0, BLSTM_E_WAIT_TIMEOUT) == 0) { ctl->detail[0] = d0; ctl->detail[1] = d1; }
-      atomicExch(&ctl->abort, 1);
-      return false;
-    }
-  }
-  return true;
-}
-template <int N> __device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
-template <int N> __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 __device__ __forceinline__ uint32_t ldg4(const void* p) { return *reinterpret_cast<const uint32_t*>(p); }
 __device__ __forceinline__ void stg4(void* p, uint32_t v) { *reinterpret_cast<uint32_t*>(p) = v; }
 __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, uint32_t (&r)[4]) {
@@ -802,10 +771,39 @@ small_bwd_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant_
 // every bit of a row's results - does not depend on the batch.
 static int small_cluster(int H) { return H <= 64 ? 1 : H <= 128 ? 4 : H <= 256 ? 8 : 16; }
 
-// Clusters that can be resident at once, one CTA per SM (a B200's GPCs hold 7 clusters of 16, 15 of 8, 33 of 4).
-static int small_cluster_capacity(int nc) {
+__global__ void one_cta_per_sm_kernel() {}
+
+// Asked of the occupancy calculator once per size from 5 CTAs on: clusters do not tile every GPC without a remainder (a
+// B200 holds 33 of 4 CTAs, 15 of 8, 7 of 16).
+int resident_clusters(int nc) {
+  static std::atomic<int> cached[17];
   const int sms = plan_sm_count();
-  return nc <= 4 ? sms * 132 / 148 / nc : nc <= 8 ? sms * 15 / 148 : sms * 7 / 148;
+  if (nc <= 4) return sms * 132 / 148 / nc;
+  int c = cached[nc].load(std::memory_order_relaxed);
+  if (c > 0) return c;
+  c = nc <= 8 ? sms * 15 / 148 : sms * 7 / 148;
+  DeviceInfo di;
+  auto kern = one_cta_per_sm_kernel;
+  if (get_device_info(&di) == BLSTM_OK && di.sm_count > 0 &&
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) == cudaSuccess &&
+      cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(nc);
+    cfg.blockDim = dim3(384);
+    cfg.dynamicSmemBytes = 200 * 1024;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = nc;
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int mc = 0;
+    if (cudaOccupancyMaxActiveClusters(&mc, kern, &cfg) == cudaSuccess && mc > 0) c = mc;
+  }
+  (void)cudaGetLastError();
+  cached[nc].store(c, std::memory_order_relaxed);
+  return c;
 }
 
 // Whether the plan beats the tcgen05 kernels.  Those take the same time for any batch of up to a few 128-row tiles, these
@@ -830,7 +828,7 @@ SmallPlan small_plan(const blstm_desc& d, int phase) {
   p.gc = cdiv(G, small_cluster(H));
   p.nc = cdiv(G, p.gc);
   if (p.nc == 1 && (d.flags & BLSTM_FLAG_TEST_NO_ARRIVE)) return p;     // (no wait that could run out)
-  const int cap = std::max(1, small_cluster_capacity(p.nc) / ((d.flags & BLSTM_FLAG_HALF_DEVICE) ? 2 : 1));
+  const int cap = std::max(1, resident_clusters(p.nc) / ((d.flags & BLSTM_FLAG_HALF_DEVICE) ? 2 : 1));
   p.ks = 2 * cdiv(H, 32);
   const int tiles = cdiv(B, 8);
   p.ncl = std::min(cap, tiles);
@@ -873,32 +871,11 @@ SmallPlan small_plan(const blstm_desc& d, int phase) {
   return p;
 }
 
-template <typename Kern, typename... Args>
-static int launch_small(Kern kern, const SmallPlan& pl, cudaStream_t st, const Args&... args) {
-  BLSTM_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
-  if (pl.nc > 8) BLSTM_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(pl.grid);
-  cfg.blockDim = dim3(pl.threads);
-  cfg.dynamicSmemBytes = pl.smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = pl.nc;
-  attr.val.clusterDim.y = 1;
-  attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = pl.nc > 1 ? 1 : 0;
-  BLSTM_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, args...));
-  count_launch();
-  return BLSTM_OK;
-}
-
 template <typename T16>
 static int small_fwd_t(const SmallPlan& pl, const CUtensorMap& tp, const CUtensorMap& th, const CUtensorMap& tc,
                        const SmallFwdParams& p, cudaStream_t st) {
 #define BLSTM_SMALL_FWD(K, N, C) \
-  if (pl.kr == K && pl.kspl == N && (pl.nc > 1) == C) return launch_small(small_fwd_kernel<K, N, C, T16>, pl, st, tp, th, tc, p);
+  if (pl.kr == K && pl.kspl == N && (pl.nc > 1) == C) return launch_clusters(small_fwd_kernel<K, N, C, T16>, pl.grid, pl.threads, pl.smem, pl.nc, st, tp, th, tc, p);
   BLSTM_SMALL_FWD(2, 1, false)
   BLSTM_SMALL_FWD(4, 1, false)
   BLSTM_SMALL_FWD(6, 1, true)
@@ -919,7 +896,7 @@ template <typename T16>
 static int small_bwd_t(const SmallPlan& pl, const CUtensorMap& tp, const CUtensorMap& tc, const CUtensorMap& to,
                        const CUtensorMap& td, const SmallBwdParams& p, cudaStream_t st) {
 #define BLSTM_SMALL_BWD(M, K, C) \
-  if (pl.mpw == M && pl.kr == K && (pl.nc > 1) == C) return launch_small(small_bwd_kernel<M, K, 1, C, T16>, pl, st, tp, tc, to, td, p);
+  if (pl.mpw == M && pl.kr == K && (pl.nc > 1) == C) return launch_clusters(small_bwd_kernel<M, K, 1, C, T16>, pl.grid, pl.threads, pl.smem, pl.nc, st, tp, tc, to, td, p);
   BLSTM_SMALL_BWD(1, 2, false)
   BLSTM_SMALL_BWD(1, 8, false)
   BLSTM_SMALL_BWD(1, 16, false)

@@ -79,3 +79,69 @@ def test_small_batch_recurrences_give_up_with_a_status_when_nothing_arrives(phas
             rc = lib.blstm_bwd_recurrence(d, out.data_ptr(), None, None, ifgo.data_ptr(), cell.data_ptr(), Wh.data_ptr(),
                                           dg.data_ptr(), dh0.data_ptr(), dc0.data_ptr(), None, ws.data_ptr(), n, s)
         assert rc == 0 and lib.blstm_read_status(ws.data_ptr(), None, s) == want
+
+
+# fp32: one CTA, clusters of 2 to 14; rows per chunk 1, 2, 4, 8; several chunks; hidden sizes that are no multiple of anything
+F32_SHAPES = [(5, 3, 7), (4, 300, 32), (6, 40, 33), (3, 600, 64), (5, 1, 100), (4, 45, 128), (5, 44, 257), (3, 9, 200),
+              (4, 100, 320), (1, 5, 96), (6, 130, 160)]
+
+
+@pytest.mark.parametrize("shape", F32_SHAPES)
+def test_fp32_cluster_recurrences_against_fp64_maths(shape):
+    lib, (T, B, H) = _lib.load(), shape
+    g = torch.Generator(device="cuda").manual_seed(B * 17 + H)
+    r = lambda *s, std=1.0: torch.randn(*s, generator=g, device="cuda") * std
+    pre, h0, c0 = r(T, B, 4 * H), r(B, H, std=0.3), r(B, H, std=0.3)
+    dout, dh_n, dc_n = r(T, B, H), r(B, H), r(B, H)
+    Wh = (torch.rand(4 * H, H, generator=g, device="cuda") * 2 - 1) / H ** 0.5
+    d = _lib.Desc(_lib.F32, T, B, H, H, 0, 0, 0)
+    ifgo, out, cell = _fwd(lib, d, pre, Wh, h0, c0)
+    W, h, c = Wh.double(), h0.double(), c0.double()
+    for t in range(T):
+        a = pre[t].double() + h @ W.T
+        i, f, gg, o = a.split(H, dim=1)
+        c = torch.sigmoid(f) * c + torch.sigmoid(i) * torch.tanh(gg)
+        h = torch.sigmoid(o) * torch.tanh(c)
+        for name, got, want in (("ifgo", ifgo[t], a), ("out", out[t + 1], h), ("cell", cell[t + 1], c)):
+            assert float((got - want).abs().max()) <= 1e-5 * max(1.0, float(want.abs().max())), (name, t)
+    infer = _fwd(lib, _lib.Desc(_lib.F32, T, B, H, H, _lib.FLAG_INFERENCE, 0, 0), pre, Wh, h0, c0)
+    assert torch.equal(infer[1], out) and torch.equal(infer[2][T], cell[T]) and torch.equal(infer[0], pre)
+    n = (B + 1) // 2
+    part = _fwd(lib, _lib.Desc(_lib.F32, T, n, H, H, 0, 0, 0), pre[:, :n].contiguous(), Wh, h0[:n].contiguous(), c0[:n].contiguous())
+    assert torch.equal(part[1], out[:, :n])
+    dg, dh0, dc0, db = _bwd(lib, d, dout, dh_n, dc_n, ifgo, cell, Wh)
+    dh, dc, want_db = dh_n.double(), dc_n.double(), 0
+    for t in reversed(range(T)):
+        pi, pf, pg, po = ifgo[t].double().split(H, dim=1)
+        si, sf, so, tg, tc = torch.sigmoid(pi), torch.sigmoid(pf), torch.sigmoid(po), torch.tanh(pg), torch.tanh(cell[t + 1].double())
+        dh = dout[t].double() + dh
+        dc = dc + dh * so * (1 - tc * tc)
+        q = torch.cat([dc * tg * si * (1 - si), dc * cell[t].double() * sf * (1 - sf), dc * si * (1 - tg * tg),
+                       dh * tc * so * (1 - so)], dim=1)
+        assert float((dg[t] - q).abs().max()) <= 1e-5 * max(1.0, float(q.abs().max())), t
+        dc, dh, want_db = dc * sf, q @ W, want_db + q.sum(0)
+    for got, want in ((dh0, dh), (dc0, dc), (db, want_db)):
+        assert float((got - want).abs().max()) <= 1e-5 * max(1.0, float(want.abs().max()))
+    again = _bwd(lib, d, dout, dh_n, dc_n, ifgo, cell, Wh)
+    assert all(torch.equal(a, b) for a, b in zip((dg, dh0, dc0, db), again))
+
+
+# (T, B, I, H): partial tiles in M, N and K, rows that allow 16-byte copies and rows that do not, K split and not
+@pytest.mark.parametrize("shape", [(3, 5, 1, 3), (1, 64, 16, 16), (40, 33, 123, 65), (64, 16, 128, 128), (10, 100, 257, 40)])
+def test_fp32_gemms_against_fp64_matmul(shape):
+    lib, (T, B, I, H) = _lib.load(), shape
+    g = torch.Generator(device="cuda").manual_seed(T + I)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    x, Wx, bx, bh, dg, out = r(T, B, I), r(4 * H, I), r(4 * H), r(4 * H), r(T, B, 4 * H), r(T + 1, B, H)
+    d = _lib.Desc(_lib.F32, T, B, I, H, 0, 0, 0)
+    s = torch.cuda.current_stream().cuda_stream
+    n = lib.blstm_workspace_bytes(d, _lib.PHASE_BWD)
+    ws = torch.zeros(n, dtype=torch.uint8, device="cuda")
+    new = lambda *sh: torch.full(sh, float("nan"), device="cuda")
+    ifgo, dx, dWx, dWh = new(T * B, 4 * H), new(T * B, I), new(4 * H, I), new(4 * H, H)
+    _lib.check(lib.blstm_input_projection(d, x.data_ptr(), Wx.data_ptr(), bx.data_ptr(), bh.data_ptr(), ifgo.data_ptr(), s))
+    _lib.check(lib.blstm_dgrad_input(d, dg.data_ptr(), Wx.data_ptr(), dx.data_ptr(), ws.data_ptr(), n, s))
+    _lib.check(lib.blstm_wgrad(d, dg.data_ptr(), x.data_ptr(), out.data_ptr(), dWx.data_ptr(), dWh.data_ptr(), ws.data_ptr(), n, s))
+    X, D, O = x.double().view(T * B, I), dg.double().view(T * B, -1), out[:-1].double().reshape(T * B, H)
+    for got, want in ((ifgo, X @ Wx.double().T + bx.double() + bh.double()), (dx, D @ Wx.double()), (dWx, D.T @ X), (dWh, D.T @ O)):
+        assert float((got - want).norm() / want.norm()) <= 1e-6
