@@ -54,12 +54,34 @@ SIGNATURES = {
     "blstm_bwd": (c_int, [DP] + [P] * 17 + [c_size_t, P]),
     "blstm_read_status": (c_int, [P, POINTER(c_int32), P]),
     "blstm_launch_count": (ctypes.c_ulonglong, []),
+    "blstm_set_mailbox": (None, [P]),
+    "blstm_repack": (c_int, [P, c_int, P]),
     "blstm_fwd_recurrence_static": (c_int, [DP, P, P, P, P, P]),
     "blstm_static_scratch_capacity": (c_size_t, []),
     "blstm_static_scratch_status": (c_int, [POINTER(c_int32), P]),
 }
 
 _lib = None
+_host = None
+
+
+def host():
+    """The CPython extension behind the operators (csrc/host.cpp), set up once; raises when it is missing."""
+    global _host
+    if _host is None:
+        load()
+        try:
+            from . import _host as ext
+        except ImportError as e:
+            raise RuntimeError("the extension fastlstm_b200._host is required and could not be loaded; build it with "
+                               "`python -m fastlstm_b200.build`") from e
+        env = os.environ.get
+        ext.configure(FLAG_FORCE_GENERIC if env("FASTLSTM_B200_FORCE_GENERIC", "0") == "1" else 0,
+                      int(env("FASTLSTM_B200_WAIT_LIMIT_US", "0")),
+                      # read the device status word (and wait for the stream) after every launch
+                      env("FASTLSTM_B200_SYNC_CHECK", "0") == "1", BlstmError)
+        _host = ext
+    return _host
 
 
 def load():

@@ -9,8 +9,10 @@
 
 #include "common.cuh"
 #include "f32_gemm.cuh"
+#include "f32_cluster.cuh"
 #include "generic.cuh"
 #include "sm100.cuh"
+#include "step.cuh"
 
 namespace blstm {
 
@@ -104,6 +106,79 @@ static BwdLayout bwd_layout(const blstm_desc& d) {
   return L;
 }
 
+size_t control_bytes(const blstm_desc& d, int phase) {
+  if (sm100_recurrence_supported(d, phase)) return round_up(sm100_recurrence_control(d, phase), 16);
+  if (sm100::f32_plan(d, phase).ok) return sizeof(Control);
+  GenericPlan pl;
+  pl.make(d, phase);
+  return pl.off_db;
+}
+
+// What the calling thread's launches tell the host through, or null (blstm_set_mailbox).
+static thread_local int* g_mailbox = nullptr;
+
+struct BeginParams {
+  uint4* ws;
+  size_t ws16;              // 16-byte pieces of control block and counters to clear
+  int* mailbox;
+  const char* src[2];       // h0, c0 or null
+  char* dst[2];             // slot 0 of out, cell
+  size_t slot_bytes;        // 0: states are in place
+  int piece;                // bytes the slot copies move at a time: 16, 4 or 2, by alignment
+};
+
+__global__ void __launch_bounds__(256) begin_kernel(const BeginParams p) {
+  const size_t i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x, n = (size_t)gridDim.x * blockDim.x;
+  for (size_t i = i0; i < p.ws16; i += n) {
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (i == 1) {           // Control::mailbox
+      const unsigned long long m = reinterpret_cast<unsigned long long>(p.mailbox);
+      v.x = (unsigned)m;
+      v.y = (unsigned)(m >> 32);
+    }
+    p.ws[i] = v;
+  }
+#pragma unroll
+  for (int s = 0; s < 2; ++s) {
+    const char* src = p.src[s];
+    char* dst = p.dst[s];
+    if (p.piece == 16)
+      for (size_t i = i0 * 16; i + 16 <= p.slot_bytes; i += n * 16)
+        *reinterpret_cast<uint4*>(dst + i) = src ? *reinterpret_cast<const uint4*>(src + i) : make_uint4(0, 0, 0, 0);
+    else if (p.piece == 4)
+      for (size_t i = i0 * 4; i < p.slot_bytes; i += n * 4)
+        *reinterpret_cast<unsigned*>(dst + i) = src ? *reinterpret_cast<const unsigned*>(src + i) : 0u;
+    const size_t tail = p.piece == 16 ? p.slot_bytes / 16 * 16 : p.piece == 4 ? p.slot_bytes : 0;
+    for (size_t i = tail + i0 * 2; i < p.slot_bytes; i += n * 2)
+      *reinterpret_cast<unsigned short*>(dst + i) = src ? *reinterpret_cast<const unsigned short*>(src + i) : (unsigned short)0;
+  }
+}
+static_assert(offsetof(Control, mailbox) == 16, "begin_kernel writes the mailbox with the second 16-byte piece");
+
+int begin_call(const blstm_desc& d, int phase, void* ws, const void* h0, const void* c0, void* out, void* cell, cudaStream_t st) {
+  BeginParams p;
+  p.ws = reinterpret_cast<uint4*>(ws);
+  p.ws16 = ws ? control_bytes(d, phase) / 16 : 0;
+  p.mailbox = g_mailbox;
+  p.src[0] = (const char*)h0; p.src[1] = (const char*)c0;
+  p.dst[0] = (char*)out; p.dst[1] = (char*)cell;
+  p.slot_bytes = out ? (size_t)d.batch * d.hidden_size * esize(d.dtype) : 0;
+  const uintptr_t m = reinterpret_cast<uintptr_t>(h0) | reinterpret_cast<uintptr_t>(c0) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(cell);
+  p.piece = (m & 15u) == 0 && (d.dtype != BLSTM_F32 || p.slot_bytes % 16 == 0) ? 16 : d.dtype == BLSTM_F32 ? 4 : 2;
+  const size_t pieces = std::max(p.ws16, p.slot_bytes / p.piece);
+  const int grid = (int)std::min<size_t>(std::max<size_t>((pieces + 1023) / 1024, 1), 296);   // four pieces a thread, two blocks per SM at most
+  begin_kernel<<<grid, 256, 0, st>>>(p);
+  BLSTM_CUDA_OK(cudaGetLastError());
+  count_launch();
+  return BLSTM_OK;
+}
+
+static int fwd_recurrence(const blstm_desc& d, void* ifgo, const void* Wh, void* out, void* cell, void* ws, size_t ws_bytes,
+                          cudaStream_t st) {
+  if (sm100_recurrence_supported(d, BLSTM_PHASE_FWD)) return sm100_fwd_recurrence(d, ifgo, Wh, out, cell, ws, ws_bytes, st);
+  return generic_fwd_recurrence(d, ifgo, Wh, out, cell, ws, ws_bytes, st);
+}
+
 }  // namespace blstm
 
 using namespace blstm;
@@ -156,6 +231,7 @@ size_t blstm_workspace_bytes(const blstm_desc* d, int phase) {
 const char* blstm_plan_name(const blstm_desc* d, int phase) {
   if (check_desc(d)) return "invalid";
   if (phase == BLSTM_PHASE_FWD_OP) {
+    if (step_supported(*d)) return "step";
     if (generic_fused_fwd_supported(*d)) return "fused";
     phase = BLSTM_PHASE_FWD;
   }
@@ -168,6 +244,11 @@ int blstm_plan_detail(const blstm_desc* d, int phase, char* buf, size_t buf_byte
   int rc = check_desc(d);
   if (rc) return rc;
   if (phase == BLSTM_PHASE_FWD_OP) {
+    if (step_supported(*d)) {
+      snprintf(buf, buf_bytes, "step fwd (projection, recurrence and gates of one timestep) units_per_cta=8 grid=%d threads=256",
+               (d->hidden_size + 7) / 8);
+      return BLSTM_OK;
+    }
     if (generic_fused_fwd_supported(*d)) {
       snprintf(buf, buf_bytes, "fused fwd (projection inside the time loop) rows_per_cta=4 grid=%d threads=%d",
                (d->batch + 3) / 4, 4 * d->hidden_size);
@@ -210,9 +291,9 @@ int blstm_fwd_recurrence(const blstm_desc* d, void* ifgo, const void* Wh, void* 
   if (!aligned16(d->dtype, ifgo, Wh, out, cell)) return BLSTM_E_INVALID_ARG;
   if (!ws_ok(workspace, workspace_bytes, blstm_workspace_bytes(d, BLSTM_PHASE_FWD))) return BLSTM_E_WORKSPACE;
   cudaStream_t st = (cudaStream_t)stream;
-  if (sm100_recurrence_supported(*d, BLSTM_PHASE_FWD))
-    return sm100_fwd_recurrence(*d, ifgo, Wh, out, cell, workspace, workspace_bytes, st);
-  return generic_fwd_recurrence(*d, ifgo, Wh, out, cell, workspace, workspace_bytes, st);
+  rc = begin_call(*d, BLSTM_PHASE_FWD, workspace, nullptr, nullptr, nullptr, nullptr, st);
+  if (rc) return rc;
+  return fwd_recurrence(*d, ifgo, Wh, out, cell, workspace, workspace_bytes, st);
 }
 
 int blstm_fwd(const blstm_desc* d, const void* x, const void* h0, const void* c0, const void* Wx,
@@ -220,26 +301,22 @@ int blstm_fwd(const blstm_desc* d, const void* x, const void* h0, const void* c0
               void* workspace, size_t workspace_bytes, void* stream) {
   int rc = check_desc(d);
   if (rc) return rc;
-  if (!x || !Wx || !Wh || !out || !cell || !ifgo) return BLSTM_E_INVALID_ARG;
+  const bool step = step_supported(*d);
+  if (!x || !Wx || !Wh || !out || !cell || (!ifgo && !(step && (d->flags & BLSTM_FLAG_INFERENCE)))) return BLSTM_E_INVALID_ARG;
   if ((h0 == nullptr) != (c0 == nullptr)) return BLSTM_E_INVALID_ARG;
   if (!aligned16(d->dtype, x, h0, c0, Wx, Wh, bx, bh, out, cell, ifgo)) return BLSTM_E_INVALID_ARG;
   cudaStream_t st = (cudaStream_t)stream;
-  const size_t slot = (size_t)d->batch * d->hidden_size * esize(d->dtype);
-  if (h0) {
-    BLSTM_CUDA_OK(cudaMemcpyAsync(out, h0, slot, cudaMemcpyDeviceToDevice, st));
-    BLSTM_CUDA_OK(cudaMemcpyAsync(cell, c0, slot, cudaMemcpyDeviceToDevice, st));
-  } else {
-    BLSTM_CUDA_OK(cudaMemsetAsync(out, 0, slot, st));
-    BLSTM_CUDA_OK(cudaMemsetAsync(cell, 0, slot, st));
-  }
-  if (generic_fused_fwd_supported(*d)) {
-    // the kernel records nothing on the device, but callers read the control block afterwards
-    if (workspace && workspace_bytes >= sizeof(Control)) BLSTM_CUDA_OK(cudaMemsetAsync(workspace, 0, sizeof(Control), st));
-    return generic_fused_fwd(*d, x, Wx, Wh, bx, bh, ifgo, out, cell, st);
-  }
+  // (the single-kernel forms record nothing on the device, but callers may read the control block afterwards)
+  const bool have_ws = ws_ok(workspace, workspace_bytes, blstm_workspace_bytes(d, BLSTM_PHASE_FWD));
+  if (step) return step_fwd(*d, x, h0, c0, Wx, Wh, bx, bh, out, cell, ifgo, have_ws ? (Control*)workspace : nullptr, st);
+  const bool fused = generic_fused_fwd_supported(*d);
+  if (!fused && !have_ws) return BLSTM_E_WORKSPACE;
+  rc = begin_call(*d, BLSTM_PHASE_FWD, have_ws ? workspace : nullptr, h0, c0, out, cell, st);
+  if (rc) return rc;
+  if (fused) return generic_fused_fwd(*d, x, Wx, Wh, bx, bh, ifgo, out, cell, st);
   rc = blstm_input_projection(d, x, Wx, bx, bh, ifgo, stream);
   if (rc) return rc;
-  return blstm_fwd_recurrence(d, ifgo, Wh, out, cell, workspace, workspace_bytes, stream);
+  return fwd_recurrence(*d, ifgo, Wh, out, cell, workspace, workspace_bytes, st);
 }
 
 int blstm_bwd_recurrence(const blstm_desc* d, const void* dout, const void* dh_n, const void* dc_n,
@@ -252,6 +329,8 @@ int blstm_bwd_recurrence(const blstm_desc* d, const void* dout, const void* dh_n
   const BwdLayout L = bwd_layout(*d);
   if (!ws_ok(workspace, workspace_bytes, L.rec_bytes)) return BLSTM_E_WORKSPACE;
   cudaStream_t st = (cudaStream_t)stream;
+  rc = begin_call(*d, BLSTM_PHASE_BWD, workspace, nullptr, nullptr, nullptr, nullptr, st);
+  if (rc) return rc;
   if (sm100_recurrence_supported(*d, BLSTM_PHASE_BWD))
     return sm100_bwd_recurrence(*d, dout, dh_n, dc_n, ifgo, cell, Wh, d_ifgo, dh0, dc0, db, workspace,
                                 L.rec_bytes, st);
@@ -340,6 +419,8 @@ int blstm_bwd(const blstm_desc* d, const void* dout, const void* dh_n, const voi
   if (dWx && dWh) rc = blstm_wgrad(d, d_ifgo, x, out, dWx, dWh, workspace, workspace_bytes, stream);
   return rc;
 }
+
+void blstm_set_mailbox(int32_t* mapped) { g_mailbox = mapped; }
 
 unsigned long long blstm_launch_count(void) { return g_launches.load(std::memory_order_relaxed); }
 

@@ -17,7 +17,7 @@ __device__ __forceinline__ void st_async16(uint32_t addr, uint4 v, uint32_t bar)
 __device__ __forceinline__ void st_shared16(uint32_t addr, uint4 v) {
   asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
-// Bounded mbarrier wait, inlined on purpose: a call would spill the weight fragments around it.
+// Bounded mbarrier wait, inlined on purpose: a call on the waiting path would spill the weight fragments around it.
 __device__ __forceinline__ bool wait_inline(uint64_t* bar, uint32_t parity, volatile int* dead, Control* ctl,
                                             unsigned long long limit_ns, int d0, int d1) {
   if (mbar_try_wait_cluster(bar, parity)) return true;
@@ -30,8 +30,7 @@ __device__ __forceinline__ bool wait_inline(uint64_t* bar, uint32_t parity, vola
     if (t0 == 0) t0 = now;
     if (now - t0 > limit_ns) {
       *dead = 1;
-      if (atomicCAS(&ctl->status, 0, BLSTM_E_WAIT_TIMEOUT) == 0) { ctl->detail[0] = d0; ctl->detail[1] = d1; }
-      atomicExch(&ctl->abort, 1);
+      record_timeout(ctl, d0, d1);
       return false;
     }
   }

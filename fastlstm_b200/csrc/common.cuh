@@ -12,14 +12,15 @@
 namespace blstm {
 
 // ---------------------------------------------------------------------------
-// Workspace control block (first 256 bytes of every workspace).  Zeroed by the
-// host entry point with a stream-ordered memset before each launch.
+// Workspace control block (first 256 bytes of every workspace).  Set up by the
+// host entry point with a stream-ordered kernel before each launch.
 // ---------------------------------------------------------------------------
 struct Control {
   int abort;        // set by the first CTA whose wait ran out; polled by all spinners
   int status;       // BLSTM_OK or BLSTM_E_WAIT_TIMEOUT
   int detail[2];    // step index, batch tile of the wait that gave up
-  int pad[60];
+  int* mailbox;     // mapped host memory that gets a copy of status and detail, or null
+  int pad[58];
 };
 static_assert(sizeof(Control) == 256, "control block is 256 bytes");
 
@@ -91,6 +92,23 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
   return t;
 }
 
+// The first wait of a launch that runs out leaves its status (and tells the host, if it listens), then every other
+// spinner leaves.
+static __device__ __noinline__ void record_timeout(Control* ctl, int d0, int d1) {
+  if (atomicCAS(&ctl->status, 0, BLSTM_E_WAIT_TIMEOUT) == 0) {
+    ctl->detail[0] = d0;
+    ctl->detail[1] = d1;
+    volatile int* m = ctl->mailbox;
+    if (m) {
+      m[2] = d0;
+      m[3] = d1;
+      __threadfence_system();
+      m[1] = BLSTM_E_WAIT_TIMEOUT;
+    }
+  }
+  atomicExch(&ctl->abort, 1);
+}
+
 // Spin until *flag >= target.  Gives up (returns false) when another CTA has
 // raised ctl->abort or when limit_ns elapsed; in the latter case it records
 // BLSTM_E_WAIT_TIMEOUT with (d0, d1) and raises abort so every other spinner
@@ -105,11 +123,7 @@ static __device__ __noinline__ bool wait_flag_ge(const int* flag, int target, Co
     if ((++spins & 31u) == 0u) {
       if (ld_relaxed_gpu(&ctl->abort) != 0) return false;
       if (globaltimer_ns() - t0 > limit_ns) {
-        if (atomicCAS(&ctl->status, 0, BLSTM_E_WAIT_TIMEOUT) == 0) {
-          ctl->detail[0] = d0;
-          ctl->detail[1] = d1;
-        }
-        atomicExch(&ctl->abort, 1);
+        record_timeout(ctl, d0, d1);
         return false;
       }
     }
@@ -121,6 +135,11 @@ static __device__ __noinline__ bool wait_flag_ge(const int* flag, int target, Co
 // ---------------------------------------------------------------------------
 void set_cuda_error(cudaError_t e, const char* where);
 void count_launch(int n = 1);  // bump the per-process kernel-launch counter
+// Every recurrence launch starts with this one kernel: clears the control block and the counters of the phase's plan
+// (control_bytes) and, for a whole forward operator, puts the initial states (zeros where h0 / c0 are null) into slot 0 of
+// out and cell.  out may be null.
+int begin_call(const blstm_desc& d, int phase, void* ws, const void* h0, const void* c0, void* out, void* cell, cudaStream_t st);
+size_t control_bytes(const blstm_desc& d, int phase);
 
 #define BLSTM_CUDA_OK(expr)                                  \
   do {                                                       \

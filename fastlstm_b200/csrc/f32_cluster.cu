@@ -515,7 +515,7 @@ F32Plan f32_plan(const blstm_desc& d, int phase) {
   p.U = (phase == BLSTM_PHASE_BWD && H > 256) ? 24 : 32;
   p.nc = cdiv(H, p.U);
   if (p.nc == 1 && (d.flags & BLSTM_FLAG_TEST_NO_ARRIVE)) return p;      // (no wait that could run out)
-  const int cap = std::max(1, resident_clusters(p.nc) / ((d.flags & BLSTM_FLAG_HALF_DEVICE) ? 2 : 1));
+  const int cap = std::max(1, resident_clusters(p.nc));
   const int per = cdiv(B, std::min(cap, B));
   p.R = per >= 5 ? 8 : per >= 3 ? 4 : per;
   p.nch = cdiv(per, p.R);
@@ -587,7 +587,6 @@ int f32_fwd_recurrence(const blstm_desc& d, const F32Plan& pl, void* ifgo, const
                        cudaStream_t st) {
   F32Params p = f32_params(d, pl, ws);
   p.Wh = (const float*)Wh; p.ifgo = (float*)ifgo; p.out = (float*)out; p.cell = (float*)cell;
-  BLSTM_CUDA_OK(cudaMemsetAsync(ws, 0, sizeof(Control), st));
   switch (pl.kj) {
     case 1: return f32_fwd_r<1>(pl, p, st);
     case 2: return f32_fwd_r<2>(pl, p, st);
@@ -609,7 +608,6 @@ int f32_bwd_recurrence(const blstm_desc& d, const F32Plan& pl, const void* dout,
   p.dout = (const float*)dout; p.dh_n = (const float*)dh_n; p.dc_n = (const float*)dc_n;
   p.d_ifgo = (float*)d_ifgo; p.dh0 = (float*)dh0; p.dc0 = (float*)dc0;
   p.db_part = db ? reinterpret_cast<float*>(static_cast<char*>(ws) + sizeof(Control)) : nullptr;
-  BLSTM_CUDA_OK(cudaMemsetAsync(ws, 0, sizeof(Control), st));
   int rc = BLSTM_E_UNSUPPORTED;
   if (pl.U == 24) rc = f32_bwd_r<24, 10>(pl, p, st);
   else if (pl.pw == 1) rc = f32_bwd_r<32, 1>(pl, p, st);

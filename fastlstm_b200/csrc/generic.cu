@@ -430,7 +430,6 @@ int generic_fwd_recurrence(const blstm_desc& d, void* ifgo, const void* Wh, void
   if (ws_bytes < pl.ws_bytes) return BLSTM_E_WORKSPACE;
   const sm100::F32Plan fp = sm100::f32_plan(d, BLSTM_PHASE_FWD);
   if (fp.ok) return f32_fwd_recurrence(d, fp, ifgo, Wh, out, cell, ws, st);
-  BLSTM_CUDA_OK(cudaMemsetAsync(ws, 0, pl.off_db, st));
   switch (d.dtype) {
     case BLSTM_F32: return launch_fwd<float>(d, pl, ifgo, Wh, out, cell, ws, st);
     case BLSTM_F16: return launch_fwd<__half>(d, pl, ifgo, Wh, out, cell, ws, st);
@@ -465,7 +464,6 @@ int generic_bwd_recurrence(const blstm_desc& d, const void* dout, const void* dh
   if (ws_bytes < pl.ws_bytes) return BLSTM_E_WORKSPACE;
   const sm100::F32Plan fp = sm100::f32_plan(d, BLSTM_PHASE_BWD);
   if (fp.ok) return f32_bwd_recurrence(d, fp, dout, dh_n, dc_n, ifgo, cell, Wh, d_ifgo, dh0, dc0, db, ws, st);
-  BLSTM_CUDA_OK(cudaMemsetAsync(ws, 0, pl.off_db, st));
   int rc = BLSTM_E_INVALID_ARG;
   switch (d.dtype) {
     case BLSTM_F32: rc = launch_bwd<float>(d, pl, dout, dh_n, dc_n, ifgo, cell, Wh, d_ifgo, dh0, dc0, ws, st); break;

@@ -19,6 +19,7 @@ int sm100_wgrad(const blstm_desc& d, const void* d_ifgo, const void* x, const vo
 // true when the tcgen05 persistent recurrence covers this problem
 bool sm100_recurrence_supported(const blstm_desc& d, int phase);
 size_t sm100_recurrence_workspace(const blstm_desc& d, int phase);
+size_t sm100_recurrence_control(const blstm_desc& d, int phase);   // ... of which this much is cleared before the launch
 int sm100_fwd_recurrence(const blstm_desc& d, void* ifgo, const void* Wh, void* out, void* cell,
                          void* ws, size_t ws_bytes, cudaStream_t st);
 int sm100_bwd_recurrence(const blstm_desc& d, const void* dout, const void* dh_n, const void* dc_n,

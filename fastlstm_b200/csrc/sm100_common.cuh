@@ -140,13 +140,7 @@ static __device__ __noinline__ bool mbar_wait_slow(uint64_t* bar, uint32_t parit
       if (w.ctl && ld_relaxed_gpu(&w.ctl->abort) != 0) { *w.dead = 1; return false; }
       if (globaltimer_ns() - t0 > w.limit_ns) {
         *w.dead = 1;
-        if (w.ctl) {
-          if (atomicCAS(&w.ctl->status, 0, BLSTM_E_WAIT_TIMEOUT) == 0) {
-            w.ctl->detail[0] = w.d0;
-            w.ctl->detail[1] = w.d1;
-          }
-          atomicExch(&w.ctl->abort, 1);
-        }
+        if (w.ctl) record_timeout(w.ctl, w.d0, w.d1);
         return false;
       }
     }
@@ -165,13 +159,7 @@ static __device__ __noinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t pa
       if (w.ctl && ld_relaxed_gpu(&w.ctl->abort) != 0) { *w.dead = 1; return false; }
       if (globaltimer_ns() - t0 > w.limit_ns) {
         *w.dead = 1;
-        if (w.ctl) {
-          if (atomicCAS(&w.ctl->status, 0, BLSTM_E_WAIT_TIMEOUT) == 0) {
-            w.ctl->detail[0] = w.d0;
-            w.ctl->detail[1] = w.d1;
-          }
-          atomicExch(&w.ctl->abort, 1);
-        }
+        if (w.ctl) record_timeout(w.ctl, w.d0, w.d1);
         return false;
       }
     }

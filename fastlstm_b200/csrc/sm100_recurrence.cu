@@ -1768,6 +1768,11 @@ size_t sm100_recurrence_workspace(const blstm_desc& d, int phase) {
   return phase == BLSTM_PHASE_BWD ? make_bwd_plan(d).ws_bytes : make_plan(d, phase).ws_bytes;
 }
 
+size_t sm100_recurrence_control(const blstm_desc& d, int phase) {
+  if (small_plan(d, phase).ok) return sizeof(Control);
+  return phase == BLSTM_PHASE_BWD ? make_bwd_plan(d).off_db : make_plan(d, phase).ws_bytes;
+}
+
 int sm100_plan_detail(const blstm_desc& d, int phase, char* buf, size_t n) {
   const SmallPlan sp = small_plan(d, phase);
   if (sp.ok) return small_plan_detail(d, sp, phase, buf, n);
@@ -1829,7 +1834,6 @@ int sm100_fwd_recurrence(const blstm_desc& d, void* ifgo, const void* Wh, void* 
       if (rc) return rc;
     }
   }
-  BLSTM_CUDA_OK(cudaMemsetAsync(ws, 0, pl.ws_bytes, st));
   FwdParams p;
   p.npb = pl.npb;
   p.ep_bytes = (int)pl.ep_bytes;
@@ -1910,7 +1914,6 @@ int sm100_bwd_recurrence(const blstm_desc& d, const void* dout, const void* dh_n
     rc = encode_tensor_map(&td, d_ifgo, 4, dims, str, box, 2, 32);
     if (rc) return rc;
   }
-  BLSTM_CUDA_OK(cudaMemsetAsync(ws, 0, pl.off_db, st));
   BwdParams p;
   p.ep_bytes = (int)pl.ep_bytes;
   p.T = T; p.B = B; p.H = H;

@@ -828,7 +828,7 @@ SmallPlan small_plan(const blstm_desc& d, int phase) {
   p.gc = cdiv(G, small_cluster(H));
   p.nc = cdiv(G, p.gc);
   if (p.nc == 1 && (d.flags & BLSTM_FLAG_TEST_NO_ARRIVE)) return p;     // (no wait that could run out)
-  const int cap = std::max(1, resident_clusters(p.nc) / ((d.flags & BLSTM_FLAG_HALF_DEVICE) ? 2 : 1));
+  const int cap = std::max(1, resident_clusters(p.nc));   // (no cluster waits for another: two launches share the device as they fit)
   p.ks = 2 * cdiv(H, 32);
   const int tiles = cdiv(B, 8);
   p.ncl = std::min(cap, tiles);
@@ -945,7 +945,6 @@ int small_fwd_recurrence(const blstm_desc& d, const SmallPlan& pl, void* ifgo, c
   p.limit_ns = d.wait_limit_us > 0 ? (unsigned long long)d.wait_limit_us * 1000ull : kDefaultWaitNs;
   p.ctl = reinterpret_cast<Control*>(ws);
   p.Wh = Wh; p.out = out; p.cell = cell;
-  BLSTM_CUDA_OK(cudaMemsetAsync(ws, 0, sizeof(Control), st));
   CUtensorMap tp, th, tc;
   int rc = gates_map(&tp, ifgo, d, pl);
   if (!rc) rc = states_map(&th, out, d, pl, d.seq_len + 1);
@@ -965,7 +964,6 @@ int small_bwd_recurrence(const blstm_desc& d, const SmallPlan& pl, const void* d
   p.ctl = reinterpret_cast<Control*>(ws);
   p.dh_n = dh_n; p.dc_n = dc_n; p.cell = cell; p.Wh = Wh; p.dh0 = dh0; p.dc0 = dc0;
   p.db_part = db ? reinterpret_cast<float*>(static_cast<char*>(ws) + sizeof(Control)) : nullptr;
-  BLSTM_CUDA_OK(cudaMemsetAsync(ws, 0, sizeof(Control), st));
   CUtensorMap tp, tc, to, td;
   int rc = gates_map(&tp, ifgo, d, pl);
   if (!rc) rc = states_map(&tc, cell, d, pl, d.seq_len + 1);

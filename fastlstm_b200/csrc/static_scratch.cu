@@ -57,8 +57,10 @@ int blstm_fwd_recurrence_static(const blstm_desc* d, void* ifgo, const void* Wh,
   int rc = static_scratch_ptr(&ws);
   if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
-  // The launchers below clear the control block and every counter they use with a
-  // stream-ordered memset before the kernel, so the previous call's contents never leak in.
+  // The control block and every counter are cleared on the stream before the kernel, so the
+  // previous call's contents never leak in.
+  rc = begin_call(*d, BLSTM_PHASE_FWD, ws, nullptr, nullptr, nullptr, nullptr, st);
+  if (rc) return rc;
   if (sm100_recurrence_supported(*d, BLSTM_PHASE_FWD))
     return sm100_fwd_recurrence(*d, ifgo, Wh, out, cell, ws, kStaticScratchBytes, st);
   return generic_fwd_recurrence(*d, ifgo, Wh, out, cell, ws, kStaticScratchBytes, st);

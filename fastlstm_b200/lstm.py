@@ -13,12 +13,14 @@ gradients through the returned (h_n, c_n), fp32 weight/bias gradients, fp32
 matmuls stay fp32 (the reference flips the global TF32 switch on import,
 fastlstm/lstm.py:15-19; this module does not).  PyTorch is used for device
 memory, streams and autograd only; every device computation goes through
-libfastlstm_b200.so and there is no fallback path.
+libfastlstm_b200.so and there is no fallback path.  What a call does on the
+host - checks, buffers, the C ABI calls - is csrc/host.cpp.
 """
 from __future__ import annotations
 
+import contextlib
+import functools
 import os
-import threading
 
 import torch
 import torch.nn as nn
@@ -27,19 +29,8 @@ from . import _lib
 
 _DTYPE_CODE = {torch.float32: _lib.F32, torch.float16: _lib.F16, torch.bfloat16: _lib.BF16}
 
-# Set FASTLSTM_B200_SYNC_CHECK=1 to read the device status word (and wait for
-# the stream) after every recurrence launch; otherwise it is read lazily.
-_SYNC_CHECK = os.environ.get("FASTLSTM_B200_SYNC_CHECK", "0") == "1"
 _FORCE_GENERIC = os.environ.get("FASTLSTM_B200_FORCE_GENERIC", "0") == "1"
 _WAIT_LIMIT_US = int(os.environ.get("FASTLSTM_B200_WAIT_LIMIT_US", "0"))
-
-
-def _ptr(t):
-    return None if t is None else t.data_ptr()
-
-
-def _stream(t):
-    return torch.cuda.current_stream(t.device).cuda_stream
 
 
 def _desc(dtype, T, B, I, H, flags=0):
@@ -50,79 +41,17 @@ def _desc(dtype, T, B, I, H, flags=0):
     return _lib.Desc(_DTYPE_CODE[dtype], T, B, I, H, flags, _WAIT_LIMIT_US, 0)
 
 
-def _require(t, name, dtype=None, shape=None, device=None):
-    if t is None:
-        return
-    if not t.is_cuda:
-        raise ValueError(f"{name} must be a CUDA tensor (there is no CPU path)")
-    if not t.is_contiguous():
-        raise ValueError(f"{name} must be contiguous")
-    if dtype is not None and t.dtype != dtype:
-        raise ValueError(f"{name} has dtype {t.dtype}, expected {dtype}")
-    if device is not None and t.device != device:
-        raise ValueError(f"{name} is on {t.device}, expected {device}")
-    if shape is not None and tuple(t.shape) != tuple(shape):
-        raise ValueError(f"{name} has shape {tuple(t.shape)}, expected {tuple(shape)}")
-
-
-# ---------------------------------------------------------------------------
-# Deferred device-status checks: each recurrence launch leaves a status word in
-# its workspace; it is copied to pinned memory on the same stream and examined
-# once the copy has completed (at a later call, or in check_status()).
-# ---------------------------------------------------------------------------
-class _StatusRing:
-    def __init__(self):
-        self.lock = threading.Lock()
-        self.pending = []   # (event, pinned tensor, label)
-        self.free = []
-
-    def push(self, ws, label):
-        with self.lock:
-            host = self.free.pop() if self.free else torch.empty(4, dtype=torch.int32, pin_memory=True)
-        host.copy_(ws[:16].view(torch.int32), non_blocking=True)
-        ev = torch.cuda.Event()
-        ev.record(torch.cuda.current_stream(ws.device))
-        with self.lock:
-            self.pending.append((ev, host, label))
-
-    def poll(self, wait=False):
-        with self.lock:
-            items, self.pending = self.pending, []
-        keep, err = [], None
-        for ev, host, label in items:
-            if wait:
-                ev.synchronize()
-            if ev.query():
-                code = int(host[1])
-                if code != 0 and err is None:
-                    err = (code, label, int(host[2]), int(host[3]))
-                with self.lock:
-                    self.free.append(host)
-            else:
-                keep.append((ev, host, label))
-        with self.lock:
-            self.pending = keep + self.pending
-        if err is not None:
-            code, label, d0, d1 = err
-            raise _lib.BlstmError(code, f"{label} (step {d0}, batch tile {d1})")
-
-
-_status = _StatusRing()
-
-
 def check_status(wait: bool = True):
     """Raise if any finished launch recorded a device-side error (a bounded wait
-    that ran out).  With wait=True, first waits for all outstanding launches."""
-    _status.poll(wait=wait)
+    that ran out).  With wait=True, first waits for all outstanding launches.  (Launches write such an
+    error to mapped host memory; every operator call looks there too.)"""
+    _lib.host().check_status(bool(wait))
 
 
-def _after_launch(desc, ws, label):
-    if _SYNC_CHECK:
-        rc = _lib.load().blstm_read_status(ws.data_ptr(), None, _stream(ws))
-        _lib.check(rc, label)
-    else:
-        _status.push(ws, label)
-        _status.poll(wait=False)
+def _profiled(name):
+    """record_function while a profiler runs, nothing otherwise (entering one costs 5 us either way)."""
+    prof = torch.autograd.profiler
+    return prof.record_function(name) if prof._is_profiler_enabled else contextlib.nullcontext()
 
 
 _PHASES = {"fwd": _lib.PHASE_FWD, "bwd": _lib.PHASE_BWD, "fwd_op": _lib.PHASE_FWD_OP}
@@ -154,33 +83,9 @@ def lstm_persistent_fwd(x, h0, c0, Wx, bx, Wh, bh, inference=False, half_device=
     inference=True: nothing is saved for backward - ifgo and cell[1..T-1] are left unwritten
     (cell[T] is still c_n), which halves the bytes each step moves.
     half_device=True: the recurrence is planned for half of the SMs (two layers side by side)."""
-    lib = _lib.load()
     if x.dim() == 2:
         x = x[None]
-    T, B, I = x.shape
-    H = Wh.shape[1]
-    dt, dev = x.dtype, x.device
-    _require(x, "x")
-    _require(Wx, "Wx", dt, (4 * H, I), dev)
-    _require(Wh, "Wh", dt, (4 * H, H), dev)
-    _require(bx, "bx", dt, (4 * H,), dev)
-    _require(bh, "bh", dt, (4 * H,), dev)
-    if (h0 is None) != (c0 is None):
-        raise ValueError("h0 and c0 must both be given or both be None")
-    _require(h0, "h0", dt, (B, H), dev)
-    _require(c0, "c0", dt, (B, H), dev)
-    d = _desc(dt, T, B, I, H, (_lib.FLAG_INFERENCE if inference else 0) | (_lib.FLAG_HALF_DEVICE if half_device else 0))
-    with torch.cuda.device(dev):
-        states = torch.empty((2, T + 1, B, H), device=dev, dtype=dt)
-        out, cell = states.unbind(0)
-        ifgo = torch.empty((T, B, 4 * H), device=dev, dtype=dt)
-        ws_bytes = lib.blstm_workspace_bytes(d, _lib.PHASE_FWD)
-        ws = torch.empty(ws_bytes, device=dev, dtype=torch.uint8)
-        rc = lib.blstm_fwd(d, _ptr(x), _ptr(h0), _ptr(c0), _ptr(Wx), _ptr(Wh), _ptr(bx), _ptr(bh),
-                           _ptr(out), _ptr(cell), _ptr(ifgo), _ptr(ws), ws_bytes, _stream(x))
-        _lib.check(rc, "blstm_fwd")
-        _after_launch(d, ws, "forward recurrence")
-    return out, cell, ifgo
+    return _lib.host().fwd(x, h0, c0, Wx, bx, Wh, bh, bool(inference), bool(half_device))
 
 
 def lstm_persistent_bwd(dh, dc_n, dh_n, x, h, cell, ifgo, Wx, Wh, need_dx=True, wgrads=None, half_device=False):
@@ -190,59 +95,13 @@ def lstm_persistent_bwd(dh, dc_n, dh_n, x, h, cell, ifgo, Wx, Wh, need_dx=True, 
     fp32, dbx is dbh.  (fastlstm/lstm.py:236-334)
     wgrads: optional flat fp32 tensor of 4H*(I+H+1) elements laid out dWx | dWh | db that the
     kernels write into (a data-parallel gradient bucket); allocated here when None."""
-    lib = _lib.load()
-    T, B, H = dh.shape
-    I = x.shape[-1]
-    dt, dev = x.dtype, x.device
-    dh = dh.contiguous()
-    _require(dh, "dh", dt, (T, B, H), dev)
-    _require(dh_n, "dh_n", dt, (B, H), dev)
-    _require(dc_n, "dc_n", dt, (B, H), dev)
-    _require(h, "h", dt, (T + 1, B, H), dev)
-    _require(cell, "cell", dt, (T + 1, B, H), dev)
-    _require(ifgo, "ifgo", dt, (T, B, 4 * H), dev)
-    d = _desc(dt, T, B, I, H, _lib.FLAG_HALF_DEVICE if half_device else 0)
-    with torch.cuda.device(dev):
-        d_ifgo = torch.empty_like(ifgo)
-        d_x = torch.empty((T, B, I), device=dev, dtype=dt) if need_dx else None
-        carries = torch.empty((2, B, H), device=dev, dtype=dt)
-        dh_0, dc_0 = carries.unbind(0)
-        if wgrads is None:
-            wgrads = torch.empty(4 * H * (I + H + 1), device=dev, dtype=torch.float32)
-        _require(wgrads, "wgrads", torch.float32, (4 * H * (I + H + 1),), dev)
-        dWx = wgrads[:4 * H * I].view(4 * H, I)
-        dWh = wgrads[4 * H * I:4 * H * (I + H)].view(4 * H, H)
-        db = wgrads[4 * H * (I + H):]
-        ws_bytes = lib.blstm_workspace_bytes(d, _lib.PHASE_BWD)
-        ws = torch.empty(ws_bytes, device=dev, dtype=torch.uint8)
-        rc = lib.blstm_bwd(d, _ptr(dh), _ptr(dh_n), _ptr(dc_n), _ptr(x), _ptr(h), _ptr(cell),
-                           _ptr(ifgo), _ptr(Wx), _ptr(Wh), _ptr(d_ifgo), _ptr(d_x), _ptr(dh_0),
-                           _ptr(dc_0), _ptr(dWx), _ptr(dWh), _ptr(db), _ptr(ws), ws_bytes, _stream(x))
-        _lib.check(rc, "blstm_bwd")
-        _after_launch(d, ws, "backward recurrence")
-    return d_x, dh_0, dc_0, dWx, db, dWh, db
+    return _lib.host().bwd(dh.contiguous(), dc_n, dh_n, x, h, cell, ifgo, Wx, Wh, bool(need_dx), wgrads, bool(half_device))
 
 
 def Wgrad(d_ifgo, x, h):
     """(dbx, dbh, dWx, dWh) from d_ifgo [T,B,4H], x [T,B,I], h = out[T+1,B,H].
     (fastlstm/lstm.py:494-501; fp32 results, no transpose copy)"""
-    lib = _lib.load()
-    T, B, G = d_ifgo.shape
-    H, I = G // 4, x.shape[-1]
-    d = _desc(x.dtype, T, B, I, H)
-    dev = x.device
-    with torch.cuda.device(dev):
-        dWx = torch.empty((G, I), device=dev, dtype=torch.float32)
-        dWh = torch.empty((G, H), device=dev, dtype=torch.float32)
-        ws_bytes = lib.blstm_workspace_bytes(d, _lib.PHASE_BWD)
-        ws = torch.empty(ws_bytes, device=dev, dtype=torch.uint8)
-        rc = lib.blstm_wgrad(d, _ptr(d_ifgo), _ptr(x), _ptr(h), _ptr(dWx), _ptr(dWh), _ptr(ws),
-                             ws_bytes, _stream(x))
-        _lib.check(rc, "blstm_wgrad")
-        db = torch.empty(G, device=dev, dtype=torch.float32)
-        rc = lib.blstm_bias_grad(d, _ptr(d_ifgo), _ptr(db), _ptr(ws), ws_bytes, _stream(x))
-        _lib.check(rc, "blstm_bias_grad")
-    return db, db, dWx, dWh
+    return _lib.host().wgrad(d_ifgo, x, h)
 
 
 # ---------------------------------------------------------------------------
@@ -252,6 +111,7 @@ def Wgrad(d_ifgo, x, h):
 # exactly 0 and it feeds nothing into the real units; padded input columns meet zero weights.  The
 # padded copies cost a few small kernels per call - far less than the CUDA-core kernels they replace.
 # ---------------------------------------------------------------------------
+@functools.lru_cache(maxsize=1024)
 def _padded_sizes(dtype, I, H, T=1, B=None):
     """(Ip, Hp) when the layer should run zero-padded on the tensor-core kernels, else None.  With a
     batch size: hidden sizes in multiples of 8 where the small-batch recurrences take them."""
@@ -260,6 +120,8 @@ def _padded_sizes(dtype, I, H, T=1, B=None):
     if max(I, H) <= 64 and T <= 12:           # tiny sizes have the fused kernel
         return None
     Ip, Hp = -(-I // 8) * 8, -(-H // 8) * 8
+    if Ip == I and H % 64 == 0:
+        return None
     if B is None or any(plan_name(dtype, T, B, Ip, Hp, phase) != "sm100" for phase in ("fwd", "bwd")):
         Hp = -(-H // 64) * 64
     if (Ip, Hp) == (I, H) or Hp > 2048:
@@ -323,7 +185,7 @@ class PersistentLSTMfn(torch.autograd.Function):
             inference = not any(ctx.needs_input_grad)
         ctx.inference = bool(inference)
         ctx.sink = sink
-        with torch.autograd.profiler.record_function("fastlstm_b200::fwd"):
+        with _profiled("fastlstm_b200::fwd"):
             out, cell, ifgo = lstm_persistent_fwd(
                 x, None if h_0 is None else h_0.contiguous(), None if c_0 is None else c_0.contiguous(),
                 Wx.contiguous(), bx, Wh.contiguous(), bh, inference=inference)
@@ -356,7 +218,7 @@ class PersistentLSTMfn(torch.autograd.Function):
         d_out = d_out.contiguous()
         d_hn = None if d_hn is None else d_hn.contiguous()
         d_cn = None if d_cn is None else d_cn.contiguous()
-        with torch.autograd.profiler.record_function("fastlstm_b200::bwd"):
+        with _profiled("fastlstm_b200::bwd"):
             d_x, dh_0, dc_0, dWx, dbx, dWh, dbh = lstm_persistent_bwd(
                 d_out, d_cn, d_hn, x, out, cell, ifgo, Wx.contiguous(), Wh.contiguous(),
                 need_dx=ctx.needs_input_grad[0],
@@ -382,6 +244,26 @@ class PersistentLSTMfn(torch.autograd.Function):
             return (d_x, dh_0, dc_0, None, None, None, None, None, None, None)
         return (d_x, dh_0, dc_0, dWx, dbx if ctx.has_bias[0] else None, dWh,
                 dbh if ctx.has_bias[1] else None, None, None, None)
+
+
+def _layer(x, h0, c0, Wx, bx, Wh, bh, inference, stacked=False):
+    """One layer on the GPU, as PersistentLSTMfn computes it (same casts, padding and gradients), with the
+    conversions in one launch and the autograd node in the host extension.  stacked: the final states come as
+    tensors [1,B,H] of their own."""
+    host = _lib.host()
+    if (h0 is None) != (c0 is None):
+        raise ValueError("h0 and c0 must both be given or both be None")
+    to = torch.get_autocast_dtype("cuda") if torch.is_autocast_enabled("cuda") else None
+    T, B, I = x.shape
+    H = Wh.shape[1]
+    Ip, Hp = _padded_sizes(x.dtype if to is None else to, I, H, T, B) or (0, 0)
+    xp, h0p, c0p, Wxp, bxp, Whp, bhp = host.prepare(x, h0, c0, Wx, bx, Wh, bh, to, Ip, Hp)
+    with _profiled("fastlstm_b200::fwd"):
+        out, cell, ifgo = lstm_persistent_fwd(xp, h0p, c0p, Wxp, bxp, Whp, bhp, inference=inference)
+    if not inference:
+        return host.attach(x, h0, c0, Wx, bx, Wh, bh, xp, Wxp, Whp, out, cell, ifgo, stacked)
+    o, h, c = out[1:, :, :H], out[-1, :, :H], cell[-1, :, :H]
+    return (o, h[None].clone(), c[None].clone()) if stacked else (o, h, c)
 
 
 _side_streams = {}
@@ -421,7 +303,7 @@ class WavefrontLSTMfn(torch.autograd.Function):
         streams[1].wait_stream(main)
         saved = [[None] * NC for _ in range(L)]
         done = [[None] * NC for _ in range(L)]
-        with torch.autograd.profiler.record_function("fastlstm_b200::wavefront_fwd"):
+        with _profiled("fastlstm_b200::wavefront_fwd"):
             for diag in range(NC + L - 1):
                 for l in range(L):
                     k = diag - l
@@ -480,7 +362,7 @@ class WavefrontLSTMfn(torch.autograd.Function):
         carry = [[None] * NC for _ in range(L)]
         done = [[None] * NC for _ in range(L)]
         acc = [None] * L
-        with torch.autograd.profiler.record_function("fastlstm_b200::wavefront_bwd"):
+        with _profiled("fastlstm_b200::wavefront_bwd"):
             for diag in range(NC + L - 1):
                 for li in range(L):
                     l = L - 1 - li
@@ -597,6 +479,8 @@ class FastLSTM(nn.Module):
         self.num_directions = 2 if bidirectional else 1
         self.proj_size = proj_size
         self._sinks = None            # per (layer, direction) gradient sinks of a GradBucket, or None
+        self._names = {(layer, d): tuple(f"{n}_l{layer}{sfx}" for n in ("weight_ih", "bias_ih", "weight_hh", "bias_hh"))
+                       for layer in range(num_layers) for d, sfx in enumerate(self._suffixes())}
         k = 1.0 / hidden_size ** 0.5
         fk = dict(device=device, dtype=dtype)
 
@@ -619,9 +503,8 @@ class FastLSTM(nn.Module):
         return ("", "_reverse") if self.bidirectional else ("",)
 
     def layer_params(self, layer, reverse=False):
-        sfx = "_reverse" if reverse else ""
-        g = lambda n: getattr(self, f"{n}_l{layer}{sfx}", None)
-        return g("weight_ih"), g("bias_ih"), g("weight_hh"), g("bias_hh")
+        own = self._parameters           # (a reparametrised weight is an attribute instead)
+        return tuple(own[n] if n in own else getattr(self, n, None) for n in self._names[layer, int(reverse)])
 
     def _projected_layer(self, x_d, h0, c0, Wx, bx, Wh, bh, Whr, inference):
         """One direction of one layer with an output projection (nn.LSTM's proj_size): the recurrent
@@ -648,9 +531,53 @@ class FastLSTM(nn.Module):
             return self._forward_packed(x, h_c_0)
         if x.dim() != 3:
             raise ValueError("expected a 3-D input [T,B,I] (or [B,T,I] with batch_first)")
+        if not torch.is_grad_enabled():
+            res = self._forward_inference(x, h_c_0)
+            if res is not None:
+                return res
         if self.batch_first:
             x = x.transpose(0, 1)
         return self._forward_padded(x, h_c_0, None)
+
+    def _forward_inference(self, x, h_c_0):
+        """Grad mode off, one direction, nothing to convert or pad: the layers without autograd nodes; a single
+        timestep, where the host is what takes the time, in one call of the host extension.  None when the
+        general path has to run."""
+        if (self.num_directions != 1 or self.proj_size > 0 or not x.is_cuda or torch.is_autocast_enabled("cuda")
+                or (self.dropout > 0.0 and self.training and self.num_layers > 1)):
+            return None
+        L, H, dt = self.num_layers, self.hidden_size, x.dtype
+        T, B = (x.shape[1], x.shape[0]) if self.batch_first else (x.shape[0], x.shape[1])
+        if T > 1 and (self._wavefront_chunks(x.transpose(0, 1) if self.batch_first else x, h_c_0, None)
+                      or any(_padded_sizes(dt, n, H, T, B) is not None for n in {x.shape[2], H})):
+            return None
+        if T == 1 and dt != torch.float32 and (H % 8 or x.shape[2] % 8):
+            return None
+        h0 = c0 = None
+        if h_c_0 is not None:
+            h0, c0 = h_c_0
+            if not (torch.is_tensor(h0) and torch.is_tensor(c0) and h0.dim() == 3 and c0.dim() == 3
+                    and h0.shape[0] == L and c0.shape[0] == L and h0.dtype == dt and c0.dtype == dt):
+                return None
+        params = []
+        for layer in range(L):
+            params += self.layer_params(layer)
+        if any(p is not None and p.dtype != dt for p in params):
+            return None
+        if T == 1:
+            out, h_n, c_n = _lib.host().infer(x, h0, c0, params, self.batch_first)
+            return out, (h_n, c_n)
+        x = (x.transpose(0, 1) if self.batch_first else x).contiguous()
+        h_n, c_n = [], []
+        for layer in range(L):
+            Wx, bx, Wh, bh = params[4 * layer:4 * layer + 4]
+            out, cell, _ = lstm_persistent_fwd(x, None if h0 is None else h0[layer].contiguous(),
+                                               None if c0 is None else c0[layer].contiguous(),
+                                               Wx.contiguous(), bx, Wh.contiguous(), bh, inference=True)
+            x = out[1:]
+            h_n.append(out[-1])
+            c_n.append(cell[-1])
+        return x.transpose(0, 1) if self.batch_first else x, (torch.stack(h_n), torch.stack(c_n))
 
     def _forward_packed(self, seq, h_c_0):
         """PackedSequence input (torch.nn.LSTM's convention; the reference lists it as missing,
@@ -673,15 +600,13 @@ class FastLSTM(nn.Module):
         The wavefront needs two or more layers of one direction on the tensor-core kernels and pays
         when a layer alone leaves the GPU latency bound: every CTA has a single batch tile on the
         whole device and at most two on half of it."""
-        if os.environ.get("FASTLSTM_B200_WAVEFRONT", "1") == "0":
-            return 0
-        if (self.num_layers < 2 or self.num_directions != 1 or self.proj_size > 0 or lengths is not None
+        if (x.shape[0] < 64 or self.num_layers < 2 or self.num_directions != 1 or self.proj_size > 0 or lengths is not None
                 or (self.dropout > 0.0 and self.training) or not x.is_cuda
                 or x.dtype not in (torch.float16, torch.bfloat16) or torch.is_autocast_enabled("cuda")):
             return 0
         T, B, I = x.shape
         H = self.hidden_size
-        if H % 64 != 0 or H > 1024 or I % 8 != 0 or T < 64:
+        if H % 64 != 0 or H > 1024 or I % 8 != 0 or os.environ.get("FASTLSTM_B200_WAVEFRONT", "1") == "0":
             return 0
         if any(p.dtype != x.dtype for p in self.parameters()):
             return 0
@@ -742,6 +667,7 @@ class FastLSTM(nn.Module):
             if len(h_0) != self.num_layers * nd or len(c_0) != self.num_layers * nd:
                 raise ValueError(f"expected {self.num_layers * nd} initial states, got {len(h_0)} / {len(c_0)}")
         h_n, c_n = [], []
+        single = (self.num_layers * nd == 1 and self.proj_size == 0 and lengths is None and self._sinks is None and x.is_cuda)
         for layer in range(self.num_layers):
             outs = []
             for d in range(nd):
@@ -760,6 +686,8 @@ class FastLSTM(nn.Module):
                     if lengths is not None:
                         h_i, c_i = at_last(o), at_last(cells)
                         o = o * valid[:, :, None].to(o.dtype)
+                elif lengths is None and sink is None and x_d.is_cuda:
+                    o, h_i, c_i = _layer(x_d, hl, cl, Wx, bx, Wh, bh, inference, single)
                 elif lengths is None:
                     o, h_i, c_i = PersistentLSTMfn.apply(x_d, hl, cl, Wx, bx, Wh, bh, inference, sink)
                 else:
@@ -774,4 +702,6 @@ class FastLSTM(nn.Module):
                 x = torch.nn.functional.dropout(x, self.dropout, True)
         if self.batch_first and lengths is None:
             x = x.transpose(0, 1)
+        if single:                        # (the layer has made the stacked tensors itself)
+            return x, (h_n[0], c_n[0])
         return x, (torch.stack(h_n), torch.stack(c_n))

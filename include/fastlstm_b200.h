@@ -129,7 +129,8 @@ int blstm_fwd_recurrence(const blstm_desc* d, void* ifgo, const void* Wh, void* 
                          void* cell, void* workspace, size_t workspace_bytes, void* stream);
 
 /* Whole forward operator: initial-state slots, projection, recurrence.
- * h0/c0 [B,H] may both be NULL (zeros).  Replaces lstm_persistent_fwd,
+ * h0/c0 [B,H] may both be NULL (zeros).  A single timestep of up to 64 rows is one launch (plan "step");
+ * with BLSTM_FLAG_INFERENCE that plan does not need ifgo (NULL allowed).  Replaces lstm_persistent_fwd,
  * fastlstm/lstm.py:31-146, including its dispatch of tiny sizes to the fully fused kernel
  * (fastlstm/lstm.py:40-47, fastlstm/kernels.py:672-819): one launch, no projected
  * pre-activations in memory, no workspace use. */
@@ -198,6 +199,26 @@ int blstm_fwd_recurrence_static(const blstm_desc* d, void* ifgo, const void* Wh,
                                 void* cell, void* stream);
 size_t blstm_static_scratch_capacity(void);
 int blstm_static_scratch_status(int32_t* detail, void* stream);
+
+/* One dense tensor [groups, rows, cols] of another row and column count and element type: the common part is
+ * copied (converted), the rest of dst is zero. */
+typedef struct blstm_repack_item {
+  const void* src;
+  void* dst;
+  int32_t src_dtype, dst_dtype;   /* BLSTM_F32 / BLSTM_F16 / BLSTM_BF16 */
+  int64_t groups;
+  int32_t src_rows, src_cols, dst_rows, dst_cols;
+} blstm_repack_item;
+
+/* Up to 8 tensors in one launch: zero padding of ragged sizes, its inverse, type conversion.
+ * Stands in for the casts of fastlstm/lstm.py:511-517. */
+int blstm_repack(const blstm_repack_item* items, int n, void* stream);
+
+/* Host memory (mapped into the device, 16 bytes: -, status, detail[2]) that the CALLING THREAD's later
+ * launches write a device-side error to as well, or NULL (default): a caller that looks there need not
+ * read control blocks back.  The status word is written last; the caller clears it.  No reference
+ * counterpart. */
+void blstm_set_mailbox(int32_t* mapped);
 
 /* Number of kernels this library has launched in this process so far (HOST
  * counter; memsets and copies are not counted).  Benchmarks report the

@@ -145,3 +145,80 @@ def test_fp32_gemms_against_fp64_matmul(shape):
     X, D, O = x.double().view(T * B, I), dg.double().view(T * B, -1), out[:-1].double().reshape(T * B, H)
     for got, want in ((ifgo, X @ Wx.double().T + bx.double() + bh.double()), (dx, D @ Wx.double()), (dWx, D.T @ X), (dWh, D.T @ O)):
         assert float((got - want).norm() / want.norm()) <= 1e-6
+
+
+# one row; a partial n-tile; the most rows; sizes the 16-byte accesses do not take (fp32); K in partial blocks of 32
+@pytest.mark.parametrize("dtype,B,I,H", [("bf16", 1, 512, 512), ("fp16", 9, 40, 72), ("bf16", 64, 136, 8), ("fp16", 33, 8, 1024),
+                                         ("fp32", 1, 16, 64), ("fp32", 7, 123, 65), ("fp32", 64, 200, 400), ("fp32", 2, 3, 5)])
+@pytest.mark.parametrize("states", [False, True])
+def test_single_timestep_kernel_against_fp64_maths(dtype, B, I, H, states):
+    lib = _lib.load()
+    dt = {"fp32": torch.float32, **TD}[dtype]
+    g = torch.Generator(device="cuda").manual_seed(B + I + H)
+    r = lambda *s, std=1.0: (torch.randn(*s, generator=g, device="cuda") * std).to(dt)
+    x, Wx, Wh, bx, bh = r(1, B, I), r(4 * H, I, std=I ** -0.5), r(4 * H, H, std=H ** -0.5), r(4 * H, std=0.1), r(4 * H, std=0.1)
+    h0, c0 = (r(B, H, std=0.3), r(B, H, std=0.3)) if states else (None, None)
+    p = lambda t: None if t is None else t.data_ptr()
+    s = torch.cuda.current_stream().cuda_stream
+    res = []
+    for flags in (0, _lib.FLAG_INFERENCE):
+        d = _lib.Desc(_lib.DTYPE_CODE[dtype], 1, B, I, H, flags, 0, 0)
+        assert lib.blstm_plan_name(d, _lib.PHASE_FWD_OP) == b"step"
+        out, cell, ifgo = (torch.full(sh, float("nan"), device="cuda", dtype=dt) for sh in ((2, B, H), (2, B, H), (1, B, 4 * H)))
+        n = lib.blstm_workspace_bytes(d, 0)
+        ws = torch.ones(n, dtype=torch.uint8, device="cuda")
+        _lib.check(lib.blstm_fwd(d, p(x), p(h0), p(c0), p(Wx), p(Wh), p(bx), p(bh), p(out), p(cell), p(ifgo) if not flags else None,
+                                 p(ws), n, s))
+        assert lib.blstm_read_status(ws.data_ptr(), None, s) == 0
+        res.append((out, cell, ifgo))
+    z = torch.zeros(B, H, device="cuda", dtype=torch.float64)
+    hp, cp = (z, z) if h0 is None else (h0.double(), c0.double())
+    a = x[0].double() @ Wx.double().T + hp @ Wh.double().T + bx.double() + bh.double()
+    i, f, gg, o = a.split(H, dim=1)
+    c = torch.sigmoid(f) * cp + torch.sigmoid(i) * torch.tanh(gg)
+    h = torch.sigmoid(o) * torch.tanh(c)
+    tol = {"fp32": 1e-5, "fp16": 3e-3, "bf16": 2e-2}[dtype]
+    out, cell, ifgo = res[0]
+    for got, want in ((out[0], hp), (cell[0], cp), (out[1], h), (cell[1], c), (ifgo[0], a)):
+        assert float((got.double() - want).abs().max()) <= tol * max(1.0, float(want.abs().max()))
+    assert torch.equal(res[1][0], out) and torch.equal(res[1][1], cell)
+
+
+def test_mailbox_hears_of_a_wait_that_ran_out():
+    """Launches of a thread that has set a mailbox also leave a device-side error there (no fault: suppressed arrivals)."""
+    lib = _lib.load()
+    T, B, H = 4, 9, 256
+    z = lambda *s: torch.zeros(*s, device="cuda", dtype=torch.bfloat16)
+    ifgo, out, cell, Wh = z(T, B, 4 * H), z(T + 1, B, H), z(T + 1, B, H), z(4 * H, H)
+    mail = torch.zeros(4, dtype=torch.int32).pin_memory()
+    s = torch.cuda.current_stream().cuda_stream
+    d = _lib.Desc(_lib.BF16, T, B, H, H, _lib.FLAG_TEST_NO_ARRIVE, 20000, 0)
+    n = lib.blstm_workspace_bytes(d, 0)
+    ws = torch.zeros(n, dtype=torch.uint8, device="cuda")
+    lib.blstm_set_mailbox(mail.data_ptr())
+    try:
+        assert lib.blstm_fwd_recurrence(d, ifgo.data_ptr(), Wh.data_ptr(), out.data_ptr(), cell.data_ptr(), ws.data_ptr(), n, s) == 0
+    finally:
+        lib.blstm_set_mailbox(None)
+    torch.cuda.synchronize()
+    assert mail[1] == _lib.E_WAIT_TIMEOUT and mail[2] >= 1
+
+
+@pytest.mark.parametrize("G,R,C,R2,C2", [(4, 65, 123, 128, 128), (4, 128, 128, 65, 123), (1, 40, 33, 40, 64), (3, 7, 8, 7, 8), (1, 5, 3, 5, 3)])
+@pytest.mark.parametrize("src,dst", [("fp32", "fp32"), ("fp32", "bf16"), ("fp16", "fp16"), ("bf16", "fp32")])
+def test_repack_pads_crops_and_converts(G, R, C, R2, C2, src, dst):
+    import ctypes
+    lib = _lib.load()
+    ty = {"fp32": torch.float32, **TD}
+    a = torch.randn(G, R, C, device="cuda").to(ty[src])
+    b = torch.full((G, R2, C2), float("nan"), device="cuda", dtype=ty[dst])
+
+    class Item(ctypes.Structure):
+        _fields_ = [("src", ctypes.c_void_p), ("dst", ctypes.c_void_p), ("sd", ctypes.c_int32), ("dd", ctypes.c_int32),
+                    ("groups", ctypes.c_int64), ("r", ctypes.c_int32), ("c", ctypes.c_int32), ("r2", ctypes.c_int32), ("c2", ctypes.c_int32)]
+    items = (Item * 1)(Item(a.data_ptr(), b.data_ptr(), _lib.DTYPE_CODE[src], _lib.DTYPE_CODE[dst], G, R, C, R2, C2))
+    _lib.check(lib.blstm_repack(items, 1, torch.cuda.current_stream().cuda_stream))
+    want = torch.zeros(G, R2, C2, device="cuda", dtype=ty[dst])
+    r, c = min(R, R2), min(C, C2)
+    want[:, :r, :c] = a[:, :r, :c].to(ty[dst])
+    assert torch.equal(b, want)
