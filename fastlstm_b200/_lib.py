@@ -56,6 +56,8 @@ SIGNATURES = {
     "blstm_launch_count": (ctypes.c_ulonglong, []),
     "blstm_set_mailbox": (None, [P]),
     "blstm_repack": (c_int, [P, c_int, P]),
+    "blstm_gather_rows": (c_int, [P, P, P, ctypes.c_int64, ctypes.c_int64, P]),
+    "blstm_packed_maps": (c_int, [P, P, P, c_int, c_int, P, P]),
     "blstm_fwd_recurrence_static": (c_int, [DP, P, P, P, P, P]),
     "blstm_static_scratch_capacity": (c_size_t, []),
     "blstm_static_scratch_status": (c_int, [POINTER(c_int32), P]),

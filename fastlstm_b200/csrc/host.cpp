@@ -399,6 +399,70 @@ py::tuple infer(const Tensor& x_in, const OptTensor& h0, const OptTensor& c0, co
   return py::make_tuple(out, hn, cn);
 }
 
+// ---------------------------------------------------------------- packed sequences
+Tensor gather_rows_impl(const Tensor& src_in, const Tensor& idx, at::IntArrayRef lead) {
+  const Tensor src = src_in.contiguous();
+  const int64_t C = src.size(-1);
+  std::vector<int64_t> shape = lead.vec();
+  shape.push_back(C);
+  const Tensor dst = at::empty(shape, src.options().requires_grad(false));
+  c10::cuda::CUDAGuard guard(src.device());
+  check(blstm_gather_rows(dst.data_ptr(), src.const_data_ptr(), (const int32_t*)idx.const_data_ptr(), idx.numel(), C * src.element_size(),
+                          at::cuda::getCurrentCUDAStream(src.device().index()).stream()),
+        "blstm_gather_rows");
+  return dst;
+}
+
+// Rows of src (its last dimension) in another order; `inv` maps every row of src to the row it went to, or -1.
+struct GatherRowsFn : public torch::autograd::Function<GatherRowsFn> {
+  static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& src, const Tensor& idx, const Tensor& inv, std::vector<int64_t> lead) {
+    ctx->save_for_backward({inv});
+    std::vector<int64_t> s = src.sizes().vec();
+    s.pop_back();
+    ctx->saved_data["lead"] = s;
+    return gather_rows_impl(src, idx, lead);
+  }
+  static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list g) {
+    const auto saved = ctx->get_saved_variables();
+    return {gather_rows_impl(g[0], saved[0], ctx->saved_data["lead"].toIntVector()), Tensor(), Tensor(), Tensor()};
+  }
+};
+
+Tensor gather_rows(const Tensor& src, const Tensor& idx, const Tensor& inv, std::vector<int64_t> lead) {
+  py::gil_scoped_release nogil;
+  return GatherRowsFn::apply(src, idx, inv, lead);
+}
+
+// The maps of blstm_packed_maps as tensors: (padded, turned, rev, inv_last, last, packed, packed_turned).
+std::vector<Tensor> packed_maps(const Tensor& batch_sizes, const OptTensor& rank, const Tensor& data) {
+  py::gil_scoped_release nogil;
+  const int64_t T = batch_sizes.numel();
+  const Tensor bs = batch_sizes.contiguous();
+  const int64_t* b = static_cast<const int64_t*>(bs.const_data_ptr());
+  const int64_t B = b[0];
+  const Tensor host = at::empty({2 * T}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
+  int32_t* h = static_cast<int32_t*>(host.data_ptr());
+  int64_t n = 0;
+  for (int64_t t = 0; t < T; ++t) {
+    h[t] = (int32_t)b[t];
+    h[T + t] = (int32_t)n;
+    n += b[t];
+  }
+  c10::cuda::CUDAGuard guard(data.device());
+  const auto i32 = data.options().requires_grad(false).dtype(at::kInt);
+  const Tensor dev = host.to(data.device(), /*non_blocking=*/true);
+  const Tensor maps = at::empty({4 * T * B + B + 2 * n}, i32);
+  check(blstm_packed_maps((const int32_t*)dev.const_data_ptr(), (const int32_t*)dev.const_data_ptr() + T,
+                          rank ? (const int64_t*)rank->const_data_ptr() : nullptr, (int)T, (int)B, (int32_t*)maps.data_ptr(),
+                          at::cuda::getCurrentCUDAStream(data.device().index()).stream()),
+        "blstm_packed_maps");
+  std::vector<Tensor> r;
+  for (int k = 0; k < 4; ++k) r.push_back(maps.narrow(0, k * T * B, T * B));
+  r.push_back(maps.narrow(0, 4 * T * B, B));
+  for (int k = 0; k < 2; ++k) r.push_back(maps.narrow(0, 4 * T * B + B + k * n, n));
+  return r;
+}
+
 void check_status(bool wait) {
   for (int dev = 0; dev < kMaxDevices; ++dev) {
     if (!g_mail[dev].load(std::memory_order_acquire)) continue;
@@ -435,5 +499,7 @@ PYBIND11_MODULE(_host, m) {
   m.def("prepare", &prepare);
   m.def("attach", &attach);
   m.def("infer", &infer);
+  m.def("gather_rows", &gather_rows);
+  m.def("packed_maps", &packed_maps);
   m.def("check_status", &check_status);
 }

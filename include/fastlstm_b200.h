@@ -214,6 +214,18 @@ typedef struct blstm_repack_item {
  * Stands in for the casts of fastlstm/lstm.py:511-517. */
 int blstm_repack(const blstm_repack_item* items, int n, void* stream);
 
+/* dst row i = src row idx[i], zeros where idx[i] < 0; n rows of row_bytes (even) bytes. */
+int blstm_gather_rows(void* dst, const void* src, const int32_t* idx, int64_t n, int64_t row_bytes, void* stream);
+
+/* Row maps between the rows of a packed batch (batch_sizes [T] and their exclusive sums `offsets` [T], device;
+ * `rank` [B]: sorted position of every sequence, or NULL) and the padded grid [T,B] it stands for:
+ *   maps = [T,B] packed row or -1 | [T,B] the same, each sequence from its end | [T,B] padded row, each sequence
+ *          reversed in place | [T,B] sequence whose last step this is, or -1 | [B] padded row of the last step |
+ *          [N] padded row | [N] padded row in the reversed grid,          N = sum of batch_sizes.
+ * No reference counterpart (packed sequences are listed as missing, README.md:92-93). */
+int blstm_packed_maps(const int32_t* batch_sizes, const int32_t* offsets, const int64_t* rank, int T, int B,
+                      int32_t* maps, void* stream);
+
 /* Host memory (mapped into the device, 16 bytes: -, status, detail[2]) that the CALLING THREAD's later
  * launches write a device-side error to as well, or NULL (default): a caller that looks there need not
  * read control blocks back.  The status word is written last; the caller clears it.  No reference

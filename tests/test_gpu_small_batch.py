@@ -222,3 +222,34 @@ def test_repack_pads_crops_and_converts(G, R, C, R2, C2, src, dst):
     r, c = min(R, R2), min(C, C2)
     want[:, :r, :c] = a[:, :r, :c].to(ty[dst])
     assert torch.equal(b, want)
+
+
+@pytest.mark.parametrize("lengths,C", [([1], 1), ([4, 9, 1, 6, 9, 2], 12), ([33] * 5, 8), ([70, 2, 41, 70], 130)])
+@pytest.mark.parametrize("dtype", ["fp32", "bf16"])
+def test_packed_row_maps_and_gathers(lengths, C, dtype):
+    """The maps between packed rows and the padded grid, forwards and turned, and the gathers they drive, against
+    torch's packing; each map's inverse carries the gradient."""
+    from torch.nn.utils.rnn import pack_padded_sequence
+    host = _lib.host()
+    ty = {"fp32": torch.float32, **TD}[dtype]
+    T, B = max(lengths), len(lengths)
+    x = torch.randn(T, B, C).to(ty)
+    turned_x = torch.zeros_like(x)
+    for b, n in enumerate(lengths):
+        x[n:, b] = 0
+        turned_x[:n, b] = x[:n, b].flip(0)
+    seq = pack_padded_sequence(x.cuda(), torch.tensor(lengths), enforce_sorted=False)
+    padded, turned, rev, inv_last, last, packed, packed_t = host.packed_maps(seq.batch_sizes, seq.unsorted_indices, seq.data)
+    data = seq.data.clone().requires_grad_(True)
+    a = host.gather_rows(data, padded, packed, [T, B])
+    b = host.gather_rows(data, turned, packed_t, [T, B])
+    assert torch.equal(a.cpu(), x) and torch.equal(b.cpu(), turned_x)
+    assert torch.equal(host.gather_rows(a, packed, padded, [data.shape[0]]), data)
+    assert torch.equal(host.gather_rows(b, packed_t, turned, [data.shape[0]]), data)
+    assert torch.equal(host.gather_rows(a, rev, rev, [T, B]).cpu(), turned_x)
+    h = host.gather_rows(a, last, inv_last, [B])
+    assert torch.equal(h.cpu(), torch.stack([x[n - 1, i] for i, n in enumerate(lengths)]))
+    h.sum().backward()
+    want = pack_padded_sequence(torch.stack([torch.arange(T) == n - 1 for n in lengths], 1)[:, :, None].expand(T, B, C).to(ty),
+                                torch.tensor(lengths), enforce_sorted=False).data
+    assert torch.equal(data.grad.cpu(), want)
