@@ -129,6 +129,19 @@ struct FwdOut {
   Tensor out, cell, ifgo;
 };
 
+// Two tensors of one shape in one allocation, each on a 16-byte boundary (which the kernels ask of 16-bit tensors).
+std::array<Tensor, 2> empty_pair(at::IntArrayRef shape, const at::TensorOptions& opt) {
+  const int64_t n = c10::multiply_integers(shape), step = (n + 7) / 8 * 8;
+  const Tensor both = at::empty({2 * step}, opt);
+  return {both.narrow(0, 0, n).view(shape), both.narrow(0, step, n).view(shape)};
+}
+
+// t contiguous and on a 16-byte boundary
+Tensor fit(const Tensor& t) {
+  const Tensor c = t.contiguous();
+  return reinterpret_cast<uintptr_t>(c.const_data_ptr()) & 15 ? c.clone() : c;
+}
+
 FwdOut fwd_impl(const Tensor& x, const OptTensor& h0, const OptTensor& c0, const Tensor& Wx, const OptTensor& bx, const Tensor& Wh,
                 const OptTensor& bh, bool inference, bool half_device) {
   require(x, "x");
@@ -147,9 +160,9 @@ FwdOut fwd_impl(const Tensor& x, const OptTensor& h0, const OptTensor& c0, const
   Call call(dev);
   const auto opt = x.options().requires_grad(false);
   FwdOut r;
-  const Tensor states = at::empty({2, T + 1, B, H}, opt);
-  r.out = states.select(0, 0);
-  r.cell = states.select(0, 1);
+  auto [out, cell] = empty_pair({T + 1, B, H}, opt);
+  r.out = out;
+  r.cell = cell;
   const bool lone = inference && T == 1 && std::string_view(blstm_plan_name(&d, BLSTM_PHASE_FWD_OP)) == "step";
   Tensor ws;
   size_t ws_bytes = 0;
@@ -197,21 +210,20 @@ BwdOut bwd_impl(const Tensor& dh, const OptTensor& dc_n, const OptTensor& dh_n, 
   const Tensor d_ifgo = at::empty({T, B, 4 * H}, opt);
   BwdOut r;
   if (need_dx) r.d_x = at::empty({T, B, I}, opt);
-  const Tensor carries = at::empty({2, B, H}, opt);
+  auto [dh_0, dc_0] = empty_pair({B, H}, opt);
+  r.dh_0 = dh_0;
+  r.dc_0 = dc_0;
   const int64_t n = 4 * H * (I + H + 1);
   r.wgrads = wgrads_in ? *wgrads_in : at::empty({n}, opt.dtype(at::kFloat));
   require(r.wgrads, "wgrads", at::kFloat, dev, {n});
   float* w = static_cast<float*>(r.wgrads.data_ptr());
   const size_t ws_bytes = blstm_workspace_bytes(&d, BLSTM_PHASE_BWD);
   const Tensor ws = at::empty({(int64_t)ws_bytes}, opt.dtype(at::kByte));
-  char* c = static_cast<char*>(carries.data_ptr());
   check(blstm_bwd(&d, ptr(dh), ptr(dh_n), ptr(dc_n), ptr(x), ptr(h), ptr(cell), ptr(ifgo), ptr(Wx), ptr(Wh), d_ifgo.data_ptr(),
-                  need_dx ? r.d_x.data_ptr() : nullptr, c, c + B * H * x.element_size(), w, w + 4 * H * I, w + 4 * H * (I + H),
+                  need_dx ? r.d_x.data_ptr() : nullptr, r.dh_0.data_ptr(), r.dc_0.data_ptr(), w, w + 4 * H * I, w + 4 * H * (I + H),
                   ws.data_ptr(), ws_bytes, call.stream),
         "blstm_bwd");
   call.done(ws, "backward recurrence");
-  r.dh_0 = carries.select(0, 0);
-  r.dc_0 = carries.select(0, 1);
   return r;
 }
 
@@ -265,7 +277,7 @@ py::tuple prepare(const Tensor& x, const OptTensor& h0, const OptTensor& c0, con
     auto move = [&](OptTensor& t, int64_t groups, int64_t rows, int64_t cols, int64_t rows_to, int64_t cols_to, std::vector<int64_t> shape) {
       if (!t) return;
       const auto ty = to.value_or(t->scalar_type());
-      if (ty == t->scalar_type() && rows == rows_to && cols == cols_to) t = t->contiguous();
+      if (ty == t->scalar_type() && rows == rows_to && cols == cols_to) t = fit(*t);
       else t = m.add(*t, ty, groups, rows, cols, rows_to, cols_to, shape);
     };
     auto last = [&](const OptTensor& t, int64_t n) { std::vector<int64_t> s = t ? t->sizes().vec() : std::vector<int64_t>(); if (t) s.back() = n; return s; };
@@ -380,15 +392,15 @@ py::tuple infer(const Tensor& x_in, const OptTensor& h0, const OptTensor& c0, co
     at::NoGradGuard no_grad;
     const int64_t L = (int64_t)params.size() / 4;
     Tensor x = batch_first ? x_in.transpose(0, 1) : x_in;
-    x = x.contiguous();
+    x = fit(x);
     std::vector<Tensor> h(L), c(L);
     for (int64_t l = 0; l < L; ++l) {
       OptTensor hl, cl;
-      if (h0) hl = h0->select(0, l).contiguous();
-      if (c0) cl = c0->select(0, l).contiguous();
+      if (h0) hl = fit(h0->select(0, l));
+      if (c0) cl = fit(c0->select(0, l));
       FwdOut r = fwd_impl(x, hl, cl, params[4 * l]->contiguous(), params[4 * l + 1], params[4 * l + 2]->contiguous(), params[4 * l + 3], true, false);
       const int64_t T = x.size(0);
-      x = r.out.narrow(0, 1, T);
+      x = fit(r.out.narrow(0, 1, T));
       h[l] = r.out.select(0, T);
       c[l] = r.cell.select(0, T);
     }

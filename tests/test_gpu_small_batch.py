@@ -253,3 +253,27 @@ def test_packed_row_maps_and_gathers(lengths, C, dtype):
     want = pack_padded_sequence(torch.stack([torch.arange(T) == n - 1 for n in lengths], 1)[:, :, None].expand(T, B, C).to(ty),
                                 torch.tensor(lengths), enforce_sorted=False).data
     assert torch.equal(data.grad.cpu(), want)
+
+
+@pytest.mark.parametrize("T,B,H,P,states", [(2, 1, 33, 7, True), (40, 9, 96, 32, True), (30, 64, 512, 128, False)])
+def test_projected_layer_matches_nn_lstm(T, B, H, P, states):
+    """The projected layer as an ordinary one with the recurrent weights W_hh W_hr."""
+    import fastlstm_b200 as F
+    torch.manual_seed(H)
+    ref = torch.nn.LSTM(20, H, proj_size=P).double()
+    with torch.no_grad():
+        for p in ref.parameters():
+            p.copy_(p.half().double())
+    m = F.FastLSTM(20, H, proj_size=P, device="cuda", dtype=torch.float16)
+    m.load_state_dict({k: v.half() for k, v in ref.state_dict().items()})
+    x, h0, c0 = (torch.randn(*s).half() * 0.5 for s in ((T, B, 20), (1, B, P), (1, B, H)))
+    res = []
+    for mod, cast in ((m, lambda t: t.cuda().requires_grad_(True)), (ref, lambda t: t.double().requires_grad_(True))):
+        xi, hi, ci = cast(x), cast(h0), cast(c0)
+        out, (hn, cn) = mod(xi, (hi, ci)) if states else mod(xi)
+        (out.float().square().sum() + hn.float().sum() + cn.float().sum()).backward()
+        grads = [xi.grad] + ([hi.grad, ci.grad] if states else []) + [p.grad for p in mod.parameters()]
+        res.append([t.detach().double().cpu() for t in (out, hn, cn, *grads)])
+    for i, (a, b) in enumerate(zip(*res)):
+        assert (a - b).norm() <= 1e-2 * b.norm() + 1e-6, i
+    F.check_status()
