@@ -258,6 +258,9 @@ int blstm_plan_detail(const blstm_desc* d, int phase, char* buf, size_t buf_byte
   }
   if (sm100_recurrence_supported(*d, phase)) {
     sm100_plan_detail(*d, phase, buf, buf_bytes);
+  } else if (const sm100::F32Plan fp = sm100::f32_plan(*d, phase); fp.ok) {
+    snprintf(buf, buf_bytes, "generic %s fp32 small-batch cluster=%d units_per_cta=%d rows_per_cluster=%d chunks=%d grid=%d threads=384 smem=%zu",
+             phase == BLSTM_PHASE_BWD ? "bwd" : "fwd", fp.nc, fp.U, fp.rows, fp.nch, fp.ncl * fp.nc, fp.smem);
   } else {
     GenericPlan pl;
     pl.make(*d, phase);

@@ -515,7 +515,7 @@ F32Plan f32_plan(const blstm_desc& d, int phase) {
   p.U = (phase == BLSTM_PHASE_BWD && H > 256) ? 24 : 32;
   p.nc = cdiv(H, p.U);
   if (p.nc == 1 && (d.flags & BLSTM_FLAG_TEST_NO_ARRIVE)) return p;      // (no wait that could run out)
-  const int cap = std::max(1, resident_clusters(p.nc));
+  const int cap = d.flags & BLSTM_FLAG_HALF_DEVICE ? (resident_clusters(p.nc) + 1) / 2 : resident_clusters(p.nc);   // (a hint: clusters are independent)
   const int per = cdiv(B, std::min(cap, B));
   p.R = per >= 5 ? 8 : per >= 3 ? 4 : per;
   p.nch = cdiv(per, p.R);

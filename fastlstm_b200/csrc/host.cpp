@@ -301,6 +301,7 @@ struct LayerState {
   Tensor x, Wx, Wh, out, cell, ifgo;
   int64_t I, H;                // the layer's own sizes
   bool stacked;                // final states as [1,B,H]
+  bool half;                   // planned for half of the device
 };
 
 struct LayerFn : public torch::autograd::Function<LayerFn> {
@@ -308,7 +309,7 @@ struct LayerFn : public torch::autograd::Function<LayerFn> {
                                                 const Tensor& Wx, const OptTensor& bx, const Tensor& Wh, const OptTensor& bh, LayerState s) {
     const int64_t T = s.out.size(0) - 1;
     ctx->saved_data["sizes"] = std::vector<int64_t>{s.I, s.H};
-    ctx->saved_data["given"] = std::vector<int64_t>{h0.has_value(), bx.has_value(), bh.has_value(), x.requires_grad(), s.stacked};
+    ctx->saved_data["given"] = std::vector<int64_t>{h0.has_value(), bx.has_value(), bh.has_value(), x.requires_grad(), s.stacked, s.half};
     Tensor y = s.out.narrow(0, 1, T), hn = s.out.select(0, T), cn = s.cell.select(0, T);
     if (s.out.size(2) != s.H) { y = y.narrow(2, 0, s.H); hn = hn.narrow(1, 0, s.H); cn = cn.narrow(1, 0, s.H); }
     if (s.stacked) {             // tensors of their own, in one copy
@@ -340,7 +341,7 @@ struct LayerFn : public torch::autograd::Function<LayerFn> {
     else dy = g[0].contiguous();
     const OptTensor dhn = state_grad(g[1]), dcn = state_grad(g[2]);
     m.run(x.device());
-    BwdOut r = bwd_impl(dy, dcn, dhn, x, out, cell, ifgo, Wx, Wh, given[3] != 0, std::nullopt, false);
+    BwdOut r = bwd_impl(dy, dcn, dhn, x, out, cell, ifgo, Wx, Wh, given[3] != 0, std::nullopt, given[5] != 0);
     Tensor dWx = r.wgrads.narrow(0, 0, 4 * Hp * Ip).view({4 * Hp, Ip}), dWh = r.wgrads.narrow(0, 4 * Hp * Ip, 4 * Hp * Hp).view({4 * Hp, Hp});
     Tensor db = r.wgrads.narrow(0, 4 * Hp * (Ip + Hp), 4 * Hp), dh0 = r.dh_0, dc0 = r.dc_0, dx = r.d_x;
     if (pad) {
@@ -359,8 +360,8 @@ struct LayerFn : public torch::autograd::Function<LayerFn> {
 
 py::tuple attach(const Tensor& x, const OptTensor& h0, const OptTensor& c0, const Tensor& Wx, const OptTensor& bx, const Tensor& Wh,
                  const OptTensor& bh, const Tensor& xp, const Tensor& Wxp, const Tensor& Whp, const Tensor& out, const Tensor& cell,
-                 const Tensor& ifgo, bool stacked) {
-  const auto r = LayerFn::apply(x, h0, c0, Wx, bx, Wh, bh, LayerState{xp, Wxp, Whp, out, cell, ifgo, x.size(-1), Wh.size(-1), stacked});
+                 const Tensor& ifgo, bool stacked, bool half) {
+  const auto r = LayerFn::apply(x, h0, c0, Wx, bx, Wh, bh, LayerState{xp, Wxp, Whp, out, cell, ifgo, x.size(-1), Wh.size(-1), stacked, half});
   return py::make_tuple(r[0], r[1], r[2]);
 }
 

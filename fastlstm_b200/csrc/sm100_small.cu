@@ -828,7 +828,8 @@ SmallPlan small_plan(const blstm_desc& d, int phase) {
   p.gc = cdiv(G, small_cluster(H));
   p.nc = cdiv(G, p.gc);
   if (p.nc == 1 && (d.flags & BLSTM_FLAG_TEST_NO_ARRIVE)) return p;     // (no wait that could run out)
-  const int cap = std::max(1, resident_clusters(p.nc));   // (no cluster waits for another: two launches share the device as they fit)
+  // (No cluster waits for another, so half a device is only a hint: two launches side by side share it as they fit.)
+  const int cap = d.flags & BLSTM_FLAG_HALF_DEVICE ? (resident_clusters(p.nc) + 1) / 2 : resident_clusters(p.nc);
   p.ks = 2 * cdiv(H, 32);
   const int tiles = cdiv(B, 8);
   p.ncl = std::min(cap, tiles);

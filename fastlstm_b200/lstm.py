@@ -246,10 +246,11 @@ class PersistentLSTMfn(torch.autograd.Function):
                 dbh if ctx.has_bias[1] else None, None, None, None)
 
 
-def _layer(x, h0, c0, Wx, bx, Wh, bh, inference, stacked=False, want_cells=False):
+def _layer(x, h0, c0, Wx, bx, Wh, bh, inference, stacked=False, want_cells=False, half=False):
     """One layer on the GPU, as PersistentLSTMfn computes it (same casts, padding and gradients), with the
     conversions in one launch and the autograd node in the host extension.  stacked: the final states come as
-    tensors [1,B,H] of their own.  want_cells: also the cell states of every step (no gradient)."""
+    tensors [1,B,H] of their own.  want_cells: also the cell states of every step (no gradient).  half: planned
+    for half of the device, another layer runs beside it."""
     host = _lib.host()
     if (h0 is None) != (c0 is None):
         raise ValueError("h0 and c0 must both be given or both be None")
@@ -259,14 +260,42 @@ def _layer(x, h0, c0, Wx, bx, Wh, bh, inference, stacked=False, want_cells=False
     Ip, Hp = _padded_sizes(x.dtype if to is None else to, I, H, T, B) or (0, 0)
     xp, h0p, c0p, Wxp, bxp, Whp, bhp = host.prepare(x, h0, c0, Wx, bx, Wh, bh, to, Ip, Hp)
     with _profiled("fastlstm_b200::fwd"):
-        out, cell, ifgo = lstm_persistent_fwd(xp, h0p, c0p, Wxp, bxp, Whp, bhp, inference=inference)
+        out, cell, ifgo = lstm_persistent_fwd(xp, h0p, c0p, Wxp, bxp, Whp, bhp, inference=inference, half_device=half)
     if not inference:
-        res = host.attach(x, h0, c0, Wx, bx, Wh, bh, xp, Wxp, Whp, out, cell, ifgo, stacked)
+        res = host.attach(x, h0, c0, Wx, bx, Wh, bh, xp, Wxp, Whp, out, cell, ifgo, stacked, half)
     else:
         res = out[1:, :, :H], out[-1, :, :H], cell[-1, :, :H]
         if stacked:
             res = res[0], res[1][None].clone(), res[2][None].clone()
     return res + (cell[1:, :, :H],) if want_cells else res
+
+
+@functools.lru_cache(maxsize=1024)
+def _shares_device(dtype, T, B, I, H):
+    """True when two launches of this layer's recurrences can run side by side to advantage: clusters that wait
+    for nothing outside themselves, and enough steps to pay for the streams (some 30 us of host time)."""
+    Ip, Hp = _padded_sizes(dtype, I, H, T, B) or (I, H)
+    return T >= 48 and all("small-batch" in plan_detail(dtype, T, B, Ip, Hp, phase) for phase in ("fwd", "bwd"))
+
+
+class _Beside:
+    """Runs the second direction of a layer, with the input x, on the side stream beside the first.  Entering makes
+    the side stream wait for everything so far - x, and the readers of memory that it frees and reuses - and join()
+    makes the current stream wait for it.  A no-op where `on` is false."""
+
+    def __init__(self, x, on):
+        self.main = torch.cuda.current_stream(x.device) if on else None
+        self.side = _side_stream(x.device) if on else None
+        if on:
+            x.record_stream(self.side)       # x comes from the main stream's memory, and backward reads it again
+            self.side.wait_stream(self.main)
+
+    def stream(self, d):
+        return torch.cuda.stream(self.side) if d and self.side is not None else contextlib.nullcontext()
+
+    def join(self):
+        if self.side is not None:
+            self.main.wait_stream(self.side)
 
 
 _side_streams = {}
@@ -630,23 +659,29 @@ class FastLSTM(nn.Module):
         padded, turned, rev, inv_last, last, packed, packed_t = host.packed_maps(seq.batch_sizes, seq.unsorted_indices, data)
         h_0, c_0 = self._initial_states(h_c_0)
         h_n, c_n, x = [], [], None
+        dt = torch.get_autocast_dtype("cuda") if torch.is_autocast_enabled("cuda") else data.dtype
         for layer in range(self.num_layers):
             outs, top = [], layer == self.num_layers - 1
-            for d in range(nd):
+            half = nd == 2 and _shares_device(dt, T, B, (data if x is None else x).shape[-1], self.hidden_size)
+            if x is None:
+                xs = [host.gather_rows(data, *maps, [T, B]) for maps in ((padded, packed), (turned, packed_t))[:nd]]
+            else:
+                xs = [x] if nd == 1 else [x, host.gather_rows(x, rev, rev, [T, B])]
+            beside = _Beside(xs[-1], half)
+            for d, x_d in enumerate(xs):
                 Wx, bx, Wh, bh = self.layer_params(layer, reverse=(d == 1))
-                if x is None:
-                    x_d = host.gather_rows(data, turned if d else padded, packed_t if d else packed, [T, B])
-                else:
-                    x_d = host.gather_rows(x, rev, rev, [T, B]) if d else x
                 hl, cl = h_0[layer * nd + d], c_0[layer * nd + d]
-                o, _, _, cells = _layer(x_d, hl, cl, Wx, bx, Wh, bh, _nothing_to_save(x_d, hl, cl, Wx, bx, Wh, bh), want_cells=True)
-                h_n.append(host.gather_rows(o, last, inv_last, [B]))       # states at each sequence's own last step
-                c_n.append(host.gather_rows(cells, last, inv_last, [B]))
-                if top:
-                    o = host.gather_rows(o, packed_t if d else packed, turned if d else padded, [data.shape[0]])
-                elif d:
-                    o = host.gather_rows(o, rev, rev, [T, B])
+                with beside.stream(d):
+                    inference = _nothing_to_save(x_d, hl, cl, Wx, bx, Wh, bh)
+                    o, _, _, cells = _layer(x_d, hl, cl, Wx, bx, Wh, bh, inference, want_cells=True, half=half)
+                    h_n.append(host.gather_rows(o, last, inv_last, [B]))       # states at each sequence's own last step
+                    c_n.append(host.gather_rows(cells, last, inv_last, [B]))
+                    if top:
+                        o = host.gather_rows(o, packed_t if d else packed, turned if d else padded, [data.shape[0]])
+                    elif d:
+                        o = host.gather_rows(o, rev, rev, [T, B])
                 outs.append(o)
+            beside.join()
             x = outs[0] if nd == 1 else torch.cat(outs, dim=-1)
             if self.dropout > 0.0 and self.training and not top:
                 x = torch.nn.functional.dropout(x, self.dropout, True)
@@ -731,10 +766,25 @@ class FastLSTM(nn.Module):
         h_0, c_0 = self._initial_states(h_c_0)
         h_n, c_n = [], []
         single = (self.num_layers * nd == 1 and self.proj_size == 0 and lengths is None and self._sinks is None and x.is_cuda)
+        dt = torch.get_autocast_dtype("cuda") if torch.is_autocast_enabled("cuda") else x.dtype
         for layer in range(self.num_layers):
             outs = []
+            half = (nd == 2 and x.is_cuda and lengths is None and self._sinks is None and self.proj_size == 0
+                    and _shares_device(dt, T, B, x.shape[2], self.hidden_size))
+            turned = x.flip(0) if half else x
+            beside = _Beside(turned, half)
             for d in range(nd):
                 Wx, bx, Wh, bh = self.layer_params(layer, reverse=(d == 1))
+                if half:
+                    hl, cl = h_0[layer * nd + d], c_0[layer * nd + d]
+                    x_d = turned if d else x
+                    with beside.stream(d):
+                        inference = _nothing_to_save(x_d, hl, cl, Wx, bx, Wh, bh)
+                        o, h_i, c_i = _layer(x_d, hl, cl, Wx, bx, Wh, bh, inference, half=True)
+                        outs.append(o.flip(0) if d else o)
+                    h_n.append(h_i)
+                    c_n.append(c_i)
+                    continue
                 # the reverse direction walks t = T-1 .. 0 (every sequence from its own end when packed)
                 x_d = x if d == 0 else (x.flip(0) if lengths is None else reverse_time(x))
                 hl, cl = h_0[layer * nd + d], c_0[layer * nd + d]
@@ -762,6 +812,7 @@ class FastLSTM(nn.Module):
                 outs.append(o if d == 0 else (o.flip(0) if lengths is None else reverse_time(o)))
                 h_n.append(h_i)
                 c_n.append(c_i)
+            beside.join()
             x = outs[0] if nd == 1 else torch.cat(outs, dim=-1)
             if self.dropout > 0.0 and self.training and layer < self.num_layers - 1:
                 x = torch.nn.functional.dropout(x, self.dropout, True)

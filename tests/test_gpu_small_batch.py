@@ -255,6 +255,36 @@ def test_packed_row_maps_and_gathers(lengths, C, dtype):
     assert torch.equal(data.grad.cpu(), want)
 
 
+@pytest.mark.parametrize("packed", [False, True])
+@pytest.mark.parametrize("T,B,H", [(48, 3, 40), (64, 32, 128), (50, 17, 320)])
+def test_directions_side_by_side_match_nn_lstm(T, B, H, packed):
+    """Both directions at once, each on half of the device, against torch.nn.LSTM in float64 - twice, so that the
+    second pass reuses the first one's memory on both streams."""
+    import fastlstm_b200 as F
+    from torch.nn.utils.rnn import pack_padded_sequence
+    torch.manual_seed(T + H)
+    ref = torch.nn.LSTM(24, H, num_layers=2, bidirectional=True).double()
+    m = F.FastLSTM(24, H, num_layers=2, bidirectional=True, device="cuda", dtype=torch.bfloat16)
+    with torch.no_grad():
+        for p in ref.parameters():
+            p.copy_(p.bfloat16().double())
+    m.load_state_dict({k: v.bfloat16() for k, v in ref.state_dict().items()})
+    lengths = torch.randint(1, T + 1, (B,))
+    lengths[B // 2] = T
+    for seed in range(2):
+        x = torch.randn(T, B, 24).bfloat16()
+        res = []
+        for mod, xi in ((m, x.cuda().requires_grad_(True)), (ref, x.double().requires_grad_(True))):
+            mod.zero_grad()
+            out, (hn, cn) = mod(pack_padded_sequence(xi, lengths, enforce_sorted=False) if packed else xi)
+            out = out.data if packed else out
+            (out.float().square().sum() + hn.float().sum()).backward()
+            res.append([t.detach().double().cpu() for t in (out, hn, cn, xi.grad, *(p.grad for p in mod.parameters()))])
+        for i, (a, b) in enumerate(zip(*res)):
+            assert (a - b).norm() <= 2e-2 * b.norm() + 1e-6, i
+    F.check_status()
+
+
 @pytest.mark.parametrize("T,B,H,P,states", [(2, 1, 33, 7, True), (40, 9, 96, 32, True), (30, 64, 512, 128, False)])
 def test_projected_layer_matches_nn_lstm(T, B, H, P, states):
     """The projected layer as an ordinary one with the recurrent weights W_hh W_hr."""
