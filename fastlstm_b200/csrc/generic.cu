@@ -343,16 +343,24 @@ gen_bwd_kernel(GenParams p, const T* __restrict__ dout, const T* __restrict__ dh
   }
 }
 
-__global__ void reduce_db_kernel(const float* __restrict__ part, int n_part, int n, float* __restrict__ db) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n) return;
+// 32 columns x 8 groups of rows per block; the groups are added up in a fixed order.
+__global__ void __launch_bounds__(256) reduce_db_kernel(const float* __restrict__ part, int n_part, int n, float* __restrict__ db) {
+  __shared__ float red[8][32];
+  const int c = threadIdx.x & 31, g = threadIdx.x >> 5, j = blockIdx.x * 32 + c;
   float s = 0.f;
-  for (int i = 0; i < n_part; ++i) s += part[(size_t)i * n + j];
-  db[j] = s;
+  if (j < n)
+    for (int i = g; i < n_part; i += 8) s += part[(size_t)i * n + j];
+  red[g][c] = s;
+  __syncthreads();
+  if (g == 0 && j < n) {
+#pragma unroll
+    for (int i = 1; i < 8; ++i) s += red[i][c];
+    db[j] = s;
+  }
 }
 
 int reduce_db(const float* part, int n_part, int n, float* db, cudaStream_t st) {
-  reduce_db_kernel<<<cdiv(n, 256), 256, 0, st>>>(part, n_part, n, db);
+  reduce_db_kernel<<<cdiv(n, 32), 256, 0, st>>>(part, n_part, n, db);
   BLSTM_CUDA_OK(cudaGetLastError());
   count_launch();
   return BLSTM_OK;

@@ -819,22 +819,27 @@ static int launch_fwd_t(const RecPlan& pl, const CUtensorMap& tw, const CUtensor
 // output units of one batch tile; CTA r of the cluster takes gate r's K range (H rows of
 // Wh, resident in shared memory as an N-major operand) and streams the matching H columns
 // of d_ifgo[t] through TMA.  Each CTA ends a step with a partial [128 x 64] fp32 product in
-// TMEM; the four partials are reduce-scattered through distributed shared memory (each CTA
-// receives the three 16-unit slices it needs, 24 KB per step) so that CTA r finishes with
-// dh for units [16r, 16r+16) of the cluster's 64 - the units whose gate maths it then
-// does (thread = batch row x 8 units: dc carried in fp32 registers, d_ifgo[t-1] written and
-// published with the same per-(step, batch tile) arrival counters as the forward kernel).
+// TMEM; the four partials are reduce-scattered through distributed shared memory by ROWS (a
+// warp reads one 32-row quarter of the accumulator anyway; each CTA receives three 8 KB slices)
+// so that CTA r finishes with dh of rows [32r, 32r+32) of the tile for all 64 units - whose gate
+// maths it then does: thread = row x 8 units, a warp = 4 rows x 64 units, so every global access
+// of the gate maths moves whole 128-byte lines.  (A split by units left 16-unit rows: 32-byte
+// pieces that went through TMA boxes, whose stores had to complete before a hand-off: T=256, B=4096,
+// H=512 took 9.5 ms a launch, 8.1 this way; T=256, B=256, H=768 2.36 -> 1.91; T=512, B=256, H=1024
+// 5.1 -> 4.5; T=1024, B=32, H=2048 11.3 -> 10.5.  Bound by the hand-off chain of a step.)  dc is
+// carried in fp32 registers, d_ifgo[t-1] is published with the same per-(step, batch tile)
+// arrival counters as in the forward kernel.
 // =====================================================================================
 constexpr int DB_PARTS = 1024;            // row groups of the bias-gradient column sum
-constexpr int XROW_BYTES = 64;            // one row of a slice: 16 fp32; its four 16-byte pieces are XOR-swizzled
-constexpr int XSLOT_BYTES = RB * XROW_BYTES;  // one exchanged slice: 128 rows x 16 fp32 = 8 KB
+constexpr int XROW_BYTES = 256;           // one row of a slice: 64 fp32; its 16-byte pieces: even ones, then odd ones, XOR-swizzled
+constexpr int XSLOT_BYTES = 32 * XROW_BYTES;  // one exchanged slice: 32 rows x 64 fp32 = 8 KB
 
 struct BwdPlan {
   bool ok;
   int nug, nbt, nb_par, ntl, TI, grid, threads, stages, ni, nl, ws, alias;
   int kr;                   // K chunks of the Wh slice that stay resident (all of them unless ws)
   int hb;                   // bytes of the d_ifgo rows in a ring stage (128 rows, or a single smaller tile's own)
-  size_t w_bytes, recv_bytes, stage_bytes, smem, ep_bytes;
+  size_t w_bytes, recv_bytes, stage_bytes, smem;
   size_t off_flags, n_flags, off_db, ws_bytes;
 };
 
@@ -875,30 +880,24 @@ static BwdPlan make_bwd_plan(const blstm_desc& d) {
   // H=2048 measured 12.5 ms with 18 of 32 chunks resident against 11.5 ms with none); the kernel handles
   // any split, `kr` chunks are resident.
   auto resident_chunks = [&](size_t) { return p.ws ? 0 : KCp; };
-  // Cluster exchange: receive slots (3 peers x 8 KB) and send staging (3 x 8 KB), one set.  With
-  // interleaved tiles a CTA tells its three peers when it has consumed an item's slices, and nobody
-  // stages or ships the next item before all three have said so (`consumed` in the kernel).
-  // Interleaved tiles also move the epilogue's gate traffic through TMA: three landing buffers per pair
-  // of epilogue warps (32 rows x 4 gates x 16 units; d_ifgo is written back in place and stored from there).
-  p.recv_bytes = (size_t)2 * 3 * XSLOT_BYTES;
-  p.ep_bytes = p.TI >= 2 ? (size_t)4 * 3 * 4096 : 0;
-  p.kr = resident_chunks(1024 + p.recv_bytes + p.ep_bytes + 1024);
-  if (1024 + (size_t)p.kr * 8192 + p.recv_bytes + p.ep_bytes + 1024 + 3 * p.stage_bytes > 232448 && p.TI >= 2) {
+  // Cluster exchange: receive slots (4 CTAs x 8 KB, this CTA's own among them) and send staging (3 x 8 KB), one
+  // set.  With interleaved tiles a CTA tells the cluster when it has consumed an item's slices, and nobody
+  // stages or ships the next item before all four have said so (`consumed` in the kernel).
+  p.recv_bytes = (size_t)(4 + 3) * XSLOT_BYTES;
+  p.kr = resident_chunks(1024 + p.recv_bytes + 1024);
+  if (1024 + (size_t)p.kr * 8192 + p.recv_bytes + 1024 + 3 * p.stage_bytes > 232448 && p.TI >= 2)
     p.TI = 1;                                               // not enough room to interleave tiles
-    p.ep_bytes = 0;
-    p.kr = resident_chunks(1024 + p.recv_bytes + 1024);
-  }
   size_t wres = (size_t)p.kr * 8192;
-  size_t fixed = 1024 + wres + p.recv_bytes + p.ep_bytes + 1024 + tail_pad;  // 1024: barriers and counters behind the ring
+  size_t fixed = 1024 + wres + p.recv_bytes + 1024 + tail_pad;  // 1024: barriers and counters behind the ring
   // warps: 1 producer + 3 MMA issuers (or 2 + a publisher warp when tiles are interleaved) + 2 epilogue
   // warpgroups = 12 (3 per SM sub-partition, 168 registers each); a 13th warp would cap every thread
   // at 128 registers.
   const int n_issuers = p.TI >= 2 ? 2 : 3;
   p.threads = 32 * 12;
   if (!pick_ring(fixed, p.stage_bytes, n_issuers, H / RK, &p.stages, &p.ni)) return p;
-  // One tile in flight and a shallow ring (H = 768, 1024: the resident weights leave three stages):
+  // One tile in flight and a shallow ring (H = 768, 1024: the resident weights leave four stages, or two):
   // the ring is idle while an item's slices cross the cluster, so the exchange buffers are laid over
-  // its first stages and the ring gets their 48 KB.  A peer may then write a slice only after this
+  // its first stages and the ring gets their 56 KB.  A peer may then write a slice only after this
   // CTA has finished the item's MMAs, which each CTA tells its peers (see `rdy` in the kernel).
   p.alias = 0;
   if (p.TI == 1 && p.stages < 6) {
@@ -919,7 +918,7 @@ static BwdPlan make_bwd_plan(const blstm_desc& d) {
   p.n_flags = (size_t)d.seq_len * p.nbt;
   p.off_flags = sizeof(Control);
   p.off_db = p.off_flags + round_up(p.n_flags * sizeof(int), 256);
-  p.ws_bytes = p.off_db + round_up((size_t)DB_PARTS * 4 * H * sizeof(float), 256);
+  p.ws_bytes = p.off_db + round_up((size_t)std::max(DB_PARTS, p.nb_par * 32) * 4 * H * sizeof(float), 256);
   p.ok = true;
   return p;
 }
@@ -939,7 +938,6 @@ struct BwdParams {
   int flag_target;          // arrivals that complete a flag: H/16 CTAs per batch tile [x 8 epilogue warps]
   int cta_publish;          // 1: one arrival per CTA and item, 0: one per epilogue warp
   int alias;                // 1: exchange buffers laid over the first ring stages (one tile in flight)
-  int ep_bytes;             // bytes of the epilogue's TMA buffers (interleaved tiles)
   unsigned long long limit_ns;
   Control* ctl;
   int* flags;               // [T][nbt]: arrivals for d_ifgo[t]
@@ -951,28 +949,12 @@ struct BwdParams {
   void* d_ifgo;             // [T,B,4H]
   void* dh0;                // [B,H]
   void* dc0;                // [B,H]
-  float* db_part;           // [nb_par * 4][4H] bias-gradient partial sums (one row per CTA group and row quarter), or null
+  float* db_part;           // [nb_par * 32][4H] bias-gradient partial sums (one row per CTA group and four rows of its tiles), or null
 };
-
-template <typename T16>
-__device__ __forceinline__ void unpack16(const uint4& v0, const uint4& v1, float (&f)[16]) {
-  const uint32_t w[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
-#pragma unroll
-  for (int u = 0; u < 8; ++u) { const float2 t = cvt2<T16>(w[u]); f[2 * u] = t.x; f[2 * u + 1] = t.y; }
-}
-template <typename T16>
-__device__ __forceinline__ void store16(T16* dst, const float (&f)[16]) {
-  uint32_t w[8];
-#pragma unroll
-  for (int u = 0; u < 8; ++u) w[u] = pk2<T16>(f[2 * u], f[2 * u + 1]);
-  stg16(dst, make_uint4(w[0], w[1], w[2], w[3]));
-  stg16(dst + 8, make_uint4(w[4], w[5], w[6], w[7]));
-}
 
 template <int TI, typename T16>
 __global__ void __launch_bounds__(384, 1)
-bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmG,
-           const __grid_constant__ CUtensorMap tmI, const __grid_constant__ CUtensorMap tmD, const BwdParams p) {
+bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmG, const BwdParams p) {
   // Warps: 0 = TMA producer, then NACC MMA issuers, then (interleaved tiles only) one PUBLISHER warp,
   // then 8 epilogue warps from warp 4 on - 12 in all either way.
   // With interleaved tiles the epilogue warps are the bottleneck, and the release that publishes an
@@ -983,12 +965,6 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
   constexpr int FIRST_EPI = 4;
   constexpr bool WRITER_FENCE = false;            // the proxy fence of the hand-off: reader (one tile) or publisher warp
   constexpr int ITEM_WARPS = 8;                   // epilogue warps, all working on every item
-  // Interleaved tiles are throughput bound and the epilogue's row-strided 16-byte global accesses were
-  // the bottleneck there: the saved pre-activations come in, and d_ifgo goes out, as TMA boxes through
-  // shared memory, one pair of landing buffers per epilogue warp (tmI: ifgo, tmD: d_ifgo, both
-  // as {unit, row, gate, step}).  The TMA store of d_ifgo[t] is also what the peers' producers read
-  // next, so a warp counts its item in only after its store has completed.
-  constexpr bool TMAEP = (TI >= 2);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int H = p.H;
@@ -997,28 +973,23 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
   uint8_t* w_s = smem;                                        // [KC][64 k rows][128 B]
   const int SB = p.stage_bytes;                               // d_ifgo chunk (16 KB) [+ Wh chunk when streamed]
   const int HB = p.hb;                                        // d_ifgo rows of a stage; a streamed Wh chunk follows
-  uint8_t* recv = smem + (size_t)p.kr * 8192;                 // [3 senders][128 rows][64 B]
-  constexpr int XB = 1;                                       // one set of exchange buffers
-  uint8_t* stage = recv + (size_t)XB * 3 * XSLOT_BYTES;      // [3 receivers][128 rows][64 B]
-  uint8_t* ep_s = stage + (size_t)XB * 3 * XSLOT_BYTES;      // epilogue TMA buffers [4 warp pairs][3][4 KB]
-  uint8_t* a_s = p.alias ? recv : ep_s + p.ep_bytes;         // ring (over the exchange buffers if aliased)
+  uint8_t* recv = smem + (size_t)p.kr * 8192;                 // [4 senders][32 rows][256 B]
+  uint8_t* stage = recv + (size_t)4 * XSLOT_BYTES;            // [3 receivers][32 rows][256 B]
+  uint8_t* a_s = p.alias ? recv : stage + (size_t)3 * XSLOT_BYTES;   // ring (over the exchange buffers if aliased)
   uint64_t* bars = reinterpret_cast<uint64_t*>(a_s + (size_t)R_STAGES * SB);
   uint64_t* full = bars;
   uint64_t* empty = bars + R_MAX_STAGES;
   uint64_t* acc_full = bars + 2 * R_MAX_STAGES;
   uint64_t* acc_empty = acc_full + 2;
   uint64_t* w_full = acc_empty + 2;
-  uint64_t* xchg = w_full + 1;                                // [2]
-  uint64_t* staged = xchg + 2;                                // [2]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(staged + 2);
+  uint64_t* xchg = w_full + 1;                                // slices of an item complete
+  uint64_t* staged = xchg + 1;                                // [4] row quarter staged by its two warps
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(staged + 4);
   volatile int* dead = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* pub_cnt = const_cast<int*>(dead) + 1;        // [4] arrivals of the epilogue warps, by item index mod 4
-  uint64_t* pub_bar = reinterpret_cast<uint64_t*>(pub_cnt + 4);   // [4] item published? by item index mod 4
+  uint64_t* pub_bar = reinterpret_cast<uint64_t*>(pub_cnt + 4);   // [4] item stored? by item index mod 4
   uint64_t* rdy = pub_bar + 4;                                 // aliased buffers: the 3 peers are done with their MMAs
-  uint64_t* consumed = rdy + 1;                                // interleaved tiles: the 3 peers' 8 warps read an item's slices
-  uint64_t* pre_full = consumed + 1;                           // [4 warp pairs][3] landing buffer filled
-  uint64_t* pre_done = pre_full + 12;                          // [4 warp pairs][3] both warps wrote their d_ifgo halves
-  uint64_t* pre_free = pre_full + 24;                          // [4 warp pairs][3] landing buffer may be refilled
+  uint64_t* consumed = rdy + 1;                                // interleaved tiles: the cluster's 32 warps read an item's slices
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t r = cluster_ctarank();                       // gate whose K range this CTA owns
@@ -1033,18 +1004,17 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
     for (int s = 0; s < R_STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], nacc); mbar_init(&acc_empty[a], ITEM_WARPS); }
     mbar_init(w_full, 1);
-    for (int j = 0; j < 2; ++j) { mbar_init(&xchg[j], 1); mbar_init(&staged[j], ITEM_WARPS); }   // xchg: one expect_tx arrival + tx bytes
+    mbar_init(xchg, 3);                             // one expect_tx arrival + tx bytes, and the two warps of the own quarter
+    for (int j = 0; j < 4; ++j) mbar_init(&staged[j], 2);
     *dead = 0;
     for (int i = 0; i < 4; ++i) pub_cnt[i] = 0;
-    for (int i = 0; i < 4; ++i) mbar_init(&pub_bar[i], TMAEP ? 4 : ITEM_WARPS);   // (interleaved: one arrival per warp pair)
+    for (int i = 0; i < 4; ++i) mbar_init(&pub_bar[i], ITEM_WARPS);
     mbar_init(rdy, 3);
-    mbar_init(consumed, 3 * ITEM_WARPS);
-    for (int i = 0; i < 24; ++i) { mbar_init(&pre_full[i], i < 12 ? 1 : 2); mbar_init(&pre_free[i], 1); }
+    mbar_init(consumed, 4 * ITEM_WARPS);
     fence_mbar_init();
     for (int s = 0; s < R_STAGES; ++s) mbar_expect_tx(&full[s], (p.ws && s % KC >= p.kr) ? SB : HB);
     tma_prefetch_desc(&tmW);
     tma_prefetch_desc(&tmG);
-    if (TMAEP) { tma_prefetch_desc(&tmI); tma_prefetch_desc(&tmD); }
   }
   if (warp == 1) tmem_alloc(tmem_slot, TMEM_COLS);
   tc_fence_before();
@@ -1143,31 +1113,6 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
           }
         }
       }
-    } else if (TMAEP && lane <= 4) {
-      // ------------------------------------------------------------ gate loaders (lanes 1..4)
-      // Lane 1+w fetches the gate boxes of the two epilogue warps of row quarter w (all 16 units: 32-byte
-      // rows), up to three gate-maths items ahead, into the pair's three landing buffers in turn; a
-      // buffer is refilled once the pair has said that the d_ifgo box it held has been written
-      // (pre_free).  Issuing these loads from here rather than from the epilogue warps matters: a TMA
-      // issue waits for room behind the producer's 16 KB boxes (about a thousand clocks), which the
-      // epilogue warps cannot afford.
-      const int w = lane - 1;
-      const int gq = w;                                         // the pair's row quarter
-      const int g_unit0 = ugc * 64 + (int)r * 16;
-      uint8_t* g_buf = ep_s + (size_t)w * 3 * 4096;
-      ItemCursor<TI> lc;
-      lc.init();
-      int n = 0;
-      bool ok = true;
-      while (ok && lc.next(pb, p.nb_par, p.nbt, n_chunks, T)) {
-        const int b = n % 3;
-        wc.d0 = T - 1 - lc.t; wc.d1 = lc.tile(pb, p.nb_par);
-        if (n >= 3 && !mbar_wait(&pre_free[3 * w + b], (uint32_t)(n / 3 - 1) & 1u, wc)) { ok = false; break; }
-        mbar_expect_tx(&pre_full[3 * w + b], 4096);
-        tma_load_4d(g_buf + b * 4096, &tmI, &pre_full[3 * w + b], g_unit0, lc.tile(pb, p.nb_par) * RB + gq * 32, 0,
-                    T - 1 - lc.t);
-        ++n;
-      }
     }
   } else if (warp < 1 + NACC) {
     // ---------------------------------------------------------------- MMA issuers (own whole chunks)
@@ -1220,26 +1165,29 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
     }
   } else {
     // ---------------------------------------------------------------- epilogue: two warpgroups
-    // thread = (batch row, 8 units): the two warpgroups split the CTA's 16 units of every item, which
-    // halves the serial path of a step (accumulator read-out, gate maths) and keeps it free of spills.
     constexpr int NU = 8;                        // units per thread
-    const int g = (warp - FIRST_EPI) >> 2;       // warpgroup = which half of the 16 units
-    const int uoff = g * NU;
-    const int q = warp & 3;
-    const int row_in_tile = q * 32 + lane;
-    const int unit0 = ugc * 64 + (int)r * 16 + uoff;
-    const int swz = (row_in_tile >> 1) & 3;   // bank swizzle of the exchanged slices
+    const int ew = warp - FIRST_EPI;
+    // accumulator read-out: thread = row `lane` of quarter q, units 32g .. 32g+31
+    const int g = ew >> 2, q = warp & 3;
+    // gate maths: thread = row grow of this CTA's quarter r, units gu .. gu+7 of the cluster's 64
+    const int grow = ew * 4 + (lane >> 3), gu = (lane & 7) * 8;
+    const int row_in_tile = (int)r * 32 + grow;
+    const int unit0 = ugc * 64 + gu;
     const size_t H4 = 4 * (size_t)H;
     const T16* ifgo = reinterpret_cast<const T16*>(p.ifgo);
     const T16* cell = reinterpret_cast<const T16*>(p.cell);
     const T16* dout = reinterpret_cast<const T16*>(p.dout);
     T16* dg = reinterpret_cast<T16*>(p.d_ifgo);
-    const bool shipper = (warp == FIRST_EPI) && lane == 0;   // sends the staged slices
+    // where the accumulator's pieces go: this CTA's own receive slot, or the staging slot of CTA q
+    uint8_t* put = (q == (int)r ? recv + (size_t)r * XSLOT_BYTES : stage + (size_t)(q < (int)r ? q : q - 1) * XSLOT_BYTES) + lane * XROW_BYTES;
+    // piece 2k of a row lies at position k, piece 2k+1 at 8+k, both XORed with the row: conflict-free for the writers
+    // (32 rows, one piece) and for the readers (a row's even or odd pieces)
+    const uint8_t* get = recv + grow * XROW_BYTES + (((lane & 7) ^ (grow & 7)) << 4);
     // Bias gradient (replaces the reduction of fastlstm/lstm.py:497 and a separate pass over d_ifgo):
     // every thread adds the d_ifgo values it stores - as stored, i.e. rounded - to 32 fp32 sums of its
     // own (4 gates x 8 units) that live in the tensor-memory columns behind the accumulators, one
-    // 32-column block per warpgroup; after the last step the 32 rows of a warp are added up with
-    // shuffles and lane 0 writes the warp's partial sums.
+    // 32-column block per warpgroup; after the last step the four rows of a warp are added up with
+    // shuffles and its first eight lanes write the warp's partial sums.
     constexpr int DB_COL = 192;                  // NACC * N <= 192 columns per accumulator buffer are in use
     const uint32_t db_taddr = tmem_base + DB_COL + g * 32 + (uint32_t(q * 32) << 16);
     const bool want_db = p.db_part != nullptr;
@@ -1254,58 +1202,42 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
     int it = 0;                 // MMA items consumed so far: TMEM buffer it & 1, on its (it >> 1)-th use
     int pub_it = 0;             // gate-maths items published so far
     bool ok = true;
-    // Interleaved tiles: the two warps of a row quarter (one per unit half) share three landing buffers
-    // [4 gates][32 rows][16 units] (32-byte rows with the 32-byte swizzle: a warp's 16-byte pieces of one
-    // gate fall into different banks), used in turn by consecutive gate-maths items.  Whole 32-byte
-    // segments matter: an SM's TMA unit is what bounds an item, and its cost goes by row segments - eight
-    // boxes of 16-byte segments in and eight out per item cost it about twice the item's 128 KB of d_ifgo
-    // chunks.  A lane of the publisher warp issues the pair's TMA loads; lane 0 of the pair's first warp
-    // issues its store once both warps have written their halves (pre_done); when the store has completed
-    // the buffer is handed back to the loader and the pair counts the item in.
-    uint8_t* pbuf = ep_s + (size_t)q * 3 * 4096;
-    uint64_t* pfull = pre_full + 3 * q;
-    uint64_t* pdone = pre_done + 3 * q;
-    auto p_off = [&](int k) { return k * 1024 + lane * 32 + ((g ^ ((lane >> 2) & 1)) * 16); };
-    uint64_t* pfree = pre_free + 3 * q;
     for (int ch = 0; ch < n_chunks && ok; ++ch) {
-      // dc is carried per interleaved tile; dh is rebuilt from the accumulator in every item, so one
+      // dc and c[t+1] are carried per interleaved tile; dh is rebuilt from the accumulator in every item, so one
       // copy serves all tiles (its first value, the gradient of h_n, is fetched in the tile's first item)
       float dc[TI][NU], dhc[NU];
-      uint4 pf[7];       // next item's inputs: gates i,f,g,o, c[t+1], c[t], dout[t]
+      uint4 cn[TI];      // c[t+1] of the tile's next item
+      uint4 pf[6];       // next item's inputs: gates i,f,g,o, c[t], dout[t]
 #pragma unroll
       for (int j = 0; j < TI; ++j) {
         const int bt = pb + (ch * TI + j) * p.nb_par;
         const int row = bt * RB + row_in_tile;
         const bool rok = bt < p.nbt && row < p.B;
+        cn[j] = make_uint4(0, 0, 0, 0);
 #pragma unroll
         for (int u = 0; u < NU; ++u) dc[j][u] = 0.f;
-        if (rok && p.dc_n) unpack8<T16>(ldg16(reinterpret_cast<const T16*>(p.dc_n) + (size_t)row * H + unit0), dc[j]);
+        if (rok) {
+          cn[j] = ldg16(cell + ((size_t)T * p.B + row) * H + unit0);
+          if (p.dc_n) unpack8<T16>(ldg16(reinterpret_cast<const T16*>(p.dc_n) + (size_t)row * H + unit0), dc[j]);
+        }
       }
       auto prefetch = [&](int t, int bt) {
         const int row = bt * RB + row_in_tile;
         if (bt < p.nbt && row < p.B) {
-          if constexpr (!TMAEP) {
-            const T16* gsrc = ifgo + ((size_t)t * p.B + row) * H4 + unit0;
+          const size_t m = (size_t)t * p.B + row;
+          const T16* gsrc = ifgo + m * H4 + unit0;
 #pragma unroll
-            for (int k = 0; k < 4; ++k) pf[k] = ldg16(gsrc + (size_t)k * H);
-          }
-          pf[4] = ldg16(cell + ((size_t)(t + 1) * p.B + row) * H + unit0);
-          pf[5] = ldg16(cell + ((size_t)t * p.B + row) * H + unit0);
-          pf[6] = ldg16(dout + ((size_t)t * p.B + row) * H + unit0);
+          for (int k = 0; k < 4; ++k) pf[k] = ldg16(gsrc + (size_t)k * H);
+          pf[4] = ldg16(cell + m * H + unit0);
+          pf[5] = ldg16(dout + m * H + unit0);
         }
       };
-      // two items ahead the same inputs are only pulled into L2 (no registers to hold them yet);
-      // a 32-byte sector covers both warpgroups' halves, so one warpgroup issues them
+      // two items ahead the same lines are only pulled into L2: lane k of a row's eight asks for the k-th of its six
       auto prefetch_far = [&](int t, int bt) {
-        const int row = bt * RB + row_in_tile;
-        if (g == 0 && bt < p.nbt && row < p.B) {
-          if constexpr (!TMAEP) {
-            const T16* gsrc = ifgo + ((size_t)t * p.B + row) * H4 + unit0;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) prefetch_l2(gsrc + (size_t)k * H);
-          }
-          prefetch_l2(cell + ((size_t)t * p.B + row) * H + unit0);
-          prefetch_l2(dout + ((size_t)t * p.B + row) * H + unit0);
+        const int row = bt * RB + row_in_tile, k = lane & 7;
+        if (k < 6 && bt < p.nbt && row < p.B) {
+          const size_t m = (size_t)t * p.B + row;
+          prefetch_l2(k < 4 ? ifgo + m * H4 + (size_t)k * H + ugc * 64 : (k == 4 ? cell : dout) + m * H + ugc * 64);
         }
       };
       // Everything in the gate maths that does not depend on dh is worked out ahead of the accumulator:
@@ -1317,48 +1249,40 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
       constexpr bool EARLY_FACTORS = (TI == 1);
       constexpr int NF = USE_FACTORS ? NU : 1;
       float fA[NF], fBi[NF], fBf[NF], fBg[NF], fBo[NF], fSf[NF], fDd[NF];
-      auto factors = [&]() {
+      // (c1: c[t+1] of the item; its c[t] takes its place for the tile's next one)
+      auto factors = [&](uint4& c1v) {
         if constexpr (USE_FACTORS) {
-        const uint32_t wi[4] = {pf[0].x, pf[0].y, pf[0].z, pf[0].w};
-        const uint32_t wf[4] = {pf[1].x, pf[1].y, pf[1].z, pf[1].w};
-        const uint32_t wg[4] = {pf[2].x, pf[2].y, pf[2].z, pf[2].w};
-        const uint32_t wo[4] = {pf[3].x, pf[3].y, pf[3].z, pf[3].w};
-        const uint32_t w1[4] = {pf[4].x, pf[4].y, pf[4].z, pf[4].w};
-        const uint32_t w0[4] = {pf[5].x, pf[5].y, pf[5].z, pf[5].w};
-        const uint32_t wd[4] = {pf[6].x, pf[6].y, pf[6].z, pf[6].w};
+          const uint32_t wi[4] = {pf[0].x, pf[0].y, pf[0].z, pf[0].w};
+          const uint32_t wf[4] = {pf[1].x, pf[1].y, pf[1].z, pf[1].w};
+          const uint32_t wg[4] = {pf[2].x, pf[2].y, pf[2].z, pf[2].w};
+          const uint32_t wo[4] = {pf[3].x, pf[3].y, pf[3].z, pf[3].w};
+          const uint32_t w1[4] = {c1v.x, c1v.y, c1v.z, c1v.w};
+          const uint32_t w0[4] = {pf[4].x, pf[4].y, pf[4].z, pf[4].w};
+          const uint32_t wd[4] = {pf[5].x, pf[5].y, pf[5].z, pf[5].w};
 #pragma unroll
-        for (int w = 0; w < 4; ++w) {
-          const float2 pi = cvt2<T16>(wi[w]), pff = cvt2<T16>(wf[w]), pg = cvt2<T16>(wg[w]), po = cvt2<T16>(wo[w]);
-          const float2 c1 = cvt2<T16>(w1[w]), c0 = cvt2<T16>(w0[w]), dd = cvt2<T16>(wd[w]);
+          for (int w = 0; w < 4; ++w) {
+            const float2 pi = cvt2<T16>(wi[w]), pff = cvt2<T16>(wf[w]), pg = cvt2<T16>(wg[w]), po = cvt2<T16>(wo[w]);
+            const float2 c1 = cvt2<T16>(w1[w]), c0 = cvt2<T16>(w0[w]), dd = cvt2<T16>(wd[w]);
 #pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const int u = 2 * w + e;
-            const float si = sigmoid_fast(e ? pi.y : pi.x), sf = sigmoid_fast(e ? pff.y : pff.x);
-            const float so = sigmoid_fast(e ? po.y : po.x);
-            const float tg = tanh_fast(e ? pg.y : pg.x), tc = tanh_fast(e ? c1.y : c1.x);
-            fA[u] = so * (1.f - tc * tc);
-            fBi[u] = tg * si * (1.f - si);
-            fBf[u] = (e ? c0.y : c0.x) * sf * (1.f - sf);
-            fBg[u] = si * (1.f - tg * tg);
-            fBo[u] = tc * so * (1.f - so);
-            fSf[u] = sf;
-            fDd[u] = e ? dd.y : dd.x;
+            for (int e = 0; e < 2; ++e) {
+              const int u = 2 * w + e;
+              const float si = sigmoid_fast(e ? pi.y : pi.x), sf = sigmoid_fast(e ? pff.y : pff.x);
+              const float so = sigmoid_fast(e ? po.y : po.x);
+              const float tg = tanh_fast(e ? pg.y : pg.x), tc = tanh_fast(e ? c1.y : c1.x);
+              fA[u] = so * (1.f - tc * tc);
+              fBi[u] = tg * si * (1.f - si);
+              fBf[u] = (e ? c0.y : c0.x) * sf * (1.f - sf);
+              fBg[u] = si * (1.f - tg * tg);
+              fBo[u] = tc * so * (1.f - so);
+              fSf[u] = sf;
+              fDd[u] = e ? dd.y : dd.x;
+            }
           }
+          c1v = pf[4];
         }
-        }
-      };
-      // interleaved tiles: the gates of the item whose maths comes next, out of its landing buffer
-      auto fetch_gates = [&]() -> bool {
-        if constexpr (TMAEP) {
-          if (!mbar_wait(&pfull[pub_it % 3], (uint32_t)(pub_it / 3) & 1u, wc)) return false;
-          const uint8_t* pbb = pbuf + (pub_it % 3) * 4096;
-#pragma unroll
-          for (int k = 0; k < 4; ++k) pf[k] = *reinterpret_cast<const uint4*>(pbb + p_off(k));
-        }
-        return true;
       };
       prefetch(T - 1, pb + (ch * TI) * p.nb_par);
-      if (USE_FACTORS && EARLY_FACTORS) factors();
+      if (USE_FACTORS && EARLY_FACTORS) factors(cn[0]);
       for (int st = 0; st <= T && ok; ++st) {
 #pragma unroll
         for (int j = 0; j < TI; ++j) {
@@ -1371,102 +1295,87 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
             const int a = it & 1;
             const uint32_t a_ph = (uint32_t)(it >> 1) & 1u;
             // one set of exchange buffers: its barriers change phase with every item
-            constexpr int xb = 0;
             const uint32_t x_ph = (uint32_t)it & 1u;
             ++it;
             wc.d0 = T - st; wc.d1 = bt;
             if (!mbar_wait(&acc_full[a], a_ph, wc)) { ok = false; break; }
             if constexpr (TI >= 2) {
-              // the previous item's slices have been read by all three peers (so the staging below
-              // overwrites nothing a copy still reads, and the peers' receive slots are free again)
+              // the previous item's slices have been read by the whole cluster (so the staging below overwrites
+              // nothing a copy still reads, and the receive slots are free again)
               // (no data rides on this barrier, so a plain CTA-scope wait will do)
               if (it > 1 && !mbar_wait(consumed, (uint32_t)it & 1u, wc)) { ok = false; break; }
             }
-            if (p.alias && shipper) {
-              // this item's MMAs are done (their reads of the ring completed before acc_full did), so
+            if (ew == 0 && lane == 0) {
+              // what this CTA is about to receive (nothing for a quarter without rows)
+              mbar_expect_tx(xchg, bt * RB + (int)r * 32 < p.B ? 3 * XSLOT_BYTES : 0);
+              // aliased: this item's MMAs are done (their reads of the ring completed before acc_full did), so
               // the ring - and the exchange buffers laid over it - is idle until the next item: tell
               // the three peers they may write their slices.  Nothing of this thread is published by
               // the signal, hence relaxed.
+              if (p.alias) {
 #pragma unroll
-              for (int dst = 0; dst < 4; ++dst)
-                if (dst != (int)r) mbar_arrive_remote_relaxed(mapa_shared(smem_u32(rdy), dst));
+                for (int dst = 0; dst < 4; ++dst)
+                  if (dst != (int)r) mbar_arrive_remote_relaxed(mapa_shared(smem_u32(rdy), dst));
+              }
             }
             tc_fence_after();
-            const uint32_t taddr = tmem_base + a * ACC_STRIDE + (uint32_t(q * 32) << 16) + uoff;
+            const bool q_ok = bt * RB + q * 32 < p.B;       // quarter q has rows
+            const uint32_t taddr = tmem_base + a * ACC_STRIDE + (uint32_t(q * 32) << 16) + g * 32;
 #pragma unroll
-            for (int dst = 0; dst < 4; ++dst) {
-              // the issuers' partial accumulators for these units: NACC loads, ONE wait
-              uint32_t v[NACC][NU];
+            for (int h = 0; h < 2; ++h) {
+              // the issuers' partial accumulators for 16 units: NACC loads, ONE wait
+              uint32_t v[NACC][16];
 #pragma unroll
-              for (int xx = 0; xx < NACC; ++xx) tmem_ld_32x8(taddr + xx * N + dst * 16, v[xx]);
+              for (int xx = 0; xx < NACC; ++xx) tmem_ld_32x16(taddr + xx * N + h * 16, v[xx]);
               tmem_ld_wait();
-              float sum[NU];
 #pragma unroll
-              for (int u = 0; u < NU; ++u) {
-                float a0 = __uint_as_float(v[0][u]);
-                if (nacc > 1) a0 += __uint_as_float(v[1][u]);
-                if (NACC > 2 && nacc > 2) a0 += __uint_as_float(v[NACC - 1][u]);
-                sum[u] = a0;
-              }
-              if (dst == (int)r) {
+              for (int c4 = 0; c4 < 4; ++c4) {
+                float sum[4];
 #pragma unroll
-                for (int u = 0; u < NU; ++u) dhc[u] = sum[u];   // last step's carry is dead by now
-              } else {
-                // stage the slice for peer `dst` locally (row = 64 B, 16-byte pieces XOR-swizzled)
-                uint8_t* sp = stage + ((size_t)xb * 3 + (dst < (int)r ? dst : dst - 1)) * XSLOT_BYTES +
-                              row_in_tile * XROW_BYTES;
-#pragma unroll
-                for (int c4 = 0; c4 < NU / 4; ++c4)
-                  *reinterpret_cast<float4*>(sp + (((uoff >> 2) + c4) ^ swz) * 16) =
-                      make_float4(sum[4 * c4], sum[4 * c4 + 1], sum[4 * c4 + 2], sum[4 * c4 + 3]);
+                for (int u = 0; u < 4; ++u) {
+                  float a0 = __uint_as_float(v[0][4 * c4 + u]);
+                  if (nacc > 1) a0 += __uint_as_float(v[1][4 * c4 + u]);
+                  if (NACC > 2 && nacc > 2) a0 += __uint_as_float(v[NACC - 1][4 * c4 + u]);
+                  sum[u] = a0;
+                }
+                const int pc = g * 8 + h * 4 + c4;          // piece of the row
+                *reinterpret_cast<float4*>(put + ((((pc >> 1) ^ (lane & 7)) + 8 * (pc & 1)) << 4)) = make_float4(sum[0], sum[1], sum[2], sum[3]);
               }
             }
             tc_fence_before();
             fence_proxy_async_smem();                 // staged slices -> visible to the bulk-copy engine
             __syncwarp();
-            if (lane == 0) { mbar_arrive(&acc_empty[a]); mbar_arrive(&staged[xb]); }
-            // one thread ships the three slices once all eight epilogue warps have staged their part
-            // (bounded mbarrier wait, never a named barrier: a warp that gave up must not strand the rest)
-            if (shipper && mbar_wait(&staged[xb], x_ph, wc) &&
-                (!p.alias || mbar_wait_cluster(rdy, x_ph, wc))) {   // aliased: every peer's ring is idle
-              mbar_expect_tx(&xchg[xb], 3 * XSLOT_BYTES);      // what this CTA is about to receive
+            if (lane == 0) {
+              mbar_arrive(&acc_empty[a]);
+              if (q == (int)r) mbar_arrive(xchg);
+              else mbar_arrive(&staged[q]);
+              // one thread of the quarter's two warps ships it once both have staged their halves
+              // (bounded mbarrier wait, never a named barrier: a warp that gave up must not strand the rest)
+              if (g == 0 && q != (int)r && mbar_wait(&staged[q], x_ph, wc) && q_ok &&
+                  (!p.alias || mbar_wait_cluster(rdy, x_ph, wc)))       // aliased: every peer's ring is idle
+                dsmem_bulk_copy(mapa_shared(smem_u32(recv) + r * XSLOT_BYTES, q), put - lane * XROW_BYTES, XSLOT_BYTES,
+                                mapa_shared(smem_u32(xchg), q));
+            }
+            __syncwarp();
+            if (USE_FACTORS && !EARLY_FACTORS && st < T) factors(cn[j]);       // fills the wait for the peers' slices
+            if (!mbar_wait_cluster(xchg, x_ph, wc)) { ok = false; break; }
 #pragma unroll
-              for (int dst = 0; dst < 4; ++dst)
-                if (dst != (int)r) {
-                  // this CTA is sender number `slot` among peer dst's three; addresses mapped on the
-                  // spot (only this thread needs them)
-                  const int slot = (int)r < dst ? (int)r : (int)r - 1;
-                  dsmem_bulk_copy(mapa_shared(smem_u32(recv) + (xb * 3 + slot) * XSLOT_BYTES, dst),
-                                  stage + ((size_t)xb * 3 + (dst < (int)r ? dst : dst - 1)) * XSLOT_BYTES,
-                                  XSLOT_BYTES, mapa_shared(smem_u32(&xchg[xb]), dst));
-                }
-            }
-            if (USE_FACTORS && !EARLY_FACTORS && st < T) {               // fills the wait for the peers' slices
-              if (!fetch_gates()) { ok = false; break; }
-              factors();
-            }
-            if (!mbar_wait_cluster(&xchg[xb], x_ph, wc)) { ok = false; break; }
-            const uint8_t* rv = recv + (size_t)xb * (3 * XSLOT_BYTES) + row_in_tile * XROW_BYTES;
+            for (int u = 0; u < NU; ++u) dhc[u] = 0.f;
 #pragma unroll
-            for (int c4 = 0; c4 < NU / 4; ++c4) {
-              const int off = (((uoff >> 2) + c4) ^ swz) * 16;
-              const float4 s0 = *reinterpret_cast<const float4*>(rv + off);
-              const float4 s1 = *reinterpret_cast<const float4*>(rv + XSLOT_BYTES + off);
-              const float4 s2 = *reinterpret_cast<const float4*>(rv + 2 * XSLOT_BYTES + off);
-              dhc[4 * c4 + 0] += s0.x + s1.x + s2.x;
-              dhc[4 * c4 + 1] += s0.y + s1.y + s2.y;
-              dhc[4 * c4 + 2] += s0.z + s1.z + s2.z;
-              dhc[4 * c4 + 3] += s0.w + s1.w + s2.w;
-            }
+            for (int s = 0; s < 4; ++s)
+#pragma unroll
+              for (int o = 0; o < 2; ++o) {
+                const float4 v = *reinterpret_cast<const float4*>(get + s * XSLOT_BYTES + o * 128);
+                dhc[4 * o] += v.x;
+                dhc[4 * o + 1] += v.y;
+                dhc[4 * o + 2] += v.z;
+                dhc[4 * o + 3] += v.w;
+              }
             if constexpr (TI >= 2) {
-              // this warp has read the item's slices (the sums above hold them): tell the three peers.
+              // this warp has read the item's slices (the sums above hold them): tell the cluster.
               // Nothing is published by the signal, hence relaxed.
               __syncwarp();
-              if (lane == 0) {
-#pragma unroll
-                for (int dst = 0; dst < 4; ++dst)
-                  if (dst != (int)r) mbar_arrive_remote_relaxed(mapa_shared(smem_u32(consumed), dst));
-              }
+              if (lane < 4) mbar_arrive_remote_relaxed(mapa_shared(smem_u32(consumed), lane));
             }
           }
           if (st == 0) {
@@ -1479,10 +1388,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
             const int t = T - 1 - st;
             uint32_t qi[4], qf[4], qg[4], qo[4];
             if constexpr (USE_FACTORS) {
-              if (!EARLY_FACTORS && st == 0) {            // later items computed them during the exchange
-                if (!fetch_gates()) { ok = false; break; }
-                factors();
-              }
+              if (!EARLY_FACTORS && st == 0) factors(cn[j]);            // later items computed them during the exchange
 #pragma unroll
               for (int w = 0; w < 4; ++w) {
                 float r_[2][4];
@@ -1504,14 +1410,14 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
               }
             } else {
               // four interleaved tiles leave no registers for the factors: all of the maths here
-              if (!fetch_gates()) { ok = false; break; }
               const uint32_t wi[4] = {pf[0].x, pf[0].y, pf[0].z, pf[0].w};
               const uint32_t wf[4] = {pf[1].x, pf[1].y, pf[1].z, pf[1].w};
               const uint32_t wg[4] = {pf[2].x, pf[2].y, pf[2].z, pf[2].w};
               const uint32_t wo[4] = {pf[3].x, pf[3].y, pf[3].z, pf[3].w};
-              const uint32_t w1[4] = {pf[4].x, pf[4].y, pf[4].z, pf[4].w};
-              const uint32_t w0[4] = {pf[5].x, pf[5].y, pf[5].z, pf[5].w};
-              const uint32_t wd[4] = {pf[6].x, pf[6].y, pf[6].z, pf[6].w};
+              const uint32_t w1[4] = {cn[j].x, cn[j].y, cn[j].z, cn[j].w};
+              const uint32_t w0[4] = {pf[4].x, pf[4].y, pf[4].z, pf[4].w};
+              const uint32_t wd[4] = {pf[5].x, pf[5].y, pf[5].z, pf[5].w};
+              cn[j] = pf[4];
 #pragma unroll
               for (int w = 0; w < 4; ++w) {
                 const float2 pi = cvt2<T16>(wi[w]), pff = cvt2<T16>(wf[w]), pg = cvt2<T16>(wg[w]), po = cvt2<T16>(wo[w]);
@@ -1537,30 +1443,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
                 qo[w] = pk2<T16>(r_[0][3], r_[1][3]);
               }
             }
-            if constexpr (TMAEP) {
-              // d_ifgo[t] goes back into the landing buffer the gates came from and leaves as one box.
-              // The PREVIOUS item's box has been written by now: its buffer takes the gates of the item
-              // two ahead, and (the peers' producers read d_ifgo next) the warp counts that item in.
-              uint8_t* pbb = pbuf + (pub_it % 3) * 4096;
-              *reinterpret_cast<uint4*>(pbb + p_off(0)) = make_uint4(qi[0], qi[1], qi[2], qi[3]);
-              *reinterpret_cast<uint4*>(pbb + p_off(1)) = make_uint4(qf[0], qf[1], qf[2], qf[3]);
-              *reinterpret_cast<uint4*>(pbb + p_off(2)) = make_uint4(qg[0], qg[1], qg[2], qg[3]);
-              *reinterpret_cast<uint4*>(pbb + p_off(3)) = make_uint4(qo[0], qo[1], qo[2], qo[3]);
-              fence_proxy_async_smem();
-              __syncwarp();
-              if (lane == 0) mbar_arrive(&pdone[pub_it % 3]);      // this warp's half of the box is in place
-              if (lane == 0 && g == 0 && mbar_wait(&pdone[pub_it % 3], (uint32_t)(pub_it / 3) & 1u, wc)) {
-                tma_store_4d(&tmD, pbb, unit0, bt * RB + q * 32, 0, t);      // (g == 0: unit0 is the pair's first unit)
-                tma_store_commit();
-                // The peers' producers read d_ifgo[t] next, so the pair counts the item in only once the
-                // store has completed, and it waits for that at once: putting the wait off by an item (when
-                // it costs nothing) lengthens every tile's hand-off chain by that item, and the chain is
-                // what bounds the step even with four tiles interleaved (B=4096, H=512: 8.28 -> 7.75 ms).
-                tma_store_wait<0>();
-                mbar_arrive(&pfree[pub_it % 3]);
-                mbar_arrive(&pub_bar[pub_it & 3]);
-              }
-            } else if (row_ok) {
+            if (row_ok) {
               T16* dstp = dg + ((size_t)t * p.B + row) * H4 + unit0;
               stg16(dstp, make_uint4(qi[0], qi[1], qi[2], qi[3]));
               stg16(dstp + (size_t)H, make_uint4(qf[0], qf[1], qf[2], qf[3]));
@@ -1575,9 +1458,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
             // (a warp can be at most four items ahead of another - the maths-only items that open a
             // chunk - so four counters never mix items)
             if (lane == 0) {
-              if constexpr (TMAEP) {
-                // counted in above, once the store has completed
-              } else if constexpr (PUBLISHER) {
+              if constexpr (PUBLISHER) {
                 mbar_arrive(&pub_bar[pub_it & 3]);      // the publisher warp releases for the CTA
               } else {
                 const bool pub = !p.cta_publish ||
@@ -1586,6 +1467,14 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
               }
             }
             ++pub_it;
+            {
+              int nj = j + 1, ns = st;
+              if (nj == TI || pb + (ch * TI + nj) * p.nb_par >= p.nbt) { nj = 0; ns = st + 1; }
+              if (ns < T) prefetch(T - 1 - ns, pb + (ch * TI + nj) * p.nb_par);
+              int fj = nj + 1, fs = ns;
+              if (fj == TI || pb + (ch * TI + fj) * p.nb_par >= p.nbt) { fj = 0; fs = ns + 1; }
+              if (fs < T) prefetch_far(T - 1 - fs, pb + (ch * TI + fj) * p.nb_par);
+            }
             // bias-gradient sums: after the publication, off the hand-off chain
             if (want_db) {   // warp-uniform: tensor-memory loads and stores need the whole warp; rows past B add 0
               const uint32_t* qs[4] = {qi, qf, qg, qo};
@@ -1604,17 +1493,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
               }
               tmem_st_wait();
             }
-            {
-              int nj = j + 1, ns = st;
-              if (nj == TI || pb + (ch * TI + nj) * p.nb_par >= p.nbt) { nj = 0; ns = st + 1; }
-              if (ns < T) {
-                prefetch(T - 1 - ns, pb + (ch * TI + nj) * p.nb_par);
-                if (USE_FACTORS && EARLY_FACTORS) factors();
-              }
-              int fj = nj + 1, fs = ns;
-              if (fj == TI || pb + (ch * TI + fj) * p.nb_par >= p.nbt) { fj = 0; fs = ns + 1; }
-              if (fs < T) prefetch_far(T - 1 - fs, pb + (ch * TI + fj) * p.nb_par);
-            }
+            if (USE_FACTORS && EARLY_FACTORS && st + 1 < T) factors(cn[0]);
           } else if (row_ok) {
             // ---- after the last step: the carries are the gradients of the initial state
             store8<T16>(reinterpret_cast<T16*>(p.dh0) + (size_t)row * H + unit0, dhc);
@@ -1624,7 +1503,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
       }
     }
     if (want_db) {
-      float* dst = p.db_part + ((size_t)pb * 4 + q) * H4 + unit0;
+      float* dst = p.db_part + (((size_t)pb * 4 + r) * ITEM_WARPS + ew) * H4 + unit0;
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         uint32_t acc[8];
@@ -1633,9 +1512,9 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
           float v = __uint_as_float(acc[u]);
-#pragma unroll
-          for (int off = 16; off >= 1; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-          if (lane == 0) dst[(size_t)k * H + u] = v;
+          v += __shfl_xor_sync(0xffffffffu, v, 8);
+          v += __shfl_xor_sync(0xffffffffu, v, 16);
+          if (lane < 8) dst[(size_t)k * H + u] = v;
         }
       }
     }
@@ -1715,8 +1594,7 @@ static int bwd_cta_capacity() {
 }
 
 template <int TI, typename T16>
-static int launch_bwd_t(const BwdPlan& pl, const CUtensorMap& tw, const CUtensorMap& tg, const CUtensorMap& ti,
-                        const CUtensorMap& td, BwdParams& p, cudaStream_t st) {
+static int launch_bwd_t(const BwdPlan& pl, const CUtensorMap& tw, const CUtensorMap& tg, BwdParams& p, cudaStream_t st) {
   auto kern = bwd_kernel<TI, T16>;
   BLSTM_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
   cudaLaunchConfig_t cfg = {};
@@ -1740,14 +1618,14 @@ static int launch_bwd_t(const BwdPlan& pl, const CUtensorMap& tw, const CUtensor
   int max_clusters = 0;
   BLSTM_CUDA_OK(cudaOccupancyMaxActiveClusters(&max_clusters, kern, &cfg));
   if (max_clusters * 4 < pl.grid) return BLSTM_E_NOT_CORESIDENT;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tw, tg, ti, td, p);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tw, tg, p);
   if (cfg.numAttrs == 2 && (e == cudaErrorNotSupported || e == cudaErrorCooperativeLaunchTooLarge)) {
     // Only when the driver refuses the cooperative + cluster combination as such is the cooperative
     // attribute dropped (co-residency then rests on the occupancy check above); any other launch error
     // is reported as it is.
     (void)cudaGetLastError();
     cfg.numAttrs = 1;
-    e = cudaLaunchKernelEx(&cfg, kern, tw, tg, ti, td, p);
+    e = cudaLaunchKernelEx(&cfg, kern, tw, tg, p);
   }
   BLSTM_CUDA_OK(e);
   count_launch();
@@ -1902,20 +1780,7 @@ int sm100_bwd_recurrence(const blstm_desc& d, const void* dout, const void* dh_n
     rc = encode_tensor_map(&tg, d_ifgo, 3, dims, str, box);
     if (rc) return rc;
   }
-  CUtensorMap ti = tg, td = tg;     // only read by the kernels that interleave tiles
-  if (pl.TI >= 2) {
-    // ifgo and d_ifgo [T,B,4H] as {unit, batch row, gate, t}: a box is a warp pair's 4 gates x 32 rows x 16 units
-    // (32-byte rows, 32-byte swizzle)
-    uint64_t dims[4] = {(uint64_t)H, (uint64_t)B, 4, (uint64_t)T};
-    uint64_t str[3] = {(uint64_t)4 * H * 2, (uint64_t)H * 2, (uint64_t)B * 4 * H * 2};
-    uint32_t box[4] = {16, 32, 4, 1};
-    rc = encode_tensor_map(&ti, ifgo, 4, dims, str, box, 2, 32);
-    if (rc) return rc;
-    rc = encode_tensor_map(&td, d_ifgo, 4, dims, str, box, 2, 32);
-    if (rc) return rc;
-  }
   BwdParams p;
-  p.ep_bytes = (int)pl.ep_bytes;
   p.T = T; p.B = B; p.H = H;
   p.nbt = pl.nbt; p.nug = pl.nug; p.nb_par = pl.nb_par; p.ntl = pl.ntl; p.stages = pl.stages; p.ni = pl.ni;
   p.nl = pl.nl;
@@ -1935,11 +1800,11 @@ int sm100_bwd_recurrence(const blstm_desc& d, const void* dout, const void* dh_n
   p.d_ifgo = d_ifgo; p.dh0 = dh0; p.dc0 = dc0;
   p.db_part = db ? reinterpret_cast<float*>(static_cast<char*>(ws) + pl.off_db) : nullptr;
   const bool bf = d.dtype == BLSTM_BF16;
-  if (pl.TI == 1)      rc = bf ? launch_bwd_t<1, __nv_bfloat16>(pl, tw, tg, ti, td, p, st) : launch_bwd_t<1, __half>(pl, tw, tg, ti, td, p, st);
-  else if (pl.TI == 2) rc = bf ? launch_bwd_t<2, __nv_bfloat16>(pl, tw, tg, ti, td, p, st) : launch_bwd_t<2, __half>(pl, tw, tg, ti, td, p, st);
-  else                 rc = bf ? launch_bwd_t<4, __nv_bfloat16>(pl, tw, tg, ti, td, p, st) : launch_bwd_t<4, __half>(pl, tw, tg, ti, td, p, st);
+  if (pl.TI == 1)      rc = bf ? launch_bwd_t<1, __nv_bfloat16>(pl, tw, tg, p, st) : launch_bwd_t<1, __half>(pl, tw, tg, p, st);
+  else if (pl.TI == 2) rc = bf ? launch_bwd_t<2, __nv_bfloat16>(pl, tw, tg, p, st) : launch_bwd_t<2, __half>(pl, tw, tg, p, st);
+  else                 rc = bf ? launch_bwd_t<4, __nv_bfloat16>(pl, tw, tg, p, st) : launch_bwd_t<4, __half>(pl, tw, tg, p, st);
   if (rc) return rc;
-  if (db) return reduce_db(p.db_part, pl.nb_par * 4, 4 * H, db, st);   // the kernel left one row per CTA group and row quarter
+  if (db) return reduce_db(p.db_part, pl.nb_par * 32, 4 * H, db, st);
   return BLSTM_OK;
 }
 
