@@ -109,14 +109,15 @@ static RecPlan make_plan(const blstm_desc& d, int phase) {
   p.ntl = cdiv(p.nbt, p.nb_par);
   p.TI = p.ntl >= 3 ? 4 : p.ntl >= 2 ? 2 : 1;     // batch tiles interleaved per CTA (state: cell rows in registers)
   p.grid = p.nh * p.nb_par;
-  p.epi_warps = (UH == 16 && p.TI == 1) ? 4 : 8;
+  p.epi_warps = 8;
   // a single 16-unit tile in flight is latency bound: four issuers next to one epilogue warpgroup
   // (9 warps); otherwise two issuers, eight epilogue warps and, for interleaved tiles, the publisher
   // (interleaved 32-unit slices: N = 128 runs the tensor pipe at full rate from ONE issuing thread, and a
   // single accumulator per item leaves tensor-memory columns for the cell rows of four tiles)
-  const int n_issuers = (UH == 16 && p.TI == 1) ? 4 : (UH == 32 && p.TI >= 2) ? 1 : 2;
+  // (streamed weights double the bytes of a chunk: a third issuer)
+  const int n_issuers = UH == 32 ? 1 : (p.TI == 1 && (size_t)p.N * H * 2 > 128 * 1024) ? 3 : 2;
   const int n_publisher = p.TI >= 2 ? 1 : 0;
-  p.threads = 32 * (1 + n_issuers + n_publisher + p.epi_warps);   // producer + MMA issuers [+ publisher] + epilogue
+  p.threads = 32 * (1 + (UH == 32 ? 1 : p.TI == 1 ? 3 : 2) + n_publisher + p.epi_warps);   // producer + MMA issuers [+ publisher] + epilogue
   // Wh slice resident in shared memory when it fits next to a useful ring; otherwise (H > 1024) it is
   // streamed through the ring with h, chunk by chunk, every step (it stays in L2).  A single batch tile
   // of fewer than 128 rows only stages its own rows (the MMA's rows past them read whatever follows:
@@ -154,8 +155,8 @@ static RecPlan make_plan(const blstm_desc& d, int phase) {
   // (B=2048: 2.55 -> 2.46 ms, B=1024: 1.89 -> 1.78 ms), a single tile on a six-stage ring with fewer
   // (H=1024: 3.89 -> 3.75 ms).
   p.nl = p.ni;
+  if (p.TI == 1) p.nl = p.stages == 6 ? 2 : 4;
   if (p.TI == 2) p.nl = UH == 32 ? 2 : 4;
-  if (p.TI == 1 && p.stages == 6) p.nl = 2;
   if (p.stages % p.nl != 0 || p.nl > H / RK) p.nl = p.ni;
   p.smem = fixed + (size_t)p.stages * p.stage_bytes;
   p.n_flags = (size_t)(d.seq_len + 1) * p.nbt;
@@ -178,8 +179,7 @@ struct FwdParams {
   int fmt;
   int no_arrive;
   int inference;            // skip the stores that only backward needs
-  int flag_target;          // arrivals that complete a flag: nh CTAs per batch tile [x epilogue warps]
-  int cta_publish;          // 1: one arrival per CTA and item, 0: one per epilogue warp
+  int flag_target;          // arrivals that complete a flag: nh CTAs per batch tile
   int npb;                  // TMA landing buffers per epilogue warp (interleaved tiles)
   int ep_bytes;             // bytes of the epilogue's TMA buffers (between the weights and the ring)
   unsigned long long limit_ns;
@@ -212,10 +212,14 @@ struct ItemCursor {
 // warps - at most 12 (3 per SM sub-partition), which leaves 168 registers per thread; a 13th would cap
 // them at 128.  The epilogue must not spill.
 template <int UH, int TI, typename T16>
-__global__ void __launch_bounds__(32 * (UH == 16 && TI == 1 ? 9 : (TI >= 2 ? (UH == 32 ? 11 : 12) : 11)), 1)
+__global__ void __launch_bounds__(32 * (UH == 16 ? 12 : 11), 1)
 fwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmH,
            const __grid_constant__ CUtensorMap tmP, const FwdParams p) {
   constexpr int N = 4 * UH;
+  // One tile in flight: h leaves through a TMA store (tmP: out as {unit, row, step}) that the warp sees completed after
+  // some 300 clocks, staged in the ring, which is idle until this CTA has counted the item in.  Plain stores cost the
+  // release behind them 1.6 k clocks (128 CTAs handing one tile on in a loop: 4.6 k clocks a hand-off with plain stores
+  // and the wide proxy fence, 3.1 k this way).
   // Interleaved tiles are throughput bound, and there the epilogue's row-strided 16-byte global
   // accesses (a thread owns a batch row: 32 sectors per warp instruction) were the bottleneck: the
   // projected pre-activations come in as TMA boxes through shared memory, one set of buffers per
@@ -227,14 +231,9 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
   // Epilogue warps.  A single tile of 16 units is latency bound and runs best as one warpgroup with
   // 16 units per thread next to four issuers (9 warps); every other shape uses two warpgroups that
   // split the CTA's units (8 or 16 per thread), which keeps interleaved tiles free of spills.
-  constexpr int EW = (UH == 16 && TI == 1) ? 4 : 8;
+  constexpr int EW = 8;
   constexpr int NU = 4 * UH / EW;                   // units per epilogue thread
   constexpr int NV = NU / 8;                        // 16-byte pieces per operand per thread
-  // Which side runs the generic->async proxy fence of the hand-off.  One tile in flight: the READER, after
-  // it has seen the counter (traced: the writers' release then waits for their h stores alone, 1.5 k clk
-  // instead of fence 1.8 k + release 1.5 k, against 0.8 k for the fence on the reading side).  Interleaved
-  // tiles: the writers' publisher warp.
-  constexpr bool WRITER_FENCE = false;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int H = p.H;
@@ -266,7 +265,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
   // stalls its thread for a memory round trip, so a PUBLISHER warp does the releasing (and the proxy
   // fence of the hand-off): the epilogue warps only arrive on a CTA-local barrier after storing h.
   constexpr bool PUBLISHER = (TI >= 2);
-  constexpr int NACC = (UH == 16 && TI == 1) ? 4 : (UH == 32 && TI >= 2) ? 1 : 2;   // issuer warps / partial accumulators
+  constexpr int NACC = UH == 32 ? 1 : TI == 1 ? 3 : 2;   // issuer warps / partial accumulators
   constexpr int FIRST_EPI = 1 + NACC + (PUBLISHER ? 1 : 0);   // first epilogue warp
   // Columns per item buffer (NACC * N <= 256).  Interleaved tiles pack the two buffers into the first
   // 256 columns and keep the tiles' cell rows (fp32, a column per unit) in the columns behind them.
@@ -284,14 +283,14 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
     mbar_init(w_full, 1);
     *dead = 0;
     for (int i = 0; i < 4; ++i) pub_cnt[i] = 0;
-    for (int i = 0; i < 4; ++i) mbar_init(&pub_bar[i], EW);
+    for (int i = 0; i < 4; ++i) mbar_init(&pub_bar[i], TI == 1 ? 1 : EW);
     for (int i = 0; i < 16; ++i) mbar_init(&pre_full[i], 1);
     fence_mbar_init();
     // (stage s is first used by chunk s; with streamed weights there are more chunks than stages)
     for (int s = 0; s < R_STAGES; ++s) mbar_expect_tx(&full[s], (p.ws && s % KC >= p.kr) ? SB : HB);
     tma_prefetch_desc(&tmW);
     tma_prefetch_desc(&tmH);
-    if (TMAEP) tma_prefetch_desc(&tmP);
+    tma_prefetch_desc(&tmP);
   }
   if (warp == 1) tmem_alloc(tmem_slot, TMEM_COLS);
   tc_fence_before();
@@ -350,10 +349,9 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
             }
             seen = __shfl_sync(0xffffffffu, seen, 0);
             if (!seen) { *dead = 1; ok = false; break; }
-            // One proxy fence must lie between the peers' generic-proxy stores and this warp's TMA
-            // reads: here for a single tile in flight, in the writers' publisher warp otherwise (this
-            // loop then streams h without a break).
-            if (!WRITER_FENCE && !PUBLISHER) fence_proxy_async();
+            // a proxy fence between the peers' arrivals (interleaved tiles: their plain stores, fenced by their publisher
+            // warps) and this warp's TMA reads
+            if (!PUBLISHER) fence_proxy_async_global();
           }
           const int row0 = bt * RB;
           if (lane < nl && lane_ok) {
@@ -394,7 +392,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
             if (bt >= p.nbt) continue;
             wc.d0 = t; wc.d1 = bt;
             if (!mbar_wait(&pub_bar[k & 3], (uint32_t)(k >> 2) & 1u, wc)) { ok = false; break; }
-            fence_proxy_async();
+            fence_proxy_async_global();
             if (!p.no_arrive) red_release_gpu_add(&p.flags[(size_t)(t + 1) * p.nbt + bt], 1);
             ++k;
           }
@@ -404,7 +402,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
   } else if (warp < 1 + NACC) {
     // ---------------------------------------------------------------- MMA issuers
     const int x = warp - 1;                 // accumulator / K-slice index of this issuer
-    if (lane == 0) {
+    if (elect_one()) {                      // (a thread chosen by `elect` issues an MMA every 55 clocks, by lane == 0 every 74)
       constexpr uint64_t descK = smem_desc_base(16, 1024);
       const uint32_t idesc = instr_desc(p.fmt, 0, 0, RB, N);
       // Every tcgen05 instruction (mma or commit) costs this thread ~150 clocks of issue time, so
@@ -631,8 +629,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
     const int row_in_tile = q * 32 + lane;
     const int unit0 = ht * UH + ug * NU;
     const size_t H4 = 4 * (size_t)H;
+    uint8_t* hbuf = a_s + ew * (64 * NU);   // this warp's 32 rows x NU units of h
     T16* ifgo = reinterpret_cast<T16*>(p.ifgo);
-    T16* out = reinterpret_cast<T16*>(p.out);
     T16* cell = reinterpret_cast<T16*>(p.cell);
     int it = 0;                             // items consumed: TMEM buffer it & 1, on its (it >> 1)-th use
     bool ok = true;
@@ -676,87 +674,71 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
           if (!mbar_wait(&acc_full[a], a_ph, wc)) { ok = false; break; }
           tc_fence_after();
           const uint32_t taddr = tmem_base + a * ACC_STRIDE + (uint32_t(q * 32) << 16) + ug * NU;
-          // The thread's NU units are worked in passes of PW: accumulator read-out (the issuers' partial
-          // sums, gate by gate, XG of them per wait so that at most 48 values are in flight), gate
-          // maths, h store.  Two interleaved tiles of 16 units per thread take two passes of 8 -
-          // a single pass would not fit the register file - and save the final pre-activations
-          // inside the pass; every other shape takes one pass and saves them after the release.
-          constexpr int PW = (NU == 16 && TI >= 2) ? 8 : NU;
-          constexpr int XG = (NACC * PW > 48) ? 2 : NACC;
+          // accumulator read-out (the issuers' partial sums, GG gates per wait: at most 48 values in flight), gate maths, h store; the final pre-activations are saved after the release
+          constexpr int GG = 2;
           const size_t o1 = ((size_t)(t + 1) * p.B + row) * H + unit0;
           T16* gdst = ifgo + ((size_t)t * p.B + row) * H4 + unit0;
-          float pa[4][PW];
+          float pa[4][NU];
 #pragma unroll
-          for (int h0 = 0; h0 < NU; h0 += PW) {
+          for (int g0 = 0; g0 < 4; g0 += GG) {
+            uint32_t v[GG][NACC][NU];
 #pragma unroll
-            for (int g = 0; g < 4; ++g) {
+            for (int g = 0; g < GG; ++g)
 #pragma unroll
-              for (int x0 = 0; x0 < NACC; x0 += XG) {
-                uint32_t v[XG][PW];
+              for (int x = 0; x < NACC; ++x)
+                if (x < nacc) tmem_ld_cols<NU>(taddr + x * N + (g0 + g) * UH, v[g][x]);
+            tmem_ld_wait();
 #pragma unroll
-                for (int x = 0; x < XG; ++x) tmem_ld_cols<PW>(taddr + (x0 + x) * N + g * UH + h0, v[x]);
-                tmem_ld_wait();
+            for (int g = 0; g < GG; ++g)
 #pragma unroll
-                for (int u = 0; u < PW; ++u) {
-                  float s0 = (x0 == 0) ? 0.f : pa[g][u];
+              for (int u = 0; u < NU; ++u) {
+                float s0 = __uint_as_float(v[g][0][u]);
 #pragma unroll
-                  for (int x = 0; x < XG; ++x)
-                    if (x0 + x < nacc) s0 += __uint_as_float(v[x][u]);
-                  pa[g][u] = s0;
-                }
+                for (int x = 1; x < NACC; ++x)
+                  if (x < nacc) s0 += __uint_as_float(v[g][x][u]);
+                pa[g0 + g][u] = s0;
               }
-            }
-            if (h0 + PW == NU) {
-              // the accumulator is in registers: hand the TMEM buffer back to the MMA warps
-              tc_fence_before();
-              __syncwarp();
-              if (lane == 0) mbar_arrive(&acc_empty[a]);
-            }
-#pragma unroll
-            for (int g = 0; g < 4; ++g)
-#pragma unroll
-              for (int v = 0; v < PW / 8; ++v) {
-                const uint4 pw4 = pre[g * NV + h0 / 8 + v];
-                const uint32_t w[4] = {pw4.x, pw4.y, pw4.z, pw4.w};
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                  const float2 f2 = cvt2<T16>(w[u]);
-                  pa[g][8 * v + 2 * u] += f2.x;
-                  pa[g][8 * v + 2 * u + 1] += f2.y;
-                }
-              }
-            float hv[PW];
-#pragma unroll
-            for (int u = 0; u < PW; ++u) {
-              const float cn = sigmoid_fast(pa[1][u]) * c[j][h0 + u] + sigmoid_fast(pa[0][u]) * tanh_fast(pa[2][u]);
-              c[j][h0 + u] = cn;
-              hv[u] = sigmoid_fast(pa[3][u]) * tanh_fast(cn);
-            }
-            if (row_ok) {
-#pragma unroll
-              for (int v = 0; v < PW / 8; ++v) store8<T16>(out + o1 + h0 + 8 * v, &hv[8 * v]);
-              if (PW < NU && !p.inference) {
-#pragma unroll
-                for (int g = 0; g < 4; ++g) store8<T16>(gdst + (size_t)g * H + h0, pa[g]);
-              }
-            }
           }
-          // publish h[t+1] first (it is all the peers wait for): generic-proxy stores -> proxy fence
-          // (here or on the reading side) -> warp-level arrival with release semantics; peers read
-          // the rows through TMA
-          if (WRITER_FENCE) fence_proxy_async();
+          // the accumulator is in registers: hand the TMEM buffer back to the MMA warps
+          tc_fence_before();
           __syncwarp();
-          // arrival per warp, or (cta_publish) one per CTA and item: the last epilogue warp to get here
-          // publishes for all (a warp can be at most two items ahead of another, so four counters
-          // never mix items)
+          if (lane == 0) mbar_arrive(&acc_empty[a]);
+#pragma unroll
+          for (int g = 0; g < 4; ++g)
+#pragma unroll
+            for (int v = 0; v < NV; ++v) {
+              const uint4 pw4 = pre[g * NV + v];
+              const uint32_t w[4] = {pw4.x, pw4.y, pw4.z, pw4.w};
+#pragma unroll
+              for (int u = 0; u < 4; ++u) {
+                const float2 f2 = cvt2<T16>(w[u]);
+                pa[g][8 * v + 2 * u] += f2.x;
+                pa[g][8 * v + 2 * u + 1] += f2.y;
+              }
+            }
+          float hv[NU];
+#pragma unroll
+          for (int u = 0; u < NU; ++u) {
+            const float cn = sigmoid_fast(pa[1][u]) * c[j][u] + sigmoid_fast(pa[0][u]) * tanh_fast(pa[2][u]);
+            c[j][u] = cn;
+            hv[u] = sigmoid_fast(pa[3][u]) * tanh_fast(cn);
+          }
+#pragma unroll
+          for (int v = 0; v < NV; ++v) store8<T16>(reinterpret_cast<T16*>(hbuf + lane * (2 * NU)) + 8 * v, &hv[8 * v]);
+          // publish h[t+1] first (it is all the peers wait for): one arrival per CTA and item, by the last epilogue warp
+          // whose rows are stored (a warp can be at most two items ahead of another, so four counters never mix items)
+          fence_proxy_async_smem();
+          __syncwarp();
           if (lane == 0) {
-            if constexpr (PUBLISHER) {
-              mbar_arrive(&pub_bar[(it - 1) & 3]);     // the publisher warp releases for the CTA
-            } else {
-              const bool pub = !p.cta_publish || (smem_count_arrive(&pub_cnt[it & 3]) & (EW - 1)) == EW - 1;
-              if (pub && !p.no_arrive) red_release_gpu_add(&p.flags[(size_t)(t + 1) * p.nbt + bt], 1);
+            tma_store_3d(&tmP, hbuf, unit0, bt * RB + q * 32, t + 1);
+            tma_store_commit();
+            tma_store_wait<0>();
+            if ((smem_count_arrive(&pub_cnt[it & 3]) & (EW - 1)) == EW - 1) {
+              if (!p.no_arrive) red_release_gpu_add(&p.flags[(size_t)(t + 1) * p.nbt + bt], 1);
+              mbar_arrive(&pub_bar[it & 3]);
             }
           }
+          __syncwarp();
           // only now (after the release: a fence would otherwise wait for these loads) fetch the NEXT
           // item's projected pre-activations; they land while the peers run their step
           {
@@ -775,17 +757,19 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
               for (int g = 0; g < 4; ++g) prefetch_l2(src + (size_t)g * H);
             }
           }
-          // off the critical path: final pre-activations and c[t+1], saved for backward
-          // (inference: only the last cell state is needed, as c_n)
+          // off the critical path: final pre-activations and c[t+1], saved for backward (inference: only the last cell
+          // state is needed, as c_n) - once the CTA has counted the item in, because the release waits for whatever
+          // stores of the SM are under way (H=1024: 4.2 k clocks instead of 1.3 k)
+          if (!mbar_wait(&pub_bar[it & 3], (uint32_t)((it - 1) >> 2) & 1u, wc)) { ok = false; break; }
           if (row_ok && (!p.inference || t == p.T - 1)) {
 #pragma unroll
             for (int v = 0; v < NV; ++v) store8<T16>(cell + o1 + 8 * v, &c[j][8 * v]);
           }
-          if (PW == NU && row_ok && !p.inference) {
+          if (row_ok && !p.inference) {
 #pragma unroll
             for (int g = 0; g < 4; ++g)
 #pragma unroll
-              for (int v = 0; v < NV; ++v) store8<T16>(gdst + (size_t)g * H + 8 * v, &pa[g][8 * (v % (PW / 8))]);
+              for (int v = 0; v < NV; ++v) store8<T16>(gdst + (size_t)g * H + 8 * v, &pa[g][8 * v]);
           }
         }
       }
@@ -831,8 +815,8 @@ static int launch_fwd_t(const RecPlan& pl, const CUtensorMap& tw, const CUtensor
 // arrival counters as in the forward kernel.
 // =====================================================================================
 constexpr int DB_PARTS = 1024;            // row groups of the bias-gradient column sum
-constexpr int XROW_BYTES = 256;           // one row of a slice: 64 fp32; its 16-byte pieces: even ones, then odd ones, XOR-swizzled
-constexpr int XSLOT_BYTES = 32 * XROW_BYTES;  // one exchanged slice: 32 rows x 64 fp32 = 8 KB
+constexpr int XROW_BYTES = 128;           // one row of half a slice: 32 fp32; its 16-byte pieces are XOR-swizzled
+constexpr int XSLOT_BYTES = 2 * 32 * XROW_BYTES;  // one exchanged slice: 2 halves x 32 rows x 32 fp32 = 8 KB
 
 struct BwdPlan {
   bool ok;
@@ -889,10 +873,9 @@ static BwdPlan make_bwd_plan(const blstm_desc& d) {
     p.TI = 1;                                               // not enough room to interleave tiles
   size_t wres = (size_t)p.kr * 8192;
   size_t fixed = 1024 + wres + p.recv_bytes + 1024 + tail_pad;  // 1024: barriers and counters behind the ring
-  // warps: 1 producer + 3 MMA issuers (or 2 + a publisher warp when tiles are interleaved) + 2 epilogue
-  // warpgroups = 12 (3 per SM sub-partition, 168 registers each); a 13th warp would cap every thread
-  // at 128 registers.
-  const int n_issuers = p.TI >= 2 ? 2 : 3;
+  // warps: 1 producer + 3 MMA issuers (or 2 + a publisher when tiles are interleaved) + 2 epilogue warpgroups = 12
+  // (3 per SM sub-partition, 168 registers each); a 13th warp would cap every thread at 128 registers.
+  const int n_issuers = p.TI == 1 && p.ws ? 3 : 2;        // (streamed weights double the bytes of a chunk)
   p.threads = 32 * 12;
   if (!pick_ring(fixed, p.stage_bytes, n_issuers, H / RK, &p.stages, &p.ni)) return p;
   // One tile in flight and a shallow ring (H = 768, 1024: the resident weights leave four stages, or two):
@@ -904,7 +887,7 @@ static BwdPlan make_bwd_plan(const blstm_desc& d) {
     int st2 = 0, ni2 = 0;
     const size_t fixed2 = 1024 + wres + 1024 + tail_pad;
     if (pick_ring(fixed2, p.stage_bytes, n_issuers, H / RK, &st2, &ni2) && st2 > p.stages &&
-        (size_t)st2 * p.stage_bytes >= p.recv_bytes) {
+        (size_t)st2 * p.stage_bytes >= p.recv_bytes + 16384) {    // (and the rows on their way out lie behind them)
       p.alias = 1; p.stages = st2; p.ni = ni2; fixed = fixed2;
     }
   }
@@ -912,7 +895,7 @@ static BwdPlan make_bwd_plan(const blstm_desc& d) {
   // (B=4096, H=512: 8.5 -> 8.1 ms), a single tile on a six-stage ring with two (H=1024: 5.33 -> 5.22 ms)
   p.nl = p.ni;
   if (p.TI == 4) p.nl = 4;
-  if (p.TI == 1 && p.stages == 6) p.nl = 2;
+  if (p.TI == 1) p.nl = p.stages == 6 ? 2 : 4;
   if (p.stages % p.nl != 0 || p.nl > H / RK) p.nl = p.ni;
   p.smem = fixed + (size_t)p.stages * p.stage_bytes;
   p.n_flags = (size_t)d.seq_len * p.nbt;
@@ -935,8 +918,7 @@ struct BwdParams {
   int stage_bytes;
   int fmt;
   int no_arrive;
-  int flag_target;          // arrivals that complete a flag: H/16 CTAs per batch tile [x 8 epilogue warps]
-  int cta_publish;          // 1: one arrival per CTA and item, 0: one per epilogue warp
+  int flag_target;          // arrivals that complete a flag: H/16 CTAs per batch tile
   int alias;                // 1: exchange buffers laid over the first ring stages (one tile in flight)
   unsigned long long limit_ns;
   Control* ctl;
@@ -954,7 +936,8 @@ struct BwdParams {
 
 template <int TI, typename T16>
 __global__ void __launch_bounds__(384, 1)
-bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmG, const BwdParams p) {
+bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmG,
+           const __grid_constant__ CUtensorMap tmD, const BwdParams p) {
   // Warps: 0 = TMA producer, then NACC MMA issuers, then (interleaved tiles only) one PUBLISHER warp,
   // then 8 epilogue warps from warp 4 on - 12 in all either way.
   // With interleaved tiles the epilogue warps are the bottleneck, and the release that publishes an
@@ -963,7 +946,6 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
   constexpr bool PUBLISHER = (TI >= 2);
   constexpr int N = 64, NACC = PUBLISHER ? 2 : 3, ACC_STRIDE = 256;   // NACC: MMA issuer warps
   constexpr int FIRST_EPI = 4;
-  constexpr bool WRITER_FENCE = false;            // the proxy fence of the hand-off: reader (one tile) or publisher warp
   constexpr int ITEM_WARPS = 8;                   // epilogue warps, all working on every item
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -983,8 +965,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
   uint64_t* acc_empty = acc_full + 2;
   uint64_t* w_full = acc_empty + 2;
   uint64_t* xchg = w_full + 1;                                // slices of an item complete
-  uint64_t* staged = xchg + 1;                                // [4] row quarter staged by its two warps
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(staged + 4);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(xchg + 1);
   volatile int* dead = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* pub_cnt = const_cast<int*>(dead) + 1;        // [4] arrivals of the epilogue warps, by item index mod 4
   uint64_t* pub_bar = reinterpret_cast<uint64_t*>(pub_cnt + 4);   // [4] item stored? by item index mod 4
@@ -1005,7 +986,6 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
     for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], nacc); mbar_init(&acc_empty[a], ITEM_WARPS); }
     mbar_init(w_full, 1);
     mbar_init(xchg, 3);                             // one expect_tx arrival + tx bytes, and the two warps of the own quarter
-    for (int j = 0; j < 4; ++j) mbar_init(&staged[j], 2);
     *dead = 0;
     for (int i = 0; i < 4; ++i) pub_cnt[i] = 0;
     for (int i = 0; i < 4; ++i) mbar_init(&pub_bar[i], ITEM_WARPS);
@@ -1015,6 +995,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
     for (int s = 0; s < R_STAGES; ++s) mbar_expect_tx(&full[s], (p.ws && s % KC >= p.kr) ? SB : HB);
     tma_prefetch_desc(&tmW);
     tma_prefetch_desc(&tmG);
+    if (TI == 1) tma_prefetch_desc(&tmD);
   }
   if (warp == 1) tmem_alloc(tmem_slot, TMEM_COLS);
   tc_fence_before();
@@ -1060,10 +1041,9 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
           }
           seen = __shfl_sync(0xffffffffu, seen, 0);
           if (!seen) { *dead = 1; ok = false; break; }
-          // One proxy fence must lie between the peers' generic-proxy stores and the TMA reads below:
-          // here for a single tile in flight (the writers' release then waits for their stores alone),
-          // in the writers' publisher warp for interleaved tiles (this loop then streams without a break).
-          if (!WRITER_FENCE && !PUBLISHER) fence_proxy_async();
+          // a proxy fence between the peers' arrivals (interleaved tiles: their plain stores, fenced by their publisher
+          // warps) and the TMA reads below
+          if (!PUBLISHER) fence_proxy_async_global();
           const int row0 = bt * RB, col0 = (int)r * H;
           bool lane_ok = true;
           const int nl = p.nl;                 // TMA-issuing lanes: lane l owns the ring stages == l (mod nl)
@@ -1107,7 +1087,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
             if (!mbar_wait(&pub_bar[k & 3], (uint32_t)(k >> 2) & 1u, wc)) { ok = false; break; }
             // the generic->async proxy fence of the hand-off runs here, on the causality path between
             // the epilogue warps' stores (ordered before this thread by the barrier) and the release
-            fence_proxy_async();
+            fence_proxy_async_global();
             if (!p.no_arrive) red_release_gpu_add(&p.flags[(size_t)(T - 1 - st) * p.nbt + bt], 1);
             ++k;
           }
@@ -1117,7 +1097,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
   } else if (warp < 1 + NACC) {
     // ---------------------------------------------------------------- MMA issuers (own whole chunks)
     const int x = warp - 1;
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint64_t descA = smem_desc_base(16, 1024);       // d_ifgo tile, K-major
       constexpr uint64_t descB = smem_desc_base(8192, 1024);     // Wh chunk, N-major (64 units wide)
       const uint32_t idesc = instr_desc(p.fmt, 0, 1, RB, N);
@@ -1163,7 +1143,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
         }
       }
     }
-  } else {
+  } else if (warp >= FIRST_EPI) {
     // ---------------------------------------------------------------- epilogue: two warpgroups
     constexpr int NU = 8;                        // units per thread
     const int ew = warp - FIRST_EPI;
@@ -1179,10 +1159,16 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
     const T16* dout = reinterpret_cast<const T16*>(p.dout);
     T16* dg = reinterpret_cast<T16*>(p.d_ifgo);
     // where the accumulator's pieces go: this CTA's own receive slot, or the staging slot of CTA q
-    uint8_t* put = (q == (int)r ? recv + (size_t)r * XSLOT_BYTES : stage + (size_t)(q < (int)r ? q : q - 1) * XSLOT_BYTES) + lane * XROW_BYTES;
-    // piece 2k of a row lies at position k, piece 2k+1 at 8+k, both XORed with the row: conflict-free for the writers
-    // (32 rows, one piece) and for the readers (a row's even or odd pieces)
-    const uint8_t* get = recv + grow * XROW_BYTES + (((lane & 7) ^ (grow & 7)) << 4);
+    // (a slot is two halves of 32 rows x 32 units, one per warpgroup, so that every warp ships its own 4 KB)
+    uint8_t* put = (q == (int)r ? recv + (size_t)r * XSLOT_BYTES : stage + (size_t)(q < (int)r ? q : q - 1) * XSLOT_BYTES) + g * (XSLOT_BYTES / 2);
+    // a half's row is 128 bytes; piece k lies at k XOR row XOR half: conflict-free for the writers (32 rows, one piece)
+    // and for the readers (a row's even, then odd pieces of both halves)
+    // one tile in flight: this warp's d_ifgo rows on their way out, in the ring, which is idle until this CTA has counted the
+    // item in (behind the exchange buffers where those lie over the ring)
+    uint8_t* obuf = a_s + (p.alias ? 7 * XSLOT_BYTES : 0) + ew * 2048 + lane * 16;
+    const int half = (lane >> 2) & 1;
+    const uint8_t* get = recv + half * (XSLOT_BYTES / 2) + grow * XROW_BYTES;
+    const int get_x = (grow & 7) ^ half;
     // Bias gradient (replaces the reduction of fastlstm/lstm.py:497 and a separate pass over d_ifgo):
     // every thread adds the d_ifgo values it stores - as stored, i.e. rounded - to 32 fp32 sums of its
     // own (4 gates x 8 units) that live in the tensor-memory columns behind the accumulators, one
@@ -1326,7 +1312,8 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
               // the issuers' partial accumulators for 16 units: NACC loads, ONE wait
               uint32_t v[NACC][16];
 #pragma unroll
-              for (int xx = 0; xx < NACC; ++xx) tmem_ld_32x16(taddr + xx * N + h * 16, v[xx]);
+              for (int xx = 0; xx < NACC; ++xx)
+                if (xx < nacc) tmem_ld_32x16(taddr + xx * N + h * 16, v[xx]);
               tmem_ld_wait();
 #pragma unroll
               for (int c4 = 0; c4 < 4; ++c4) {
@@ -1338,8 +1325,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
                   if (NACC > 2 && nacc > 2) a0 += __uint_as_float(v[NACC - 1][4 * c4 + u]);
                   sum[u] = a0;
                 }
-                const int pc = g * 8 + h * 4 + c4;          // piece of the row
-                *reinterpret_cast<float4*>(put + ((((pc >> 1) ^ (lane & 7)) + 8 * (pc & 1)) << 4)) = make_float4(sum[0], sum[1], sum[2], sum[3]);
+                *reinterpret_cast<float4*>(put + lane * XROW_BYTES + (((h * 4 + c4) ^ (lane & 7) ^ g) << 4)) = make_float4(sum[0], sum[1], sum[2], sum[3]);
               }
             }
             tc_fence_before();
@@ -1348,12 +1334,8 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
             if (lane == 0) {
               mbar_arrive(&acc_empty[a]);
               if (q == (int)r) mbar_arrive(xchg);
-              else mbar_arrive(&staged[q]);
-              // one thread of the quarter's two warps ships it once both have staged their halves
-              // (bounded mbarrier wait, never a named barrier: a warp that gave up must not strand the rest)
-              if (g == 0 && q != (int)r && mbar_wait(&staged[q], x_ph, wc) && q_ok &&
-                  (!p.alias || mbar_wait_cluster(rdy, x_ph, wc)))       // aliased: every peer's ring is idle
-                dsmem_bulk_copy(mapa_shared(smem_u32(recv) + r * XSLOT_BYTES, q), put - lane * XROW_BYTES, XSLOT_BYTES,
+              else if (q_ok && (!p.alias || mbar_wait_cluster(rdy, x_ph, wc)))       // aliased: every peer's ring is idle
+                dsmem_bulk_copy(mapa_shared(smem_u32(recv) + r * XSLOT_BYTES + g * (XSLOT_BYTES / 2), q), put, XSLOT_BYTES / 2,
                                 mapa_shared(smem_u32(xchg), q));
             }
             __syncwarp();
@@ -1365,7 +1347,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
             for (int s = 0; s < 4; ++s)
 #pragma unroll
               for (int o = 0; o < 2; ++o) {
-                const float4 v = *reinterpret_cast<const float4*>(get + s * XSLOT_BYTES + o * 128);
+                const float4 v = *reinterpret_cast<const float4*>(get + s * XSLOT_BYTES + (((2 * (lane & 3) + o) ^ get_x) << 4));
                 dhc[4 * o] += v.x;
                 dhc[4 * o + 1] += v.y;
                 dhc[4 * o + 2] += v.z;
@@ -1443,29 +1425,38 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
                 qo[w] = pk2<T16>(r_[0][3], r_[1][3]);
               }
             }
-            if (row_ok) {
+            if constexpr (TI == 1) {
+              // one tile in flight: out through a TMA store (a box of 4 gates x 4 rows x 64 units a warp) that the warp
+              // sees completed after some 300 clocks; plain stores cost the release behind them 1.6 k
+              stg16(obuf, make_uint4(qi[0], qi[1], qi[2], qi[3]));
+              stg16(obuf + 512, make_uint4(qf[0], qf[1], qf[2], qf[3]));
+              stg16(obuf + 1024, make_uint4(qg[0], qg[1], qg[2], qg[3]));
+              stg16(obuf + 1536, make_uint4(qo[0], qo[1], qo[2], qo[3]));
+              fence_proxy_async_smem();
+            } else if (row_ok) {
               T16* dstp = dg + ((size_t)t * p.B + row) * H4 + unit0;
               stg16(dstp, make_uint4(qi[0], qi[1], qi[2], qi[3]));
               stg16(dstp + (size_t)H, make_uint4(qf[0], qf[1], qf[2], qf[3]));
               stg16(dstp + 2 * (size_t)H, make_uint4(qg[0], qg[1], qg[2], qg[3]));
               stg16(dstp + 3 * (size_t)H, make_uint4(qo[0], qo[1], qo[2], qo[3]));
             }
-            // publish d_ifgo[t] rows of this warp, then (after the release) fetch the next item's inputs
-            if (WRITER_FENCE) fence_proxy_async();
+            // publish d_ifgo[t] rows of this warp, then (after the release) fetch the next item's inputs: one arrival per
+            // CTA and item, by the publisher warp (interleaved tiles) or the last epilogue warp whose rows are stored
+            // (a warp can be at most four items ahead of another - the maths-only items that open a chunk - so four
+            // counters never mix items)
             __syncwarp();
-            // interleaved tiles: hand the item to the publisher warp.  One tile: arrival per warp, or
-            // (cta_publish) one per CTA and item - the last epilogue warp to get here publishes for all
-            // (a warp can be at most four items ahead of another - the maths-only items that open a
-            // chunk - so four counters never mix items)
             if (lane == 0) {
               if constexpr (PUBLISHER) {
-                mbar_arrive(&pub_bar[pub_it & 3]);      // the publisher warp releases for the CTA
+                mbar_arrive(&pub_bar[pub_it & 3]);
               } else {
-                const bool pub = !p.cta_publish ||
-                                 (smem_count_arrive(&pub_cnt[pub_it & 3]) & (ITEM_WARPS - 1)) == ITEM_WARPS - 1;
+                tma_store_4d(&tmD, obuf - lane * 16, ugc * 64, bt * RB + (int)r * 32 + ew * 4, 0, t);
+                tma_store_commit();
+                tma_store_wait<0>();
+                const bool pub = (smem_count_arrive(&pub_cnt[pub_it & 3]) & (ITEM_WARPS - 1)) == ITEM_WARPS - 1;
                 if (pub && !p.no_arrive) red_release_gpu_add(&p.flags[(size_t)t * p.nbt + bt], 1);
               }
             }
+            __syncwarp();
             ++pub_it;
             {
               int nj = j + 1, ns = st;
@@ -1594,7 +1585,8 @@ static int bwd_cta_capacity() {
 }
 
 template <int TI, typename T16>
-static int launch_bwd_t(const BwdPlan& pl, const CUtensorMap& tw, const CUtensorMap& tg, BwdParams& p, cudaStream_t st) {
+static int launch_bwd_t(const BwdPlan& pl, const CUtensorMap& tw, const CUtensorMap& tg, const CUtensorMap& td, BwdParams& p,
+                        cudaStream_t st) {
   auto kern = bwd_kernel<TI, T16>;
   BLSTM_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
   cudaLaunchConfig_t cfg = {};
@@ -1618,14 +1610,14 @@ static int launch_bwd_t(const BwdPlan& pl, const CUtensorMap& tw, const CUtensor
   int max_clusters = 0;
   BLSTM_CUDA_OK(cudaOccupancyMaxActiveClusters(&max_clusters, kern, &cfg));
   if (max_clusters * 4 < pl.grid) return BLSTM_E_NOT_CORESIDENT;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tw, tg, p);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tw, tg, td, p);
   if (cfg.numAttrs == 2 && (e == cudaErrorNotSupported || e == cudaErrorCooperativeLaunchTooLarge)) {
     // Only when the driver refuses the cooperative + cluster combination as such is the cooperative
     // attribute dropped (co-residency then rests on the occupancy check above); any other launch error
     // is reported as it is.
     (void)cudaGetLastError();
     cfg.numAttrs = 1;
-    e = cudaLaunchKernelEx(&cfg, kern, tw, tg, p);
+    e = cudaLaunchKernelEx(&cfg, kern, tw, tg, td, p);
   }
   BLSTM_CUDA_OK(e);
   count_launch();
@@ -1700,10 +1692,16 @@ int sm100_fwd_recurrence(const blstm_desc& d, void* ifgo, const void* Wh, void* 
     rc = encode_tensor_map(&th, out, 3, dims, str, box);
     if (rc) return rc;
   }
-  CUtensorMap tp = th;              // only read by the kernels that interleave tiles
-  if (pl.TI >= 2) {
+  CUtensorMap tp;
+  {
     const int NU = 4 * pl.UH / pl.epi_warps;
-    {  // ifgo [T,B,4H] as {unit, batch row, gate, t}: a box is one warp's 4 gates x 32 rows x NU units;
+    if (pl.TI == 1) {  // out [T+1,B,H] as {unit, batch row, t}: a box is one warp's 32 rows x NU units
+      uint64_t dims[3] = {(uint64_t)H, (uint64_t)B, (uint64_t)(T + 1)};
+      uint64_t str[2] = {(uint64_t)H * 2, (uint64_t)B * H * 2};
+      uint32_t box[3] = {(uint32_t)NU, 32, 1};
+      rc = encode_tensor_map(&tp, out, 3, dims, str, box, 2, 0);
+      if (rc) return rc;
+    } else {  // ifgo [T,B,4H] as {unit, batch row, gate, t}: a box is one warp's 4 gates x 32 rows x NU units;
        // the box's inner extent equals the swizzle span (32 bytes) or is a single 16-byte piece (none)
       uint64_t dims[4] = {(uint64_t)H, (uint64_t)B, 4, (uint64_t)T};
       uint64_t str[3] = {(uint64_t)4 * H * 2, (uint64_t)H * 2, (uint64_t)B * 4 * H * 2};
@@ -1727,12 +1725,7 @@ int sm100_fwd_recurrence(const blstm_desc& d, void* ifgo, const void* Wh, void* 
   p.fmt = d.dtype == BLSTM_BF16 ? 1 : 0;
   p.no_arrive = (d.flags & BLSTM_FLAG_TEST_NO_ARRIVE) ? 1 : 0;
   p.inference = (d.flags & BLSTM_FLAG_INFERENCE) ? 1 : 0;
-  // One arrival per CTA and item (the last epilogue warp to finish publishes for all; with interleaved
-  // tiles the publisher warp).  Measured 3-7 % faster than one arrival per warp from 64 arrivals per
-  // counter on (B=512 H=512: 1.43 -> 1.33 ms; H=1024: 4.06 -> 3.95 ms; H=2048: 9.4 -> 9.0 ms): the
-  // same-address reductions serialise in L2 and the counter completes with the slowest of them.
-  p.cta_publish = (pl.nh * pl.epi_warps >= 64 || pl.TI >= 2) ? 1 : 0;
-  p.flag_target = p.cta_publish ? pl.nh : pl.nh * pl.epi_warps;
+  p.flag_target = pl.nh;            // one arrival per CTA and item
   p.limit_ns = d.wait_limit_us > 0 ? (unsigned long long)d.wait_limit_us * 1000ull : kDefaultWaitNs;
   p.ctl = reinterpret_cast<Control*>(ws);
   p.flags = reinterpret_cast<int*>(static_cast<char*>(ws) + pl.off_flags);
@@ -1745,7 +1738,6 @@ int sm100_fwd_recurrence(const blstm_desc& d, void* ifgo, const void* Wh, void* 
   BLSTM_FWD_CASE(16, 1)
   BLSTM_FWD_CASE(16, 2)
   BLSTM_FWD_CASE(16, 4)
-  BLSTM_FWD_CASE(32, 1)
   BLSTM_FWD_CASE(32, 2)
   BLSTM_FWD_CASE(32, 4)
 #undef BLSTM_FWD_CASE
@@ -1780,6 +1772,14 @@ int sm100_bwd_recurrence(const blstm_desc& d, const void* dout, const void* dh_n
     rc = encode_tensor_map(&tg, d_ifgo, 3, dims, str, box);
     if (rc) return rc;
   }
+  CUtensorMap td;
+  {  // d_ifgo [T,B,4H] as {unit, batch row, gate, t}: a box is one warp's 4 gates x 4 rows x 64 units
+    uint64_t dims[4] = {(uint64_t)H, (uint64_t)B, 4, (uint64_t)T};
+    uint64_t str[3] = {(uint64_t)4 * H * 2, (uint64_t)H * 2, (uint64_t)B * 4 * H * 2};
+    uint32_t box[4] = {64, 4, 4, 1};
+    rc = encode_tensor_map(&td, d_ifgo, 4, dims, str, box, 2, 0);
+    if (rc) return rc;
+  }
   BwdParams p;
   p.T = T; p.B = B; p.H = H;
   p.nbt = pl.nbt; p.nug = pl.nug; p.nb_par = pl.nb_par; p.ntl = pl.ntl; p.stages = pl.stages; p.ni = pl.ni;
@@ -1788,11 +1788,7 @@ int sm100_bwd_recurrence(const blstm_desc& d, const void* dout, const void* dh_n
   p.alias = pl.alias;
   p.fmt = d.dtype == BLSTM_BF16 ? 1 : 0;
   p.no_arrive = (d.flags & BLSTM_FLAG_TEST_NO_ARRIVE) ? 1 : 0;
-  // One arrival per epilogue warp up to about a thousand per counter, one per CTA beyond that and
-  // whenever tiles are interleaved.  (Unlike in the forward kernel, per-CTA arrivals measured 2-5 %
-  // SLOWER here below that size: eight warps elect the publisher instead of four.)
-  p.cta_publish = ((H / 16) * 8 >= 1024 || pl.TI >= 2) ? 1 : 0;
-  p.flag_target = p.cta_publish ? H / 16 : (H / 16) * 8;
+  p.flag_target = H / 16;           // one arrival per CTA and item
   p.limit_ns = d.wait_limit_us > 0 ? (unsigned long long)d.wait_limit_us * 1000ull : kDefaultWaitNs;
   p.ctl = reinterpret_cast<Control*>(ws);
   p.flags = reinterpret_cast<int*>(static_cast<char*>(ws) + pl.off_flags);
@@ -1800,9 +1796,9 @@ int sm100_bwd_recurrence(const blstm_desc& d, const void* dout, const void* dh_n
   p.d_ifgo = d_ifgo; p.dh0 = dh0; p.dc0 = dc0;
   p.db_part = db ? reinterpret_cast<float*>(static_cast<char*>(ws) + pl.off_db) : nullptr;
   const bool bf = d.dtype == BLSTM_BF16;
-  if (pl.TI == 1)      rc = bf ? launch_bwd_t<1, __nv_bfloat16>(pl, tw, tg, p, st) : launch_bwd_t<1, __half>(pl, tw, tg, p, st);
-  else if (pl.TI == 2) rc = bf ? launch_bwd_t<2, __nv_bfloat16>(pl, tw, tg, p, st) : launch_bwd_t<2, __half>(pl, tw, tg, p, st);
-  else                 rc = bf ? launch_bwd_t<4, __nv_bfloat16>(pl, tw, tg, p, st) : launch_bwd_t<4, __half>(pl, tw, tg, p, st);
+  if (pl.TI == 1)      rc = bf ? launch_bwd_t<1, __nv_bfloat16>(pl, tw, tg, td, p, st) : launch_bwd_t<1, __half>(pl, tw, tg, td, p, st);
+  else if (pl.TI == 2) rc = bf ? launch_bwd_t<2, __nv_bfloat16>(pl, tw, tg, td, p, st) : launch_bwd_t<2, __half>(pl, tw, tg, td, p, st);
+  else                 rc = bf ? launch_bwd_t<4, __nv_bfloat16>(pl, tw, tg, td, p, st) : launch_bwd_t<4, __half>(pl, tw, tg, td, p, st);
   if (rc) return rc;
   if (db) return reduce_db(p.db_part, pl.nb_par * 32, 4 * H, db, st);
   return BLSTM_OK;
