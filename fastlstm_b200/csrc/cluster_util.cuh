@@ -2,6 +2,8 @@
 // a call, register shares.
 #pragma once
 
+#include <cstdlib>
+
 #include "sm100_common.cuh"
 
 namespace blstm {
@@ -60,6 +62,44 @@ inline int launch_clusters(Kern kern, int grid, int threads, size_t smem, int nc
   cfg.attrs = &attr;
   cfg.numAttrs = nc > 1 ? 1 : 0;
   BLSTM_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, args...));
+  count_launch();
+  return BLSTM_OK;
+}
+
+// Launches `kern` on clusters of nc CTAs that wait for one another across clusters: the whole grid has to be resident at
+// once.  FASTLSTM_B200_NO_COOP=1 drops the cooperative attribute (profilers that replay kernels refuse a cooperative
+// cluster launch); co-residency then rests on the occupancy check alone.
+template <typename Kern, typename... Args>
+inline int launch_coresident(Kern kern, int grid, int threads, size_t smem, int nc, cudaStream_t st, const Args&... args) {
+  BLSTM_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attrs[2];
+  attrs[0].id = cudaLaunchAttributeClusterDimension;
+  attrs[0].val.clusterDim.x = nc;
+  attrs[0].val.clusterDim.y = 1;
+  attrs[0].val.clusterDim.z = 1;
+  attrs[1].id = cudaLaunchAttributeCooperative;
+  attrs[1].val.cooperative = 1;
+  cfg.attrs = attrs;
+  static const bool no_coop = [] { const char* e = getenv("FASTLSTM_B200_NO_COOP"); return e && e[0] == '1'; }();
+  cfg.numAttrs = no_coop ? 1 : 2;
+  int max_clusters = 0;
+  BLSTM_CUDA_OK(cudaOccupancyMaxActiveClusters(&max_clusters, kern, &cfg));
+  if (max_clusters * nc < grid) return BLSTM_E_NOT_CORESIDENT;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, args...);
+  if (cfg.numAttrs == 2 && (e == cudaErrorNotSupported || e == cudaErrorCooperativeLaunchTooLarge)) {
+    // Only when the driver refuses the cooperative + cluster combination as such is the cooperative
+    // attribute dropped (co-residency then rests on the occupancy check above); any other launch error
+    // is reported as it is.
+    (void)cudaGetLastError();
+    cfg.numAttrs = 1;
+    e = cudaLaunchKernelEx(&cfg, kern, args...);
+  }
+  BLSTM_CUDA_OK(e);
   count_launch();
   return BLSTM_OK;
 }

@@ -30,6 +30,8 @@
 #include "sm100_common.cuh"
 #include "sm100_rec_util.cuh"
 #include "sm100_small.cuh"
+#include "sm100_resident.cuh"
+#include "cluster_util.cuh"
 
 namespace blstm {
 namespace sm100 {
@@ -1520,7 +1522,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
   cluster_sync_all();   // no CTA leaves while a peer may still write into its shared memory
 }
 
-// Column sums of d_ifgo [rows, cols] (16-bit) over DB_PARTS interleaved row groups -> part[DB_PARTS][cols].
+// Column sums of d_ifgo [rows, cols] (16-bit) over gridDim.y interleaved row groups -> part[gridDim.y][cols].
 // HBM-bound (the whole d_ifgo is read once): a thread owns 8 adjacent columns (one 16-byte load per
 // row, a warp covers 512 contiguous bytes) and keeps 8 row loads in flight.
 template <typename T16>
@@ -1528,14 +1530,15 @@ __global__ void __launch_bounds__(128) colsum_kernel(const T16* __restrict__ g, 
   const int col = (blockIdx.x * 128 + threadIdx.x) * 8;
   if (col >= cols) return;
   float s[8];
+  const int DB = gridDim.y;
 #pragma unroll
   for (int u = 0; u < 8; ++u) s[u] = 0.f;
   const T16* src = g + col;
   int rr = blockIdx.y;
-  for (; rr + 7 * DB_PARTS < rows; rr += 8 * DB_PARTS) {
+  for (; rr + 7 * DB < rows; rr += 8 * DB) {
     uint4 v[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = ldg16(src + (size_t)(rr + i * DB_PARTS) * cols);
+    for (int i = 0; i < 8; ++i) v[i] = ldg16(src + (size_t)(rr + i * DB) * cols);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const uint32_t w[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
@@ -1543,7 +1546,7 @@ __global__ void __launch_bounds__(128) colsum_kernel(const T16* __restrict__ g, 
       for (int u = 0; u < 4; ++u) { const float2 f = cvt2<T16>(w[u]); s[2 * u] += f.x; s[2 * u + 1] += f.y; }
     }
   }
-  for (; rr < rows; rr += DB_PARTS) {
+  for (; rr < rows; rr += DB) {
     const uint4 v = ldg16(src + (size_t)rr * cols);
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
@@ -1587,41 +1590,7 @@ static int bwd_cta_capacity() {
 template <int TI, typename T16>
 static int launch_bwd_t(const BwdPlan& pl, const CUtensorMap& tw, const CUtensorMap& tg, const CUtensorMap& td, BwdParams& p,
                         cudaStream_t st) {
-  auto kern = bwd_kernel<TI, T16>;
-  BLSTM_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(pl.grid);
-  cfg.blockDim = dim3(pl.threads);
-  cfg.dynamicSmemBytes = pl.smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attrs[2];
-  attrs[0].id = cudaLaunchAttributeClusterDimension;
-  attrs[0].val.clusterDim.x = 4;
-  attrs[0].val.clusterDim.y = 1;
-  attrs[0].val.clusterDim.z = 1;
-  attrs[1].id = cudaLaunchAttributeCooperative;
-  attrs[1].val.cooperative = 1;
-  cfg.attrs = attrs;
-  // FASTLSTM_B200_NO_COOP=1 drops the cooperative attribute (profilers that replay kernels refuse
-  // a cooperative cluster launch); co-residency then rests on the occupancy check below alone.
-  static const bool no_coop = [] { const char* e = getenv("FASTLSTM_B200_NO_COOP"); return e && e[0] == '1'; }();
-  cfg.numAttrs = no_coop ? 1 : 2;
-  // every CTA spins on its peers: the whole grid has to be resident at once
-  int max_clusters = 0;
-  BLSTM_CUDA_OK(cudaOccupancyMaxActiveClusters(&max_clusters, kern, &cfg));
-  if (max_clusters * 4 < pl.grid) return BLSTM_E_NOT_CORESIDENT;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tw, tg, td, p);
-  if (cfg.numAttrs == 2 && (e == cudaErrorNotSupported || e == cudaErrorCooperativeLaunchTooLarge)) {
-    // Only when the driver refuses the cooperative + cluster combination as such is the cooperative
-    // attribute dropped (co-residency then rests on the occupancy check above); any other launch error
-    // is reported as it is.
-    (void)cudaGetLastError();
-    cfg.numAttrs = 1;
-    e = cudaLaunchKernelEx(&cfg, kern, tw, tg, td, p);
-  }
-  BLSTM_CUDA_OK(e);
-  count_launch();
-  return BLSTM_OK;
+  return launch_coresident(bwd_kernel<TI, T16>, pl.grid, pl.threads, pl.smem, 4, st, tw, tg, td, p);
 }
 
 }  // namespace sm100
@@ -1629,23 +1598,26 @@ static int launch_bwd_t(const BwdPlan& pl, const CUtensorMap& tw, const CUtensor
 using namespace sm100;
 
 bool sm100_recurrence_supported(const blstm_desc& d, int phase) {
-  if (small_plan(d, phase).ok) return true;
+  if (small_plan(d, phase).ok || resident_plan(d, phase).ok) return true;
   return phase == BLSTM_PHASE_BWD ? make_bwd_plan(d).ok : make_plan(d, phase).ok;
 }
 size_t sm100_recurrence_workspace(const blstm_desc& d, int phase) {
   const SmallPlan sp = small_plan(d, phase);
   if (sp.ok) return small_workspace(d, sp, phase);
+  if (const ResPlan rp = resident_plan(d, phase); rp.ok) return rp.ws_bytes;
   return phase == BLSTM_PHASE_BWD ? make_bwd_plan(d).ws_bytes : make_plan(d, phase).ws_bytes;
 }
 
 size_t sm100_recurrence_control(const blstm_desc& d, int phase) {
   if (small_plan(d, phase).ok) return sizeof(Control);
+  if (const ResPlan rp = resident_plan(d, phase); rp.ok) return rp.off_db;
   return phase == BLSTM_PHASE_BWD ? make_bwd_plan(d).off_db : make_plan(d, phase).ws_bytes;
 }
 
 int sm100_plan_detail(const blstm_desc& d, int phase, char* buf, size_t n) {
   const SmallPlan sp = small_plan(d, phase);
   if (sp.ok) return small_plan_detail(d, sp, phase, buf, n);
+  if (const ResPlan rp = resident_plan(d, phase); rp.ok) return resident_plan_detail(rp, phase, buf, n);
   if (phase == BLSTM_PHASE_BWD) {
     const BwdPlan p = make_bwd_plan(d);
     if (!p.ok) return 0;
@@ -1669,6 +1641,10 @@ int sm100_fwd_recurrence(const blstm_desc& d, void* ifgo, const void* Wh, void* 
                          size_t ws_bytes, cudaStream_t st) {
   const SmallPlan sp = small_plan(d, BLSTM_PHASE_FWD);
   if (sp.ok) return small_fwd_recurrence(d, sp, ifgo, Wh, out, cell, ws, st);
+  if (const ResPlan rp = resident_plan(d, BLSTM_PHASE_FWD); rp.ok) {
+    if (ws_bytes < rp.ws_bytes) return BLSTM_E_WORKSPACE;
+    return resident_fwd_recurrence(d, rp, ifgo, Wh, out, cell, ws, st);
+  }
   const RecPlan pl = make_plan(d, BLSTM_PHASE_FWD);
   if (!pl.ok) return BLSTM_E_UNSUPPORTED;
   if (ws_bytes < pl.ws_bytes) return BLSTM_E_WORKSPACE;
@@ -1749,6 +1725,10 @@ int sm100_bwd_recurrence(const blstm_desc& d, const void* dout, const void* dh_n
                          float* db, void* ws, size_t ws_bytes, cudaStream_t st) {
   const SmallPlan sp = small_plan(d, BLSTM_PHASE_BWD);
   if (sp.ok) return small_bwd_recurrence(d, sp, dout, dh_n, dc_n, ifgo, cell, Wh, d_ifgo, dh0, dc0, db, ws, st);
+  if (const ResPlan rp = resident_plan(d, BLSTM_PHASE_BWD); rp.ok) {
+    if (ws_bytes < rp.ws_bytes) return BLSTM_E_WORKSPACE;
+    return resident_bwd_recurrence(d, rp, dout, dh_n, dc_n, ifgo, cell, Wh, d_ifgo, dh0, dc0, db, ws, st);
+  }
   const BwdPlan pl = make_bwd_plan(d);
   if (!pl.ok) return BLSTM_E_UNSUPPORTED;
   if (ws_bytes < pl.ws_bytes) return BLSTM_E_WORKSPACE;
@@ -1805,17 +1785,17 @@ int sm100_bwd_recurrence(const blstm_desc& d, const void* dout, const void* dh_n
 }
 
 int sm100_bias_grad(const blstm_desc& d, const void* d_ifgo, float* db, void* ws, size_t ws_bytes, cudaStream_t st) {
-  const BwdPlan pl = make_bwd_plan(d);
-  if (!pl.ok) return BLSTM_E_UNSUPPORTED;
-  if (ws_bytes < pl.ws_bytes) return BLSTM_E_WORKSPACE;
-  float* part = reinterpret_cast<float*>(static_cast<char*>(ws) + pl.off_db);
+  // as many partial rows as the backward recurrence's workspace has room for, behind the control block
   const int rows = d.seq_len * d.batch, cols = 4 * d.hidden_size;
-  dim3 grid(cdiv(cols, 1024), DB_PARTS);
+  const int parts = (int)std::min<size_t>(DB_PARTS, (ws_bytes - sizeof(Control)) / (cols * sizeof(float)));
+  if (parts < 1) return BLSTM_E_WORKSPACE;
+  float* part = reinterpret_cast<float*>(static_cast<char*>(ws) + sizeof(Control));
+  dim3 grid(cdiv(cols, 1024), parts);
   if (d.dtype == BLSTM_BF16) colsum_kernel<__nv_bfloat16><<<grid, 128, 0, st>>>((const __nv_bfloat16*)d_ifgo, rows, cols, part);
   else                       colsum_kernel<__half><<<grid, 128, 0, st>>>((const __half*)d_ifgo, rows, cols, part);
   BLSTM_CUDA_OK(cudaGetLastError());
   count_launch();
-  return reduce_db(part, DB_PARTS, cols, db, st);
+  return reduce_db(part, parts, cols, db, st);
 }
 
 }  // namespace blstm

@@ -1,0 +1,31 @@
+// Plans and launchers of the recurrences whose weights stay on the chip (16-bit, large hidden sizes).
+#pragma once
+#include "common.cuh"
+
+namespace blstm {
+namespace sm100 {
+
+constexpr int RES_MIN_H = 576;
+
+struct ResPlan {
+  bool ok;
+  int ks, own, mt, ng;      // CTAs per cluster (parts of K); of these, owners of batch rows; M tiles; groups of rows
+  int rows, N;              // batch rows per group; N of the MMAs
+  int kc_total, kcm, nt;    // chunks of K; most of a CTA; of these in tensor memory
+  int ni;                   // MMA issuers
+  int grid;
+  size_t smem, off_db, ws_bytes;
+};
+
+ResPlan resident_plan(const blstm_desc& d, int phase);
+
+}  // namespace sm100
+
+int resident_fwd_recurrence(const blstm_desc& d, const sm100::ResPlan& pl, void* ifgo, const void* Wh, void* out, void* cell, void* ws,
+                            cudaStream_t st);
+int resident_bwd_recurrence(const blstm_desc& d, const sm100::ResPlan& pl, const void* dout, const void* dh_n, const void* dc_n,
+                            const void* ifgo, const void* cell, const void* Wh, void* d_ifgo, void* dh0, void* dc0, float* db,
+                            void* ws, cudaStream_t st);
+int resident_plan_detail(const sm100::ResPlan& pl, int phase, char* buf, size_t n);
+
+}  // namespace blstm

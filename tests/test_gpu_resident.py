@@ -1,0 +1,72 @@
+"""Recurrences whose weights stay on the chip (large hidden sizes) against the fp32 step-by-step evaluation."""
+import pytest
+import torch
+
+from fastlstm_b200 import _lib
+from test_gpu_recurrence import TD, _bwd, _cmp, _desc, _fwd, _torch_bwd, _torch_fwd
+
+pytestmark = pytest.mark.gpu
+
+# N = 16, 32, 64; one row, ragged rows and groups; half an M tile in backward (H % 128 == 64); K split over 1 and 2 (forward),
+# 4, 5 and 6 (backward, one issuer) CTAs; weights that fit tensor memory and weights that do not
+SHAPES = [(4, 1, 768), (3, 65, 704), (5, 100, 768), (3, 250, 768), (4, 256, 1024), (2, 130, 960), (3, 33, 1088), (3, 64, 1536),
+          (4, 32, 2048), (3, 17, 1984), (2, 9, 2048)]
+
+
+@pytest.mark.parametrize("dtype", ["fp16", "bf16"])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_resident_recurrences_against_fp32_maths(dtype, shape):
+    lib = _lib.load()
+    T, B, H = shape
+    dt = TD[dtype]
+    g = torch.Generator(device="cuda").manual_seed(B + H)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    d = _desc(dtype, T, B, H)
+    Wh = ((torch.rand(4 * H, H, generator=g, device="cuda") * 2 - 1) / H ** 0.5).to(dt)
+    pre, h0, c0 = rnd(T, B, 4 * H).to(dt), (rnd(B, H) * 0.3).to(dt), rnd(B, H).to(dt)
+    ifgo, out, cell = _fwd(lib, d, pre, Wh, h0, c0)
+    want = _torch_fwd(pre, Wh, h0, c0)
+    tol = 8e-3 if dtype == "bf16" else 2e-3
+    _cmp("ifgo", ifgo, want[0], 4 * tol)
+    _cmp("out", out[1:], want[1], tol)
+    _cmp("cell", cell[1:], want[2], 2 * tol)
+    again = _fwd(lib, d, pre, Wh, h0, c0)
+    assert torch.equal(out, again[1]) and torch.equal(ifgo, again[0])
+    ifgo, cell, dout = rnd(T, B, 4 * H).to(dt), (rnd(T + 1, B, H) * 0.7).to(dt), rnd(T, B, H).to(dt)
+    dh, dc = rnd(B, H).to(dt), rnd(B, H).to(dt)
+    got = _bwd(lib, d, dout, dh, dc, ifgo, cell, Wh)
+    for name, a, b in zip(("d_ifgo", "dh0", "dc0", "db"), got, _torch_bwd(dout, dh, dc, ifgo, cell, Wh)):
+        _cmp(name, a, b, (1e-2 if dtype == "bf16" else 3e-3) * float(b.abs().max()))
+    assert all(torch.equal(a, b) for a, b in zip(got, _bwd(lib, d, dout, dh, dc, ifgo, cell, Wh)))
+
+
+@pytest.mark.parametrize("phase", [0, 1])
+@pytest.mark.parametrize("B,H", [(32, 1024), (32, 1536)])
+def test_resident_recurrences_give_up_with_a_status_when_nothing_arrives(phase, B, H):
+    lib = _lib.load()
+    T = 3
+    z = lambda *s: torch.zeros(*s, device="cuda", dtype=torch.bfloat16)
+    d = _lib.Desc(_lib.BF16, T, B, H, H, _lib.FLAG_TEST_NO_ARRIVE, 20000, 0)
+    n = lib.blstm_workspace_bytes(d, phase)
+    ws, s = torch.zeros(n, dtype=torch.uint8, device="cuda"), torch.cuda.current_stream().cuda_stream
+    ifgo, Wh, out, cell, c = z(T, B, 4 * H), z(4 * H, H), z(T + 1, B, H), z(T + 1, B, H), z(2, B, H)
+    if phase == 0:
+        rc = lib.blstm_fwd_recurrence(d, ifgo.data_ptr(), Wh.data_ptr(), out.data_ptr(), cell.data_ptr(), ws.data_ptr(), n, s)
+    else:
+        rc = lib.blstm_bwd_recurrence(d, out.data_ptr(), None, None, ifgo.data_ptr(), cell.data_ptr(), Wh.data_ptr(), z(T, B, 4 * H).data_ptr(),
+                                      c[0].data_ptr(), c[1].data_ptr(), None, ws.data_ptr(), n, s)
+    assert rc == 0
+    assert lib.blstm_read_status(ws.data_ptr(), None, s) == _lib.E_WAIT_TIMEOUT
+
+
+@pytest.mark.parametrize("B,H", [(16, 64), (40, 512), (64, 1024), (200, 512)])
+def test_bias_grad_for_every_backward_plan(B, H):
+    lib = _lib.load()
+    T = 7
+    d = _desc("bf16", T, B, H)
+    dg, db = torch.randn(T, B, 4 * H, device="cuda").bfloat16(), torch.empty(4 * H, device="cuda")
+    n = lib.blstm_workspace_bytes(d, _lib.PHASE_BWD)
+    ws = torch.zeros(n, dtype=torch.uint8, device="cuda")
+    _lib.check(lib.blstm_bias_grad(d, dg.data_ptr(), db.data_ptr(), ws.data_ptr(), n, torch.cuda.current_stream().cuda_stream))
+    want = dg.double().sum((0, 1))
+    assert float((db.double() - want).abs().max()) <= 1e-4 * float(want.abs().max())
