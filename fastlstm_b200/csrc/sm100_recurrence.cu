@@ -116,10 +116,9 @@ static RecPlan make_plan(const blstm_desc& d, int phase) {
   // (9 warps); otherwise two issuers, eight epilogue warps and, for interleaved tiles, the publisher
   // (interleaved 32-unit slices: N = 128 runs the tensor pipe at full rate from ONE issuing thread, and a
   // single accumulator per item leaves tensor-memory columns for the cell rows of four tiles)
-  // (streamed weights double the bytes of a chunk: a third issuer)
-  const int n_issuers = UH == 32 ? 1 : (p.TI == 1 && (size_t)p.N * H * 2 > 128 * 1024) ? 3 : 2;
+  const int n_issuers = UH == 32 ? 1 : 2;
   const int n_publisher = p.TI >= 2 ? 1 : 0;
-  p.threads = 32 * (1 + (UH == 32 ? 1 : p.TI == 1 ? 3 : 2) + n_publisher + p.epi_warps);   // producer + MMA issuers [+ publisher] + epilogue
+  p.threads = 32 * (1 + n_issuers + n_publisher + p.epi_warps);   // producer + MMA issuers [+ publisher] + epilogue
   // Wh slice resident in shared memory when it fits next to a useful ring; otherwise (H > 1024) it is
   // streamed through the ring with h, chunk by chunk, every step (it stays in L2).  A single batch tile
   // of fewer than 128 rows only stages its own rows (the MMA's rows past them read whatever follows:
@@ -214,7 +213,7 @@ struct ItemCursor {
 // warps - at most 12 (3 per SM sub-partition), which leaves 168 registers per thread; a 13th would cap
 // them at 128.  The epilogue must not spill.
 template <int UH, int TI, typename T16>
-__global__ void __launch_bounds__(32 * (UH == 16 ? 12 : 11), 1)
+__global__ void __launch_bounds__(32 * (UH == 16 && TI >= 2 ? 12 : 11), 1)
 fwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmH,
            const __grid_constant__ CUtensorMap tmP, const FwdParams p) {
   constexpr int N = 4 * UH;
@@ -267,7 +266,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
   // stalls its thread for a memory round trip, so a PUBLISHER warp does the releasing (and the proxy
   // fence of the hand-off): the epilogue warps only arrive on a CTA-local barrier after storing h.
   constexpr bool PUBLISHER = (TI >= 2);
-  constexpr int NACC = UH == 32 ? 1 : TI == 1 ? 3 : 2;   // issuer warps / partial accumulators
+  constexpr int NACC = UH == 32 ? 1 : 2;   // issuer warps / partial accumulators
   constexpr int FIRST_EPI = 1 + NACC + (PUBLISHER ? 1 : 0);   // first epilogue warp
   // Columns per item buffer (NACC * N <= 256).  Interleaved tiles pack the two buffers into the first
   // 256 columns and keep the tiles' cell rows (fp32, a column per unit) in the columns behind them.
@@ -285,7 +284,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
     mbar_init(w_full, 1);
     *dead = 0;
     for (int i = 0; i < 4; ++i) pub_cnt[i] = 0;
-    for (int i = 0; i < 4; ++i) mbar_init(&pub_bar[i], TI == 1 ? 1 : EW);
+    for (int i = 0; i < 4; ++i) mbar_init(&pub_bar[i], EW);
     for (int i = 0; i < 16; ++i) mbar_init(&pre_full[i], 1);
     fence_mbar_init();
     // (stage s is first used by chunk s; with streamed weights there are more chunks than stages)
@@ -676,8 +675,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
           if (!mbar_wait(&acc_full[a], a_ph, wc)) { ok = false; break; }
           tc_fence_after();
           const uint32_t taddr = tmem_base + a * ACC_STRIDE + (uint32_t(q * 32) << 16) + ug * NU;
-          // accumulator read-out (the issuers' partial sums, GG gates per wait: at most 48 values in flight), gate maths, h store; the final pre-activations are saved after the release
-          constexpr int GG = 2;
+          // accumulator read-out (the issuers' partial sums, GG gates per wait: 64 values in flight), gate maths, h store; the final pre-activations are saved after the release
+          constexpr int GG = 4;
           const size_t o1 = ((size_t)(t + 1) * p.B + row) * H + unit0;
           T16* gdst = ifgo + ((size_t)t * p.B + row) * H4 + unit0;
           float pa[4][NU];
@@ -687,8 +686,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
 #pragma unroll
             for (int g = 0; g < GG; ++g)
 #pragma unroll
-              for (int x = 0; x < NACC; ++x)
-                if (x < nacc) tmem_ld_cols<NU>(taddr + x * N + (g0 + g) * UH, v[g][x]);
+              for (int x = 0; x < NACC; ++x) tmem_ld_cols<NU>(taddr + x * N + (g0 + g) * UH, v[g][x]);
             tmem_ld_wait();
 #pragma unroll
             for (int g = 0; g < GG; ++g)
@@ -736,8 +734,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
             tma_store_commit();
             tma_store_wait<0>();
             if ((smem_count_arrive(&pub_cnt[it & 3]) & (EW - 1)) == EW - 1) {
-              if (!p.no_arrive) red_release_gpu_add(&p.flags[(size_t)(t + 1) * p.nbt + bt], 1);
-              mbar_arrive(&pub_bar[it & 3]);
+              if (!p.no_arrive) red_relaxed_gpu_add(&p.flags[(size_t)(t + 1) * p.nbt + bt], 1);
             }
           }
           __syncwarp();
@@ -760,9 +757,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
             }
           }
           // off the critical path: final pre-activations and c[t+1], saved for backward (inference: only the last cell
-          // state is needed, as c_n) - once the CTA has counted the item in, because the release waits for whatever
-          // stores of the SM are under way (H=1024: 4.2 k clocks instead of 1.3 k)
-          if (!mbar_wait(&pub_bar[it & 3], (uint32_t)((it - 1) >> 2) & 1u, wc)) { ok = false; break; }
+          // state is needed, as c_n)
           if (row_ok && (!p.inference || t == p.T - 1)) {
 #pragma unroll
             for (int v = 0; v < NV; ++v) store8<T16>(cell + o1 + 8 * v, &c[j][8 * v]);
@@ -875,9 +870,9 @@ static BwdPlan make_bwd_plan(const blstm_desc& d) {
     p.TI = 1;                                               // not enough room to interleave tiles
   size_t wres = (size_t)p.kr * 8192;
   size_t fixed = 1024 + wres + p.recv_bytes + 1024 + tail_pad;  // 1024: barriers and counters behind the ring
-  // warps: 1 producer + 3 MMA issuers (or 2 + a publisher when tiles are interleaved) + 2 epilogue warpgroups = 12
+  // warps: 1 producer + 2 MMA issuers + a publisher (idle unless tiles are interleaved) + 2 epilogue warpgroups = 12
   // (3 per SM sub-partition, 168 registers each); a 13th warp would cap every thread at 128 registers.
-  const int n_issuers = p.TI == 1 && p.ws ? 3 : 2;        // (streamed weights double the bytes of a chunk)
+  const int n_issuers = 2;
   p.threads = 32 * 12;
   if (!pick_ring(fixed, p.stage_bytes, n_issuers, H / RK, &p.stages, &p.ni)) return p;
   // One tile in flight and a shallow ring (H = 768, 1024: the resident weights leave four stages, or two):
@@ -946,7 +941,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
   // item stalls its thread for a memory round trip: there a thread of its own does the releasing
   // (the epilogue warps only arrive on a CTA-local barrier after their stores), which costs one issuer.
   constexpr bool PUBLISHER = (TI >= 2);
-  constexpr int N = 64, NACC = PUBLISHER ? 2 : 3, ACC_STRIDE = 256;   // NACC: MMA issuer warps
+  constexpr int N = 64, NACC = 2, ACC_STRIDE = 256;   // NACC: MMA issuer warps
   constexpr int FIRST_EPI = 4;
   constexpr int ITEM_WARPS = 8;                   // epilogue warps, all working on every item
   extern __shared__ uint8_t smem_raw[];
@@ -1314,8 +1309,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
               // the issuers' partial accumulators for 16 units: NACC loads, ONE wait
               uint32_t v[NACC][16];
 #pragma unroll
-              for (int xx = 0; xx < NACC; ++xx)
-                if (xx < nacc) tmem_ld_32x16(taddr + xx * N + h * 16, v[xx]);
+              for (int xx = 0; xx < NACC; ++xx) tmem_ld_32x16(taddr + xx * N + h * 16, v[xx]);
               tmem_ld_wait();
 #pragma unroll
               for (int c4 = 0; c4 < 4; ++c4) {
@@ -1324,7 +1318,6 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
                 for (int u = 0; u < 4; ++u) {
                   float a0 = __uint_as_float(v[0][4 * c4 + u]);
                   if (nacc > 1) a0 += __uint_as_float(v[1][4 * c4 + u]);
-                  if (NACC > 2 && nacc > 2) a0 += __uint_as_float(v[NACC - 1][4 * c4 + u]);
                   sum[u] = a0;
                 }
                 *reinterpret_cast<float4*>(put + lane * XROW_BYTES + (((h * 4 + c4) ^ (lane & 7) ^ g) << 4)) = make_float4(sum[0], sum[1], sum[2], sum[3]);
@@ -1455,7 +1448,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
                 tma_store_commit();
                 tma_store_wait<0>();
                 const bool pub = (smem_count_arrive(&pub_cnt[pub_it & 3]) & (ITEM_WARPS - 1)) == ITEM_WARPS - 1;
-                if (pub && !p.no_arrive) red_release_gpu_add(&p.flags[(size_t)t * p.nbt + bt], 1);
+                if (pub && !p.no_arrive) red_relaxed_gpu_add(&p.flags[(size_t)t * p.nbt + bt], 1);
               }
             }
             __syncwarp();

@@ -12,8 +12,9 @@
 // owner and step on the group's counter, and the whole K slice of the next step is fetched at once (no ring).
 // Batch rows are divided over groups of CTAs that know nothing of each other.
 //
-// us per step, the recurrences with the batch on the M side -> these (B200): forward B=32 H=2048 7.9 -> 4.7, B=256 H=1024
-// 7.2 -> 6.2, B=128 H=1024 4.2, B=256 H=768 6.7 -> 4.7; backward B=32 H=2048 10.0 -> 7.4, B=32 H=1536 4.8, B=128 H=1024 5.1.
+// us per step, the recurrences with the batch on the M side -> these (B200): forward B=32 H=2048 7.9 -> 3.9, B=256 H=1024
+// 7.2 -> 4.9, B=128 H=1024 3.7, B=256 H=768 6.7 -> 4.2; backward B=32 H=2048 10.0 -> 6.6, B=256 H=1024 7.6 -> 5.6, B=256 H=768
+// 6.8 -> 5.0, B=32 H=1536 4.2.
 // Bound by the chain of a step: hand-off through L2, fetch of N rows, 64 MMAs of some 50 clocks, exchange, gate maths.
 #include <algorithm>
 #include <cstdio>
@@ -105,8 +106,7 @@ resident_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
   uint64_t* w_full = full + RES_MAX_KC;
   uint64_t* acc_full = w_full + 1;
   uint64_t* xchg = acc_full + 1;
-  uint64_t* pub_bar = xchg + 1;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pub_bar + 1);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(xchg + 1);
   volatile int* dead = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* pub_cnt = const_cast<int*>(dead) + 1;
 
@@ -122,7 +122,6 @@ resident_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
     mbar_init(w_full, 1);
     mbar_init(acc_full, NI);
     mbar_init(xchg, 1 + EW);
-    mbar_init(pub_bar, 1);
     *dead = 0;
     *pub_cnt = 0;
     fence_mbar_init();
@@ -249,14 +248,21 @@ resident_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
     const uint32_t tx = owner ? (uint32_t)(KS - 1) * 4 * BLK : 0u;
     bool ok = true;
 
+    // where this warp's half of the accumulator's columns goes: RW_ rows each for NB receivers
+    constexpr int NB = OWN > 1 ? OWN / 2 : 1, RW_ = N / 2 / NB, C = RW_ < 16 ? 8 : 16;
+    const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + g * (N / 2);
+    uint8_t* put[NB];
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+      const int dst = OWN > 1 ? g * NB + i : 0;
+      put[i] = (dst == r ? recv + (size_t)r * 4 * BLK : stage + (size_t)dst * 4 * BLK) + q * BLK + (OWN > 1 ? 0 : g * RW_ * 128) + lane * 4;
+    }
     // the cluster's products of item s, summed: acc[G][UP]
     constexpr int G = BWD ? 1 : 4;
     auto exchange = [&](int s, float (&sum)[G][UP]) -> bool {
       if (ew == 0 && lane == 0) mbar_expect_tx(xchg, tx);
       if (!mbar_wait(acc_full, s & 1, wc)) return false;
       tc_fence_after();
-      const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + g * (N / 2);
-      constexpr int C = N / 2 < 16 ? 8 : 16;
 #pragma unroll
       for (int c0 = 0; c0 < N / 2; c0 += C) {
         uint32_t a0[C], a1[C];
@@ -264,11 +270,9 @@ resident_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         if constexpr (NI > 1) tmem_ld_cols<C>(taddr + N + c0, a1);
         tmem_ld_wait();
 #pragma unroll
-        for (int c = 0; c < C; ++c) {
-          const int b = g * (N / 2) + c0 + c, dst = b / RO;
-          uint8_t* to = (dst == r ? recv + (size_t)r * 4 * BLK : stage + (size_t)dst * 4 * BLK) + q * BLK + (b % RO) * 128 + lane * 4;
-          *reinterpret_cast<float*>(to) = NI > 1 ? __uint_as_float(a0[c]) + __uint_as_float(a1[c]) : __uint_as_float(a0[c]);
-        }
+        for (int c = 0; c < C; ++c)
+          *reinterpret_cast<float*>(put[(c0 + c) / RW_] + ((c0 + c) % RW_) * 128) =
+              NI > 1 ? __uint_as_float(a0[c]) + __uint_as_float(a1[c]) : __uint_as_float(a0[c]);
       }
       tc_fence_before();
       fence_proxy_async_smem();
@@ -276,8 +280,8 @@ resident_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
       if (lane == 0) {
         if constexpr (OWN > 1) {
 #pragma unroll
-          for (int i = 0; i < OWN / 2; ++i) {
-            const int dst = g * (OWN / 2) + i;
+          for (int i = 0; i < NB; ++i) {
+            const int dst = g * NB + i;
             if (dst != r)
               dsmem_bulk_copy(mapa_shared(smem_u32(recv) + (r * 4 + q) * BLK, dst), stage + (size_t)(dst * 4 + q) * BLK, BLK,
                               mapa_shared(smem_u32(xchg), dst));
@@ -304,7 +308,6 @@ resident_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
       return true;
     };
     // the warp's box is complete in shared memory: store it, and count the CTA in on flag t once all eight have
-    int n_pub = 0;
     auto publish = [&](int t) {
       fence_proxy_async_smem();
       __syncwarp();
@@ -316,11 +319,9 @@ resident_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
           tma_store_wait<0>();
         }
         if ((smem_count_arrive(pub_cnt) & (EW - 1)) == EW - 1) {
-          if (!p.no_arrive) red_release_gpu_add(&p.flags[(size_t)t * p.n_groups + grp], 1);
-          mbar_arrive(pub_bar);
+          if (!p.no_arrive) red_relaxed_gpu_add(&p.flags[(size_t)t * p.n_groups + grp], 1);
         }
       }
-      ++n_pub;
     };
     if constexpr (!BWD) {
       float c[UP];
@@ -361,8 +362,7 @@ resident_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         st_words<W>(mine, hw);
         publish(t + 1);
         load_pre(t + 1);
-        // what only backward needs, behind the release (which waits for the stores of the whole SM)
-        if (!mbar_wait(pub_bar, (n_pub - 1) & 1, wc)) break;
+        // what only backward needs
         if (ok_cell && !p.inference) {
 #pragma unroll
           for (int gg = 0; gg < 4; ++gg) {
@@ -530,8 +530,7 @@ ResPlan resident_plan(const blstm_desc& d, int phase) {
     p.ng = cdiv(B, p.rows);
     p.own = bwd ? 4 : p.ks;
     p.N = p.rows <= 16 && p.own != 2 ? 16 : p.rows <= 32 ? 32 : 64;
-    // (backward at 64 rows per group: the gate maths of 8 units a thread spill; slower than 128-row tiles)
-    if (p.rows > (bwd ? 32 : 64)) continue;
+    if (p.rows > 64) continue;
     p.kcm = cdiv(p.kc_total, p.ks);
     const size_t x = (size_t)p.kcm * p.N * 128;
     // (one issuer is a little slower, but its one accumulator may leave tensor memory for the chunk that would not fit)
