@@ -35,6 +35,7 @@ struct ResParams {
   int T, B, H;
   int mt, ks, rows;                        // M tiles; CTAs per cluster; batch rows per group
   int kcm, nt;                             // most chunks of a K slice; chunks in tensor memory
+  int x_bytes;                             // shared memory of the batch rows, or of what is laid over them if that is more
   int kc_total;
   int fmt, no_arrive, inference, flag_target, n_groups;
   unsigned long long limit_ns;
@@ -98,7 +99,7 @@ resident_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
   const int H = p.H, T = p.T, KS = p.ks;
   uint8_t* w_s = smem;                                              // [kcm - nt][16 KB]
   uint8_t* x_s = w_s + (size_t)(p.kcm - p.nt) * 16384;              // [kcm][N rows][128 B]
-  uint8_t* recv = x_s + (size_t)p.kcm * N * 128;                    // [KS senders][4][RO][32] fp32
+  uint8_t* recv = x_s + p.x_bytes;                                  // [KS senders][4][RO][32] fp32
   // in the x slots, which are idle from the item's last MMA until the CTA's rows have been counted in:
   uint8_t* stage = x_s;                                             // [OWN receivers][4][RO][32] fp32
   uint8_t* o_s = x_s + N * 512;                                     // rows on their way out
@@ -532,7 +533,8 @@ ResPlan resident_plan(const blstm_desc& d, int phase) {
     p.N = p.rows <= 16 && p.own != 2 ? 16 : p.rows <= 32 ? 32 : 64;
     if (p.rows > 64) continue;
     p.kcm = cdiv(p.kc_total, p.ks);
-    const size_t x = (size_t)p.kcm * p.N * 128;
+    const size_t x = std::max((size_t)p.kcm * p.N * 128, (size_t)p.N * 512 + (size_t)(p.N / p.own) * (bwd ? 1024 : 64));
+    p.x_bytes = (int)x;
     // (one issuer is a little slower, but its one accumulator may leave tensor memory for the chunk that would not fit)
     for (p.ni = 2; p.ni >= 1; --p.ni) {
       p.nt = std::min(p.kcm, (512 - p.ni * p.N) / 32);
@@ -540,7 +542,6 @@ ResPlan resident_plan(const blstm_desc& d, int phase) {
       if (p.smem <= 232448 || !(bwd && p.N == 32)) break;
     }
     if (p.smem > 232448 || p.ni < 1 || p.kcm > RES_MAX_KC) continue;
-    if (x < (size_t)p.N * 512 + (size_t)(p.N / p.own) * (bwd ? 1024 : 64)) continue;
     p.grid = p.ng * p.mt * p.ks;
     p.off_db = sizeof(Control) + round_up((size_t)(d.seq_len + 1) * p.ng * sizeof(int), 256);
     p.ws_bytes = p.off_db + (bwd ? (size_t)p.ng * p.N * 4 * H * sizeof(float) : 0);
@@ -558,7 +559,7 @@ static int launch_t(const ResPlan& pl, const CUtensorMap& tw, const CUtensorMap&
 static int launch(const blstm_desc& d, const ResPlan& pl, bool bwd, void* x, ResParams& p, void* ws, cudaStream_t st) {
   const int H = d.hidden_size, B = d.batch, T = d.seq_len;
   p.T = T; p.B = B; p.H = H;
-  p.mt = pl.mt; p.ks = pl.ks; p.rows = pl.rows; p.kcm = pl.kcm; p.nt = pl.nt; p.kc_total = pl.kc_total;
+  p.mt = pl.mt; p.ks = pl.ks; p.rows = pl.rows; p.kcm = pl.kcm; p.nt = pl.nt; p.x_bytes = pl.x_bytes; p.kc_total = pl.kc_total;
   p.fmt = d.dtype == BLSTM_BF16 ? 1 : 0;
   p.no_arrive = (d.flags & BLSTM_FLAG_TEST_NO_ARRIVE) ? 1 : 0;
   p.inference = (d.flags & BLSTM_FLAG_INFERENCE) ? 1 : 0;

@@ -5,13 +5,14 @@
 namespace blstm {
 namespace sm100 {
 
-constexpr int RES_MIN_H = 576;
+constexpr int RES_MIN_H = 256;         // (smaller sizes have the small-batch kernels or several 128-row tiles a CTA)
 
 struct ResPlan {
   bool ok;
   int ks, own, mt, ng;      // CTAs per cluster (parts of K); of these, owners of batch rows; M tiles; groups of rows
   int rows, N;              // batch rows per group; N of the MMAs
   int kc_total, kcm, nt;    // chunks of K; most of a CTA; of these in tensor memory
+  int x_bytes;
   int ni;                   // MMA issuers
   int grid;
   size_t smem, off_db, ws_bytes;

@@ -806,16 +806,18 @@ int resident_clusters(int nc) {
   return c;
 }
 
-// Whether the plan beats the tcgen05 kernels.  Those take the same time for any batch of up to a few 128-row tiles, these
-// about the same for every chunk after the first, so the line is a number of chunks per cluster.  Forward, us per
-// step (T = 128, B200): H = 64, B = 64: 1.9 -> 0.59; H = 256, B = 64 / 256 / 512 / 1024: 2.9 / 4.5 / 4.5 / 5.3 -> 1.0 / 2.2
-// / 3.3 / 5.6 (the last not taken); H = 320, B = 32: 4.1 -> 0.95; H = 512, B = 32 / 128 / 256: 4.2 / 5.2 / 5.2 -> 1.6 / 3.4 / 5.6 (kept
-// there too: a shard of a batch then sums in the same order); H = 768, B = 32: 4.8 -> 2.5.  Backward: H = 64: 6.1 -> 0.73;
-// H = 256, B = 64 / 1024: 6.7 / 8.3 -> 1.0 / 6.0; H = 512, B = 32 / 256: 6.7 / 8.9 -> 1.5 / 4.1; H = 640, B = 64: 7.6 -> 3.3.
+// Whether the plan beats the tcgen05 kernels: those with resident weights (multiples of 64 from 256 on; smaller sizes: the
+// general ones) take nearly the same time for any batch of up to several hundred rows, these about the same for
+// every chunk of 8 rows after the first, so the line is a number of chunks per cluster.  us per step (B200), these against
+// resident weights, forward: H = 256, B = 128 / 256 / 512: 1.3 / 2.1 / 3.3 against 2.2 / 2.3 / 2.6; H = 320, B = 128 / 256: 2.1 / 3.4
+// against 2.3 / 2.7; H = 512, B = 32 / 64 / 128 / 256: 1.6 / 2.3 / 3.2 / 5.3 against 2.6 / 2.6 / 2.6 / 2.9; H = 640, B = 16 / 64: 2.2 / 4.2
+// against 2.7 / 2.7.  Backward: H = 256, B = 256 / 512: 2.1 / 3.4 against 2.6 / 3.2; H = 512, B = 128 / 256: 2.6 / 4.1 against 3.0 / 3.5.
+// (Backward from H = 448 on the line lies before B = 128, so that the halves of a batch of 256 sum in its order.)
+// (General kernels, forward: H = 64, B = 64: 1.9 -> 0.59; H = 192: 4.4 a step at any of these batches.)
 static bool small_plan_pays(int H, const SmallPlan& p, int phase) {
   if (H <= 128) return true;
-  if (phase == BLSTM_PHASE_BWD) return true;                             // (what fits in shared memory)
-  return p.nch <= (H <= 256 ? 8 : H <= 512 ? 5 : 2);
+  if (phase == BLSTM_PHASE_BWD) return H < 256 || p.nch <= (H <= 384 ? 4 : 2);
+  return p.nch <= (H < 256 ? 8 : H <= 320 ? 3 : H <= 512 ? 2 : 1);
 }
 
 SmallPlan small_plan(const blstm_desc& d, int phase) {

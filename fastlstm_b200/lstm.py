@@ -64,10 +64,10 @@ def plan_name(dtype, T, B, I, H, phase="fwd"):
     return _lib.load().blstm_plan_name(d, _PHASES[phase]).decode()
 
 
-def plan_detail(dtype, T, B, I, H, phase="fwd"):
-    """One-line description of the launch geometry the library picks for this problem."""
+def plan_detail(dtype, T, B, I, H, phase="fwd", half_device=False):
+    """One-line description of the launch geometry the library picks for this problem (on half of the SMs)."""
     import ctypes
-    d = _desc(dtype, T, B, I, H)
+    d = _desc(dtype, T, B, I, H, _lib.FLAG_HALF_DEVICE if half_device else 0)
     buf = ctypes.create_string_buffer(512)
     _lib.check(_lib.load().blstm_plan_detail(d, _PHASES[phase], buf, 512), "blstm_plan_detail")
     return buf.value.decode()
@@ -276,6 +276,18 @@ def _shares_device(dtype, T, B, I, H):
     for nothing outside themselves, and enough steps to pay for the streams (some 30 us of host time)."""
     Ip, Hp = _padded_sizes(dtype, I, H, T, B) or (I, H)
     return T >= 48 and all("small-batch" in plan_detail(dtype, T, B, Ip, Hp, phase) for phase in ("fwd", "bwd"))
+
+
+@functools.lru_cache(maxsize=1024)
+def _wavefront_pays(dtype, T, B, H, grad):
+    """False where a layer alone has recurrences with resident weights or the small-batch ones: those leave little to hide,
+    and a training step's launches for every chunk cost more than that (two layers, forward and backward: T=256, B=512,
+    H=512 6.8 ms as a wavefront, 6.4 without; T=256, B=32, H=256 1.8 and 1.25; T=128, B=200, H=768 3.4 both).  Inference
+    gains from 128 steps on where half of the device has them too (T=256, B=128, H=512: 1.44 -> 1.15 ms)."""
+    def on_chip(half):
+        return all(any(w in plan_detail(dtype, T, B, H, H, phase, half) for w in ("resident weights", "small-batch"))
+                   for phase in (("fwd", "bwd") if grad else ("fwd",)))
+    return not on_chip(False) or (not grad and T >= 128 and on_chip(True))
 
 
 class _Beside:
@@ -599,7 +611,7 @@ class FastLSTM(nn.Module):
             return None
         L, H, dt = self.num_layers, self.hidden_size, x.dtype
         T, B = (x.shape[1], x.shape[0]) if self.batch_first else (x.shape[0], x.shape[1])
-        if T > 1 and (self._wavefront_chunks(x.transpose(0, 1) if self.batch_first else x, h_c_0, None)
+        if T > 1 and (self._wavefront_chunks(x.transpose(0, 1) if self.batch_first else x, h_c_0, None) and _wavefront_pays(dt, T, B, H, False)
                       or any(_padded_sizes(dt, n, H, T, B) is not None for n in {x.shape[2], H})):
             return None
         if T == 1 and dt != torch.float32 and (H % 8 or x.shape[2] % 8):
@@ -747,6 +759,9 @@ class FastLSTM(nn.Module):
     def _forward_padded(self, x, h_c_0, lengths):
         """x [T,B,I]; lengths: None, or the [B] valid lengths (device tensor) of padded sequences."""
         n_chunks = self._wavefront_chunks(x, h_c_0, lengths)
+        if n_chunks and not _wavefront_pays(x.dtype, x.shape[0], x.shape[1], self.hidden_size,
+                                                torch.is_grad_enabled()):
+            n_chunks = 0
         if n_chunks:
             return self._forward_wavefront(x, h_c_0, n_chunks)
         nd = self.num_directions

@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 # CTAs; K split over two warps (11 to 16 CTAs, K steps in odd halves); weights partly in shared memory; batches of
 # one row, one row past a chunk, chunks shared by replicas
 SHAPES = [(5, 3, 8), (4, 9, 24), (9, 1300, 64), (3, 1, 64), (5, 33, 72), (6, 270, 128), (4, 17, 136), (7, 120, 200),
-          (5, 400, 256), (1, 9, 256), (6, 8, 264), (4, 57, 288), (5, 130, 384), (3, 40, 448), (6, 250, 512), (2, 1, 512),
+          (5, 360, 256), (1, 9, 256), (6, 8, 264), (4, 57, 288), (5, 100, 384), (3, 40, 448), (6, 110, 512), (2, 1, 512),
           (4, 15, 520), (3, 50, 640), (4, 9, 768)]
 
 
