@@ -1591,19 +1591,21 @@ static int launch_bwd_t(const BwdPlan& pl, const CUtensorMap& tw, const CUtensor
 using namespace sm100;
 
 bool sm100_recurrence_supported(const blstm_desc& d, int phase) {
-  if (small_plan(d, phase).ok || resident_plan(d, phase).ok) return true;
+  if (small_plan(d, phase).ok || resident_plan(d, phase).ok || tiles_plan(d, phase).ok) return true;
   return phase == BLSTM_PHASE_BWD ? make_bwd_plan(d).ok : make_plan(d, phase).ok;
 }
 size_t sm100_recurrence_workspace(const blstm_desc& d, int phase) {
   const SmallPlan sp = small_plan(d, phase);
   if (sp.ok) return small_workspace(d, sp, phase);
   if (const ResPlan rp = resident_plan(d, phase); rp.ok) return rp.ws_bytes;
+  if (const TilesPlan tp = tiles_plan(d, phase); tp.ok) return tp.ws_bytes;
   return phase == BLSTM_PHASE_BWD ? make_bwd_plan(d).ws_bytes : make_plan(d, phase).ws_bytes;
 }
 
 size_t sm100_recurrence_control(const blstm_desc& d, int phase) {
   if (small_plan(d, phase).ok) return sizeof(Control);
   if (const ResPlan rp = resident_plan(d, phase); rp.ok) return rp.off_db;
+  if (const TilesPlan tp = tiles_plan(d, phase); tp.ok) return tp.off_db;
   return phase == BLSTM_PHASE_BWD ? make_bwd_plan(d).off_db : make_plan(d, phase).ws_bytes;
 }
 
@@ -1611,6 +1613,7 @@ int sm100_plan_detail(const blstm_desc& d, int phase, char* buf, size_t n) {
   const SmallPlan sp = small_plan(d, phase);
   if (sp.ok) return small_plan_detail(d, sp, phase, buf, n);
   if (const ResPlan rp = resident_plan(d, phase); rp.ok) return resident_plan_detail(rp, phase, buf, n);
+  if (const TilesPlan tp = tiles_plan(d, phase); tp.ok) return tiles_plan_detail(tp, buf, n);
   if (phase == BLSTM_PHASE_BWD) {
     const BwdPlan p = make_bwd_plan(d);
     if (!p.ok) return 0;
@@ -1721,6 +1724,10 @@ int sm100_bwd_recurrence(const blstm_desc& d, const void* dout, const void* dh_n
   if (const ResPlan rp = resident_plan(d, BLSTM_PHASE_BWD); rp.ok) {
     if (ws_bytes < rp.ws_bytes) return BLSTM_E_WORKSPACE;
     return resident_bwd_recurrence(d, rp, dout, dh_n, dc_n, ifgo, cell, Wh, d_ifgo, dh0, dc0, db, ws, st);
+  }
+  if (const TilesPlan tp = tiles_plan(d, BLSTM_PHASE_BWD); tp.ok) {
+    if (ws_bytes < tp.ws_bytes) return BLSTM_E_WORKSPACE;
+    return tiles_bwd_recurrence(d, tp, dout, dh_n, dc_n, ifgo, cell, Wh, d_ifgo, dh0, dc0, db, ws, st);
   }
   const BwdPlan pl = make_bwd_plan(d);
   if (!pl.ok) return BLSTM_E_UNSUPPORTED;

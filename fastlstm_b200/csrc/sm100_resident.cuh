@@ -20,6 +20,17 @@ struct ResPlan {
 
 ResPlan resident_plan(const blstm_desc& d, int phase);
 
+// ... backward, for batches of several 64-row tiles per group
+struct TilesPlan {
+  bool ok;
+  int mt, ng, nbt;          // M tiles; groups; batch tiles
+  int kc, s2;               // K chunks of a CTA; ring stages per issuer
+  int grid;
+  size_t smem, off_db, ws_bytes;
+};
+
+TilesPlan tiles_plan(const blstm_desc& d, int phase);
+
 }  // namespace sm100
 
 int resident_fwd_recurrence(const blstm_desc& d, const sm100::ResPlan& pl, void* ifgo, const void* Wh, void* out, void* cell, void* ws,
@@ -27,6 +38,10 @@ int resident_fwd_recurrence(const blstm_desc& d, const sm100::ResPlan& pl, void*
 int resident_bwd_recurrence(const blstm_desc& d, const sm100::ResPlan& pl, const void* dout, const void* dh_n, const void* dc_n,
                             const void* ifgo, const void* cell, const void* Wh, void* d_ifgo, void* dh0, void* dc0, float* db,
                             void* ws, cudaStream_t st);
+int tiles_bwd_recurrence(const blstm_desc& d, const sm100::TilesPlan& pl, const void* dout, const void* dh_n, const void* dc_n,
+                         const void* ifgo, const void* cell, const void* Wh, void* d_ifgo, void* dh0, void* dc0, float* db, void* ws,
+                         cudaStream_t st);
+int tiles_plan_detail(const sm100::TilesPlan& pl, char* buf, size_t n);
 int resident_plan_detail(const sm100::ResPlan& pl, int phase, char* buf, size_t n);
 
 }  // namespace blstm

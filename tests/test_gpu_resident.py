@@ -10,7 +10,9 @@ pytestmark = pytest.mark.gpu
 # N = 16, 32, 64; one row, ragged rows and groups; half an M tile in backward (H % 128 == 64); K split over 1 and 2 (forward),
 # 4, 5 and 6 (backward, one issuer) CTAs; weights that fit tensor memory and weights that do not
 SHAPES = [(4, 1, 768), (3, 65, 704), (5, 100, 768), (3, 250, 768), (4, 256, 1024), (2, 130, 960), (3, 33, 1088), (3, 64, 1536),
-          (4, 32, 2048), (3, 17, 1984), (2, 9, 2048)]
+          (4, 32, 2048), (3, 17, 1984), (2, 9, 2048),
+          # several tiles a group in backward: four, five and eight, a partial last tile, half an M tile, odd numbers of K chunks
+          (3, 1600, 512), (3, 4096, 512), (5, 2300, 448), (3, 3210, 320), (3, 4000, 256), (1, 2047, 512)]
 
 
 @pytest.mark.parametrize("dtype", ["fp16", "bf16"])
@@ -41,7 +43,7 @@ def test_resident_recurrences_against_fp32_maths(dtype, shape):
 
 
 @pytest.mark.parametrize("phase", [0, 1])
-@pytest.mark.parametrize("B,H", [(32, 1024), (32, 1536)])
+@pytest.mark.parametrize("B,H", [(32, 1024), (32, 1536), (2048, 512)])
 def test_resident_recurrences_give_up_with_a_status_when_nothing_arrives(phase, B, H):
     lib = _lib.load()
     T = 3
