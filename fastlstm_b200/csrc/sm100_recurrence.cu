@@ -19,7 +19,7 @@
 //   warps 1..NACC tcgen05.mma issuers (each owns whole K chunks and its own TMEM
 //                 accumulator; warp 1 owns the TMEM allocation)
 //   next warp     publisher (interleaved tiles only): proxy fence + release per item
-//   last 4 or 8   epilogue: thread = batch row x 8 or 16 hidden units x 4 gates
+//   last 8        epilogue: thread = batch row x 8 or 16 hidden units x 4 gates
 #include <stdio.h>
 #include <algorithm>
 #include <atomic>
@@ -112,10 +112,9 @@ static RecPlan make_plan(const blstm_desc& d, int phase) {
   p.TI = p.ntl >= 3 ? 4 : p.ntl >= 2 ? 2 : 1;     // batch tiles interleaved per CTA (state: cell rows in registers)
   p.grid = p.nh * p.nb_par;
   p.epi_warps = 8;
-  // a single 16-unit tile in flight is latency bound: four issuers next to one epilogue warpgroup
-  // (9 warps); otherwise two issuers, eight epilogue warps and, for interleaved tiles, the publisher
-  // (interleaved 32-unit slices: N = 128 runs the tensor pipe at full rate from ONE issuing thread, and a
-  // single accumulator per item leaves tensor-memory columns for the cell rows of four tiles)
+  // two issuers, eight epilogue warps and, for interleaved tiles, the publisher (32-unit slices: N = 128 runs the
+  // tensor pipe at full rate from ONE issuing thread, and a single accumulator per item leaves tensor-memory columns
+  // for the cell rows of four tiles)
   const int n_issuers = UH == 32 ? 1 : 2;
   const int n_publisher = p.TI >= 2 ? 1 : 0;
   p.threads = 32 * (1 + n_issuers + n_publisher + p.epi_warps);   // producer + MMA issuers [+ publisher] + epilogue
@@ -209,7 +208,7 @@ struct ItemCursor {
 };
 
 // UH: hidden units per CTA (16 or 32).  TI: batch tiles interleaved per CTA (1, 2 or 4).
-// Warps: 1 TMA producer, NACC MMA issuers, with interleaved tiles one publisher warp, 4 or 8 epilogue
+// Warps: 1 TMA producer, NACC MMA issuers, with interleaved tiles one publisher warp, 8 epilogue
 // warps - at most 12 (3 per SM sub-partition), which leaves 168 registers per thread; a 13th would cap
 // them at 128.  The epilogue must not spill.
 template <int UH, int TI, typename T16>
@@ -229,9 +228,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
   // twelve 16-byte accesses a thread makes per 8 units.  h keeps its direct stores (they are what
   // the step hand-off orders) and so do the cell rows (a buffer for them would cost a ring stage).
   constexpr bool TMAEP = (TI >= 2);
-  // Epilogue warps.  A single tile of 16 units is latency bound and runs best as one warpgroup with
-  // 16 units per thread next to four issuers (9 warps); every other shape uses two warpgroups that
-  // split the CTA's units (8 or 16 per thread), which keeps interleaved tiles free of spills.
+  // Epilogue warps: two warpgroups that split the CTA's units (8 or 16 per thread, free of spills).
   constexpr int EW = 8;
   constexpr int NU = 4 * UH / EW;                   // units per epilogue thread
   constexpr int NV = NU / 8;                        // 16-byte pieces per operand per thread
@@ -259,9 +256,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int ht = blockIdx.x % p.nh, pb = blockIdx.x / p.nh;
-  // One thread can issue a tcgen05.mma only every ~150 clocks whatever its shape, far below
-  // what these small-N shapes need, so NACC warps issue concurrently: warp x takes the x-th
-  // K=16 slice(s) of every chunk into its own TMEM accumulator, and the epilogue adds them up.
+  // NACC warps issue MMAs concurrently, each for whole chunks into its own TMEM accumulator, and the epilogue adds them
+  // up: a thread issues one every 55 clocks at best, but loses some hundred to every chunk's barriers.
   // With interleaved tiles the epilogue warps are the bottleneck and the release that publishes an item
   // stalls its thread for a memory round trip, so a PUBLISHER warp does the releasing (and the proxy
   // fence of the hand-off): the epilogue warps only arrive on a CTA-local barrier after storing h.
@@ -406,9 +402,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
     if (elect_one()) {                      // (a thread chosen by `elect` issues an MMA every 55 clocks, by lane == 0 every 74)
       constexpr uint64_t descK = smem_desc_base(16, 1024);
       const uint32_t idesc = instr_desc(p.fmt, 0, 0, RB, N);
-      // Every tcgen05 instruction (mma or commit) costs this thread ~150 clocks of issue time, so
-      // issuer x owns WHOLE chunks (kc = x, x+NACC, ...): four MMAs and one commit per chunk,
-      // in parallel with the other issuers, each into its own accumulator.
+      // issuer x owns WHOLE chunks (kc = x, x+NACC, ...): four MMAs and one commit per chunk
       bool ok = (x < nacc) && (p.kr == 0 || mbar_wait(w_full, 0, wc));
       int gs = 0;
       uint32_t gph = 0;
@@ -952,8 +946,8 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
   uint8_t* w_s = smem;                                        // [KC][64 k rows][128 B]
   const int SB = p.stage_bytes;                               // d_ifgo chunk (16 KB) [+ Wh chunk when streamed]
   const int HB = p.hb;                                        // d_ifgo rows of a stage; a streamed Wh chunk follows
-  uint8_t* recv = smem + (size_t)p.kr * 8192;                 // [4 senders][32 rows][256 B]
-  uint8_t* stage = recv + (size_t)4 * XSLOT_BYTES;            // [3 receivers][32 rows][256 B]
+  uint8_t* recv = smem + (size_t)p.kr * 8192;                 // [4 senders][2 halves][32 rows][128 B]
+  uint8_t* stage = recv + (size_t)4 * XSLOT_BYTES;            // [3 receivers][2 halves][32 rows][128 B]
   uint8_t* a_s = p.alias ? recv : stage + (size_t)3 * XSLOT_BYTES;   // ring (over the exchange buffers if aliased)
   uint64_t* bars = reinterpret_cast<uint64_t*>(a_s + (size_t)R_STAGES * SB);
   uint64_t* full = bars;
