@@ -83,13 +83,12 @@ __device__ __forceinline__ int ld_relaxed_gpu(const int* p) {
   asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
+// Counts in on data that other SMs read behind ld_acquire_gpu.  Also where the data left through TMA stores that this
+// thread, or warps it has synchronised with, waited for: the wait makes them visible to the waiting thread, and only a
+// release carries that on to the reader.  Its fence takes 700 clocks when no store of the SM is under way, 1.2 k behind
+// the stores of other warps (a relaxed reduction: 40); on the chain of a step that is 0.5 to 0.6 us.
 __device__ __forceinline__ void red_release_gpu_add(int* p, int v) {
   asm volatile("red.release.gpu.global.add.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-// Counts in on data that this thread has seen COMPLETED at the point of coherence (TMA stores it has waited for): there is
-// nothing for a release to wait for, and its fence costs 1.3 k clocks all the same.
-__device__ __forceinline__ void red_relaxed_gpu_add(int* p, int v) {
-  asm volatile("red.relaxed.gpu.global.add.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 __device__ __forceinline__ unsigned long long globaltimer_ns() {
   unsigned long long t;

@@ -728,7 +728,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
             tma_store_commit();
             tma_store_wait<0>();
             if ((smem_count_arrive(&pub_cnt[it & 3]) & (EW - 1)) == EW - 1) {
-              if (!p.no_arrive) red_relaxed_gpu_add(&p.flags[(size_t)(t + 1) * p.nbt + bt], 1);
+              if (!p.no_arrive) red_release_gpu_add(&p.flags[(size_t)(t + 1) * p.nbt + bt], 1);
             }
           }
           __syncwarp();
@@ -1442,7 +1442,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
                 tma_store_commit();
                 tma_store_wait<0>();
                 const bool pub = (smem_count_arrive(&pub_cnt[pub_it & 3]) & (ITEM_WARPS - 1)) == ITEM_WARPS - 1;
-                if (pub && !p.no_arrive) red_relaxed_gpu_add(&p.flags[(size_t)t * p.nbt + bt], 1);
+                if (pub && !p.no_arrive) red_release_gpu_add(&p.flags[(size_t)t * p.nbt + bt], 1);
               }
             }
             __syncwarp();

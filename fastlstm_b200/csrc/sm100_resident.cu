@@ -12,10 +12,11 @@
 // owner and step on the group's counter, and the whole K slice of the next step is fetched at once (no ring).
 // Batch rows are divided over groups of CTAs that know nothing of each other.
 //
-// us per step, the recurrences with the batch on the M side -> these (B200): forward B=32 H=2048 7.9 -> 3.9, B=256 H=1024
-// 7.2 -> 4.9, B=128 H=1024 3.7, B=256 H=768 6.7 -> 4.2; backward B=32 H=2048 10.0 -> 6.6, B=256 H=1024 7.6 -> 5.6, B=256 H=768
-// 6.8 -> 5.0, B=32 H=1536 4.2.
-// Bound by the chain of a step: hand-off through L2, fetch of N rows, 64 MMAs of some 50 clocks, exchange, gate maths.
+// us per step, the recurrences with the batch on the M side -> these (B200): forward B=32 H=2048 7.9 -> 4.4, B=256 H=1024
+// 7.2 -> 5.7, B=128 H=1024 4.3, B=256 H=768 6.7 -> 4.8; backward B=32 H=2048 10.0 -> 6.9, B=256 H=1024 7.6 -> 6.2, B=256 H=768
+// 6.8 -> 5.7, B=32 H=1536 4.6.
+// Bound by the chain of a step: hand-off through L2 (its release alone 0.5 us), fetch of N rows, 64 MMAs of some 50 clocks,
+// exchange, gate maths.
 #include <algorithm>
 #include <cstdio>
 
@@ -267,7 +268,7 @@ resident_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
           tma_store_wait<0>();
         }
         if ((smem_count_arrive(pub_cnt) & (EW - 1)) == EW - 1) {
-          if (!p.no_arrive) red_relaxed_gpu_add(&p.flags[(size_t)t * p.n_groups + grp], 1);
+          if (!p.no_arrive) red_release_gpu_add(&p.flags[(size_t)t * p.n_groups + grp], 1);
         }
       }
     };

@@ -9,8 +9,8 @@
 // accumulators leave.  Two issuers take every other tile, each with its own accumulator and its own half of the ring.
 // Shared memory holds no weights, so the ring is what the exchange leaves: 2 x 4 stages of 8 KB.  A CTA has 128 units where the
 // kernel with the batch on the M side had 64 a cluster, which halves what a step reads of d_ifgo (67 MB at B = 4096, H = 512).
-// us per step, that kernel -> this: B = 4096, H = 512: 25.5 -> 21.4; B = 3000: 20.4 -> 16.1; B = 2048: 12.9 -> 11.9; B = 4096, H = 256:
-// 12.5 -> 9.5; B = 3000, H = 384: 19.1 -> 11.9.  Not for three tiles a group (B = 1200, H = 512: 9.7, here 10.8: the chain of a
+// us per step, that kernel -> this, launched alone: B = 4096, H = 512: 25.5 -> 21.7 to 23 (it runs into the power cap; 25.5 inside a
+// training step); B = 3000: 20.4 -> 16.0; B = 2048: 12.9 -> 12.3; B = 4096, H = 256: 12.5 -> 9.4; B = 3000, H = 384: 19.1 -> 11.8.  Not for three tiles a group (B = 1200, H = 512: 9.7, here 10.8: the chain of a
 // step shows); the same thing forward was slower (14.7, 17.8), sixteen epilogue warps of half the cells no faster (22.4).
 #include <algorithm>
 #include <cstdio>
@@ -190,8 +190,8 @@ tiles_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
         tma_store_4d(&tmO, boxes + b * BOX, mt * 128, tile * N + r * RO, 0, t);
         tma_store_commit();
         tma_store_wait<0>();
-        if (!p.no_arrive) red_relaxed_gpu_add(&p.flags[(size_t)t * p.nbt + tile], 1);
         mbar_arrive(&box_free[b]);
+        if (!p.no_arrive) red_release_gpu_add(&p.flags[(size_t)t * p.nbt + tile], 1);
         if (++j == NT) { j = 0; ++s; }
       }
     }

@@ -1,4 +1,8 @@
 """Host-side behaviour of the module that needs no GPU."""
+import glob
+import os
+import re
+
 import pytest
 import torch
 import torch.nn as nn
@@ -172,3 +176,18 @@ def test_proj_size_plumbing_matches_nn_lstm(monkeypatch, bidirectional):
         mod.FastLSTM(I, H, proj_size=H)
     with pytest.raises(ValueError):
         mod.FastLSTM(I, H, proj_size=-1)
+
+
+def test_every_hand_off_through_global_memory_is_a_release():
+    # what a CTA counts in on a global counter other SMs read behind ld.acquire.gpu: without a release on this side nothing
+    # orders the data before the count, whatever was waited for locally
+    import fastlstm_b200
+    counted = 0
+    for path in glob.glob(os.path.join(os.path.dirname(fastlstm_b200.__file__), "csrc", "*.cu*")):
+        with open(path) as f:
+            code = re.sub(r"//.*", "", f.read())
+        assert not re.search(r"\b(red|atom)\.(async\.)?relaxed", code), path
+        for call in re.findall(r"(\w+)\(&p\.flags\[", code):
+            assert call in ("red_release_gpu_add", "wait_flag_ge", "ld_acquire_gpu"), (path, call)
+            counted += call == "red_release_gpu_add"
+    assert counted >= 7
