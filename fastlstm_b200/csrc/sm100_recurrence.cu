@@ -345,6 +345,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
               seen = wait_flag_ge(&p.flags[(size_t)t * p.nbt + bt], p.flag_target, p.ctl, p.limit_ns, t, bt) ? 1 : 0;
             }
             seen = __shfl_sync(0xffffffffu, seen, 0);
+            __syncwarp();      // (a shuffle orders no memory: the issuing lanes come behind the acquire)
             if (!seen) { *dead = 1; ok = false; break; }
             // a proxy fence between the peers' arrivals (interleaved tiles: their plain stores, fenced by their publisher
             // warps) and this warp's TMA reads
@@ -1031,6 +1032,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
             seen = wait_flag_ge(&p.flags[(size_t)tg * p.nbt + bt], p.flag_target, p.ctl, p.limit_ns, tg, bt) ? 1 : 0;
           }
           seen = __shfl_sync(0xffffffffu, seen, 0);
+          __syncwarp();      // (a shuffle orders no memory: the issuing lanes come behind the acquire)
           if (!seen) { *dead = 1; ok = false; break; }
           // a proxy fence between the peers' arrivals (interleaved tiles: their plain stores, fenced by their publisher
           // warps) and the TMA reads below

@@ -136,6 +136,7 @@ resident_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         int seen = 1;
         if (lane == 0) seen = wait_flag_ge(&p.flags[(size_t)t * p.n_groups + grp], p.flag_target, p.ctl, p.limit_ns, t, grp) ? 1 : 0;
         seen = __shfl_sync(0xffffffffu, seen, 0);
+        __syncwarp();      // (a shuffle orders no memory: the issuing lanes come behind the acquire)
         if (!seen) { *dead = 1; break; }
         fence_proxy_async_global();
       }

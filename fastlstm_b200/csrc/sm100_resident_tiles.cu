@@ -125,6 +125,7 @@ tiles_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
       if (lane == 0 && early_now < p.flag_target)
         seen = wait_flag_ge(&p.flags[(size_t)t * p.nbt + tile], p.flag_target, p.ctl, p.limit_ns, t, tile) ? 1 : 0;
       seen = __shfl_sync(0xffffffffu, seen, 0);
+      __syncwarp();      // (a shuffle orders no memory: the issuing lanes come behind the acquire)
       if (!seen) { *dead = 1; break; }
       fence_proxy_async_global();
       bool ok = true;

@@ -191,3 +191,16 @@ def test_every_hand_off_through_global_memory_is_a_release():
             assert call in ("red_release_gpu_add", "wait_flag_ge", "ld_acquire_gpu"), (path, call)
             counted += call == "red_release_gpu_add"
     assert counted >= 7
+
+
+def test_the_lanes_that_fetch_come_behind_the_lane_that_acquired():
+    # one lane acquires a hand-off counter, others issue the loads: the shuffle that hands its finding on orders no memory
+    import fastlstm_b200
+    found = 0
+    for path in glob.glob(os.path.join(os.path.dirname(fastlstm_b200.__file__), "csrc", "*.cu")):
+        with open(path) as f:
+            code = re.sub(r"//.*", "", f.read())
+        for follows in re.findall(r"seen = __shfl_sync\(0xffffffffu, seen, 0\);\s*(\S+)", code):
+            assert follows == "__syncwarp();", path
+            found += 1
+    assert found >= 4
