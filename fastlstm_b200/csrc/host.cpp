@@ -301,15 +301,16 @@ struct LayerState {
   Tensor x, Wx, Wh, out, cell, ifgo;
   int64_t I, H;                // the layer's own sizes
   bool stacked;                // final states as [1,B,H]
-  bool half;                   // planned for half of the device
-};
+  std::optional<std::array<int64_t, 3>> main;   // planned for half of the device, another layer beside it: the stream (id, device
+};                                              // index and type) that the gradients are used on, whichever one backward runs on
 
 struct LayerFn : public torch::autograd::Function<LayerFn> {
   static torch::autograd::variable_list forward(torch::autograd::AutogradContext* ctx, const Tensor& x, const OptTensor& h0, const OptTensor& c0,
                                                 const Tensor& Wx, const OptTensor& bx, const Tensor& Wh, const OptTensor& bh, LayerState s) {
     const int64_t T = s.out.size(0) - 1;
     ctx->saved_data["sizes"] = std::vector<int64_t>{s.I, s.H};
-    ctx->saved_data["given"] = std::vector<int64_t>{h0.has_value(), bx.has_value(), bh.has_value(), x.requires_grad(), s.stacked, s.half, (int64_t)x.scalar_type()};
+    ctx->saved_data["given"] = std::vector<int64_t>{h0.has_value(), bx.has_value(), bh.has_value(), x.requires_grad(), s.stacked, s.main.has_value(), (int64_t)x.scalar_type()};
+    if (s.main) ctx->saved_data["main"] = std::vector<int64_t>(s.main->begin(), s.main->end());
     Tensor y = s.out.narrow(0, 1, T), hn = s.out.select(0, T), cn = s.cell.select(0, T);
     if (s.out.size(2) != s.H) { y = y.narrow(2, 0, s.H); hn = hn.narrow(1, 0, s.H); cn = cn.narrow(1, 0, s.H); }
     if (s.stacked) {             // tensors of their own, in one copy
@@ -356,6 +357,12 @@ struct LayerFn : public torch::autograd::Function<LayerFn> {
       dc0 = dc0.narrow(1, 0, H);
     }
     m.run(x.device());
+    if (given[5]) {
+      const auto on = ctx->saved_data["main"].toIntVector();
+      const auto main = c10::Stream::unpack3(on[0], (c10::DeviceIndex)on[1], (c10::DeviceType)on[2]);
+      for (Tensor* t : {&dx, &dh0, &dc0, &dWx, &dWh, &db})
+        if (t->defined()) t->record_stream(main);
+    }
     const Tensor none;
     return {dx, given[0] ? dh0 : none, given[0] ? dc0 : none, dWx, given[1] ? db : none, dWh, given[2] ? db : none, none};
   }
@@ -363,8 +370,8 @@ struct LayerFn : public torch::autograd::Function<LayerFn> {
 
 py::tuple attach(const Tensor& x, const OptTensor& h0, const OptTensor& c0, const Tensor& Wx, const OptTensor& bx, const Tensor& Wh,
                  const OptTensor& bh, const Tensor& xp, const Tensor& Wxp, const Tensor& Whp, const Tensor& out, const Tensor& cell,
-                 const Tensor& ifgo, bool stacked, bool half) {
-  const auto r = LayerFn::apply(x, h0, c0, Wx, bx, Wh, bh, LayerState{xp, Wxp, Whp, out, cell, ifgo, x.size(-1), Wh.size(-1), stacked, half});
+                 const Tensor& ifgo, bool stacked, std::optional<std::array<int64_t, 3>> main) {
+  const auto r = LayerFn::apply(x, h0, c0, Wx, bx, Wh, bh, LayerState{xp, Wxp, Whp, out, cell, ifgo, x.size(-1), Wh.size(-1), stacked, main});
   return py::make_tuple(r[0], r[1], r[2]);
 }
 

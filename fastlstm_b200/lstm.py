@@ -246,11 +246,11 @@ class PersistentLSTMfn(torch.autograd.Function):
                 dbh if ctx.has_bias[1] else None, None, None, None)
 
 
-def _layer(x, h0, c0, Wx, bx, Wh, bh, inference, stacked=False, want_cells=False, half=False):
+def _layer(x, h0, c0, Wx, bx, Wh, bh, inference, stacked=False, want_cells=False, main=None):
     """One layer on the GPU, as PersistentLSTMfn computes it (same casts, padding and gradients), with the
     conversions in one launch and the autograd node in the host extension.  stacked: the final states come as
-    tensors [1,B,H] of their own.  want_cells: also the cell states of every step (no gradient).  half: planned
-    for half of the device, another layer runs beside it."""
+    tensors [1,B,H] of their own.  want_cells: also the cell states of every step (no gradient).  main: planned
+    for half of the device, another layer runs beside it; the stream that the gradients will be used on."""
     host = _lib.host()
     if (h0 is None) != (c0 is None):
         raise ValueError("h0 and c0 must both be given or both be None")
@@ -260,9 +260,10 @@ def _layer(x, h0, c0, Wx, bx, Wh, bh, inference, stacked=False, want_cells=False
     Ip, Hp = _padded_sizes(x.dtype if to is None else to, I, H, T, B) or (0, 0)
     xp, h0p, c0p, Wxp, bxp, Whp, bhp = host.prepare(x, h0, c0, Wx, bx, Wh, bh, to, Ip, Hp)
     with _profiled("fastlstm_b200::fwd"):
-        out, cell, ifgo = lstm_persistent_fwd(xp, h0p, c0p, Wxp, bxp, Whp, bhp, inference=inference, half_device=half)
+        out, cell, ifgo = lstm_persistent_fwd(xp, h0p, c0p, Wxp, bxp, Whp, bhp, inference=inference, half_device=main is not None)
     if not inference:
-        res = host.attach(x, h0, c0, Wx, bx, Wh, bh, xp, Wxp, Whp, out, cell, ifgo, stacked, half)
+        on = None if main is None else (main.stream_id, main.device_index, main.device_type)
+        res = host.attach(x, h0, c0, Wx, bx, Wh, bh, xp, Wxp, Whp, out, cell, ifgo, stacked, on)
     else:
         res = out[1:, :, :H], out[-1, :, :H], cell[-1, :, :H]
         if stacked:
@@ -291,15 +292,20 @@ def _wavefront_pays(dtype, T, B, H, grad):
 
 
 class _Beside:
-    """Runs the second direction of a layer, with the input x, on the side stream beside the first.  Entering makes
-    the side stream wait for everything so far - x, and the readers of memory that it frees and reuses - and join()
-    makes the current stream wait for it.  A no-op where `on` is false."""
+    """Runs the second direction of a layer on the side stream beside the first.  Entering makes the side stream wait for
+    everything so far, join() makes the current stream wait for the side stream, and release(), behind the readers of what
+    the side stream has made, the side stream for them: it may get that memory back before they have run.  The other way
+    round the last holder of a tensor can be a backward node of the side stream, so what that stream reads of the current
+    one's memory - the input, row maps, weights that are not parameters - is recorded with the allocator, and so are the
+    gradients its nodes hand out (LayerState in csrc/host.cpp).  A no-op where `on` is false."""
 
-    def __init__(self, x, on):
-        self.main = torch.cuda.current_stream(x.device) if on else None
-        self.side = _side_stream(x.device) if on else None
+    def __init__(self, device, on, *reads):
+        self.main = torch.cuda.current_stream(device) if on else None
+        self.side = _side_stream(device) if on else None
         if on:
-            x.record_stream(self.side)       # x comes from the main stream's memory, and backward reads it again
+            for t in reads:
+                if t is not None and not isinstance(t, nn.Parameter):     # (parameters outlive the graph)
+                    t.record_stream(self.side)
             self.side.wait_stream(self.main)
 
     def stream(self, d):
@@ -308,6 +314,10 @@ class _Beside:
     def join(self):
         if self.side is not None:
             self.main.wait_stream(self.side)
+
+    def release(self):
+        if self.side is not None:
+            self.side.wait_stream(self.main)
 
 
 _side_streams = {}
@@ -370,13 +380,13 @@ class WavefrontLSTMfn(torch.autograd.Function):
                         saved[l][k] = (xc, out, cell, None if inference else ifgo)
                         done[l][k] = torch.cuda.Event()
                         done[l][k].record(st)
-            # every later use (the concatenation below, backward, the allocator) comes after both streams
             main.wait_stream(streams[1])
-            streams[1].wait_stream(main)
             top = saved[L - 1]
             y = torch.cat([top[k][1][1:] for k in range(NC)], dim=0) if NC > 1 else top[0][1][1:].clone()
             h_n = torch.stack([saved[l][NC - 1][1][-1] for l in range(L)])
             c_n = torch.stack([saved[l][NC - 1][2][-1] for l in range(L)])
+            # (the side stream may get its memory back before the reads above have run)
+            streams[1].wait_stream(main)
         ctx.inference = bool(inference)
         if not inference:
             ctx.saved = saved
@@ -448,7 +458,6 @@ class WavefrontLSTMfn(torch.autograd.Function):
                         done[l][k] = torch.cuda.Event()
                         done[l][k].record(st)
             main.wait_stream(streams[1])
-            streams[1].wait_stream(main)
             d_x = None
             if need_dx0:
                 d_x = torch.cat(dx[0], dim=0) if NC > 1 else dx[0][0]
@@ -456,6 +465,9 @@ class WavefrontLSTMfn(torch.autograd.Function):
             if ctx.had_state:
                 dh0 = torch.stack([carry[l][0][0] for l in range(L)])
                 dc0 = torch.stack([carry[l][0][1] for l in range(L)])
+            streams[1].wait_stream(main)
+            for l in range(1, L, 2):
+                acc[l].record_stream(main)       # (the parameters' gradients are used there)
         grads = []
         for l in range(L):
             Wx, bx, Wh, bh = params[4 * l:4 * l + 4]
@@ -679,13 +691,14 @@ class FastLSTM(nn.Module):
                 xs = [host.gather_rows(data, *maps, [T, B]) for maps in ((padded, packed), (turned, packed_t))[:nd]]
             else:
                 xs = [x] if nd == 1 else [x, host.gather_rows(x, rev, rev, [T, B])]
-            beside = _Beside(xs[-1], half)
+            params = [self.layer_params(layer, reverse=(d == 1)) for d in range(nd)]
+            beside = _Beside(data.device, half, xs[-1], turned, *params[-1])        # (the maps are views of one tensor)
             for d, x_d in enumerate(xs):
-                Wx, bx, Wh, bh = self.layer_params(layer, reverse=(d == 1))
+                Wx, bx, Wh, bh = params[d]
                 hl, cl = h_0[layer * nd + d], c_0[layer * nd + d]
                 with beside.stream(d):
                     inference = _nothing_to_save(x_d, hl, cl, Wx, bx, Wh, bh)
-                    o, _, _, cells = _layer(x_d, hl, cl, Wx, bx, Wh, bh, inference, want_cells=True, half=half)
+                    o, _, _, cells = _layer(x_d, hl, cl, Wx, bx, Wh, bh, inference, want_cells=True, main=beside.main)
                     h_n.append(host.gather_rows(o, last, inv_last, [B]))       # states at each sequence's own last step
                     c_n.append(host.gather_rows(cells, last, inv_last, [B]))
                     if top:
@@ -695,10 +708,12 @@ class FastLSTM(nn.Module):
                 outs.append(o)
             beside.join()
             x = outs[0] if nd == 1 else torch.cat(outs, dim=-1)
+            if top:
+                states = torch.stack(h_n), torch.stack(c_n)
+            beside.release()
             if self.dropout > 0.0 and self.training and not top:
                 x = torch.nn.functional.dropout(x, self.dropout, True)
-        return (PackedSequence(x, seq.batch_sizes, seq.sorted_indices, seq.unsorted_indices),
-                (torch.stack(h_n), torch.stack(c_n)))
+        return PackedSequence(x, seq.batch_sizes, seq.sorted_indices, seq.unsorted_indices), states
 
     def _initial_states(self, h_c_0):
         """One (h_0, c_0) per layer and direction, or Nones."""
@@ -787,15 +802,16 @@ class FastLSTM(nn.Module):
             half = (nd == 2 and x.is_cuda and lengths is None and self._sinks is None and self.proj_size == 0
                     and _shares_device(dt, T, B, x.shape[2], self.hidden_size))
             turned = x.flip(0) if half else x
-            beside = _Beside(turned, half)
+            params = [self.layer_params(layer, reverse=(d == 1)) for d in range(nd)]
+            beside = _Beside(x.device, half, turned, *params[-1])
             for d in range(nd):
-                Wx, bx, Wh, bh = self.layer_params(layer, reverse=(d == 1))
+                Wx, bx, Wh, bh = params[d]
                 if half:
                     hl, cl = h_0[layer * nd + d], c_0[layer * nd + d]
                     x_d = turned if d else x
                     with beside.stream(d):
                         inference = _nothing_to_save(x_d, hl, cl, Wx, bx, Wh, bh)
-                        o, h_i, c_i = _layer(x_d, hl, cl, Wx, bx, Wh, bh, inference, half=True)
+                        o, h_i, c_i = _layer(x_d, hl, cl, Wx, bx, Wh, bh, inference, main=beside.main)
                         outs.append(o.flip(0) if d else o)
                     h_n.append(h_i)
                     c_n.append(c_i)
@@ -829,10 +845,12 @@ class FastLSTM(nn.Module):
                 c_n.append(c_i)
             beside.join()
             x = outs[0] if nd == 1 else torch.cat(outs, dim=-1)
+            if layer == self.num_layers - 1:
+                # (a single layer has made the stacked tensors itself)
+                states = (h_n[0], c_n[0]) if single else (torch.stack(h_n), torch.stack(c_n))
+            beside.release()
             if self.dropout > 0.0 and self.training and layer < self.num_layers - 1:
                 x = torch.nn.functional.dropout(x, self.dropout, True)
         if self.batch_first and lengths is None:
             x = x.transpose(0, 1)
-        if single:                        # (the layer has made the stacked tensors itself)
-            return x, (h_n[0], c_n[0])
-        return x, (torch.stack(h_n), torch.stack(c_n))
+        return x, states

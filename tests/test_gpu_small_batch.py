@@ -285,6 +285,36 @@ def test_directions_side_by_side_match_nn_lstm(T, B, H, packed):
     F.check_status()
 
 
+@pytest.mark.parametrize("packed", [False, True])
+def test_directions_side_by_side_when_nothing_but_the_weights_needs_a_gradient(packed):
+    """No input gradient, no kept states: the last holders of what the directions share are nodes of the backward pass.
+    Passes on different batches back to back, nothing waited for in between, give bit for bit the gradients of each
+    batch on its own."""
+    import fastlstm_b200 as F
+    from torch.nn.utils.rnn import pack_padded_sequence
+    torch.manual_seed(3)
+    T, B, H = 64, 24, 128
+    m = F.FastLSTM(24, H, num_layers=2, bidirectional=True, device="cuda", dtype=torch.bfloat16)
+    xs, lens = [torch.randn(T, B, 24, device="cuda").bfloat16() for _ in range(6)], [torch.randint(1, T + 1, (B,)) for _ in range(6)]
+    for n in lens:
+        n[0] = T
+
+    def grads(k):
+        m.zero_grad()
+        out = m(pack_padded_sequence(xs[k], lens[k], enforce_sorted=False) if packed else xs[k])[0]
+        out = out.data if packed else out
+        torch.autograd.backward([out], [torch.ones_like(out)])
+        return [p.grad for p in m.parameters()]
+    alone = []
+    for k in range(6):
+        alone.append([g.clone() for g in grads(k)])
+        torch.cuda.synchronize()
+    for _ in range(3):
+        for g, want in zip([grads(k) for k in range(6)], alone):
+            assert all(torch.equal(a, b) for a, b in zip(g, want))
+    F.check_status()
+
+
 @pytest.mark.parametrize("T,B,H,P,states", [(2, 1, 33, 7, True), (40, 9, 96, 32, True), (30, 64, 512, 128, False)])
 def test_projected_layer_matches_nn_lstm(T, B, H, P, states):
     """The projected layer as an ordinary one with the recurrent weights W_hh W_hr."""

@@ -204,3 +204,92 @@ def test_the_lanes_that_fetch_come_behind_the_lane_that_acquired():
             assert follows == "__syncwarp();", path
             found += 1
     assert found >= 4
+
+
+@pytest.mark.parametrize("packed", [False, True])
+def test_memory_that_two_streams_share_is_not_reused_under_a_queued_read(monkeypatch, packed):
+    """The directions of a layer on two streams (fakes; the operators by plain torch): what the side stream reads of the main
+    stream's memory is recorded there - backward's last holder may be a node on either - and the side stream comes behind
+    the main stream's last read of what it has made."""
+    import contextlib
+    from torch.nn.utils import parametrize
+    from torch.nn.utils.rnn import pack_padded_sequence
+    from fastlstm_b200 import _lib, lstm
+    log, made_on, recorded, reads = [], {}, set(), []
+    key = lambda t: t.untyped_storage().data_ptr()
+
+    class Stream:
+        stream_id = device_index = device_type = 0
+
+        def __init__(self, name):
+            self.name = name
+
+        def wait_stream(self, other):
+            log.append((self.name, "waits for", other.name))
+    main, side, now = Stream("main"), Stream("side"), []
+    now.append(main)
+
+    @contextlib.contextmanager
+    def on(stream):
+        now.append(stream)
+        yield
+        now.pop()
+
+    keep = []
+
+    def op(out, *used):                    # an operator of the current stream
+        reads.extend((now[-1].name, t) for t in used if t is not None)
+        for t in out:
+            made_on[key(t)] = now[-1].name
+            keep.append(t)
+        return out
+
+    class Host:
+        def packed_maps(self, batch_sizes, rank, data):
+            T, B = batch_sizes.numel(), int(batch_sizes[0])
+            maps = torch.zeros(4 * T * B + B + 2 * data.shape[0], dtype=torch.long)
+            op([maps])
+            return list(maps.split([T * B] * 4 + [B] + [data.shape[0]] * 2))
+
+        def gather_rows(self, src, idx, inv, lead):
+            return op([src.reshape(-1, src.shape[-1])[idx].view(*lead, -1).clone()], src, idx, inv)[0]
+
+    def layer(x, h0, c0, Wx, bx, Wh, bh, inference, want_cells=False, **_):
+        out, cells = x @ Wx.t()[:, :Wh.shape[1]], x @ Wx.t()[:, -Wh.shape[1]:]
+        h, c = out[-1].clone(), cells[-1].clone()
+        op([out, cells, h, c], x, Wx, Wh, bx, bh)
+        return (out, h, c) + ((cells,) if want_cells else ())
+
+    class Twice(nn.Module):
+        def forward(self, w):
+            return 2 * w
+    m = FastLSTM(6, 4, num_layers=2, bidirectional=True)
+    parametrize.register_parametrization(m, "weight_ih_l0_reverse", Twice())
+    params = {key(p) for p in m.parameters()}
+    monkeypatch.setattr(_lib, "host", lambda: Host())
+    monkeypatch.setattr(lstm, "_layer", layer)
+    monkeypatch.setattr(lstm, "_shares_device", lambda *a: True)
+    monkeypatch.setattr(lstm, "_side_stream", lambda d: side)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda d=None: now[-1])
+    monkeypatch.setattr(torch.cuda, "stream", on)
+    monkeypatch.setattr(torch.Tensor, "is_cuda", True)
+    monkeypatch.setattr(torch.Tensor, "record_stream", lambda t, s: recorded.add((key(t), s.name)))
+    for name in ("cat", "stack"):
+        f = getattr(torch, name)
+        monkeypatch.setattr(torch, name, lambda ts, dim=0, f=f, name=name: log.append(("main", name)) or f(ts, dim=dim))
+    x = torch.randn(5, 3, 6)
+    if packed:
+        m._forward_packed_rows(pack_padded_sequence(x, [5, 4, 2]), None)
+    else:
+        m._forward_padded(x, None, None)
+    shared = [t for who, t in reads if who == "side" and made_on.get(key(t), "main") == "main" and key(t) not in params]
+    assert len(shared) >= (8 if packed else 3)
+    for t in shared:
+        assert (key(t), "side") in recorded, t.shape
+    assert log[-1] == ("side", "waits for", "main") and ("main", "waits for", "side") in log
+    last = max(i for i, e in enumerate(log) if e[0] == "main" and e[1] in ("cat", "stack"))
+    assert log.index(("main", "waits for", "side")) < last < len(log) - 1
+    # every layer's concatenation too, before the next layer's work may free what it read
+    for i, e in enumerate(log):
+        if e == ("main", "cat"):
+            assert ("side", "waits for", "main") in log[i + 1:i + 4]
