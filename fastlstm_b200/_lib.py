@@ -15,6 +15,7 @@ ABI_VERSION = 1
 F32, F16, BF16 = 0, 1, 2
 DTYPE_CODE = {"fp32": F32, "fp16": F16, "bf16": BF16}
 PHASE_FWD, PHASE_BWD, PHASE_FWD_OP = 0, 1, 2
+FAMILY_GENERIC, FAMILY_SMALL_BATCH, FAMILY_RESIDENT, FAMILY_BATCH_TILES = 1, 5, 6, 7
 FLAG_FORCE_GENERIC = 1
 FLAG_INFERENCE = 8
 FLAG_NO_FUSED = 32        # blstm_fwd: keep tiny sizes on projection + recurrence
@@ -43,6 +44,7 @@ SIGNATURES = {
     "blstm_device_check": (c_int, [c_int]),
     "blstm_workspace_bytes": (c_size_t, [DP, c_int]),
     "blstm_plan_name": (c_char_p, [DP, c_int]),
+    "blstm_plan_family": (c_int, [DP, c_int]),
     "blstm_plan_detail": (c_int, [DP, c_int, ctypes.c_char_p, c_size_t]),
     "blstm_input_projection": (c_int, [DP, P, P, P, P, P, P]),
     "blstm_fwd_recurrence": (c_int, [DP, P, P, P, P, P, c_size_t, P]),

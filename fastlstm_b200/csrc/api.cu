@@ -228,14 +228,26 @@ size_t blstm_workspace_bytes(const blstm_desc* d, int phase) {
   return 0;
 }
 
-const char* blstm_plan_name(const blstm_desc* d, int phase) {
-  if (check_desc(d)) return "invalid";
+int blstm_plan_family(const blstm_desc* d, int phase) {
+  if (check_desc(d)) return BLSTM_FAMILY_NONE;
   if (phase == BLSTM_PHASE_FWD_OP) {
-    if (step_supported(*d)) return "step";
-    if (generic_fused_fwd_supported(*d)) return "fused";
+    if (step_supported(*d)) return BLSTM_FAMILY_STEP;
+    if (generic_fused_fwd_supported(*d)) return BLSTM_FAMILY_FUSED;
     phase = BLSTM_PHASE_FWD;
   }
-  return sm100_recurrence_supported(*d, phase) ? "sm100" : "generic";
+  if (const int family = sm100_plan_family(*d, phase)) return family;
+  return sm100::f32_plan(*d, phase).ok ? BLSTM_FAMILY_F32_CLUSTER : BLSTM_FAMILY_GENERIC;
+}
+
+const char* blstm_plan_name(const blstm_desc* d, int phase) {
+  switch (blstm_plan_family(d, phase)) {
+    case BLSTM_FAMILY_NONE: return "invalid";
+    case BLSTM_FAMILY_STEP: return "step";
+    case BLSTM_FAMILY_FUSED: return "fused";
+    case BLSTM_FAMILY_GENERIC:
+    case BLSTM_FAMILY_F32_CLUSTER: return "generic";
+    default: return "sm100";
+  }
 }
 
 int blstm_plan_detail(const blstm_desc* d, int phase, char* buf, size_t buf_bytes) {

@@ -163,7 +163,7 @@ FwdOut fwd_impl(const Tensor& x, const OptTensor& h0, const OptTensor& c0, const
   auto [out, cell] = empty_pair({T + 1, B, H}, opt);
   r.out = out;
   r.cell = cell;
-  const bool lone = inference && T == 1 && std::string_view(blstm_plan_name(&d, BLSTM_PHASE_FWD_OP)) == "step";
+  const bool lone = inference && T == 1 && blstm_plan_family(&d, BLSTM_PHASE_FWD_OP) == BLSTM_FAMILY_STEP;
   Tensor ws;
   size_t ws_bytes = 0;
   if (!lone) {

@@ -26,6 +26,8 @@ int sm100_bwd_recurrence(const blstm_desc& d, const void* dout, const void* dh_n
                          const void* ifgo, const void* cell, const void* Wh, void* d_ifgo, void* dh0,
                          void* dc0, float* db, void* ws, size_t ws_bytes, cudaStream_t st);
 
+// which of the recurrences a phase uses (BLSTM_FAMILY_*; BLSTM_FAMILY_NONE when the tcgen05 kernels do not cover it)
+int sm100_plan_family(const blstm_desc& d, int phase);
 // one-line description of the launch plan of a phase ("" when the tcgen05 kernels do not cover it)
 int sm100_plan_detail(const blstm_desc& d, int phase, char* buf, size_t n);
 

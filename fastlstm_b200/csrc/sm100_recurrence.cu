@@ -1586,10 +1586,12 @@ static int launch_bwd_t(const BwdPlan& pl, const CUtensorMap& tw, const CUtensor
 
 using namespace sm100;
 
-bool sm100_recurrence_supported(const blstm_desc& d, int phase) {
-  if (small_plan(d, phase).ok || resident_plan(d, phase).ok || tiles_plan(d, phase).ok) return true;
-  return phase == BLSTM_PHASE_BWD ? make_bwd_plan(d).ok : make_plan(d, phase).ok;
+int sm100_plan_family(const blstm_desc& d, int phase) {
+  if (small_plan(d, phase).ok) return BLSTM_FAMILY_SMALL_BATCH;
+  if (resident_plan(d, phase).ok || tiles_plan(d, phase).ok) return BLSTM_FAMILY_RESIDENT;
+  return (phase == BLSTM_PHASE_BWD ? make_bwd_plan(d).ok : make_plan(d, phase).ok) ? BLSTM_FAMILY_BATCH_TILES : BLSTM_FAMILY_NONE;
 }
+bool sm100_recurrence_supported(const blstm_desc& d, int phase) { return sm100_plan_family(d, phase) != BLSTM_FAMILY_NONE; }
 size_t sm100_recurrence_workspace(const blstm_desc& d, int phase) {
   const SmallPlan sp = small_plan(d, phase);
   if (sp.ok) return small_workspace(d, sp, phase);

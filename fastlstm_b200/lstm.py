@@ -64,6 +64,11 @@ def plan_name(dtype, T, B, I, H, phase="fwd"):
     return _lib.load().blstm_plan_name(d, _PHASES[phase]).decode()
 
 
+def _family(dtype, T, B, I, H, phase, half_device=False):
+    """Which kernels (_lib.FAMILY_*) the library picks for this problem, on half of the SMs where half_device."""
+    return _lib.load().blstm_plan_family(_desc(dtype, T, B, I, H, _lib.FLAG_HALF_DEVICE if half_device else 0), _PHASES[phase])
+
+
 def plan_detail(dtype, T, B, I, H, phase="fwd", half_device=False):
     """One-line description of the launch geometry the library picks for this problem (on half of the SMs)."""
     import ctypes
@@ -276,7 +281,7 @@ def _shares_device(dtype, T, B, I, H):
     """True when two launches of this layer's recurrences can run side by side to advantage: clusters that wait
     for nothing outside themselves, and enough steps to pay for the streams (some 30 us of host time)."""
     Ip, Hp = _padded_sizes(dtype, I, H, T, B) or (I, H)
-    return T >= 48 and all("small-batch" in plan_detail(dtype, T, B, Ip, Hp, phase) for phase in ("fwd", "bwd"))
+    return T >= 48 and all(_family(dtype, T, B, Ip, Hp, phase) == _lib.FAMILY_SMALL_BATCH for phase in ("fwd", "bwd"))
 
 
 @functools.lru_cache(maxsize=1024)
@@ -286,7 +291,7 @@ def _wavefront_pays(dtype, T, B, H, grad):
     H=512 6.8 ms as a wavefront, 6.4 without; T=256, B=32, H=256 1.8 and 1.25; T=128, B=200, H=768 3.4 both).  Inference
     gains from 128 steps on where half of the device has them too (T=256, B=128, H=512: 1.44 -> 1.15 ms)."""
     def on_chip(half):
-        return all(any(w in plan_detail(dtype, T, B, H, H, phase, half) for w in ("resident weights", "small-batch"))
+        return all(_family(dtype, T, B, H, H, phase, half) in (_lib.FAMILY_RESIDENT, _lib.FAMILY_SMALL_BATCH)
                    for phase in (("fwd", "bwd") if grad else ("fwd",)))
     return not on_chip(False) or (not grad and T >= 128 and on_chip(True))
 

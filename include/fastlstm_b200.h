@@ -109,6 +109,20 @@ size_t blstm_workspace_bytes(const blstm_desc* d, int phase);
  * choice, fastlstm/configs.py:146-276 (prune_persistent_configs) and :29-58. */
 const char* blstm_plan_name(const blstm_desc* d, int phase);
 
+/* The kernels behind a plan, for callers that arrange launches around them (which fit beside each other, which leave
+ * something to overlap).  BLSTM_FAMILY_NONE: invalid arguments. */
+enum {
+  BLSTM_FAMILY_NONE = 0,
+  BLSTM_FAMILY_GENERIC = 1,     /* CUDA cores, any size                                                    */
+  BLSTM_FAMILY_STEP = 2,        /* one timestep as one launch (BLSTM_PHASE_FWD_OP)                         */
+  BLSTM_FAMILY_FUSED = 3,       /* projection inside the time loop (BLSTM_PHASE_FWD_OP)                    */
+  BLSTM_FAMILY_F32_CLUSTER = 4, /* fp32, clusters that wait for nothing outside themselves                 */
+  BLSTM_FAMILY_SMALL_BATCH = 5, /* 16-bit, the same                                                        */
+  BLSTM_FAMILY_RESIDENT = 6,    /* 16-bit, weights in tensor memory, grid-wide hand-off                    */
+  BLSTM_FAMILY_BATCH_TILES = 7  /* 16-bit, 128 batch rows on the M side, grid-wide hand-off                */
+};
+int blstm_plan_family(const blstm_desc* d, int phase);
+
 /* Writes a one-line, human-readable description of the launch geometry the phase will use
  * (tile sizes, interleaved batch tiles, grid, ring depth) into the HOST buffer `buf`.
  * Read-only; stands in for inspecting the reference's chosen autotune config

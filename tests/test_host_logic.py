@@ -293,3 +293,30 @@ def test_memory_that_two_streams_share_is_not_reused_under_a_queued_read(monkeyp
     for i, e in enumerate(log):
         if e == ("main", "cat"):
             assert ("side", "waits for", "main") in log[i + 1:i + 4]
+
+
+def test_how_a_layer_runs_does_not_hang_on_the_words_of_a_plan(monkeypatch):
+    # plan_detail is text for people; the family behind it is what the host arranges launches by
+    from fastlstm_b200 import _lib, lstm
+    cases = [(dt, T, B, H) for dt in (torch.float16, torch.bfloat16, torch.float32) for T in (8, 64, 256)
+             for B in (8, 64, 512, 1500, 4096) for H in (64, 128, 192, 320, 512, 576, 1088)]
+    words = {"small-batch": _lib.FAMILY_SMALL_BATCH, "resident weights": _lib.FAMILY_RESIDENT, "TI=": _lib.FAMILY_BATCH_TILES, "generic": _lib.FAMILY_GENERIC}
+    seen = set()
+    for dt, T, B, H in cases:
+        if dt == torch.float32:
+            continue
+        for phase in ("fwd", "bwd"):
+            for half in (False, True):
+                want = next(f for w, f in words.items() if w in lstm.plan_detail(dt, T, B, H, H, phase, half))
+                assert lstm._family(dt, T, B, H, H, phase, half) == want
+                seen.add(want)
+    assert len(seen) == 4
+
+    def ways():
+        lstm._shares_device.cache_clear()
+        lstm._wavefront_pays.cache_clear()
+        return [(lstm._shares_device(dt, T, B, H, H), lstm._wavefront_pays(dt, T, B, H, True), lstm._wavefront_pays(dt, T, B, H, False))
+                for dt, T, B, H in cases]
+    before = ways()
+    monkeypatch.setattr(lstm, "plan_detail", lambda *a, **k: "reworded")
+    assert ways() == before and len(set(before)) > 2
