@@ -809,15 +809,20 @@ int resident_clusters(int nc) {
 // Whether the plan beats the tcgen05 kernels: those with resident weights (multiples of 64 from 256 on; smaller sizes: the
 // general ones) take nearly the same time for any batch of up to several hundred rows, these about the same for
 // every chunk of 8 rows after the first, so the line is a number of chunks per cluster.  us per step (B200), these against
-// resident weights, forward: H = 256, B = 128 / 256 / 512: 1.3 / 2.1 / 3.3 against 2.2 / 2.3 / 2.6; H = 320, B = 128 / 256: 2.1 / 3.4
-// against 2.3 / 2.7; H = 512, B = 32 / 64 / 128 / 256: 1.6 / 2.3 / 3.2 / 5.3 against 2.6 / 2.6 / 2.6 / 2.9; H = 640, B = 16 / 64: 2.2 / 4.2
-// against 2.7 / 2.7.  Backward: H = 256, B = 256 / 512: 2.1 / 3.4 against 2.6 / 3.2; H = 512, B = 128 / 256: 2.6 / 4.1 against 3.0 / 3.5.
-// (Backward from H = 448 on the line lies before B = 128, so that the halves of a batch of 256 sum in its order.)
+// the others at 1, 2, 3, ... chunks, a dash where the line lies.
+// Forward: H = 192: 8: 3.5 / 5.5 (nothing saved: 4.5) - 10: 4.4 / 5.6 (4.6), 12: 5.3 / 5.6 (4.6; and two layers as a wavefront beat both);
+// H = 256: 3: 2.1 / 2.8, 4: 2.4 / 3.1 - 5: 3.3 / 3.1; H = 320: 3: 2.0 / 2.8, 4: 2.7 / 2.9 - 5: 3.4 / 3.2; H = 384: 2: 1.7 / 2.9, 3: 2.4 / 2.9 -
+// 4: 3.3 / 3.3; H = 448: 3: 2.8 / 3.1 - 4: 3.7 / 3.4; H = 512: 1: 1.6 / 3.0, 2: 2.2 / 3.1 - 3: 3.2 / 3.1 to 3.5, 5: 5.3 / 3.5;
+// H = 576: 1: 1.9 / 3.2 - 2: 3.7 / 3.2; H = 640: 1: 2.2 / 3.2 - 2: 4.2 / 3.2; H = 768: 1: 2.5 / 3.4.
+// Backward: H = 192: 8: 4.7 / 5.0 - 9: 5.2 / 5.0; H = 256: 5: 3.3 / 3.6, 6: 3.9 / 4.9; H = 320: 4: 3.3 / 3.6 - 5: 4.0 / 3.6; H = 384: 4: 3.1 / 3.7 -
+// 5: 3.8 / 3.7; H = 448: 4: 3.7 / 3.9 - 5: 4.2 / 3.9; H = 512: 3: 2.5 / 3.4, 4: 3.3 / 3.9, 5: 4.05 / 3.91; H = 576: 2: 3.3 / 3.5; H = 640: 2: 3.3 / 3.6
+// (more does not fit).  At H = 512 five chunks are a tie but for 4 %, and taken so that a batch of 256 rows and its
+// halves go through the same kernels and agree bit for bit, which they do not across a line.
 // (General kernels, forward: H = 64, B = 64: 1.9 -> 0.59; H = 192: 4.4 a step at any of these batches.)
 static bool small_plan_pays(int H, const SmallPlan& p, int phase) {
   if (H <= 128) return true;
-  if (phase == BLSTM_PHASE_BWD) return H < 256 || p.nch <= (H <= 384 ? 4 : 2);
-  return p.nch <= (H < 256 ? 8 : H <= 320 ? 3 : H <= 512 ? 2 : 1);
+  if (phase == BLSTM_PHASE_BWD) return p.nch <= (H < 256 ? 8 : H == 256 ? 6 : H <= 448 ? 4 : H <= 512 ? 5 : 2);
+  return p.nch <= (H < 256 ? 8 : H <= 320 ? 4 : H <= 448 ? 3 : H <= 512 ? 2 : 1);
 }
 
 SmallPlan small_plan(const blstm_desc& d, int phase) {

@@ -15,7 +15,9 @@ pytestmark = pytest.mark.gpu
 # one row, one row past a chunk, chunks shared by replicas
 SHAPES = [(5, 3, 8), (4, 9, 24), (9, 1300, 64), (3, 1, 64), (5, 33, 72), (6, 270, 128), (4, 17, 136), (7, 120, 200),
           (5, 360, 256), (1, 9, 256), (6, 8, 264), (4, 57, 288), (5, 100, 384), (3, 40, 448), (6, 110, 512), (2, 1, 512),
-          (4, 15, 520), (3, 50, 640), (4, 9, 768)]
+          (4, 15, 520), (3, 50, 640), (4, 9, 768),
+          # as many chunks a cluster as the dispatch gives them: 4 and 3
+          (4, 480, 256), (4, 224, 320), (3, 168, 448)]
 
 
 def _plan(d, phase):

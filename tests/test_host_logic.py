@@ -320,3 +320,14 @@ def test_how_a_layer_runs_does_not_hang_on_the_words_of_a_plan(monkeypatch):
     before = ways()
     monkeypatch.setattr(lstm, "plan_detail", lambda *a, **k: "reworded")
     assert ways() == before and len(set(before)) > 2
+
+
+def test_small_batch_kernels_where_they_measured_faster():
+    # hidden size -> most rows (forward, backward) that the small-batch recurrences get: 15 clusters of 8 CTAs at 256, 7 of 16
+    # above, eight rows a chunk.  At 512 a batch of 256 and its halves stay in the same backward kernel.
+    from fastlstm_b200 import _lib, lstm
+    for H, most in {192: (960, 960), 256: (480, 720), 384: (168, 224), 512: (112, 280), 576: (56, 112)}.items():
+        for phase, n in zip(("fwd", "bwd"), most):
+            for B in (8, n // 2, n, n + 1):
+                small = lstm._family(torch.bfloat16, 64, B, H, H, phase) == _lib.FAMILY_SMALL_BATCH
+                assert small == (B <= n), (H, B, phase)
