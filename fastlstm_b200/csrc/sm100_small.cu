@@ -15,7 +15,7 @@
 //   - results go to the peers' shared memory with st.async, whose bytes complete the peers' mbarriers: one way
 //     through the cluster takes ~0.5 k clocks (an all-to-all of 16 x 512 B, 1.3 k clocks with the waits), where
 //     store -> release -> counter -> poll -> TMA through L2 takes 4-6 k.
-// Rows are worked in chunks of 8 or 16 with barriers of their own, so that with several chunks per cluster one
+// Rows are worked in chunks of 8 with barriers of their own, so that with several chunks per cluster one
 // chunk's exchange hides behind the others' products.
 // What it measured: at small_plan_pays below.
 #include <stdio.h>
@@ -107,7 +107,7 @@ template <int KR, int KSPL, bool CL, typename T16>
 __global__ void __launch_bounds__(384, 1)
 small_fwd_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUtensorMap tmH,
                  const __grid_constant__ CUtensorMap tmC, const SmallFwdParams p) {
-  constexpr int NTC = 1, CR = 8;                                // n-tiles and rows of a chunk
+  constexpr int CR = 8;                                         // rows of a chunk
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   const int H = p.H, T = p.T, B = p.B, KS = p.ks, gc = p.gc;
@@ -128,7 +128,7 @@ small_fwd_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant_
   const uint32_t part = (uint32_t)CR * gc * 16, slot_b = 6 * part;
   const uint32_t h_off = (uint32_t)S * slot_b;
   const uint32_t c_off = h_off + (uint32_t)p.nch * 2 * CR * pitch;
-  const uint32_t w_off = c_off + (uint32_t)p.nch * gc * 256 * NTC;
+  const uint32_t w_off = c_off + (uint32_t)p.nch * gc * 256;
   const uint32_t b_off = w_off + (uint32_t)gc * (KSPL == 2 ? 2 : KS - KR) * 1024;
   uint64_t* hbar = reinterpret_cast<uint64_t*>(smem + b_off);   // [chunk][parity] h complete
   uint64_t* full = hbar + 2 * SB_MAX_CHUNKS;                    // [S] slot filled
@@ -136,7 +136,7 @@ small_fwd_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant_
   uint64_t* pbar = staged + SB_MAX_SLOTS;                       // [gl][item parity] partial sums passed on
   volatile int* dead = reinterpret_cast<volatile int*>(pbar + 8);
   float4* psum = reinterpret_cast<float4*>(smem + w_off) + gl * 64 + lane;   // [item parity][gl][tile][lane] (K split; no weights there)
-  float2* cst = reinterpret_cast<float2*>(smem + c_off) + gl * NTC * 32 + lane;   // [chunk][gl][NTC][lane]
+  float2* cst = reinterpret_cast<float2*>(smem + c_off) + gl * 32 + lane;   // [chunk][gl][lane]
   const uint4* w_s = reinterpret_cast<const uint4*>(smem + w_off) + (size_t)gl * (KS - KR) * 64 + lane;
   const uint32_t sbase = smem_u32(smem);
   const T16* out = reinterpret_cast<const T16*>(p.out);
@@ -220,13 +220,11 @@ small_fwd_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant_
         }
   }
   // ---- own cell states
-  for (int ch = rep; ch < nch; ch += p.rpl)
-#pragma unroll
-    for (int nt = 0; nt < NTC; ++nt) {
-      const int r = ch * CR + nt * 8 + u;
-      const uint32_t v = (live && r < rows) ? ldg4(cell + (size_t)(row0 + r) * H + unit0 + 2 * c) : 0u;
-      cst[(ch * gc * NTC + nt) * 32] = cvt2<T16>(transpose8x8(v));
-    }
+  for (int ch = rep; ch < nch; ch += p.rpl) {
+    const int r = ch * CR + u;
+    const uint32_t v = (live && r < rows) ? ldg4(cell + (size_t)(row0 + r) * H + unit0 + 2 * c) : 0u;
+    cst[ch * gc * 32] = cvt2<T16>(transpose8x8(v));
+  }
   // the shared-memory weights are in place (all computing warps come here, before anything can give up)
   asm volatile("bar.sync 1, %0;" ::"r"(32 * gc * KSPL * p.rpl) : "memory");
   // shared::cluster addresses of this lane's destinations: CTAs c, c+4, c+8, c+12
@@ -246,10 +244,8 @@ small_fwd_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant_
     if (finish && !wait_inline(&full[k & (S - 1)], (uint32_t)(k / S) & 1u, dead, p.ctl, p.limit_ns, t, cl)) break;
     uint32_t pw[4] = {0, 0, 0, 0};
     if (finish) ldmatrix_x4_trans(sl + so_g, pw);
-    float acc[2][2][NTC][4] = {};                               // [K parity][tile][n-tile]
-    float2 cs[NTC];
-#pragma unroll
-    for (int nt = 0; nt < NTC; ++nt) cs[nt] = cst[(ch * gc * NTC + nt) * 32];
+    float acc[2][2][4] = {};                                    // [K parity][tile]
+    float2 cs = cst[ch * gc * 32];
     if (t > 0) {
       uint64_t* bar = &hbar[2 * ch + par];
       if (!wait_inline(bar, (uint32_t)((t - 1) >> 1) & 1u, dead, p.ctl, p.limit_ns, t, cl)) break;
@@ -258,25 +254,20 @@ small_fwd_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant_
     // operand fetches run ahead of the MMAs (one at a time they cost as much as the MMAs)
     const uint32_t hb = sbase + h_off + (uint32_t)((ch * 2 + par) * CR + (lane & 7)) * pitch + (lane >> 3) * 16 + kh * KR * 32;
     constexpr int AH = KR / 2 < 3 ? KR / 2 : 3;
-    uint32_t b[AH + 1][NTC][4];
+    uint32_t b[AH + 1][4];
 #pragma unroll
     for (int i = 0; i < AH; ++i)
-#pragma unroll
-      for (int nt = 0; nt < NTC; ++nt) ldmatrix_x4(hb + nt * 8 * pitch + i * 64, b[i][nt]);
+      ldmatrix_x4(hb + i * 64, b[i]);
 #pragma unroll
     for (int i = 0; i < KR / 2; ++i) {
       if (i + AH < KR / 2) {
-#pragma unroll
-        for (int nt = 0; nt < NTC; ++nt) ldmatrix_x4(hb + nt * 8 * pitch + (i + AH) * 64, b[(i + AH) % (AH + 1)][nt]);
+        ldmatrix_x4(hb + (i + AH) * 64, b[(i + AH) % (AH + 1)]);
       }
-#pragma unroll
-      for (int nt = 0; nt < NTC; ++nt) {
-        const uint32_t(&bb)[4] = b[i % (AH + 1)][nt];
-        mma16816<T16>(acc[0][0][nt], w[2 * i][0], bb[0], bb[1]);
-        mma16816<T16>(acc[0][1][nt], w[2 * i][1], bb[0], bb[1]);
-        mma16816<T16>(acc[1][0][nt], w[2 * i + 1][0], bb[2], bb[3]);
-        mma16816<T16>(acc[1][1][nt], w[2 * i + 1][1], bb[2], bb[3]);
-      }
+      const uint32_t(&bb)[4] = b[i % (AH + 1)];
+      mma16816<T16>(acc[0][0], w[2 * i][0], bb[0], bb[1]);
+      mma16816<T16>(acc[0][1], w[2 * i][1], bb[0], bb[1]);
+      mma16816<T16>(acc[1][0], w[2 * i + 1][0], bb[2], bb[3]);
+      mma16816<T16>(acc[1][1], w[2 * i + 1][1], bb[2], bb[3]);
     }
     if constexpr (KSPL == 1) {
 #pragma unroll 2
@@ -287,26 +278,23 @@ small_fwd_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant_
           const uint4 v = w_s[((ks - KR) * 2 + i) * 32];
           a[i >> 1][i & 1][0] = v.x; a[i >> 1][i & 1][1] = v.y; a[i >> 1][i & 1][2] = v.z; a[i >> 1][i & 1][3] = v.w;
         }
-#pragma unroll
-        for (int nt = 0; nt < NTC; ++nt) {
-          uint32_t bb[4];
-          ldmatrix_x4(hb + nt * 8 * pitch + ks * 32, bb);
-          mma16816<T16>(acc[0][0][nt], a[0][0], bb[0], bb[1]);
-          mma16816<T16>(acc[0][1][nt], a[0][1], bb[0], bb[1]);
-          mma16816<T16>(acc[1][0][nt], a[1][0], bb[2], bb[3]);
-          mma16816<T16>(acc[1][1][nt], a[1][1], bb[2], bb[3]);
-        }
+        uint32_t bb[4];
+        ldmatrix_x4(hb + ks * 32, bb);
+        mma16816<T16>(acc[0][0], a[0][0], bb[0], bb[1]);
+        mma16816<T16>(acc[0][1], a[0][1], bb[0], bb[1]);
+        mma16816<T16>(acc[1][0], a[1][0], bb[2], bb[3]);
+        mma16816<T16>(acc[1][1], a[1][1], bb[2], bb[3]);
       }
     } else {
       // the other half's partial sums: passed on through shared memory, or taken
 #pragma unroll
       for (int tile = 0; tile < 2; ++tile)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) acc[0][tile][0][e] += acc[1][tile][0][e];
+        for (int e = 0; e < 4; ++e) acc[0][tile][e] += acc[1][tile][e];
       float4* ps = psum + (k & 1) * gc * 64;
       if (!finish) {
-        ps[0] = make_float4(acc[0][0][0][0], acc[0][0][0][1], acc[0][0][0][2], acc[0][0][0][3]);
-        ps[32] = make_float4(acc[0][1][0][0], acc[0][1][0][1], acc[0][1][0][2], acc[0][1][0][3]);
+        ps[0] = make_float4(acc[0][0][0], acc[0][0][1], acc[0][0][2], acc[0][0][3]);
+        ps[32] = make_float4(acc[0][1][0], acc[0][1][1], acc[0][1][2], acc[0][1][3]);
         __syncwarp();
         if (lane == 0) mbar_arrive(&pbar[2 * gl + (k & 1)]);
         if (ch == last_ch) { ch = rep; ++t; } else ch += p.rpl;
@@ -314,54 +302,50 @@ small_fwd_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant_
       }
       if (!wait_inline(&pbar[2 * gl + (k & 1)], (uint32_t)(k >> 1) & 1u, dead, p.ctl, p.limit_ns, t, cl)) break;
       const float4 o0 = ps[0], o1 = ps[32];
-      acc[1][0][0][0] = o0.x; acc[1][0][0][1] = o0.y; acc[1][0][0][2] = o0.z; acc[1][0][0][3] = o0.w;
-      acc[1][1][0][0] = o1.x; acc[1][1][0][1] = o1.y; acc[1][1][0][2] = o1.z; acc[1][1][0][3] = o1.w;
-      cs[0] = cst[ch * gc * 32];                                // (the other half may have written it)
+      acc[1][0][0] = o0.x; acc[1][0][1] = o0.y; acc[1][0][2] = o0.z; acc[1][0][3] = o0.w;
+      acc[1][1][0] = o1.x; acc[1][1][1] = o1.y; acc[1][1][2] = o1.z; acc[1][1][3] = o1.w;
+      cs = cst[ch * gc * 32];                                // (the other half may have written it)
     }
-    uint32_t gw[NTC][4];
+    uint32_t gw[4];
+    float g4[4][2];
 #pragma unroll
-    for (int nt = 0; nt < NTC; ++nt) {
-      float g4[4][2];
-#pragma unroll
-      for (int g = 0; g < 4; ++g)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const float2 f = cvt2<T16>(pw[g]);
-          g4[g][e] = acc[0][g >> 1][nt][(g & 1) * 2 + e] + acc[1][g >> 1][nt][(g & 1) * 2 + e] + (e ? f.y : f.x);
-        }
-      float hv[2], cv[2];
+    for (int g = 0; g < 4; ++g)
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        cv[e] = sigmoid_fast(g4[1][e]) * (e ? cs[nt].y : cs[nt].x) + sigmoid_fast(g4[0][e]) * tanh_fast(g4[2][e]);
-        hv[e] = sigmoid_fast(g4[3][e]) * tanh_fast(cv[e]);
+        const float2 f = cvt2<T16>(pw[g]);
+        g4[g][e] = acc[0][g >> 1][(g & 1) * 2 + e] + acc[1][g >> 1][(g & 1) * 2 + e] + (e ? f.y : f.x);
       }
-      // h and c as rows of 8 units (16 bytes); row u's h goes to the whole cluster
-      stmatrix_x2_trans(sl + so_hc + nt * gc * 128, pk2<T16>(hv[0], hv[1]), pk2<T16>(cv[0], cv[1]));
-      __syncwarp();
-      const uint4 v = ld_shared16(sl + so_h + nt * gc * 128);
-      const uint32_t ho = h_off + (uint32_t)((ch * 2 + (par ^ 1)) * CR + nt * 8 + u) * pitch + unit0 * 2;
-      if (live && ch * CR + nt * 8 + u < rows && t + 1 < T && !p.no_arrive) {
-        if (CL) {
-          const uint32_t bo = b_off + (uint32_t)(2 * ch + (par ^ 1)) * 8;
+    float hv[2], cv[2];
 #pragma unroll
-          for (int i = 0; i < 4; ++i)
-            if (c + 4 * i < p.nc) st_async16(peer[i] + ho, v, peer[i] + bo);
-        } else if (c == 0) {
-          st_shared16(sbase + ho, v);
-        }
-      }
-      cst[(ch * gc * NTC + nt) * 32] = make_float2(cv[0], cv[1]);
-#pragma unroll
-      for (int g = 0; g < 4; ++g) gw[nt][g] = pk2<T16>(g4[g][0], g4[g][1]);
+    for (int e = 0; e < 2; ++e) {
+      cv[e] = sigmoid_fast(g4[1][e]) * (e ? cs.y : cs.x) + sigmoid_fast(g4[0][e]) * tanh_fast(g4[2][e]);
+      hv[e] = sigmoid_fast(g4[3][e]) * tanh_fast(cv[e]);
     }
+    // h and c as rows of 8 units (16 bytes); row u's h goes to the whole cluster
+    stmatrix_x2_trans(sl + so_hc, pk2<T16>(hv[0], hv[1]), pk2<T16>(cv[0], cv[1]));
+    __syncwarp();
+    const uint4 v = ld_shared16(sl + so_h);
+    const uint32_t ho = h_off + (uint32_t)((ch * 2 + (par ^ 1)) * CR + u) * pitch + unit0 * 2;
+    if (live && ch * CR + u < rows && t + 1 < T && !p.no_arrive) {
+      if (CL) {
+        const uint32_t bo = b_off + (uint32_t)(2 * ch + (par ^ 1)) * 8;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (c + 4 * i < p.nc) st_async16(peer[i] + ho, v, peer[i] + bo);
+      } else if (c == 0) {
+        st_shared16(sbase + ho, v);
+      }
+    }
+    cst[ch * gc * 32] = make_float2(cv[0], cv[1]);
+#pragma unroll
+    for (int g = 0; g < 4; ++g) gw[g] = pk2<T16>(g4[g][0], g4[g][1]);
     if (!CL) {
       __syncwarp();
       if (lane == 0) mbar_arrive(&hbar[2 * ch + (par ^ 1)]);
     }
     // off the chain: the final pre-activations in place, and the previous item's boxes on their way
     if (!p.inference) {
-#pragma unroll
-      for (int nt = 0; nt < NTC; ++nt) stmatrix_x4_trans(sl + so_g + nt * gc * 128, gw[nt][0], gw[nt][1], gw[nt][2], gw[nt][3]);
+      stmatrix_x4_trans(sl + so_g, gw[0], gw[1], gw[2], gw[3]);
     }
     __syncwarp();
     if (lane == 0) mbar_arrive(&staged[k & (S - 1)]);
@@ -384,17 +368,21 @@ small_fwd_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant_
 // The two meet at barriers over two operand buffers, so with several chunks both are busy.  Global traffic as in
 // the forward kernel: slots [gate i f g o | c | dout][row][units], d_ifgo written back over the gates.
 // =====================================================================================
-template <int MPW, int KR, int NTC, bool CL, typename T16>
+template <int MPW, int KR, bool CL, typename T16>
 __global__ void __launch_bounds__(512, 1)
 small_bwd_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUtensorMap tmC,
                  const __grid_constant__ CUtensorMap tmO, const __grid_constant__ CUtensorMap tmD, const SmallBwdParams p) {
-  constexpr int CR = 8 * NTC;
+  constexpr int CR = 8;                                         // rows of a chunk
   constexpr int S = 8;                                          // slots of the ring
   // A single tile per warp splits its K steps over two accumulators (a chain of 16 MMAs takes 350 clocks)
   constexpr int NA = MPW == 1 ? 2 : 1;
+  // All K steps in registers but for five groups of units a CTA and, in one CTA, fewer than eight: there the number of
+  // groups follows from KR, and a step with addresses known at compile time takes 5 to 11 % less (H = 384, B = 32: 1.23 ->
+  // 1.15 us, H = 512, B = 128: 2.8 -> 2.5; H = 512, B = 32 5 % more).
+  constexpr bool TAIL = CL ? MPW == 5 : KR < 16;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  const int H = p.H, T = p.T, B = p.B, gc = p.gc;
+  const int H = p.H, T = p.T, B = p.B, gc = TAIL ? p.gc : KR / 2;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int u = lane >> 2, c = lane & 3;
   const int rank = CL ? (int)cluster_ctarank() : 0;
@@ -403,19 +391,17 @@ small_bwd_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant_
   const int rows = min(p.rows, B - row0);
   const int nch = rows > 0 ? (rows + CR - 1) / CR : 0;
   const int pitch = gc * 64 + 16;
-  const int nm = p.mgroups * p.ksp;                             // product warps
-  const int nsrc = p.nc * p.ksp;
+  const int nm = p.mgroups;                                     // product warps
   const int lunits = min(gc * 8, max(0, H - rank * gc * 8));    // units this CTA owns
-  const int pairs = (gc + p.ksp - 1) / p.ksp;                   // pairs of K steps (one unit group each) of a product warp
 
-  // shared memory: ring | operand buffers [2][CR][pitch] | partial sums [chunk][parity][src][NTC][gc*8][8] | states | weights | barriers
+  // shared memory: ring | operand buffers [2][CR][pitch] | partial sums [chunk][parity][src][gc*8][8] | states | weights | barriers
   const uint32_t part = (uint32_t)CR * gc * 16, slot_b = 6 * part;
-  const uint32_t src_b = (uint32_t)NTC * gc * 256;              // bytes of one source's partial sums
+  const uint32_t src_b = (uint32_t)gc * 256;                    // bytes of one source's partial sums
   const uint32_t d_off = S * slot_b;
   const uint32_t r_off = d_off + 2u * CR * pitch;
-  const uint32_t s_off = r_off + (uint32_t)p.nch * 2 * nsrc * src_b;
-  const uint32_t w_off = s_off + (uint32_t)p.nch * gc * NTC * 512;
-  const uint32_t b_off = w_off + (uint32_t)nm * MPW * (pairs - KR / 2) * 1024;
+  const uint32_t s_off = r_off + (uint32_t)p.nch * 2 * p.nc * src_b;
+  const uint32_t w_off = s_off + (uint32_t)p.nch * gc * 512;
+  const uint32_t b_off = w_off + (uint32_t)nm * MPW * (gc - KR / 2) * 1024;
   uint64_t* xbar = reinterpret_cast<uint64_t*>(smem + b_off);   // [chunk][parity] partial sums complete
   uint64_t* full = xbar + 2 * SB_MAX_CHUNKS;                    // [S] slot filled
   uint64_t* staged = full + S;                                  // [S] slot's d_ifgo in place
@@ -428,7 +414,7 @@ small_bwd_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant_
   for (uint32_t i = threadIdx.x; i < (w_off - d_off) / 16; i += blockDim.x)
     *reinterpret_cast<uint4*>(smem + d_off + (size_t)i * 16) = make_uint4(0, 0, 0, 0);
   auto expect = [&](int ch) {                                   // bytes a chunk's partial sums bring in
-    return nsrc * lunits * 16 * ((min(CR, rows - ch * CR) + 3) / 4);
+    return p.nc * lunits * 16 * ((min(CR, rows - ch * CR) + 3) / 4);
   };
   if (threadIdx.x == 0) {
     *dead = 0;
@@ -487,27 +473,25 @@ small_bwd_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant_
     // ---------------------------------------------------------------- gate maths
     const int unit0 = (rank * gc + warp) * 8;
     const bool live = unit0 < H;
-    float4* st_s = reinterpret_cast<float4*>(smem + s_off) + warp * NTC * 32 + lane;   // [chunk][gl][NTC][lane]: dc, c[t+1] (2 rows each)
-    for (int ch = 0; ch < nch; ++ch)
-#pragma unroll
-      for (int nt = 0; nt < NTC; ++nt) {
-        const int r = ch * CR + nt * 8 + u;
-        const bool rok = live && r < rows;
-        const size_t o = (size_t)(row0 + r) * H + unit0 + 2 * c;
-        const uint32_t v = (rok && p.dc_n) ? ldg4(reinterpret_cast<const T16*>(p.dc_n) + o) : 0u;
-        const uint32_t v1 = rok ? ldg4(reinterpret_cast<const T16*>(p.cell) + (size_t)T * B * H + o) : 0u;
-        const float2 d2 = cvt2<T16>(transpose8x8(v)), c2 = cvt2<T16>(transpose8x8(v1));
-        st_s[(ch * gc * NTC + nt) * 32] = make_float4(d2.x, d2.y, c2.x, c2.y);
-      }
+    float4* st_s = reinterpret_cast<float4*>(smem + s_off) + warp * 32 + lane;   // [chunk][gl][lane]: dc, c[t+1] (2 rows each)
+    for (int ch = 0; ch < nch; ++ch) {
+      const int r = ch * CR + u;
+      const bool rok = live && r < rows;
+      const size_t o = (size_t)(row0 + r) * H + unit0 + 2 * c;
+      const uint32_t v = (rok && p.dc_n) ? ldg4(reinterpret_cast<const T16*>(p.dc_n) + o) : 0u;
+      const uint32_t v1 = rok ? ldg4(reinterpret_cast<const T16*>(p.cell) + (size_t)T * B * H + o) : 0u;
+      const float2 d2 = cvt2<T16>(transpose8x8(v)), c2 = cvt2<T16>(transpose8x8(v1));
+      st_s[ch * gc * 32] = make_float4(d2.x, d2.y, c2.x, c2.y);
+    }
     const uint32_t so_g = swz((lane >> 3) * part + (lane & 7) * gc * 16 + warp * 16, gc);
     const uint32_t so_cd = swz((4 + ((lane >> 3) & 1)) * part + (lane & 7) * gc * 16 + warp * 16, gc);
     // dh of this lane's unit and rows: the sum of the sources' partial sums
-    auto gather = [&](int st, int ch, int nt, float (&dh)[2]) {
-      const float2* src = reinterpret_cast<const float2*>(smem + r_off + (size_t)(ch * 2 + ((st - 1) & 1)) * nsrc * src_b +
-                                                          ((size_t)nt * gc * 8 + warp * 8) * 32) + lane;
+    auto gather = [&](int st, int ch, float (&dh)[2]) {
+      const float2* src = reinterpret_cast<const float2*>(smem + r_off + (size_t)(ch * 2 + ((st - 1) & 1)) * p.nc * src_b +
+                                                          warp * 256) + lane;
       dh[0] = dh[1] = 0.f;
 #pragma unroll 8
-      for (int s = 0; s < nsrc; ++s) {
+      for (int s = 0; s < p.nc; ++s) {
         const float2 v = src[(size_t)s * (src_b / 8)];
         dh[0] += v.x;
         dh[1] += v.y;
@@ -522,82 +506,67 @@ small_bwd_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant_
         const uint32_t sl = sbase + (uint32_t)(k & (S - 1)) * slot_b;
         if (!wait_inline(&full[k & (S - 1)], (uint32_t)(k / S) & 1u, dead, p.ctl, p.limit_ns, T - 1 - st, cl)) { ok = false; break; }
         // all that does not depend on dh
-        float4 sv[NTC];
-        float2 cv[NTC], dv[NTC];
-        float fA[NTC][2], fO[NTC][2], fI[NTC][2], fF[NTC][2], fG[NTC][2], sF[NTC][2];
+        float fA[2], fO[2], fI[2], fF[2], fG[2], sF[2];
+        uint32_t pw[4], pc, pd;
+        ldmatrix_x4_trans(sl + so_g, pw);
+        ldmatrix_x2_trans(sl + so_cd, pc, pd);
+        const float4 sv = st_s[ch * gc * 32];
+        const float2 cv = cvt2<T16>(pc), dv = cvt2<T16>(pd);
+        const float2 x0 = cvt2<T16>(pw[0]), x1 = cvt2<T16>(pw[1]), x2 = cvt2<T16>(pw[2]), x3 = cvt2<T16>(pw[3]);
 #pragma unroll
-        for (int nt = 0; nt < NTC; ++nt) {
-          uint32_t pw[4], pc, pd;
-          ldmatrix_x4_trans(sl + so_g + nt * gc * 128, pw);
-          ldmatrix_x2_trans(sl + so_cd + nt * gc * 128, pc, pd);
-          sv[nt] = st_s[(ch * gc * NTC + nt) * 32];
-          cv[nt] = cvt2<T16>(pc);
-          dv[nt] = cvt2<T16>(pd);
-          const float2 x0 = cvt2<T16>(pw[0]), x1 = cvt2<T16>(pw[1]), x2 = cvt2<T16>(pw[2]), x3 = cvt2<T16>(pw[3]);
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const float si = sigmoid_fast(e ? x0.y : x0.x), sf = sigmoid_fast(e ? x1.y : x1.x), so = sigmoid_fast(e ? x3.y : x3.x);
-            const float tg = tanh_fast(e ? x2.y : x2.x), tc = tanh_fast(e ? sv[nt].w : sv[nt].z);
-            fA[nt][e] = so * (1.f - tc * tc);
-            fI[nt][e] = tg * si * (1.f - si);
-            fF[nt][e] = (e ? cv[nt].y : cv[nt].x) * sf * (1.f - sf);
-            fG[nt][e] = si * (1.f - tg * tg);
-            fO[nt][e] = tc * so * (1.f - so);
-            sF[nt][e] = sf;
-          }
+        for (int e = 0; e < 2; ++e) {
+          const float si = sigmoid_fast(e ? x0.y : x0.x), sf = sigmoid_fast(e ? x1.y : x1.x), so = sigmoid_fast(e ? x3.y : x3.x);
+          const float tg = tanh_fast(e ? x2.y : x2.x), tc = tanh_fast(e ? sv.w : sv.z);
+          fA[e] = so * (1.f - tc * tc);
+          fI[e] = tg * si * (1.f - si);
+          fF[e] = (e ? cv.y : cv.x) * sf * (1.f - sf);
+          fG[e] = si * (1.f - tg * tg);
+          fO[e] = tc * so * (1.f - so);
+          sF[e] = sf;
         }
         if (st > 0) {
           uint64_t* bar = &xbar[2 * ch + ((st - 1) & 1)];
           if (!wait_inline(bar, (uint32_t)((st - 1) >> 1) & 1u, dead, p.ctl, p.limit_ns, T - 1 - st, cl)) { ok = false; break; }
           if (CL && warp == 0 && lane == 0 && st + 1 < T) mbar_expect_tx(bar, expect(ch));
         }
-        float q[NTC][4][2];
-#pragma unroll
-        for (int nt = 0; nt < NTC; ++nt) {
-          float dh[2] = {0.f, 0.f};
-          if (st > 0) gather(st, ch, nt, dh);
-          else if (p.dh_n) {
-            const int r = ch * CR + nt * 8 + u;
-            const uint32_t v = (live && r < rows) ? ldg4(reinterpret_cast<const T16*>(p.dh_n) + (size_t)(row0 + r) * H + unit0 + 2 * c) : 0u;
-            const float2 f = cvt2<T16>(transpose8x8(v));
-            dh[0] = f.x;
-            dh[1] = f.y;
-          }
-          float dcn[2];
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const float d = (e ? dv[nt].y : dv[nt].x) + dh[e];
-            const float dcv = fmaf(d, fA[nt][e], e ? sv[nt].y : sv[nt].x);
-            q[nt][0][e] = dcv * fI[nt][e];
-            q[nt][1][e] = dcv * fF[nt][e];
-            q[nt][2][e] = dcv * fG[nt][e];
-            q[nt][3][e] = d * fO[nt][e];
-            dcn[e] = dcv * sF[nt][e];
-          }
-          st_s[(ch * gc * NTC + nt) * 32] = make_float4(dcn[0], dcn[1], cv[nt].x, cv[nt].y);
+        float q[4][2];
+        float dh[2] = {0.f, 0.f};
+        if (st > 0) gather(st, ch, dh);
+        else if (p.dh_n) {
+          const int r = ch * CR + u;
+          const uint32_t v = (live && r < rows) ? ldg4(reinterpret_cast<const T16*>(p.dh_n) + (size_t)(row0 + r) * H + unit0 + 2 * c) : 0u;
+          const float2 f = cvt2<T16>(transpose8x8(v));
+          dh[0] = f.x;
+          dh[1] = f.y;
         }
+        float dcn[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const float d = (e ? dv.y : dv.x) + dh[e];
+          const float dcv = fmaf(d, fA[e], e ? sv.y : sv.x);
+          q[0][e] = dcv * fI[e];
+          q[1][e] = dcv * fF[e];
+          q[2][e] = dcv * fG[e];
+          q[3][e] = d * fO[e];
+          dcn[e] = dcv * sF[e];
+        }
+        st_s[ch * gc * 32] = make_float4(dcn[0], dcn[1], cv.x, cv.y);
         // operand buffer `par` is free once the product two items ago has read it
         if (k >= 2 && !wait_inline(&dempty[par], (uint32_t)((k >> 1) - 1) & 1u, dead, p.ctl, p.limit_ns, T - 1 - st, cl)) { ok = false; break; }
         const uint32_t dgs = sbase + d_off + (uint32_t)(par * CR) * pitch + warp * 64;
-        uint32_t w16[NTC][4];
+        uint32_t w16[4];
 #pragma unroll
-        for (int nt = 0; nt < NTC; ++nt) {
-#pragma unroll
-          for (int g = 0; g < 4; ++g) w16[nt][g] = pk2<T16>(q[nt][g][0], q[nt][g][1]);
-          stmatrix_x4_trans(dgs + (uint32_t)(nt * 8 + (lane & 7)) * pitch + (lane >> 3) * 16, w16[nt][0], w16[nt][1], w16[nt][2], w16[nt][3]);
-        }
+        for (int g = 0; g < 4; ++g) w16[g] = pk2<T16>(q[g][0], q[g][1]);
+        stmatrix_x4_trans(dgs + (uint32_t)(lane & 7) * pitch + (lane >> 3) * 16, w16[0], w16[1], w16[2], w16[3]);
         __syncwarp();
         if (lane == 0) mbar_arrive(&dfull[par]);
         // off the chain: d_ifgo for the TMA store, the bias gradient's sums (of the values as stored), the previous item's boxes
+        stmatrix_x4_trans(sl + so_g, w16[0], w16[1], w16[2], w16[3]);
+        const int rc = ch * CR + 2 * c;                         // this lane's two rows
 #pragma unroll
-        for (int nt = 0; nt < NTC; ++nt) {
-          stmatrix_x4_trans(sl + so_g + nt * gc * 128, w16[nt][0], w16[nt][1], w16[nt][2], w16[nt][3]);
-          const int rc = ch * CR + nt * 8 + 2 * c;              // this lane's two rows
-#pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            const float2 f = cvt2<T16>(w16[nt][g]);
-            db[g] += (rc < rows ? f.x : 0.f) + (rc + 1 < rows ? f.y : 0.f);
-          }
+        for (int g = 0; g < 4; ++g) {
+          const float2 f = cvt2<T16>(w16[g]);
+          db[g] += (rc < rows ? f.x : 0.f) + (rc + 1 < rows ? f.y : 0.f);
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&staged[k & (S - 1)]);
@@ -606,18 +575,15 @@ small_bwd_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant_
     // ---- gradients of the initial states
     for (int ch = 0; ch < nch && ok; ++ch) {
       if (!wait_inline(&xbar[2 * ch + ((T - 1) & 1)], (uint32_t)((T - 1) >> 1) & 1u, dead, p.ctl, p.limit_ns, -1, cl)) break;
-#pragma unroll
-      for (int nt = 0; nt < NTC; ++nt) {
-        float dh[2];
-        gather(T, ch, nt, dh);
-        const float4 sv = st_s[(ch * gc * NTC + nt) * 32];
-        const uint32_t hw = transpose8x8(pk2<T16>(dh[0], dh[1])), cw = transpose8x8(pk2<T16>(sv.x, sv.y));
-        const int r = ch * CR + nt * 8 + u;
-        if (live && r < rows) {
-          const size_t o = (size_t)(row0 + r) * H + unit0 + 2 * c;
-          stg4(reinterpret_cast<T16*>(p.dh0) + o, hw);
-          stg4(reinterpret_cast<T16*>(p.dc0) + o, cw);
-        }
+      float dh[2];
+      gather(T, ch, dh);
+      const float4 sv = st_s[ch * gc * 32];
+      const uint32_t hw = transpose8x8(pk2<T16>(dh[0], dh[1])), cw = transpose8x8(pk2<T16>(sv.x, sv.y));
+      const int r = ch * CR + u;
+      if (live && r < rows) {
+        const size_t o = (size_t)(row0 + r) * H + unit0 + 2 * c;
+        stg4(reinterpret_cast<T16*>(p.dh0) + o, hw);
+        stg4(reinterpret_cast<T16*>(p.dc0) + o, cw);
       }
     }
     if (p.db_part) {
@@ -637,22 +603,20 @@ small_bwd_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant_
   if (CL) regs_inc<176>(); else regs_inc<232>();
   if (warp < 8 + nm) {
     // ---------------------------------------------------------------- products
-    const int mw = warp - 8;
-    const int mg = mw % p.mgroups, kh = mw / p.mgroups;         // M tiles mg, mg+mgroups, ...; K part kh of ksp
-    const int kp0 = gc * kh / p.ksp, kp1 = gc * (kh + 1) / p.ksp;
-    const int kmem = pairs - KR / 2;                            // pairs kept in shared memory
-    uint4* w_s = reinterpret_cast<uint4*>(smem + w_off) + (size_t)mw * MPW * kmem * 64 + lane;
+    const int mg = warp - 8;                                    // M tiles mg, mg+mgroups, ...
+    const int kmem = gc - KR / 2;                               // pairs of K steps (one unit group each) kept in shared memory
+    uint4* w_s = reinterpret_cast<uint4*>(smem + w_off) + (size_t)mg * MPW * kmem * 64 + lane;
     // weights: A[unit][k], k = 32*(local group) + 8*gate + unit of the group
     uint32_t w[MPW][KR][4];
     {
-      auto frag = [&](int i, int ks, uint32_t (&a)[4]) {        // ks: K step from kp0 on
+      auto frag = [&](int i, int ks, uint32_t (&a)[4]) {        // ks: K step
         const int m = (mg + i * p.mgroups) * 16 + u;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const int mm = m + (j & 1) * 8, kg = kp0 + (ks >> 1), gate = (ks & 1) * 2 + (j >> 1);
+          const int mm = m + (j & 1) * 8, kg = ks >> 1, gate = (ks & 1) * 2 + (j >> 1);
           const int ku = (rank * gc + kg) * 8 + 2 * c;
           uint32_t v = 0;
-          if (mm < H && kg < kp1 && ku < H) {
+          if (mm < H && kg < gc && ku < H) {
             const unsigned short* src = reinterpret_cast<const unsigned short*>(Wh) + ((size_t)gate * H + ku) * H + mm;
             v = (uint32_t)src[0] | ((uint32_t)src[H] << 16);
           }
@@ -674,14 +638,13 @@ small_bwd_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant_
     // where this lane's 16 bytes of every M tile go: an even lane sends the tile's first 8 units, an odd one its second
     uint32_t dst[MPW];
     uint32_t there = 0, owners = 0;
-    const int src = rank * p.ksp + kh;
 #pragma unroll
     for (int i = 0; i < MPW; ++i) {
       const int grp = 2 * (mg + i * p.mgroups) + (c & 1);
       const int owner = grp / gc, lg = grp - owner * gc;
       if (grp * 8 < H && !p.no_arrive) there |= 1u << i;
       owners |= (uint32_t)min(owner, p.nc - 1) << (4 * i);
-      dst[i] = (CL ? mapa_shared(sbase, min(owner, p.nc - 1)) : sbase) + r_off + src * src_b + (lg * 8 + u) * 32 + (c >> 1) * 16;
+      dst[i] = (CL ? mapa_shared(sbase, min(owner, p.nc - 1)) : sbase) + r_off + rank * src_b + (lg * 8 + u) * 32 + (c >> 1) * 16;
     }
     bool ok = true;
     int k = 0;
@@ -689,67 +652,51 @@ small_bwd_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant_
       for (int ch = 0; ch < nch; ++ch, ++k) {
         const int par = k & 1;
         if (!wait_inline(&dfull[par], (uint32_t)(k >> 1) & 1u, dead, p.ctl, p.limit_ns, T - 1 - st, cl)) { ok = false; break; }
-        float acc[MPW * NA][NTC][4];
+        float acc[MPW * NA][4];
 #pragma unroll
         for (int i = 0; i < MPW * NA; ++i)
 #pragma unroll
-          for (int nt = 0; nt < NTC; ++nt)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) acc[i][nt][e] = 0.f;
-        const uint32_t da = sbase + d_off + (uint32_t)(par * CR + (lane & 7)) * pitch + (lane >> 3) * 16 + kp0 * 64;
-        uint32_t bf[2][NTC][4];
-#pragma unroll
-        for (int nt = 0; nt < NTC; ++nt) ldmatrix_x4(da + nt * 8 * pitch, bf[0][nt]);
+          for (int e = 0; e < 4; ++e) acc[i][e] = 0.f;
+        const uint32_t da = sbase + d_off + (uint32_t)(par * CR + (lane & 7)) * pitch + (lane >> 3) * 16;
+        uint32_t bf[2][4];
+        ldmatrix_x4(da, bf[0]);
 #pragma unroll
         for (int kk = 0; kk < KR / 2; ++kk) {
           if (kk + 1 < KR / 2) {
-#pragma unroll
-            for (int nt = 0; nt < NTC; ++nt) ldmatrix_x4(da + nt * 8 * pitch + (kk + 1) * 64, bf[(kk + 1) & 1][nt]);
+            ldmatrix_x4(da + (kk + 1) * 64, bf[(kk + 1) & 1]);
           }
 #pragma unroll
-          for (int nt = 0; nt < NTC; ++nt) {
+          for (int i = 0; i < MPW; ++i) mma16816<T16>(acc[i], w[i][2 * kk], bf[kk & 1][0], bf[kk & 1][1]);
 #pragma unroll
-            for (int i = 0; i < MPW; ++i) mma16816<T16>(acc[i][nt], w[i][2 * kk], bf[kk & 1][nt][0], bf[kk & 1][nt][1]);
-#pragma unroll
-            for (int i = 0; i < MPW; ++i) mma16816<T16>(acc[i + NA - 1][nt], w[i][2 * kk + 1], bf[kk & 1][nt][2], bf[kk & 1][nt][3]);
-          }
+          for (int i = 0; i < MPW; ++i) mma16816<T16>(acc[i + NA - 1], w[i][2 * kk + 1], bf[kk & 1][2], bf[kk & 1][3]);
         }
-        for (int kk = KR / 2; kp0 + kk < kp1; ++kk) {
-          uint32_t b[NTC][4];
-#pragma unroll
-          for (int nt = 0; nt < NTC; ++nt) ldmatrix_x4(da + nt * 8 * pitch + kk * 64, b[nt]);
+        for (int kk = KR / 2; TAIL && kk < gc; ++kk) {
+          uint32_t b[4];
+          ldmatrix_x4(da + kk * 64, b);
 #pragma unroll
           for (int i = 0; i < MPW; ++i) {
             const uint4 v0 = w_s[(i * 2 * kmem + 2 * kk - KR) * 32], v1 = w_s[(i * 2 * kmem + 2 * kk - KR + 1) * 32];
             const uint32_t a0[4] = {v0.x, v0.y, v0.z, v0.w}, a1[4] = {v1.x, v1.y, v1.z, v1.w};
-#pragma unroll
-            for (int nt = 0; nt < NTC; ++nt) {
-              mma16816<T16>(acc[i][nt], a0, b[nt][0], b[nt][1]);
-              mma16816<T16>(acc[i + NA - 1][nt], a1, b[nt][2], b[nt][3]);
-            }
+            mma16816<T16>(acc[i], a0, b[0], b[1]);
+            mma16816<T16>(acc[i + NA - 1], a1, b[2], b[3]);
           }
         }
         if (NA == 2) {
 #pragma unroll
-          for (int nt = 0; nt < NTC; ++nt)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) acc[0][nt][e] += acc[MPW * NA - 1][nt][e];
+          for (int e = 0; e < 4; ++e) acc[0][e] += acc[MPW * NA - 1][e];
         }
-        const uint32_t bufo = (uint32_t)(ch * 2 + (st & 1)) * nsrc * src_b;
+        const uint32_t bufo = (uint32_t)(ch * 2 + (st & 1)) * p.nc * src_b;
         const uint32_t bo = sbase + b_off + (uint32_t)(2 * ch + (st & 1)) * 8;
         const int valid = rows - ch * CR;
 #pragma unroll
         for (int i = 0; i < MPW; ++i) {
-#pragma unroll
-          for (int nt = 0; nt < NTC; ++nt) {
-            const float s0 = (c & 1) ? acc[i][nt][0] : acc[i][nt][2], s1 = (c & 1) ? acc[i][nt][1] : acc[i][nt][3];
-            const float r0 = __shfl_xor_sync(0xffffffffu, s0, 1), r1 = __shfl_xor_sync(0xffffffffu, s1, 1);
-            const uint4 v = (c & 1) ? make_uint4(__float_as_uint(r0), __float_as_uint(r1), __float_as_uint(acc[i][nt][2]), __float_as_uint(acc[i][nt][3]))
-                                    : make_uint4(__float_as_uint(acc[i][nt][0]), __float_as_uint(acc[i][nt][1]), __float_as_uint(r0), __float_as_uint(r1));
-            if ((there >> i & 1u) && nt * 8 + 4 * (c >> 1) < valid) {
-              const uint32_t a = dst[i] + bufo + (uint32_t)nt * gc * 256;
-              if (CL) st_async16(a, v, mapa_shared(bo, owners >> (4 * i) & 15u)); else st_shared16(a, v);
-            }
+          const float s0 = (c & 1) ? acc[i][0] : acc[i][2], s1 = (c & 1) ? acc[i][1] : acc[i][3];
+          const float r0 = __shfl_xor_sync(0xffffffffu, s0, 1), r1 = __shfl_xor_sync(0xffffffffu, s1, 1);
+          const uint4 v = (c & 1) ? make_uint4(__float_as_uint(r0), __float_as_uint(r1), __float_as_uint(acc[i][2]), __float_as_uint(acc[i][3]))
+                                  : make_uint4(__float_as_uint(acc[i][0]), __float_as_uint(acc[i][1]), __float_as_uint(r0), __float_as_uint(r1));
+          if ((there >> i & 1u) && 4 * (c >> 1) < valid) {
+            const uint32_t a = dst[i] + bufo;
+            if (CL) st_async16(a, v, mapa_shared(bo, owners >> (4 * i) & 15u)); else st_shared16(a, v);
           }
         }
         __syncwarp();
@@ -856,7 +803,6 @@ SmallPlan small_plan(const blstm_desc& d, int phase) {
   } else {
     if (H > 640) return p;
     const int mt = cdiv(H, 16);
-    p.ksp = 1;
     p.mpw = p.nc == 1 ? 1 : cdiv(mt, 8);
     p.mgroups = cdiv(mt, p.mpw);
     p.nch = cdiv(tiles, p.ncl);
@@ -865,8 +811,8 @@ SmallPlan small_plan(const blstm_desc& d, int phase) {
     else if (p.nc <= 4) p.kr = p.gc == 4 ? 8 : 6;
     else p.kr = p.gc == 5 ? 6 : 2 * p.gc;
     p.smem = fixed + (size_t)8 * 768 * p.gc + (size_t)2 * 8 * (p.gc * 64 + 16) +
-             (size_t)p.nch * 2 * p.nc * p.ksp * p.gc * 256 + (size_t)p.nch * p.gc * 512 +
-             (size_t)p.mgroups * p.ksp * p.mpw * (cdiv(p.gc, p.ksp) - p.kr / 2) * 1024;
+             (size_t)p.nch * 2 * p.nc * p.gc * 256 + (size_t)p.nch * p.gc * 512 +
+             (size_t)p.mgroups * p.mpw * (p.gc - p.kr / 2) * 1024;
   }
   p.rows = 8 * p.nch;
   p.ncl = p.nparts = cdiv(B, p.rows);
@@ -874,7 +820,6 @@ SmallPlan small_plan(const blstm_desc& d, int phase) {
     while (p.ncl * p.nc % 4 != 0) ++p.ncl;                               // whole groups of four CTAs; the extra clusters have no rows
   p.grid = p.ncl * p.nc;
   if (p.smem > 232448 || p.nch > SB_MAX_CHUNKS) return p;
-  p.fits = true;
   p.ok = small_plan_pays(H, p, phase);
   return p;
 }
@@ -904,7 +849,7 @@ template <typename T16>
 static int small_bwd_t(const SmallPlan& pl, const CUtensorMap& tp, const CUtensorMap& tc, const CUtensorMap& to,
                        const CUtensorMap& td, const SmallBwdParams& p, cudaStream_t st) {
 #define BLSTM_SMALL_BWD(M, K, C) \
-  if (pl.mpw == M && pl.kr == K && (pl.nc > 1) == C) return launch_clusters(small_bwd_kernel<M, K, 1, C, T16>, pl.grid, pl.threads, pl.smem, pl.nc, st, tp, tc, to, td, p);
+  if (pl.mpw == M && pl.kr == K && (pl.nc > 1) == C && ((C ? M == 5 : K < 16) || pl.gc == K / 2)) return launch_clusters(small_bwd_kernel<M, K, C, T16>, pl.grid, pl.threads, pl.smem, pl.nc, st, tp, tc, to, td, p);
   BLSTM_SMALL_BWD(1, 2, false)
   BLSTM_SMALL_BWD(1, 8, false)
   BLSTM_SMALL_BWD(1, 16, false)
@@ -966,7 +911,7 @@ int small_bwd_recurrence(const blstm_desc& d, const SmallPlan& pl, const void* d
                          float* db, void* ws, cudaStream_t st) {
   SmallBwdParams p;
   p.T = d.seq_len; p.B = d.batch; p.H = d.hidden_size;
-  p.nc = pl.nc; p.gc = pl.gc; p.rows = pl.rows; p.nch = pl.nch; p.ksp = pl.ksp; p.mgroups = pl.mgroups;
+  p.nc = pl.nc; p.gc = pl.gc; p.rows = pl.rows; p.nch = pl.nch; p.mgroups = pl.mgroups;
   p.no_arrive = (d.flags & BLSTM_FLAG_TEST_NO_ARRIVE) ? 1 : 0;
   p.limit_ns = d.wait_limit_us > 0 ? (unsigned long long)d.wait_limit_us * 1000ull : kDefaultWaitNs;
   p.ctl = reinterpret_cast<Control*>(ws);
@@ -987,7 +932,7 @@ int small_plan_detail(const blstm_desc& d, const SmallPlan& p, int phase, char* 
   (void)d;
   if (phase == BLSTM_PHASE_BWD)
     return snprintf(buf, n, "sm100 bwd small-batch cluster=%d units_per_cta=%d rows_per_cluster=%d chunks=%d m_tiles_per_warp=%d "
-                    "k_split=%d register_steps=%d grid=%d threads=%d smem=%zu", p.nc, p.gc * 8, p.rows, p.nch, p.mpw, p.ksp, p.kr,
+                    "register_steps=%d grid=%d threads=%d smem=%zu", p.nc, p.gc * 8, p.rows, p.nch, p.mpw, p.kr,
                     p.grid, p.threads, p.smem);
   return snprintf(buf, n, "sm100 fwd small-batch cluster=%d units_per_cta=%d rows_per_cluster=%d chunks=%d k_split=%d replicas=%d "
                   "register_steps=%d/%d grid=%d threads=%d smem=%zu", p.nc, p.gc * 8, p.rows, p.nch, p.kspl, p.rpl,

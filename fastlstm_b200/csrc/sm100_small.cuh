@@ -7,15 +7,14 @@ namespace blstm {
 namespace sm100 {
 
 struct SmallPlan {
-  bool fits;                // the kernels cover the shape
-  bool ok;                  // ... and are the faster ones for it
+  bool ok;                  // the kernels cover the shape and are the faster ones for it
   int nc, gc;               // CTAs per cluster; groups of 8 hidden units per CTA
   int ks;                   // K steps of 16 (an even number)
   int kr;                   // K steps whose weights live in registers
   int rows, ncl;            // batch rows per cluster, clusters
   int nch;                  // chunks of 8 rows per cluster
   int rpl, kspl, slots;     // forward: replicas of the gc warps, K parts, item slots of the ring
-  int ksp, mgroups, mpw;    // backward: K parts, M tiles worked at once, M tiles per warp
+  int mgroups, mpw;         // backward: M tiles worked at once, M tiles per warp
   int nparts;               // backward: rows of bias-gradient partial sums
   int threads, grid;
   size_t smem;
@@ -34,7 +33,7 @@ struct SmallFwdParams {
 
 struct SmallBwdParams {
   int T, B, H;
-  int nc, gc, rows, nch, ksp, mgroups;
+  int nc, gc, rows, nch, mgroups;
   int no_arrive;
   unsigned long long limit_ns;
   Control* ctl;
