@@ -49,8 +49,7 @@ def _run(cmd, what, verbose):
 
     def finish():
         log, _ = p.communicate()
-        if verbose or p.returncode != 0:
-            sys.stderr.write(log)
+        sys.stderr.write(log)                 # (silent but for warnings and errors)
         if p.returncode != 0:
             raise RuntimeError(f"compiler failed building {what}")
     return finish
@@ -60,7 +59,7 @@ def _host_cmd():
     import torch
     from torch.utils import cpp_extension as ext
     lib_dirs = [os.path.join(os.path.dirname(torch.__file__), "lib"), os.path.join(os.path.dirname(_nvcc()), "..", "lib64")]
-    return ([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", "-w",
+    return ([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", "-Wall",
              f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-DTORCH_EXTENSION_NAME=_host"]
             + [f"-I{d}" for d in ext.include_paths(device_type="cuda") + [sysconfig.get_paths()["include"]]]
             + ["-o", HOST_PATH, HOST_SRC, f"-L{PKG_DIR}", "-l:libfastlstm_b200.so", "-Wl,-rpath,$ORIGIN"]

@@ -196,7 +196,6 @@ resident_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
     const bool box_ok = owner && box_grow < p.rows && box_unit < H;
     const float* rd = reinterpret_cast<const float*>(recv) + lr * 32 + (BWD ? (u >> 5) * (BLK / 4) + (u & 31) : u);
     const uint32_t tx = owner ? (uint32_t)(KS - 1) * 4 * BLK : 0u;
-    bool ok = true;
 
     // where this warp's half of the accumulator's columns goes: RW_ rows each for NB receivers
     constexpr int NB = OWN > 1 ? OWN / 2 : 1, RW_ = N / 2 / NB, C = RW_ < 16 ? 8 : 16;

@@ -59,3 +59,11 @@ def test_host_only_entry_points():
 
 def test_desc_struct_layout_matches_header():
     assert ctypes.sizeof(_lib.Desc) == 32
+
+
+def test_the_build_hides_no_warnings(capfd):
+    import sys
+    from fastlstm_b200 import build
+    assert "-w" not in build._host_cmd() and not any("disable-warnings" in f or "diag-suppress" in f for f in build.NVCC_FLAGS)
+    build._run([sys.executable, "-c", "print('warning: seen')"], "nothing", verbose=False)()
+    assert "warning: seen" in capfd.readouterr().err
