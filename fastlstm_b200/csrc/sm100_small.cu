@@ -720,15 +720,15 @@ static int small_cluster(int H) { return H <= 64 ? 1 : H <= 128 ? 4 : H <= 256 ?
 
 __global__ void one_cta_per_sm_kernel() {}
 
-// Asked of the occupancy calculator once per size from 5 CTAs on: clusters do not tile every GPC without a remainder (a
-// B200 holds 33 of 4 CTAs, 15 of 8, 7 of 16).
+// Asked of the occupancy calculator once per size from 5 CTAs on: clusters do not tile every GPC without a remainder.
 int resident_clusters(int nc) {
   static std::atomic<int> cached[17];
+  static const int b200[17] = {0, 148, 74, 45, 33, 26, 22, 15, 15, 15, 11, 7, 7, 7, 7, 7, 7};     // its answers with 148 SMs
   const int sms = plan_sm_count();
   if (nc <= 4) return sms * 132 / 148 / nc;
   int c = cached[nc].load(std::memory_order_relaxed);
   if (c > 0) return c;
-  c = nc <= 8 ? sms * 15 / 148 : sms * 7 / 148;
+  c = sms * b200[nc] / 148;
   DeviceInfo di;
   auto kern = one_cta_per_sm_kernel;
   if (get_device_info(&di) == BLSTM_OK && di.sm_count > 0 &&

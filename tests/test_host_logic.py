@@ -331,3 +331,10 @@ def test_small_batch_kernels_where_they_measured_faster():
             for B in (8, n // 2, n, n + 1):
                 small = lstm._family(torch.bfloat16, 64, B, H, H, phase) == _lib.FAMILY_SMALL_BATCH
                 assert small == (B <= n), (H, B, phase)
+
+
+def test_plans_without_a_device_are_those_of_a_b200():
+    # 22 clusters of six CTAs are resident at once on 148 SMs, so the largest backward plan fits over six
+    from fastlstm_b200 import plan_detail
+    s = plan_detail(torch.bfloat16, 8, 32, 2048, 2048, "bwd")
+    assert "resident weights cluster=6 " in s and "grid=96 " in s, s
