@@ -460,20 +460,24 @@ resident_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
   if (KS > 1) cluster_sync_all();     // no CTA leaves while a peer may still write into its shared memory
 }
 
-// The smallest split of K whose slice fits the chip, and as many groups of rows as fit beside each other.  Backward at
-// H = 2048 with 17 to 32 rows is the one size that fits with one issuer only, over six CTAs: 6.9 us a step against 5.3
-// at H = 1984 with two.  Seven ways two would fit, but a B200 holds 15 clusters of seven or eight CTAs and 16 M tiles need
-// 16; the kernel with the batch on the M side takes 8.6.
+// The smallest split of K whose slice fits the chip, and as many groups of rows as fit beside each other.  Backward, a slice
+// of 22 chunks and 32 rows fits with one issuer only (one accumulator instead of two leaves tensor memory for the chunk
+// that would not fit); one more CTA a cluster makes room for two, which is worth it while a group keeps to 32 rows.  us a
+// step: H = 1728, B = 32: 6.9 -> 5.0, H = 1408, B = 64: 6.9 -> 5.0, but B = 96, then 48 rows a group, 6.9 -> 7.3.
+// H = 2048 with 17 to 32 rows is left with one issuer over six CTAs (6.9; two take 5.3 at H = 1984): a B200 holds
+// 15 clusters of seven or eight CTAs and 16 M tiles need 16; the kernel with the batch on the M side takes 8.6.
 ResPlan resident_plan(const blstm_desc& d, int phase) {
-  ResPlan p{};
   const int H = d.hidden_size, B = d.batch;
   const bool bwd = phase == BLSTM_PHASE_BWD;
-  if ((d.flags & BLSTM_FLAG_FORCE_GENERIC) || (d.dtype != BLSTM_F16 && d.dtype != BLSTM_BF16)) return p;
-  if (phase != BLSTM_PHASE_FWD && !bwd) return p;
-  if (H % 64 != 0 || H < RES_MIN_H || H > 2048) return p;
-  p.mt = bwd ? cdiv(H, 128) : H / 32;
-  p.kc_total = bwd ? H / 16 : H / 64;
-  for (p.ks = bwd ? 4 : 1; p.ks <= (bwd ? 8 : 2); ++p.ks) {
+  if ((d.flags & BLSTM_FLAG_FORCE_GENERIC) || (d.dtype != BLSTM_F16 && d.dtype != BLSTM_BF16)) return ResPlan{};
+  if (phase != BLSTM_PHASE_FWD && !bwd) return ResPlan{};
+  if (H % 64 != 0 || H < RES_MIN_H || H > 2048) return ResPlan{};
+  ResPlan one{};                         // what fits with one issuer
+  for (int ks = bwd ? 4 : 1; ks <= (bwd ? 8 : 2); ++ks) {
+    ResPlan p{};
+    p.ks = ks;
+    p.mt = bwd ? cdiv(H, 128) : H / 32;
+    p.kc_total = bwd ? H / 16 : H / 64;
     int cap = p.ks == 1 ? plan_sm_count() : resident_clusters(p.ks);
     if (d.flags & BLSTM_FLAG_HALF_DEVICE) cap /= 2;
     p.ng = cap / p.mt;
@@ -486,20 +490,21 @@ ResPlan resident_plan(const blstm_desc& d, int phase) {
     p.kcm = cdiv(p.kc_total, p.ks);
     const size_t x = std::max((size_t)p.kcm * p.N * 128, (size_t)p.N * 512 + (size_t)(p.N / p.own) * (bwd ? 1024 : 64));
     p.x_bytes = (int)x;
-    // (one accumulator instead of two may leave tensor memory for the chunk that would not fit)
     for (p.ni = 2; p.ni >= 1; --p.ni) {
       p.nt = std::min(p.kcm, (512 - p.ni * p.N) / 32);
       p.smem = 1024 + (size_t)(p.kcm - p.nt) * 16384 + x + (size_t)p.ks * 4 * (p.N / p.own) * 128 + 512;
       if (p.smem <= 232448 || !(bwd && p.N == 32)) break;
     }
     if (p.smem > 232448 || p.ni < 1 || p.kcm > RES_MAX_KC) continue;
+    if (one.ok && (p.ni < 2 || p.N > 32)) continue;
     p.grid = p.ng * p.mt * p.ks;
     p.off_db = sizeof(Control) + round_up((size_t)(d.seq_len + 1) * p.ng * sizeof(int), 256);
     p.ws_bytes = p.off_db + (bwd ? (size_t)p.ng * p.N * 4 * H * sizeof(float) : 0);
     p.ok = true;
-    return p;
+    if (p.ni == 2) return p;
+    one = p;
   }
-  return p;
+  return one;
 }
 
 template <bool BWD, int N, int OWN, int NI, typename T16>

@@ -8,9 +8,9 @@ from test_gpu_recurrence import TD, _bwd, _cmp, _desc, _fwd, _torch_bwd, _torch_
 pytestmark = pytest.mark.gpu
 
 # N = 16, 32, 64; one row, ragged rows and groups; half an M tile in backward (H % 128 == 64); K split over 1 and 2 (forward),
-# 4, 5 and 6 (backward, one issuer) CTAs; weights that fit tensor memory and weights that do not
+# 4 (one issuer too), 5 and 6 (the same) CTAs backward; weights that fit tensor memory and weights that do not
 SHAPES = [(4, 1, 768), (3, 65, 704), (5, 100, 768), (3, 250, 768), (4, 256, 1024), (2, 130, 960), (3, 33, 1088), (3, 64, 1536),
-          (4, 32, 2048), (3, 17, 1984), (2, 9, 2048),
+          (4, 32, 2048), (3, 17, 1984), (2, 9, 2048), (3, 29, 1728), (3, 61, 1408), (3, 90, 1408),
           # several tiles a group in backward: four, five and eight, a partial last tile, half an M tile, odd numbers of K chunks
           (3, 1600, 512), (3, 4096, 512), (5, 2300, 448), (3, 3210, 320), (3, 4000, 256), (1, 2047, 512)]
 

@@ -338,3 +338,7 @@ def test_plans_without_a_device_are_those_of_a_b200():
     from fastlstm_b200 import plan_detail
     s = plan_detail(torch.bfloat16, 8, 32, 2048, 2048, "bwd")
     assert "resident weights cluster=6 " in s and "grid=96 " in s, s
+    # a second issuer is worth a CTA more a cluster where the rows of a group stay within 32, and only there
+    for H, B, want in ((1728, 32, "cluster=6"), (1728, 17, "cluster=6"), (1408, 64, "cluster=5"), (1408, 96, "cluster=4"), (1664, 32, "cluster=5")):
+        s = plan_detail(torch.bfloat16, 8, B, H, H, "bwd")
+        assert want in s and ("issuers=2" in s) == (B != 96), (H, B, s)
