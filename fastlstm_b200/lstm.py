@@ -286,14 +286,24 @@ def _shares_device(dtype, T, B, I, H):
 
 @functools.lru_cache(maxsize=1024)
 def _wavefront_pays(dtype, T, B, H, grad):
-    """False where a layer alone has recurrences with resident weights or the small-batch ones: those leave little to hide,
-    and a training step's launches for every chunk cost more than that (two layers, forward and backward: T=256, B=512,
-    H=512 6.8 ms as a wavefront, 6.4 without; T=256, B=32, H=256 1.8 and 1.25; T=128, B=200, H=768 3.4 both).  Inference
-    gains from 128 steps on where half of the device has them too (T=256, B=128, H=512: 1.44 -> 1.15 ms)."""
-    def on_chip(half):
-        return all(_family(dtype, T, B, H, H, phase, half) in (_lib.FAMILY_RESIDENT, _lib.FAMILY_SMALL_BATCH)
-                   for phase in (("fwd", "bwd") if grad else ("fwd",)))
-    return not on_chip(False) or (not grad and T >= 128 and on_chip(True))
+    """Whether a stack that could run as a wavefront should.  Two layers, ms layer after layer / as a wavefront (B200):
+
+    Without gradients the small-batch recurrences leave nothing to hide, on a few SMs of either half (T=256, B=64, H=256:
+    0.56 / 0.64; T=128, B=1000, H=64: 0.23 / 0.5); resident weights gain from 128 steps on where half of the device has
+    them too (T=128 and 256: B=128, H=512 0.91 / 0.81 and 1.73 / 1.40; B=440, H=320 0.98 / 0.98 and 1.87 / 1.75), the kernels
+    with several 128-row tiles always (T=128, B=1000, H=192: 1.31 / 1.05).
+
+    A training step's launches for every chunk cost more, so not where both directions stay on the chip (T=256, B=512, H=512
+    6.4 / 6.8; T=256, B=32, H=256 1.25 / 1.8) nor for few steps (T=64, B=712, H=320: 1.78 / 1.95, T=128: 3.27 / 3.3, T=256:
+    6.30 / 6.00; B=768, H=384: 2.18 / 2.22, 4.10 / 3.88, 7.97 / 7.15; B=968, H=192: 1.78 / 1.82, T=96: 2.54 / 2.33, T=256 6.33 / 5.37), and not at H=576, where half
+    of the device gives backward four tiles a CTA (B=392: T=128 4.13 / 4.64, T=256 8.02 / 8.55, T=512 15.8 / 16.4)."""
+    on_chip = (_lib.FAMILY_RESIDENT, _lib.FAMILY_SMALL_BATCH)
+    fwd = _family(dtype, T, B, H, H, "fwd")
+    if grad:
+        return T >= (96 if H < 320 else 128) and H <= 384 and not (fwd in on_chip and _family(dtype, T, B, H, H, "bwd") in on_chip)
+    if fwd == _lib.FAMILY_RESIDENT:
+        return T >= 128 and _family(dtype, T, B, H, H, "fwd", True) in on_chip
+    return fwd != _lib.FAMILY_SMALL_BATCH
 
 
 class _Beside:

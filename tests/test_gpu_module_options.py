@@ -192,14 +192,17 @@ def test_proj_size_matches_nn_lstm(dtype, bidirectional, H, P):
             assert max_rel(got[k], want[k]) <= 5e-2, k
 
 
-@pytest.mark.parametrize("B,states", [(512, False), (300, True), (64, True)])
-def test_layer_wavefront_matches_the_sequential_stack(monkeypatch, B, states):
+@pytest.mark.parametrize("B,states,T,H", [(512, False, 96, 512), (300, True, 96, 512), (64, True, 96, 512),
+                                          # (these run as a wavefront; the others' layers are faster one after the other)
+                                          (968, True, 128, 192), (1500, False, 100, 192)])
+def test_layer_wavefront_matches_the_sequential_stack(monkeypatch, B, states, T, H):
     """Two layers, few batch tiles: the stack runs as a wavefront over time chunks on two streams
     (layer 1 on chunk k beside layer 0 on chunk k+1).  Same results as the layers run one after the
     other, up to the cell state crossing chunk boundaries in bf16; gradients of inputs, initial states
     and parameters included."""
     import fastlstm_b200 as F
-    T, I, H, L = 96, 512, 512, 2
+    from fastlstm_b200 import lstm
+    I, L = 512, 2
     dt = torch.bfloat16
     torch.manual_seed(5)
     m = F.FastLSTM(I, H, num_layers=L, device="cuda", dtype=dt)
@@ -210,6 +213,7 @@ def test_layer_wavefront_matches_the_sequential_stack(monkeypatch, B, states):
     h0 = (torch.randn(L, B, H, generator=g, device="cuda") * 0.1).to(dt)
     c0 = (torch.randn(L, B, H, generator=g, device="cuda") * 0.1).to(dt)
     assert m._wavefront_chunks(x.requires_grad_(True), None, None) == 4
+    assert lstm._wavefront_pays(dt, T, B, H, True) == (H != 512)
 
     def run(on):
         monkeypatch.setenv("FASTLSTM_B200_WAVEFRONT", "1" if on else "0")

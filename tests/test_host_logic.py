@@ -342,3 +342,13 @@ def test_plans_without_a_device_are_those_of_a_b200():
     for H, B, want in ((1728, 32, "cluster=6"), (1728, 17, "cluster=6"), (1408, 64, "cluster=5"), (1408, 96, "cluster=4"), (1664, 32, "cluster=5")):
         s = plan_detail(torch.bfloat16, 8, B, H, H, "bwd")
         assert want in s and ("issuers=2" in s) == (B != 96), (H, B, s)
+
+
+def test_wavefront_where_it_measured_faster():
+    from fastlstm_b200 import lstm
+    bf = torch.bfloat16
+    for grad, T, B, H, want in ((True, 256, 968, 192, True), (True, 128, 768, 384, True), (True, 64, 768, 384, False),
+                                (True, 256, 392, 576, False), (True, 256, 512, 512, False), (True, 256, 32, 256, False),
+                                (False, 256, 64, 64, False), (False, 256, 64, 256, False), (False, 128, 64, 512, False),
+                                (False, 128, 128, 512, True), (False, 64, 128, 512, False), (False, 128, 1000, 192, True)):
+        assert lstm._wavefront_pays(bf, T, B, H, grad) == want, (grad, T, B, H)
