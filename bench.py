@@ -405,9 +405,9 @@ def main():
     # launching stream); the slower one is the dominant kernel of the step and goes in "roofline"
     hbm_gbs, tflops, which = peaks()
     es = ESIZE[cfg["dtype"]]
-    # small shards of a stack run as a layer wavefront (two layers side by side, each recurrence planned
-    # for half of the SMs): the kernels are then timed, and their plans reported, as the step runs them
-    wave = model._wavefront_chunks(x_dev, None, None) if hasattr(model, "_wavefront_chunks") else 0
+    # a stack that runs as a layer wavefront (two layers side by side, each recurrence planned for half of the
+    # SMs): the kernels are then timed, and their plans reported, as the step runs them
+    wave = model._wavefront(x_dev, None, None, cfg["bwd"]) if hasattr(model, "_wavefront") else 0
     kflags = (0 if cfg["bwd"] else _lib.FLAG_INFERENCE) | (_lib.FLAG_HALF_DEVICE if wave else 0)
     d = _lib.Desc(_lib.DTYPE_CODE[cfg["dtype"]], T, B, H, H, kflags, 0, 0)
     st = torch.cuda.current_stream().cuda_stream

@@ -638,7 +638,7 @@ class FastLSTM(nn.Module):
             return None
         L, H, dt = self.num_layers, self.hidden_size, x.dtype
         T, B = (x.shape[1], x.shape[0]) if self.batch_first else (x.shape[0], x.shape[1])
-        if T > 1 and (self._wavefront_chunks(x.transpose(0, 1) if self.batch_first else x, h_c_0, None) and _wavefront_pays(dt, T, B, H, False)
+        if T > 1 and (self._wavefront(x.transpose(0, 1) if self.batch_first else x, h_c_0, None, False)
                       or any(_padded_sizes(dt, n, H, T, B) is not None for n in {x.shape[2], H})):
             return None
         if T == 1 and dt != torch.float32 and (H % 8 or x.shape[2] % 8):
@@ -766,6 +766,11 @@ class FastLSTM(nn.Module):
             return 0
         return max(1, min(int(os.environ.get("FASTLSTM_B200_WAVEFRONT_CHUNKS", "4")), T // 16))
 
+    def _wavefront(self, x, h_c_0, lengths, grad):
+        """Number of time chunks that this call runs as a wavefront over, or 0."""
+        n = self._wavefront_chunks(x, h_c_0, lengths)
+        return n if n and _wavefront_pays(x.dtype, x.shape[0], x.shape[1], self.hidden_size, grad) else 0
+
     def _forward_wavefront(self, x, h_c_0, n_chunks):
         h0 = c0 = None
         if h_c_0 is not None:
@@ -788,10 +793,7 @@ class FastLSTM(nn.Module):
 
     def _forward_padded(self, x, h_c_0, lengths):
         """x [T,B,I]; lengths: None, or the [B] valid lengths (device tensor) of padded sequences."""
-        n_chunks = self._wavefront_chunks(x, h_c_0, lengths)
-        if n_chunks and not _wavefront_pays(x.dtype, x.shape[0], x.shape[1], self.hidden_size,
-                                                torch.is_grad_enabled()):
-            n_chunks = 0
+        n_chunks = self._wavefront(x, h_c_0, lengths, torch.is_grad_enabled())
         if n_chunks:
             return self._forward_wavefront(x, h_c_0, n_chunks)
         nd = self.num_directions

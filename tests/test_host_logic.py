@@ -352,3 +352,8 @@ def test_wavefront_where_it_measured_faster():
                                 (False, 256, 64, 64, False), (False, 256, 64, 256, False), (False, 128, 64, 512, False),
                                 (False, 128, 128, 512, True), (False, 64, 128, 512, False), (False, 128, 1000, 192, True)):
         assert lstm._wavefront_pays(bf, T, B, H, grad) == want, (grad, T, B, H)
+        if H <= 512 and B > 8:
+            # ... and it is what the module asks before it runs, and the benchmark before it reports
+            x = type("OnGpu", (), dict(is_cuda=True, shape=(T, B, H), dtype=bf))
+            m = FastLSTM(H, H, num_layers=2, device="meta", dtype=bf)
+            assert bool(m._wavefront(x, None, None, grad)) == want
