@@ -9,9 +9,10 @@
 // accumulators leave.  Two issuers take every other tile, each with its own accumulator and its own half of the ring.
 // Shared memory holds no weights, so the ring is what the exchange leaves: 2 x 4 stages of 8 KB.  A CTA has 128 units where the
 // kernel with the batch on the M side had 64 a cluster, which halves what a step reads of d_ifgo (67 MB at B = 4096, H = 512).
-// us per step, that kernel -> this, launched alone: B = 4096, H = 512: 25.5 -> 21.7 to 23 (it runs into the power cap; 25.5 inside a
-// training step); B = 3000: 20.4 -> 16.0; B = 2048: 12.9 -> 12.3; B = 4096, H = 256: 12.5 -> 9.4; B = 3000, H = 384: 19.1 -> 11.8.  Not for three tiles a group (B = 1200, H = 512: 9.7, here 10.8: the chain of a
-// step shows); the same thing forward was slower (14.7, 17.8), sixteen epilogue warps of half the cells no faster (22.4).
+// us per step, that kernel -> this, launched alone: B = 4096, H = 512: 25.5 -> 21.7 to 23 (it runs into the power cap; 24.5 inside a
+// training step); B = 3000: 20.4 -> 16.0; B = 2048: 12.9 -> 12.3; B = 4096, H = 256: 12.5 -> 9.4; B = 3000, H = 384: 19.1 -> 11.8.
+// Not for three tiles a group (B = 1200, H = 512: 9.7, here 10.8: the chain of a step shows); the same thing forward was slower
+// (14.7, 17.8), sixteen epilogue warps of half the cells no faster (22.4).
 #include <algorithm>
 #include <cstdio>
 
