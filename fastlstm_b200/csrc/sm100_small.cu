@@ -768,6 +768,7 @@ int resident_clusters(int nc) {
 // (General kernels, forward: H = 64, B = 64: 1.9 -> 0.59; H = 192: 4.4 a step at any of these batches.)
 static bool small_plan_pays(int H, const SmallPlan& p, int phase) {
   if (H <= 128) return true;
+  if (phase == BLSTM_PHASE_BWD && H < 256 && H % 64 != 0) return true;      // (the others would be the CUDA-core kernels)
   if (phase == BLSTM_PHASE_BWD) return p.nch <= (H < 256 ? 8 : H == 256 ? 6 : H <= 448 ? 4 : H <= 512 ? 5 : 2);
   return p.nch <= (H < 256 ? 8 : H <= 320 ? 4 : H <= 448 ? 3 : H <= 512 ? 2 : 1);
 }

@@ -331,6 +331,8 @@ def test_small_batch_kernels_where_they_measured_faster():
             for B in (8, n // 2, n, n + 1):
                 small = lstm._family(torch.bfloat16, 64, B, H, H, phase) == _lib.FAMILY_SMALL_BATCH
                 assert small == (B <= n), (H, B, phase)
+    # (a size that only the CUDA-core kernels would take instead)
+    assert lstm._family(torch.bfloat16, 64, 1100, 200, 200, "bwd") == _lib.FAMILY_SMALL_BATCH
 
 
 def test_plans_without_a_device_are_those_of_a_b200():
