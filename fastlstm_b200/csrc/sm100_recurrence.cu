@@ -939,7 +939,8 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
   int* pub_cnt = const_cast<int*>(dead) + 1;        // [4] arrivals of the epilogue warps, by item index mod 4
   uint64_t* pub_bar = reinterpret_cast<uint64_t*>(pub_cnt + 4);   // [4] item stored? by item index mod 4
   uint64_t* rdy = pub_bar + 4;                                 // aliased buffers: the 3 peers are done with their MMAs
-  uint64_t* consumed = rdy + 1;                                // interleaved tiles: the cluster's 32 warps read an item's slices
+  uint64_t* consumed = rdy + 1;                                // interleaved tiles: the cluster's four CTAs read an item's slices
+  uint64_t* taken = consumed + 1;                              // ... this CTA's eight warps did
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t r = cluster_ctarank();                       // gate whose K range this CTA owns
@@ -959,7 +960,8 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
     for (int i = 0; i < 4; ++i) pub_cnt[i] = 0;
     for (int i = 0; i < 4; ++i) mbar_init(&pub_bar[i], ITEM_WARPS);
     mbar_init(rdy, 3);
-    mbar_init(consumed, 4 * ITEM_WARPS);
+    mbar_init(consumed, 4);
+    mbar_init(taken, ITEM_WARPS);
     fence_mbar_init();
     for (int s = 0; s < R_STAGES; ++s) mbar_expect_tx(&full[s], SB);
     tma_prefetch_desc(&tmW);
@@ -1040,20 +1042,29 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
     }
   } else if (PUBLISHER && warp == 1 + NACC) {
     // ---------------------------------------------------------------- publisher
-    // Walks the gate-maths items in the epilogue's order; when all eight epilogue warps have stored
-    // an item's d_ifgo rows (their arrival on pub_bar is a CTA-scope release, this wait the acquire),
-    // one release at GPU scope counts this CTA in on the item's arrival counter.  An epilogue warp can
+    // Walks the items in the epilogue's order.  When all eight epilogue warps have read an item's slices, one fence at
+    // cluster scope and an arrival per CTA tell the cluster (a release by every warp stalls them 0.7 k clocks and more).  When
+    // all eight have stored an item's d_ifgo rows (their arrival on pub_bar is a CTA-scope release, this wait the
+    // acquire), one release at GPU scope counts this CTA in on the item's arrival counter.  An epilogue warp can
     // be at most four items ahead of the slowest (it needs the counters this thread completes), so
-    // four barriers never mix items.
+    // four barriers never mix items; and it needs this thread's arrival for an item before it reads the next one's slices.
     if (lane == 0) {
-      int k = 0;
+      int k = 0, it = 0;
       bool ok = true;
       for (int ch = 0; ch < n_chunks && ok; ++ch) {
-        for (int st = 0; st < T && ok; ++st) {
+        for (int st = 0; st <= T && ok; ++st) {
           for (int j = 0; j < TI && ok; ++j) {
             const int bt = pb + (ch * TI + j) * p.nb_par;
             if (bt >= p.nbt) continue;
             wc.d0 = T - 1 - st; wc.d1 = bt;
+            if (st > 0) {
+              if (!mbar_wait(taken, (uint32_t)it & 1u, wc)) { ok = false; break; }
+              ++it;
+              fence_acq_rel_cluster();
+#pragma unroll
+              for (int dst = 0; dst < 4; ++dst) mbar_arrive_remote_relaxed(mapa_shared(smem_u32(consumed), dst));
+            }
+            if (st == T) continue;
             if (!mbar_wait(&pub_bar[k & 3], (uint32_t)(k >> 2) & 1u, wc)) { ok = false; break; }
             // the generic->async proxy fence of the hand-off runs here, on the causality path between
             // the epilogue warps' stores (ordered before this thread by the barrier) and the release
@@ -1258,8 +1269,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
             if constexpr (TI >= 2) {
               // the previous item's slices have been read by the whole cluster (so the staging below overwrites
               // nothing a copy still reads, and the receive slots are free again)
-              // (no data rides on this barrier, so a plain CTA-scope wait will do)
-              if (it > 1 && !mbar_wait(consumed, (uint32_t)it & 1u, wc)) { ok = false; break; }
+              if (it > 1 && !mbar_wait_cluster(consumed, (uint32_t)it & 1u, wc)) { ok = false; break; }
             }
             if (ew == 0 && lane == 0) {
               // what this CTA is about to receive (nothing for a quarter without rows)
@@ -1322,10 +1332,9 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
                 dhc[4 * o + 3] += v.w;
               }
             if constexpr (TI >= 2) {
-              // this warp has read the item's slices (the sums above hold them): tell the cluster.
-              // Nothing is published by the signal, hence relaxed.
+              // this warp has read the item's slices: the publisher tells the cluster once all eight have
               __syncwarp();
-              if (lane < 4) mbar_arrive_remote_relaxed(mapa_shared(smem_u32(consumed), lane));
+              if (lane == 0) mbar_arrive(taken);
             }
           }
           if (st == 0) {

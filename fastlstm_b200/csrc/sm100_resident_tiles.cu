@@ -73,7 +73,8 @@ tiles_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
   uint64_t* consumed = xchg + 2;                                    // receive slots read by all owners
   uint64_t* box_full = consumed + 2;
   uint64_t* box_free = box_full + 2;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(box_free + 2);
+  uint64_t* taken = box_free + 2;                                   // receive slots read by this CTA's warps
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(taken + 2);
   volatile int* dead = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -88,7 +89,8 @@ tiles_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
       mbar_init(&acc_full[i], 1);
       mbar_init(&acc_empty[i], EW);
       mbar_init(&xchg[i], EW + 1);
-      mbar_init(&consumed[i], KS * EW);
+      mbar_init(&consumed[i], KS);
+      mbar_init(&taken[i], EW);
       mbar_init(&box_full[i], EW);
       mbar_init(&box_free[i], 1);
     }
@@ -181,12 +183,24 @@ tiles_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
       }
     }
   } else if (warp == 3) {
-    // ---------------------------------------------------------------- publisher: stores a tile's rows, counts the CTA in
+    // ---------------------------------------------------------------- publisher: stores a tile's rows, counts the CTA in,
+    // and tells the cluster when all eight warps have read an item's receive slots (for all of them: a release at cluster
+    // scope stalls its thread for 0.7 k clocks and more)
     if (lane == 0) {
       const int items = total;            // (of steps T-1 .. 0: as many as have a product)
       int s = 0, j = 0;
-      for (int m = 0; m < items; ++m) {
-        const int t = T - 1 - s, tile = tile_of(j), b = m & 1;
+      for (int m = 0; m < items + NT; ++m) {
+        const int n = m - NT, b = m & 1;
+        if (n >= 0 && n + 2 < total) {
+          const int c = n & 1;
+          wc.d0 = n;
+          if (!mbar_wait(&taken[c], (uint32_t)(n >> 1) & 1u, wc)) break;
+          fence_acq_rel_cluster();
+#pragma unroll
+          for (int dst = 0; dst < KS; ++dst) mbar_arrive_remote_relaxed(mapa_shared(smem_u32(&consumed[c]), dst));
+        }
+        if (m >= items) continue;
+        const int t = T - 1 - s, tile = tile_of(j);
         wc.d0 = t; wc.d1 = tile;
         if (!mbar_wait(&box_full[b], (uint32_t)(m >> 1) & 1u, wc)) break;
         tma_store_4d(&tmO, boxes + b * BOX, mt * 128, tile * N + r * RO, 0, t);
@@ -228,7 +242,7 @@ tiles_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
       const int b = n & 1;
       const uint32_t k = (uint32_t)(n >> 1) & 1u;
       if (ew == 0 && lane == 0) mbar_expect_tx(&xchg[b], 3 * 4 * BLK);
-      if (n >= 2 && !mbar_wait(&consumed[b], k ^ 1u, wc)) return false;
+      if (n >= 2 && !mbar_wait_cluster(&consumed[b], k ^ 1u, wc)) return false;
       if (!mbar_wait(&acc_full[b], k, wc)) return false;
       tc_fence_after();
 #pragma unroll
@@ -273,7 +287,7 @@ tiles_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CU
           sum[i + 3] += v.w;
         }
       __syncwarp();
-      if (lane < KS) mbar_arrive_remote_relaxed(mapa_shared(smem_u32(&consumed[b]), lane));
+      if (lane == 0) mbar_arrive(&taken[b]);
       return true;
     };
     // the box of the m-th tile handed on: free to write / written
