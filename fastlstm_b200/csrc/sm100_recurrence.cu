@@ -938,7 +938,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
   volatile int* dead = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* pub_cnt = const_cast<int*>(dead) + 1;        // [4] arrivals of the epilogue warps, by item index mod 4
   uint64_t* pub_bar = reinterpret_cast<uint64_t*>(pub_cnt + 4);   // [4] item stored? by item index mod 4
-  uint64_t* rdy = pub_bar + 4;                                 // aliased buffers: the 3 peers are done with their MMAs
+  uint64_t* rdy = pub_bar + 4;                                 // aliased buffers: the 3 peers' issuers are done with their MMAs
   uint64_t* consumed = rdy + 1;                                // interleaved tiles: the cluster's four CTAs read an item's slices
   uint64_t* taken = consumed + 1;                              // ... this CTA's eight warps did
 
@@ -959,7 +959,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
     *dead = 0;
     for (int i = 0; i < 4; ++i) pub_cnt[i] = 0;
     for (int i = 0; i < 4; ++i) mbar_init(&pub_bar[i], ITEM_WARPS);
-    mbar_init(rdy, 3);
+    mbar_init(rdy, 3 * nacc);
     mbar_init(consumed, 4);
     mbar_init(taken, ITEM_WARPS);
     fence_mbar_init();
@@ -1118,6 +1118,9 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
               umma_commit(&empty[s]);
             }
             if (ok) umma_commit(&acc_full[a]);
+            // aliased: once these MMAs have read it the ring, and the exchange buffers laid over it, is idle until the
+            // next item: the three peers may write their slices
+            if (TI == 1 && ok && p.alias) umma_commit_multicast(rdy, (uint16_t)(0xF ^ (1u << r)));
             gs += KC;
             while (gs >= R_STAGES) { gs -= R_STAGES; gph ^= 1; }
           }
@@ -1274,15 +1277,6 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
             if (ew == 0 && lane == 0) {
               // what this CTA is about to receive (nothing for a quarter without rows)
               mbar_expect_tx(xchg, bt * RB + (int)r * 32 < p.B ? 3 * XSLOT_BYTES : 0);
-              // aliased: this item's MMAs are done (their reads of the ring completed before acc_full did), so
-              // the ring - and the exchange buffers laid over it - is idle until the next item: tell
-              // the three peers they may write their slices.  Nothing of this thread is published by
-              // the signal, hence relaxed.
-              if (p.alias) {
-#pragma unroll
-                for (int dst = 0; dst < 4; ++dst)
-                  if (dst != (int)r) mbar_arrive_remote_relaxed(mapa_shared(smem_u32(rdy), dst));
-              }
             }
             tc_fence_after();
             const bool q_ok = bt * RB + q * 32 < p.B;       // quarter q has rows

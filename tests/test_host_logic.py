@@ -193,6 +193,23 @@ def test_every_hand_off_through_global_memory_is_a_release():
     assert counted >= 7
 
 
+def test_signals_to_the_cluster_carry_the_reads_before_them():
+    # a CTA that says its reads are done lets a peer overwrite what was read: a relaxed arrival needs a fence in front, and the
+    # peer an acquire at cluster scope
+    import fastlstm_b200
+    relaxed = waits = 0
+    for path in glob.glob(os.path.join(os.path.dirname(fastlstm_b200.__file__), "csrc", "*.cu")):
+        with open(path) as f:
+            code = re.sub(r"//.*", "", f.read())
+        for before in re.findall(r"((?:.*\n){3}).*mbar_arrive_remote_relaxed\(", code):
+            assert "fence_acq_rel_cluster();" in before, path
+            relaxed += 1
+        for wait in re.findall(r"(\w+)\(&?(?:consumed|rdy)\b[^)]*, wc\)", code):
+            assert wait == "mbar_wait_cluster", (path, wait)
+            waits += 1
+    assert relaxed >= 2 and waits >= 3
+
+
 def test_the_lanes_that_fetch_come_behind_the_lane_that_acquired():
     # one lane acquires a hand-off counter, others issue the loads: the shuffle that hands its finding on orders no memory
     import fastlstm_b200
