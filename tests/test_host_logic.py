@@ -204,7 +204,7 @@ def test_signals_to_the_cluster_carry_the_reads_before_them():
         for before in re.findall(r"((?:.*\n){3}).*mbar_arrive_remote_relaxed\(", code):
             assert "fence_acq_rel_cluster();" in before, path
             relaxed += 1
-        for wait in re.findall(r"(\w+)\(&?(?:consumed|rdy)\b[^)]*, wc\)", code):
+        for wait in re.findall(r"(\w+)\(&?(?:consumed|rdy)\b.*?, wc\)", code):
             assert wait == "mbar_wait_cluster", (path, wait)
             waits += 1
     assert relaxed >= 2 and waits >= 3
