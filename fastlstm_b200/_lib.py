@@ -45,6 +45,8 @@ SIGNATURES = {
     "blstm_workspace_bytes": (c_size_t, [DP, c_int]),
     "blstm_plan_name": (c_char_p, [DP, c_int]),
     "blstm_plan_family": (c_int, [DP, c_int]),
+    "blstm_plan_turns": (c_int, [DP, c_int]),
+    "blstm_plan_beside": (c_int, [DP, c_int]),
     "blstm_plan_detail": (c_int, [DP, c_int, ctypes.c_char_p, c_size_t]),
     "blstm_input_projection": (c_int, [DP, P, P, P, P, P, P]),
     "blstm_fwd_recurrence": (c_int, [DP, P, P, P, P, P, c_size_t, P]),

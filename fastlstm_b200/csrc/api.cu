@@ -239,6 +239,9 @@ int blstm_plan_family(const blstm_desc* d, int phase) {
   return sm100::f32_plan(*d, phase).ok ? BLSTM_FAMILY_F32_CLUSTER : BLSTM_FAMILY_GENERIC;
 }
 
+int blstm_plan_turns(const blstm_desc* d, int phase) { return check_desc(d) ? 0 : sm100_plan_turns(*d, phase); }
+int blstm_plan_beside(const blstm_desc* d, int phase) { return check_desc(d) ? 0 : sm100_plan_beside(*d, phase); }
+
 const char* blstm_plan_name(const blstm_desc* d, int phase) {
   switch (blstm_plan_family(d, phase)) {
     case BLSTM_FAMILY_NONE: return "invalid";

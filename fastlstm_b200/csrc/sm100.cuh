@@ -28,6 +28,9 @@ int sm100_bwd_recurrence(const blstm_desc& d, const void* dout, const void* dh_n
 
 // which of the recurrences a phase uses (BLSTM_FAMILY_*; BLSTM_FAMILY_NONE when the tcgen05 kernels do not cover it)
 int sm100_plan_family(const blstm_desc& d, int phase);
+// small-batch recurrences: chunks of rows a cluster works through, launches that are resident at once (0: another family)
+int sm100_plan_turns(const blstm_desc& d, int phase);
+int sm100_plan_beside(const blstm_desc& d, int phase);
 // one-line description of the launch plan of a phase ("" when the tcgen05 kernels do not cover it)
 int sm100_plan_detail(const blstm_desc& d, int phase, char* buf, size_t n);
 

@@ -1571,6 +1571,14 @@ int sm100_plan_family(const blstm_desc& d, int phase) {
   if (resident_plan(d, phase).ok || tiles_plan(d, phase).ok) return BLSTM_FAMILY_RESIDENT;
   return (phase == BLSTM_PHASE_BWD ? make_bwd_plan(d).ok : make_plan(d, phase).ok) ? BLSTM_FAMILY_BATCH_TILES : BLSTM_FAMILY_NONE;
 }
+int sm100_plan_turns(const blstm_desc& d, int phase) {
+  const SmallPlan p = small_plan(d, phase);
+  return p.ok ? p.nch : 0;
+}
+int sm100_plan_beside(const blstm_desc& d, int phase) {
+  const SmallPlan p = small_plan(d, phase);
+  return p.ok ? resident_clusters(p.nc) / p.ncl : 0;
+}
 bool sm100_recurrence_supported(const blstm_desc& d, int phase) { return sm100_plan_family(d, phase) != BLSTM_FAMILY_NONE; }
 size_t sm100_recurrence_workspace(const blstm_desc& d, int phase) {
   const SmallPlan sp = small_plan(d, phase);

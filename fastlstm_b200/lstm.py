@@ -288,8 +288,14 @@ def _shares_device(dtype, T, B, I, H):
 def _wavefront_pays(dtype, T, B, H, grad):
     """Whether a stack that could run as a wavefront should.  Two layers, ms layer after layer / as a wavefront (B200):
 
-    Without gradients the small-batch recurrences leave nothing to hide, on a few SMs of either half (T=256, B=64, H=256:
-    0.56 / 0.64; T=128, B=1000, H=64: 0.23 / 0.5); resident weights gain from 128 steps on where half of the device has
+    Without gradients the small-batch recurrences have SMs to spare only while a layer's clusters fit beside the other's
+    with no more rows to work through in turn; the launches of a wavefront then take some 0.45 ms of the host
+    (B=64, H=64: T=256 0.33 / 0.42, T=512 0.59 / 0.50, T=1024 1.10 / 0.83; B=16, H=128: T=256 0.38 / 0.42, T=512 0.69 / 0.57; B=8,
+    H=512: T=128 0.47 / 0.45, T=512 1.61 / 1.16; but B=64, H=192: T=1024 1.58 / 1.70, B=1000, H=64: 1.37 / 1.78).  Where a cluster has
+    four chunks in turn, from H = 384 on three, and half of the device would have resident weights, 32 rows to a group of H / 32 CTAs at
+    most, these win (T=256: B=200, H=320 1.50 / 1.30; B=130, H=448 1.50 / 1.37; B=150, H=384 1.33 / 1.33, T=512 2.57 / 2.41; but
+    B=400, H=256, 48 rows, 1.32 / 1.59; B=100, H=512, two chunks, 1.26 / 1.37).
+    Resident weights gain from 128 steps on where half of the device has
     them too (T=128 and 256: B=128, H=512 0.91 / 0.81 and 1.73 / 1.40; B=440, H=320 0.98 / 0.98 and 1.87 / 1.75), the kernels
     with several 128-row tiles always (T=128, B=1000, H=192: 1.31 / 1.05).
 
@@ -301,9 +307,18 @@ def _wavefront_pays(dtype, T, B, H, grad):
     fwd = _family(dtype, T, B, H, H, "fwd")
     if grad:
         return T >= (96 if H < 320 else 128) and H <= 384 and not (fwd in on_chip and _family(dtype, T, B, H, H, "bwd") in on_chip)
+    if fwd == _lib.FAMILY_BATCH_TILES:
+        return True
+    half = _family(dtype, T, B, H, H, "fwd", True)
     if fwd == _lib.FAMILY_RESIDENT:
-        return T >= 128 and _family(dtype, T, B, H, H, "fwd", True) in on_chip
-    return fwd != _lib.FAMILY_SMALL_BATCH
+        return T >= 128 and half in on_chip
+    lib, whole, part = _lib.load(), _desc(dtype, T, B, H, H), _desc(dtype, T, B, H, H, _lib.FLAG_HALF_DEVICE)
+    turns = lib.blstm_plan_turns(whole, _lib.PHASE_FWD)
+    if half == _lib.FAMILY_SMALL_BATCH:
+        return (T >= (128 if H >= 512 else 192) and T * (H + 64) >= 65536
+                and turns == lib.blstm_plan_turns(part, _lib.PHASE_FWD) and lib.blstm_plan_beside(part, _lib.PHASE_FWD) >= 2)
+    long_enough = T >= 128 if turns >= 4 else turns == 3 and H >= 384 and T >= 256
+    return half == _lib.FAMILY_RESIDENT and long_enough and B <= 32 * (74 // (H // 32))
 
 
 class _Beside:

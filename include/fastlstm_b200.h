@@ -123,6 +123,11 @@ enum {
 };
 int blstm_plan_family(const blstm_desc* d, int phase);
 
+/* BLSTM_FAMILY_SMALL_BATCH: how many chunks of batch rows a cluster works through in turn, and how many launches of the
+ * plan the device holds at once.  0 for the other families. */
+int blstm_plan_turns(const blstm_desc* d, int phase);
+int blstm_plan_beside(const blstm_desc* d, int phase);
+
 /* Writes a one-line, human-readable description of the launch geometry the phase will use
  * (tile sizes, interleaved batch tiles, grid, ring depth) into the HOST buffer `buf`.
  * Read-only; stands in for inspecting the reference's chosen autotune config

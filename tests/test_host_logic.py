@@ -369,7 +369,11 @@ def test_wavefront_where_it_measured_faster():
     for grad, T, B, H, want in ((True, 256, 968, 192, True), (True, 128, 768, 384, True), (True, 64, 768, 384, False),
                                 (True, 256, 392, 576, False), (True, 256, 512, 512, False), (True, 256, 32, 256, False),
                                 (False, 256, 64, 64, False), (False, 256, 64, 256, False), (False, 128, 64, 512, False),
-                                (False, 128, 128, 512, True), (False, 64, 128, 512, False), (False, 128, 1000, 192, True)):
+                                (False, 128, 128, 512, True), (False, 64, 128, 512, False), (False, 128, 1000, 192, True),
+                                # (long sequences of few rows: the clusters of two layers fit beside each other)
+                                (False, 1024, 64, 64, True), (False, 256, 8, 256, True), (False, 128, 8, 256, False),
+                                (False, 1024, 64, 192, False), (False, 1024, 1000, 64, False), (False, 1024, 100, 512, False),
+                                (False, 256, 200, 320, True), (False, 256, 400, 256, False)):
         assert lstm._wavefront_pays(bf, T, B, H, grad) == want, (grad, T, B, H)
         if H <= 512 and B > 8:
             # ... and it is what the module asks before it runs, and the benchmark before it reports
