@@ -200,10 +200,9 @@ __global__ void __launch_bounds__(32 * (UH == 16 && TI >= 2 ? 12 : 11), 1)
 fwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmH,
            const __grid_constant__ CUtensorMap tmP, const FwdParams p) {
   constexpr int N = 4 * UH;
-  // One tile in flight: h leaves through a TMA store (tmP: out as {unit, row, step}) that the warp sees completed after
-  // some 300 clocks, staged in the ring, which is idle until this CTA has counted the item in.  Plain stores cost the
-  // release behind them 1.6 k clocks (128 CTAs handing one tile on in a loop: 4.6 k clocks a hand-off with plain stores
-  // and the wide proxy fence, 3.1 k this way).
+  // One tile in flight: plain stores of h, the release behind them, then what only backward needs (the release waits for
+  // every store of the SM that is under way).  TMA stores that the warps wait for in front of the release cost 0.1 to
+  // 0.3 us a step more (H = 1536, B = 128: 8.8 -> 8.6; H = 1088, B = 200: 7.8 -> 7.5).
   // Interleaved tiles are throughput bound, and there the epilogue's row-strided 16-byte global
   // accesses (a thread owns a batch row: 32 sectors per warp instruction) were the bottleneck: the
   // projected pre-activations come in as TMA boxes through shared memory, one set of buffers per
@@ -270,7 +269,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
     for (int s = 0; s < R_STAGES; ++s) mbar_expect_tx(&full[s], SB);
     tma_prefetch_desc(&tmW);
     tma_prefetch_desc(&tmH);
-    tma_prefetch_desc(&tmP);
+    if (TMAEP) tma_prefetch_desc(&tmP);
   }
   if (warp == 1) tmem_alloc(tmem_slot, TMEM_COLS);
   tc_fence_before();
@@ -608,8 +607,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
     const int row_in_tile = q * 32 + lane;
     const int unit0 = ht * UH + ug * NU;
     const size_t H4 = 4 * (size_t)H;
-    uint8_t* hbuf = a_s + ew * (64 * NU);   // this warp's 32 rows x NU units of h
     T16* ifgo = reinterpret_cast<T16*>(p.ifgo);
+    T16* out = reinterpret_cast<T16*>(p.out);
     T16* cell = reinterpret_cast<T16*>(p.cell);
     int it = 0;                             // items consumed: TMEM buffer it & 1, on its (it >> 1)-th use
     bool ok = true;
@@ -701,20 +700,15 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
             c[j][u] = cn;
             hv[u] = sigmoid_fast(pa[3][u]) * tanh_fast(cn);
           }
+          if (row_ok) {
 #pragma unroll
-          for (int v = 0; v < NV; ++v) store8<T16>(reinterpret_cast<T16*>(hbuf + lane * (2 * NU)) + 8 * v, &hv[8 * v]);
+            for (int v = 0; v < NV; ++v) store8<T16>(out + o1 + 8 * v, &hv[8 * v]);
+          }
           // publish h[t+1] first (it is all the peers wait for): one arrival per CTA and item, by the last epilogue warp
           // whose rows are stored (a warp can be at most two items ahead of another, so four counters never mix items)
-          fence_proxy_async_smem();
           __syncwarp();
-          if (lane == 0) {
-            tma_store_3d(&tmP, hbuf, unit0, bt * RB + q * 32, t + 1);
-            tma_store_commit();
-            tma_store_wait<0>();
-            if ((smem_count_arrive(&pub_cnt[it & 3]) & (EW - 1)) == EW - 1) {
-              if (!p.no_arrive) red_release_gpu_add(&p.flags[(size_t)(t + 1) * p.nbt + bt], 1);
-            }
-          }
+          if (lane == 0 && (smem_count_arrive(&pub_cnt[it & 3]) & (EW - 1)) == EW - 1 && !p.no_arrive)
+            red_release_gpu_add(&p.flags[(size_t)(t + 1) * p.nbt + bt], 1);
           __syncwarp();
           // only now (after the release: a fence would otherwise wait for these loads) fetch the NEXT
           // item's projected pre-activations; they land while the peers run their step
@@ -857,7 +851,7 @@ static BwdPlan make_bwd_plan(const blstm_desc& d) {
     int st2 = 0, ni2 = 0;
     const size_t fixed2 = 1024 + wres + 1024 + tail_pad;
     if (pick_ring(fixed2, p.stage_bytes, n_issuers, H / RK, &st2, &ni2) && st2 > p.stages &&
-        (size_t)st2 * p.stage_bytes >= p.recv_bytes + 16384) {    // (and the rows on their way out lie behind them)
+        (size_t)st2 * p.stage_bytes >= p.recv_bytes) {
       p.alias = 1; p.stages = st2; p.ni = ni2; fixed = fixed2;
     }
   }
@@ -905,8 +899,7 @@ struct BwdParams {
 
 template <int TI, typename T16>
 __global__ void __launch_bounds__(384, 1)
-bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmG,
-           const __grid_constant__ CUtensorMap tmD, const BwdParams p) {
+bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmG, const BwdParams p) {
   // Warps: 0 = TMA producer, then NACC MMA issuers, then (interleaved tiles only) one PUBLISHER warp,
   // then 8 epilogue warps from warp 4 on - 12 in all either way.
   // With interleaved tiles the epilogue warps are the bottleneck, and the release that publishes an
@@ -966,7 +959,6 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
     for (int s = 0; s < R_STAGES; ++s) mbar_expect_tx(&full[s], SB);
     tma_prefetch_desc(&tmW);
     tma_prefetch_desc(&tmG);
-    if (TI == 1) tma_prefetch_desc(&tmD);
   }
   if (warp == 1) tmem_alloc(tmem_slot, TMEM_COLS);
   tc_fence_before();
@@ -1147,9 +1139,6 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
     uint8_t* put = (q == (int)r ? recv + (size_t)r * XSLOT_BYTES : stage + (size_t)(q < (int)r ? q : q - 1) * XSLOT_BYTES) + g * (XSLOT_BYTES / 2);
     // a half's row is 128 bytes; piece k lies at k XOR row XOR half: conflict-free for the writers (32 rows, one piece)
     // and for the readers (a row's even, then odd pieces of both halves)
-    // one tile in flight: this warp's d_ifgo rows on their way out, in the ring, which is idle until this CTA has counted the
-    // item in (behind the exchange buffers where those lie over the ring)
-    uint8_t* obuf = a_s + (p.alias ? 7 * XSLOT_BYTES : 0) + ew * 2048 + lane * 16;
     const int half = (lane >> 2) & 1;
     const uint8_t* get = recv + half * (XSLOT_BYTES / 2) + grow * XROW_BYTES;
     const int get_x = (grow & 7) ^ half;
@@ -1396,15 +1385,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
                 qo[w] = pk2<T16>(r_[0][3], r_[1][3]);
               }
             }
-            if constexpr (TI == 1) {
-              // one tile in flight: out through a TMA store (a box of 4 gates x 4 rows x 64 units a warp) that the warp
-              // sees completed after some 300 clocks; plain stores cost the release behind them 1.6 k
-              stg16(obuf, make_uint4(qi[0], qi[1], qi[2], qi[3]));
-              stg16(obuf + 512, make_uint4(qf[0], qf[1], qf[2], qf[3]));
-              stg16(obuf + 1024, make_uint4(qg[0], qg[1], qg[2], qg[3]));
-              stg16(obuf + 1536, make_uint4(qo[0], qo[1], qo[2], qo[3]));
-              fence_proxy_async_smem();
-            } else if (row_ok) {
+            if (row_ok) {
               T16* dstp = dg + ((size_t)t * p.B + row) * H4 + unit0;
               stg16(dstp, make_uint4(qi[0], qi[1], qi[2], qi[3]));
               stg16(dstp + (size_t)H, make_uint4(qf[0], qf[1], qf[2], qf[3]));
@@ -1420,9 +1401,6 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUte
               if constexpr (PUBLISHER) {
                 mbar_arrive(&pub_bar[pub_it & 3]);
               } else {
-                tma_store_4d(&tmD, obuf - lane * 16, ugc * 64, bt * RB + (int)r * 32 + ew * 4, 0, t);
-                tma_store_commit();
-                tma_store_wait<0>();
                 const bool pub = (smem_count_arrive(&pub_cnt[pub_it & 3]) & (ITEM_WARPS - 1)) == ITEM_WARPS - 1;
                 if (pub && !p.no_arrive) red_release_gpu_add(&p.flags[(size_t)t * p.nbt + bt], 1);
               }
@@ -1557,9 +1535,8 @@ static int bwd_cta_capacity() {
 }
 
 template <int TI, typename T16>
-static int launch_bwd_t(const BwdPlan& pl, const CUtensorMap& tw, const CUtensorMap& tg, const CUtensorMap& td, BwdParams& p,
-                        cudaStream_t st) {
-  return launch_coresident(bwd_kernel<TI, T16>, pl.grid, pl.threads, pl.smem, 4, st, tw, tg, td, p);
+static int launch_bwd_t(const BwdPlan& pl, const CUtensorMap& tw, const CUtensorMap& tg, BwdParams& p, cudaStream_t st) {
+  return launch_coresident(bwd_kernel<TI, T16>, pl.grid, pl.threads, pl.smem, 4, st, tw, tg, p);
 }
 
 }  // namespace sm100
@@ -1647,12 +1624,8 @@ int sm100_fwd_recurrence(const blstm_desc& d, void* ifgo, const void* Wh, void* 
   CUtensorMap tp;
   {
     const int NU = 4 * pl.UH / pl.epi_warps;
-    if (pl.TI == 1) {  // out [T+1,B,H] as {unit, batch row, t}: a box is one warp's 32 rows x NU units
-      uint64_t dims[3] = {(uint64_t)H, (uint64_t)B, (uint64_t)(T + 1)};
-      uint64_t str[2] = {(uint64_t)H * 2, (uint64_t)B * H * 2};
-      uint32_t box[3] = {(uint32_t)NU, 32, 1};
-      rc = encode_tensor_map(&tp, out, 3, dims, str, box, 2, 0);
-      if (rc) return rc;
+    if (pl.TI == 1) {
+      tp = th;         // (not used)
     } else {  // ifgo [T,B,4H] as {unit, batch row, gate, t}: a box is one warp's 4 gates x 32 rows x NU units;
        // the box's inner extent equals the swizzle span (32 bytes) or is a single 16-byte piece (none)
       uint64_t dims[4] = {(uint64_t)H, (uint64_t)B, 4, (uint64_t)T};
@@ -1731,14 +1704,6 @@ int sm100_bwd_recurrence(const blstm_desc& d, const void* dout, const void* dh_n
     rc = encode_tensor_map(&tg, d_ifgo, 3, dims, str, box);
     if (rc) return rc;
   }
-  CUtensorMap td;
-  {  // d_ifgo [T,B,4H] as {unit, batch row, gate, t}: a box is one warp's 4 gates x 4 rows x 64 units
-    uint64_t dims[4] = {(uint64_t)H, (uint64_t)B, 4, (uint64_t)T};
-    uint64_t str[3] = {(uint64_t)4 * H * 2, (uint64_t)H * 2, (uint64_t)B * 4 * H * 2};
-    uint32_t box[4] = {64, 4, 4, 1};
-    rc = encode_tensor_map(&td, d_ifgo, 4, dims, str, box, 2, 0);
-    if (rc) return rc;
-  }
   BwdParams p;
   p.T = T; p.B = B; p.H = H;
   p.nbt = pl.nbt; p.nug = pl.nug; p.nb_par = pl.nb_par; p.ntl = pl.ntl; p.stages = pl.stages; p.ni = pl.ni;
@@ -1755,9 +1720,9 @@ int sm100_bwd_recurrence(const blstm_desc& d, const void* dout, const void* dh_n
   p.d_ifgo = d_ifgo; p.dh0 = dh0; p.dc0 = dc0;
   p.db_part = db ? reinterpret_cast<float*>(static_cast<char*>(ws) + pl.off_db) : nullptr;
   const bool bf = d.dtype == BLSTM_BF16;
-  if (pl.TI == 1)      rc = bf ? launch_bwd_t<1, __nv_bfloat16>(pl, tw, tg, td, p, st) : launch_bwd_t<1, __half>(pl, tw, tg, td, p, st);
-  else if (pl.TI == 2) rc = bf ? launch_bwd_t<2, __nv_bfloat16>(pl, tw, tg, td, p, st) : launch_bwd_t<2, __half>(pl, tw, tg, td, p, st);
-  else                 rc = bf ? launch_bwd_t<4, __nv_bfloat16>(pl, tw, tg, td, p, st) : launch_bwd_t<4, __half>(pl, tw, tg, td, p, st);
+  if (pl.TI == 1)      rc = bf ? launch_bwd_t<1, __nv_bfloat16>(pl, tw, tg, p, st) : launch_bwd_t<1, __half>(pl, tw, tg, p, st);
+  else if (pl.TI == 2) rc = bf ? launch_bwd_t<2, __nv_bfloat16>(pl, tw, tg, p, st) : launch_bwd_t<2, __half>(pl, tw, tg, p, st);
+  else                 rc = bf ? launch_bwd_t<4, __nv_bfloat16>(pl, tw, tg, p, st) : launch_bwd_t<4, __half>(pl, tw, tg, p, st);
   if (rc) return rc;
   if (db) return reduce_db(p.db_part, pl.nb_par * 32, 4 * H, db, st);
   return BLSTM_OK;
