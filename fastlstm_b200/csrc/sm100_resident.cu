@@ -14,8 +14,8 @@
 // Batch rows are divided over groups of CTAs that know nothing of each other.
 //
 // us per step, the recurrences with the batch on the M side -> these (B200): forward B=32 H=2048 7.9 -> 4.4, B=256 H=1024
-// 7.2 -> 5.7, B=128 H=1024 4.3, B=256 H=768 6.7 -> 4.8; backward B=32 H=2048 10.0 -> 6.9, B=256 H=1024 7.6 -> 6.2, B=256 H=768
-// 6.8 -> 5.7, B=32 H=1536 4.6.
+// 7.2 -> 5.7, B=128 H=1024 4.2, B=256 H=768 6.7 -> 4.7; backward B=32 H=2048 10.0 -> 6.8, B=256 H=1024 7.6 -> 6.1, B=256 H=768
+// 6.8 -> 5.6, B=32 H=1536 4.5.
 // Bound by the chain of a step: hand-off through L2 (its release alone 0.5 us), fetch of N rows, 64 MMAs of some 50 clocks,
 // exchange, gate maths.
 #include <algorithm>
@@ -452,8 +452,8 @@ resident_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
 // The smallest split of K whose slice fits the chip, and as many groups of rows as fit beside each other.  Backward, a slice
 // of 22 chunks and 32 rows fits with one issuer only (one accumulator instead of two leaves tensor memory for the chunk
 // that would not fit); one more CTA a cluster makes room for two, which is worth it while a group keeps to 32 rows.  us a
-// step: H = 1728, B = 32: 6.9 -> 5.0, H = 1408, B = 64: 6.9 -> 5.0, but B = 96, then 48 rows a group, 6.9 -> 7.3.
-// H = 2048 with 17 to 32 rows is left with one issuer over six CTAs (6.9; two take 5.3 at H = 1984): a B200 holds
+// step: H = 1728, B = 32: 6.8 -> 4.9, H = 1408, B = 64: 6.8 -> 4.8, but B = 96, then 48 rows a group, 6.7 -> 7.1.
+// H = 2048 with 17 to 32 rows is left with one issuer over six CTAs (6.8; two take 5.2 at H = 1984): a B200 holds
 // 15 clusters of seven or eight CTAs and 16 M tiles need 16; the kernel with the batch on the M side takes 8.6.
 ResPlan resident_plan(const blstm_desc& d, int phase) {
   const int H = d.hidden_size, B = d.batch;

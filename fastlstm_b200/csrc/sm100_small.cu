@@ -376,9 +376,9 @@ small_bwd_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant_
   constexpr int S = 8;                                          // slots of the ring
   // A single tile per warp splits its K steps over two accumulators (a chain of 16 MMAs takes 350 clocks)
   constexpr int NA = MPW == 1 ? 2 : 1;
-  // All K steps in registers but for five groups of units a CTA and, in one CTA, fewer than eight: there the number of
-  // groups follows from KR, and a step with addresses known at compile time takes 5 to 11 % less (H = 384, B = 32: 1.23 ->
-  // 1.15 us, H = 512, B = 128: 2.8 -> 2.5; H = 512, B = 32 5 % more).
+  // All K steps in registers but for five groups of units a CTA and, in one CTA, fewer than eight: elsewhere the number of
+  // groups follows from KR, and a step with addresses known at compile time takes less (us, H = 384, B = 168: 2.30 -> 2.07; H = 256,
+  // B = 64: 0.95 -> 0.89; H = 512, B = 128: 2.40 both; with five groups H = 640, B = 50: 2.25 -> 2.15, B = 100: 3.0 -> 3.2).
   constexpr bool TAIL = CL ? MPW == 5 : KR < 16;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -491,8 +491,8 @@ small_bwd_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant_
                                                           warp * 256) + lane;
       dh[0] = dh[1] = 0.f;
 #pragma unroll 8
-      for (int s = 0; s < p.nc; ++s) {
-        const float2 v = src[(size_t)s * (src_b / 8)];
+      for (int s = 0; s < p.nc; ++s, src += src_b / 8) {
+        const float2 v = *src;
         dh[0] += v.x;
         dh[1] += v.y;
       }
@@ -658,18 +658,19 @@ small_bwd_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant_
 #pragma unroll
           for (int e = 0; e < 4; ++e) acc[i][e] = 0.f;
         const uint32_t da = sbase + d_off + (uint32_t)(par * CR + (lane & 7)) * pitch + (lane >> 3) * 16;
-        uint32_t bf[2][4];
-        ldmatrix_x4(da, bf[0]);
+        constexpr int AH = KR / 2 <= 4 ? KR / 2 : 2;             // operand fetches run ahead of the MMAs
+        uint32_t bf[AH][4];
+#pragma unroll
+        for (int kk = 0; kk < (AH == KR / 2 ? AH : 1); ++kk) ldmatrix_x4(da + kk * 64, bf[kk]);
 #pragma unroll
         for (int kk = 0; kk < KR / 2; ++kk) {
-          if (kk + 1 < KR / 2) {
-            ldmatrix_x4(da + (kk + 1) * 64, bf[(kk + 1) & 1]);
-          }
+          if (AH < KR / 2 && kk + 1 < KR / 2) ldmatrix_x4(da + (kk + 1) * 64, bf[(kk + 1) & 1]);
 #pragma unroll
-          for (int i = 0; i < MPW; ++i) mma16816<T16>(acc[i], w[i][2 * kk], bf[kk & 1][0], bf[kk & 1][1]);
+          for (int i = 0; i < MPW; ++i) mma16816<T16>(acc[i], w[i][2 * kk], bf[kk % AH][0], bf[kk % AH][1]);
 #pragma unroll
-          for (int i = 0; i < MPW; ++i) mma16816<T16>(acc[i + NA - 1], w[i][2 * kk + 1], bf[kk & 1][2], bf[kk & 1][3]);
+          for (int i = 0; i < MPW; ++i) mma16816<T16>(acc[i + NA - 1], w[i][2 * kk + 1], bf[kk % AH][2], bf[kk % AH][3]);
         }
+#pragma unroll 1
         for (int kk = KR / 2; TAIL && kk < gc; ++kk) {
           uint32_t b[4];
           ldmatrix_x4(da + kk * 64, b);
@@ -757,14 +758,15 @@ int resident_clusters(int nc) {
 // general ones) take nearly the same time for any batch of up to several hundred rows, these about the same for
 // every chunk of 8 rows after the first, so the line is a number of chunks per cluster.  us per step (B200), these against
 // the others at 1, 2, 3, ... chunks, a dash where the line lies.
-// Forward: H = 192: 8: 3.5 / 5.5 (nothing saved: 4.5) - 10: 4.4 / 5.6 (4.6), 12: 5.3 / 5.6 (4.6; and two layers as a wavefront beat both);
-// H = 256: 3: 2.1 / 2.8, 4: 2.4 / 3.1 - 5: 3.3 / 3.1; H = 320: 3: 2.0 / 2.8, 4: 2.7 / 2.9 - 5: 3.4 / 3.2; H = 384: 2: 1.7 / 2.9, 3: 2.4 / 2.9 -
-// 4: 3.3 / 3.3; H = 448: 3: 2.8 / 3.1 - 4: 3.7 / 3.4; H = 512: 1: 1.6 / 3.0, 2: 2.2 / 3.1 - 3: 3.2 / 3.1 to 3.5, 5: 5.3 / 3.5;
-// H = 576: 1: 1.9 / 3.2 - 2: 3.7 / 3.2; H = 640: 1: 2.2 / 3.2 - 2: 4.2 / 3.2; H = 768: 1: 2.5 / 3.4.
-// Backward: H = 192: 8: 4.7 / 5.0 - 9: 5.2 / 5.0; H = 256: 5: 3.3 / 3.6, 6: 3.9 / 4.9; H = 320: 4: 3.3 / 3.6 - 5: 4.0 / 3.6; H = 384: 4: 3.1 / 3.7 -
-// 5: 3.8 / 3.7; H = 448: 4: 3.7 / 3.9 - 5: 4.2 / 3.9; H = 512: 3: 2.5 / 3.4, 4: 3.3 / 3.9, 5: 4.05 / 3.91; H = 576: 2: 3.3 / 3.5; H = 640: 2: 3.3 / 3.6
-// (more does not fit).  At H = 512 five chunks are a tie but for 4 %, and taken so that a batch of 256 rows and its
-// halves go through the same kernels and agree bit for bit, which they do not across a line.
+// Forward: H = 192: 8: 3.5 / 5.3 (nothing saved: 4.6) - 10: 4.3 / 5.4 (4.7), 12: 5.2 / 5.4 (4.7; and two layers as a wavefront beat both);
+// H = 256: 3: 2.1 / 2.7, 4: 2.3 / 3.1 - 5: 3.2 / 3.1; H = 320: 3: 2.0 / 2.8, 4: 2.7 / 2.8 - 5: 3.4 / 3.2; H = 384: 2: 1.7 / 2.9, 3: 2.3 / 2.9 -
+// 4: 3.1 / 3.2; H = 448: 3: 2.7 / 3.3 - 4: 3.6 / 3.3; H = 512: 1: 1.6 / 3.0, 2: 2.2 / 3.1 - 3: 3.1 to 3.2 / 3.1 to 3.4, 5: 5.3 / 3.5;
+// H = 576: 1: 1.9 / 3.1 - 2: 3.8 / 3.1; H = 640: 1: 2.2 / 3.2 - 2: 4.1 / 3.2; H = 768: 1: 2.5 / 3.4.
+// Backward: H = 192: 8: 4.4 / 4.9 - 9: 4.95 / 4.95; H = 256: 5: 3.0 / 3.5, 6: 3.6 / 4.8; H = 320: 4: 3.1 / 3.5 - 5: 3.6 / 3.5; H = 384: 4: 2.8 / 3.6 -
+// 5: 3.5 / 3.6; H = 448: 4: 3.5 / 3.8 - 5: 3.9 / 3.8; H = 512: 3: 2.6 / 3.3, 4: 3.4 / 3.8, 5: 4.1 / 3.8 (B = 256), 4.1 / 5.3 (B = 280); H = 576: 2: 3.4
+// to 3.9 / 3.4 to 3.9; H = 640: 2: 3.4 / 3.5 to 3.9 (more does not fit).  At H = 512 the fifth chunk costs 9 % up to 256 rows and is
+// taken there so that a batch of 256 rows and its halves go through the same kernels and agree bit for bit, which they do not
+// across a line.
 // (General kernels, forward: H = 64, B = 64: 1.9 -> 0.59; H = 192: 4.4 a step at any of these batches.)
 static bool small_plan_pays(int H, const SmallPlan& p, int phase) {
   if (H <= 128) return true;
