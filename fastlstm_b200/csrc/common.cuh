@@ -86,7 +86,7 @@ __device__ __forceinline__ int ld_relaxed_gpu(const int* p) {
 // Counts in on data that other SMs read behind ld_acquire_gpu.  Also where the data left through TMA stores that this
 // thread, or warps it has synchronised with, waited for: the wait makes them visible to the waiting thread, and only a
 // release carries that on to the reader.  Its fence takes 700 clocks when no store of the SM is under way, 1.2 k behind
-// the stores of other warps (a relaxed reduction: 40); on the chain of a step that is 0.5 to 0.6 us.
+// the stores of other warps (a relaxed reduction: 40); on the chain of a step that is 0.4 to 0.6 us.
 __device__ __forceinline__ void red_release_gpu_add(int* p, int v) {
   asm volatile("red.release.gpu.global.add.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
