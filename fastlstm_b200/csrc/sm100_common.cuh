@@ -180,6 +180,14 @@ __device__ __forceinline__ bool mbar_wait_spin(uint64_t* bar, uint32_t parity, c
   return mbar_wait_slow(bar, parity, w);
 }
 
+// Every lane waits for a barrier of its own; the answer is the warp's.
+__device__ __forceinline__ bool warp_wait_all(uint64_t* bar, uint32_t parity, const WaitCtx& w) {
+#pragma unroll 1
+  for (int i = 0; i < 4096; ++i)
+    if (__all_sync(0xffffffffu, mbar_test_wait(bar, parity))) return true;
+  return __all_sync(0xffffffffu, mbar_wait_slow(bar, parity, w));
+}
+
 // ---------------------------------------------------------------- fences
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async;" ::: "memory"); }
 // For global memory only, which is all a hand-off through global memory needs: 12 clocks where the fence over every

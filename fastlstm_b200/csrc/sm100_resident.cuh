@@ -10,10 +10,11 @@ constexpr int RES_MIN_H = 256;         // (smaller sizes have the small-batch ke
 struct ResPlan {
   bool ok;
   int ks, own, mt, ng;      // CTAs per cluster (parts of K); of these, owners of batch rows; M tiles; groups of rows
-  int rows, N;              // batch rows per group; N of the MMAs
+  int ti, rows, N;          // tiles per group, in turn; batch rows of a tile; N of the MMAs
   int kc_total, kcm, nt;    // chunks of K; most of a CTA; of these in tensor memory
   int x_bytes;
   int ni;                   // MMA issuers
+  int group;                // chunks at once
   int grid;
   size_t smem, off_db, ws_bytes;
 };

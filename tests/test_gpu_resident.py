@@ -42,6 +42,14 @@ def test_resident_recurrences_against_fp32_maths(dtype, shape):
     assert all(torch.equal(a, b) for a, b in zip(got, _bwd(lib, d, dout, dh, dc, ifgo, cell, Wh)))
 
 
+# Where a group of rows becomes two tiles: 16 and 17 rows, a last group whose second tile has no rows, tiles of 16 rows with one
+# issuer and with two, of 32 rows, K in two parts forward, enough steps for the tiles to take turns
+@pytest.mark.parametrize("shape", [(9, 64, 1024), (9, 65, 1024), (9, 17, 2048), (9, 32, 2048), (9, 100, 768), (9, 257, 512), (9, 250, 768)])
+def test_tiles_that_take_turns(shape):
+    test_resident_recurrences_against_fp32_maths("bf16", shape)
+    test_resident_recurrences_against_fp32_maths("fp16", shape)
+
+
 @pytest.mark.parametrize("phase", [0, 1])
 @pytest.mark.parametrize("B,H", [(32, 1024), (32, 1536), (2048, 512)])
 def test_resident_recurrences_give_up_with_a_status_when_nothing_arrives(phase, B, H):
