@@ -6,9 +6,10 @@
 // many: 64 x 64 outputs by 64 threads of 8 x 8 (four 16-byte shared-memory reads per 64 FMAs, which are issued in pairs),
 // six or more per SM; where those do not fill the GPU, K is split over blocks too.  A
 // four-stage cp.async pipeline of 16 K steps feeds them; operands contiguous along K are transposed on the way in by
-// 4-byte copies, the others move in 16-byte copies where their rows allow it.  Bound by FFMA issue and, below a wave of
-// blocks, by latency.  Measured (B200; 64 x 64 x 16 blocks of 4 x 4 per thread without pipeline before): T*B = 16384, H = I =
-// 256: 327 / 358 / 3386 -> 215 / 210 / 437 us (41 TFLOP/s of 74); T*B = 4400, H = I = 257: 109 / 128 / 619 -> 73 / 97 / 201 us.
+// 4-byte copies, the others move in 16-byte copies where their rows allow it.  Bound by the FMAs' register operands (without any
+// shared-memory read in the loop 48 TFLOP/s, one FMA an issue slot 39) and, below a wave of blocks, by latency.  Measured (B200; every copy
+// with checks and a 64-bit product of its own before; projection, input gradient, both weight gradients): T*B = 16384, H = I = 256:
+// 214 / 211 / 435 -> 191 / 193 / 377 us (45 TFLOP/s of 74); T*B = 4400, H = I = 257: 72 / 97 / 201 -> 69 / 86 / 164 us.
 #include "f32_gemm.cuh"
 
 namespace blstm {
@@ -26,6 +27,12 @@ struct F32GemmParams {
   int a_vec, b_vec, c_vec;  // rows allow 16-byte accesses (operands: those contiguous along M / N)
 };
 
+__device__ __forceinline__ void cp_async4(uint32_t dst, const float* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async16(uint32_t dst, const float* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
 __device__ __forceinline__ void cp_async4(uint32_t dst, const float* src, bool ok) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(ok ? 4 : 0) : "memory");
 }
@@ -33,10 +40,31 @@ __device__ __forceinline__ void cp_async16z(uint32_t dst, const float* src, bool
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
 }
 
-// One operand's 64 x 16 tile into shared memory as [k][64 + 4].
+// One operand's 64 x 16 tile into shared memory as [k][64 + 4].  A tile that lies inside the operand is fetched from
+// addresses that differ between the copies by the same amount for all threads; checks and 64-bit products for each copy took as many
+// issue slots as the FMAs left.
 template <bool KC>
 __device__ __forceinline__ void load_tile(uint32_t dst, const float* base, long long ld, int m0, int M, int k0, int k1, int vec) {
-  if constexpr (KC) {
+  const int t = threadIdx.x;
+  if (m0 + FM <= M && k0 + FK <= k1) {
+    if constexpr (KC) {
+      const float* src = base + m0 * ld + k0;
+      const int at = (t / FK) * (int)ld + t % FK;
+      const uint32_t d = dst + ((t % FK) * FP + t / FK) * 4;
+#pragma unroll
+      for (int i = 0; i < FM * FK / 64; ++i) cp_async4(d + i * (64 / FK) * 4, src + (long long)(i * (64 / FK)) * ld + at);
+    } else if (vec) {
+      const float* src = base + k0 * ld + m0;
+      const int at = (t / (FM / 4)) * (int)ld + 4 * (t % (FM / 4));
+      const uint32_t d = dst + ((t / (FM / 4)) * FP + 4 * (t % (FM / 4))) * 4;
+#pragma unroll
+      for (int i = 0; i < FM * FK / 4 / 64; ++i) cp_async16(d + i * (256 / FM) * FP * 4, src + (long long)(i * (256 / FM)) * ld + at);
+    } else {
+      const float* src = base + k0 * ld + m0;
+#pragma unroll
+      for (int i = 0; i < FK; ++i) cp_async4(dst + (i * FP + t) * 4, src + (long long)i * ld + t);
+    }
+  } else if constexpr (KC) {
 #pragma unroll
     for (int i = 0; i < FM * FK / 64; ++i) {
       const int idx = threadIdx.x + i * 64, k = idx % FK, m = idx / FK;
