@@ -117,12 +117,12 @@ static __device__ __noinline__ void record_timeout(Control* ctl, int d0, int d1)
 // raised ctl->abort or when limit_ns elapsed; in the latter case it records
 // BLSTM_E_WAIT_TIMEOUT with (d0, d1) and raises abort so every other spinner
 // leaves promptly.  Never traps, never spins unbounded.
-// A counter that two waiters share is 16 bits of the word from `shift` on.
+// Counters that share a word are the eight bits from `shift` on.
 static __device__ __noinline__ bool wait_flag_ge(const int* flag, int target, Control* ctl,
                                           unsigned long long limit_ns, int d0, int d1, int shift = -1) {
   auto reached = [&] {
     const int v = ld_acquire_gpu(flag);
-    return (shift < 0 ? v : (int)((unsigned)v >> shift & 0xffffu)) >= target;
+    return (shift < 0 ? v : (int)((unsigned)v >> shift & 0xffu)) >= target;
   };
   if (reached()) return true;
   const unsigned long long t0 = globaltimer_ns();

@@ -1545,7 +1545,7 @@ using namespace sm100;
 
 int sm100_plan_family(const blstm_desc& d, int phase) {
   if (small_plan(d, phase).ok) return BLSTM_FAMILY_SMALL_BATCH;
-  if (resident_plan(d, phase).ok || tiles_plan(d, phase).ok) return BLSTM_FAMILY_RESIDENT;
+  if (resident_plan(d, phase).ok || tiles_plan(d, phase).ok || fwd_tiles_plan(d, phase).ok) return BLSTM_FAMILY_RESIDENT;
   return (phase == BLSTM_PHASE_BWD ? make_bwd_plan(d).ok : make_plan(d, phase).ok) ? BLSTM_FAMILY_BATCH_TILES : BLSTM_FAMILY_NONE;
 }
 int sm100_plan_turns(const blstm_desc& d, int phase) {
@@ -1562,6 +1562,7 @@ size_t sm100_recurrence_workspace(const blstm_desc& d, int phase) {
   if (sp.ok) return small_workspace(d, sp, phase);
   if (const ResPlan rp = resident_plan(d, phase); rp.ok) return rp.ws_bytes;
   if (const TilesPlan tp = tiles_plan(d, phase); tp.ok) return tp.ws_bytes;
+  if (const FwdTilesPlan fp = fwd_tiles_plan(d, phase); fp.ok) return fp.ws_bytes;
   return phase == BLSTM_PHASE_BWD ? make_bwd_plan(d).ws_bytes : make_plan(d, phase).ws_bytes;
 }
 
@@ -1569,6 +1570,7 @@ size_t sm100_recurrence_control(const blstm_desc& d, int phase) {
   if (small_plan(d, phase).ok) return sizeof(Control);
   if (const ResPlan rp = resident_plan(d, phase); rp.ok) return rp.off_db;
   if (const TilesPlan tp = tiles_plan(d, phase); tp.ok) return tp.off_db;
+  if (const FwdTilesPlan fp = fwd_tiles_plan(d, phase); fp.ok) return fp.ws_bytes;
   return phase == BLSTM_PHASE_BWD ? make_bwd_plan(d).off_db : make_plan(d, phase).ws_bytes;
 }
 
@@ -1577,6 +1579,7 @@ int sm100_plan_detail(const blstm_desc& d, int phase, char* buf, size_t n) {
   if (sp.ok) return small_plan_detail(d, sp, phase, buf, n);
   if (const ResPlan rp = resident_plan(d, phase); rp.ok) return resident_plan_detail(rp, phase, buf, n);
   if (const TilesPlan tp = tiles_plan(d, phase); tp.ok) return tiles_plan_detail(tp, buf, n);
+  if (const FwdTilesPlan fp = fwd_tiles_plan(d, phase); fp.ok) return fwd_tiles_plan_detail(fp, buf, n);
   if (phase == BLSTM_PHASE_BWD) {
     const BwdPlan p = make_bwd_plan(d);
     if (!p.ok) return 0;
@@ -1597,6 +1600,10 @@ int sm100_fwd_recurrence(const blstm_desc& d, void* ifgo, const void* Wh, void* 
   if (const ResPlan rp = resident_plan(d, BLSTM_PHASE_FWD); rp.ok) {
     if (ws_bytes < rp.ws_bytes) return BLSTM_E_WORKSPACE;
     return resident_fwd_recurrence(d, rp, ifgo, Wh, out, cell, ws, st);
+  }
+  if (const FwdTilesPlan fp = fwd_tiles_plan(d, BLSTM_PHASE_FWD); fp.ok) {
+    if (ws_bytes < fp.ws_bytes) return BLSTM_E_WORKSPACE;
+    return fwd_tiles_recurrence(d, fp, ifgo, Wh, out, cell, ws, st);
   }
   const RecPlan pl = make_plan(d, BLSTM_PHASE_FWD);
   if (!pl.ok) return BLSTM_E_UNSUPPORTED;

@@ -48,7 +48,7 @@ struct ResParams {
   int fmt, no_arrive, inference, flag_target, n_groups;
   unsigned long long limit_ns;
   Control* ctl;
-  int* flags;                              // [T+1][groups], a half word for each tile
+  int* flags;                              // [T+1][groups], a byte for each tile
   const void* Wh;
   void* ifgo;                              // forward: in/out; backward: in
   void* cell;
@@ -150,7 +150,7 @@ resident_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
       const int s = it / TI, j = it % TI, t = BWD ? T - 1 - s : s;
       if (BWD || t > 0) {
         int seen = 1;
-        if (lane == 0) seen = wait_flag_ge(&p.flags[(size_t)t * p.n_groups + grp], p.flag_target, p.ctl, p.limit_ns, t, tile0 + j, 16 * j) ? 1 : 0;
+        if (lane == 0) seen = wait_flag_ge(&p.flags[(size_t)t * p.n_groups + grp], p.flag_target, p.ctl, p.limit_ns, t, tile0 + j, 8 * j) ? 1 : 0;
         seen = __shfl_sync(0xffffffffu, seen, 0);
         __syncwarp();      // (a shuffle orders no memory: the issuing lanes come behind the acquire)
         if (!seen) { *dead = 1; break; }
@@ -214,7 +214,7 @@ resident_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
       int ok = 1;
       if (lane == 0) {
         ok = mbar_wait_spin(&stored[j], s & 1, wc);
-        if (ok && !p.no_arrive) red_release_gpu_add(&p.flags[(size_t)t * p.n_groups + grp], 1 << 16 * j);
+        if (ok && !p.no_arrive) red_release_gpu_add(&p.flags[(size_t)t * p.n_groups + grp], 1 << 8 * j);
       }
       if (!__shfl_sync(0xffffffffu, ok, 0)) break;
     }
@@ -309,7 +309,7 @@ resident_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
       if (lane == 0) {
         if constexpr (PUBLISHER) mbar_arrive(&stored[j]);
         else if ((smem_count_arrive(&pub_cnt[j]) & (EW - 1)) == EW - 1 && !p.no_arrive)
-          red_release_gpu_add(&p.flags[(size_t)t * p.n_groups + grp], 1 << 16 * j);
+          red_release_gpu_add(&p.flags[(size_t)t * p.n_groups + grp], 1 << 8 * j);
       }
       __syncwarp();
     };

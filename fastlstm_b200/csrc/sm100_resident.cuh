@@ -32,6 +32,17 @@ struct TilesPlan {
 
 TilesPlan tiles_plan(const blstm_desc& d, int phase);
 
+// ... and forward, for batches of several 32-row tiles per group
+struct FwdTilesPlan {
+  bool ok;
+  int mt, ng, nbt;          // M tiles; groups; batch tiles
+  int kc, nt, w_col, group; // K chunks; of these in tensor memory, from which column on; at once
+  int grid;
+  size_t smem, ws_bytes;
+};
+
+FwdTilesPlan fwd_tiles_plan(const blstm_desc& d, int phase);
+
 }  // namespace sm100
 
 int resident_fwd_recurrence(const blstm_desc& d, const sm100::ResPlan& pl, void* ifgo, const void* Wh, void* out, void* cell, void* ws,
@@ -42,6 +53,9 @@ int resident_bwd_recurrence(const blstm_desc& d, const sm100::ResPlan& pl, const
 int tiles_bwd_recurrence(const blstm_desc& d, const sm100::TilesPlan& pl, const void* dout, const void* dh_n, const void* dc_n,
                          const void* ifgo, const void* cell, const void* Wh, void* d_ifgo, void* dh0, void* dc0, float* db, void* ws,
                          cudaStream_t st);
+int fwd_tiles_recurrence(const blstm_desc& d, const sm100::FwdTilesPlan& pl, void* ifgo, const void* Wh, void* out, void* cell, void* ws,
+                         cudaStream_t st);
+int fwd_tiles_plan_detail(const sm100::FwdTilesPlan& pl, char* buf, size_t n);
 int tiles_plan_detail(const sm100::TilesPlan& pl, char* buf, size_t n);
 int resident_plan_detail(const sm100::ResPlan& pl, int phase, char* buf, size_t n);
 

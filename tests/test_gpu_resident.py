@@ -69,6 +69,36 @@ def test_resident_recurrences_give_up_with_a_status_when_nothing_arrives(phase, 
     assert lib.blstm_read_status(ws.data_ptr(), None, s) == _lib.E_WAIT_TIMEOUT
 
 
+# Several 32-row tiles per group, forward: three, four, six, eight (all of tensor memory and of shared memory taken) and sixteen, groups
+# with one tile less, a last tile of one row, weights past tensor memory, an odd number of K chunks
+@pytest.mark.parametrize("dtype", ["fp16", "bf16"])
+@pytest.mark.parametrize("shape", [(9, 289, 1024), (6, 1023, 1024), (3, 1700, 512), (4, 2300, 256), (3, 2849, 768), (5, 400, 832), (1, 600, 960)])
+def test_forward_tiles_against_fp32_maths(dtype, shape):
+    lib = _lib.load()
+    T, B, H = shape
+    dt = TD[dtype]
+    g = torch.Generator(device="cuda").manual_seed(B + H)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    d = _desc(dtype, T, B, H)
+    Wh = ((torch.rand(4 * H, H, generator=g, device="cuda") * 2 - 1) / H ** 0.5).to(dt)
+    pre, h0, c0 = rnd(T, B, 4 * H).to(dt), (rnd(B, H) * 0.3).to(dt), rnd(B, H).to(dt)
+    ifgo, out, cell = _fwd(lib, d, pre, Wh, h0, c0)
+    want = _torch_fwd(pre, Wh, h0, c0)
+    tol = 8e-3 if dtype == "bf16" else 2e-3          # as above
+    _cmp("ifgo", ifgo, want[0], 4 * tol)
+    _cmp("out", out[1:], want[1], tol)
+    _cmp("cell", cell[1:], want[2], 2 * tol)
+    again = _fwd(lib, d, pre, Wh, h0, c0)
+    assert torch.equal(out, again[1]) and torch.equal(ifgo, again[0]) and torch.equal(cell, again[2])
+    # without gradients: outputs and the last cell state only
+    inf = _fwd(lib, _desc(dtype, T, B, H, _lib.FLAG_INFERENCE), pre, Wh, h0, c0)
+    assert torch.equal(out, inf[1]) and torch.equal(cell[T], inf[2][T])
+
+
+def test_forward_tiles_give_up_with_a_status_when_nothing_arrives():
+    test_resident_recurrences_give_up_with_a_status_when_nothing_arrives(0, 1024, 512)
+
+
 @pytest.mark.parametrize("B,H", [(16, 64), (40, 512), (64, 1024), (200, 512)])
 def test_bias_grad_for_every_backward_plan(B, H):
     lib = _lib.load()
