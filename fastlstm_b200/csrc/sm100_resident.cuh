@@ -21,11 +21,12 @@ struct ResPlan {
 
 ResPlan resident_plan(const blstm_desc& d, int phase);
 
-// ... backward, for batches of several 64-row tiles per group
+// ... backward, for batches of several tiles per group
 struct TilesPlan {
   bool ok;
-  int mt, ng, nbt;          // M tiles; groups; batch tiles
-  int kc, s2;               // K chunks of a CTA; ring stages per issuer
+  int mt, ng, nbt, N;       // M tiles; groups; batch tiles; their rows
+  int kc, nt, w_col;        // K chunks of a CTA; of these in tensor memory, from which column on
+  int s2, group;            // ring stages per issuer; chunks of a stage
   int grid;
   size_t smem, off_db, ws_bytes;
 };

@@ -95,6 +95,30 @@ def test_forward_tiles_against_fp32_maths(dtype, shape):
     assert torch.equal(out, inf[1]) and torch.equal(cell[T], inf[2][T])
 
 
+# Several 32-row tiles per group, backward: three, four, eight (with weights in shared memory) and sixteen, groups with one tile less,
+# half an M tile, K chunks that do not divide into stages
+@pytest.mark.parametrize("dtype", ["fp16", "bf16"])
+@pytest.mark.parametrize("shape", [(5, 300, 1024), (4, 1023, 1024), (5, 1024, 512), (3, 1990, 896), (5, 521, 832), (4, 600, 768), (1, 700, 960), (4, 1400, 384)])
+def test_backward_tiles_against_fp32_maths(dtype, shape):
+    lib = _lib.load()
+    T, B, H = shape
+    dt = TD[dtype]
+    g = torch.Generator(device="cuda").manual_seed(B + H)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    d = _desc(dtype, T, B, H)
+    Wh = ((torch.rand(4 * H, H, generator=g, device="cuda") * 2 - 1) / H ** 0.5).to(dt)
+    ifgo, cell, dout = rnd(T, B, 4 * H).to(dt), (rnd(T + 1, B, H) * 0.7).to(dt), rnd(T, B, H).to(dt)
+    dh, dc = rnd(B, H).to(dt), rnd(B, H).to(dt)
+    got = _bwd(lib, d, dout, dh, dc, ifgo, cell, Wh)
+    for name, a, b in zip(("d_ifgo", "dh0", "dc0", "db"), got, _torch_bwd(dout, dh, dc, ifgo, cell, Wh)):
+        _cmp(name, a, b, (1e-2 if dtype == "bf16" else 3e-3) * float(b.abs().max()))          # as above
+    assert all(torch.equal(a, b) for a, b in zip(got, _bwd(lib, d, dout, dh, dc, ifgo, cell, Wh)))
+
+
+def test_backward_tiles_give_up_with_a_status_when_nothing_arrives():
+    test_resident_recurrences_give_up_with_a_status_when_nothing_arrives(1, 600, 1024)
+
+
 def test_forward_tiles_give_up_with_a_status_when_nothing_arrives():
     test_resident_recurrences_give_up_with_a_status_when_nothing_arrives(0, 1024, 512)
 
