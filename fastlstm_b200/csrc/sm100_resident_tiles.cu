@@ -152,9 +152,10 @@ tiles_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
       bool ok = true;
       int pos = gs[0], po = ph[0];
       if (x) { pos = gs[1]; po = ph[1]; }
-      if (lane < 2) {
-        // lane l owns the ring's stages == l (mod 2)
-        for (int kg = (lane + pos) & 1; kg < n_kg; kg += 2) {
+      if (lane == 0) {
+        // One lane fills the stages in the order in which they are consumed: a wait for a parity cannot tell a stage's next turn from the
+        // one after it, so two lanes that met in a stage - a ring of one has no other - could overtake one another.
+        for (int kg = 0; kg < n_kg; ++kg) {
           int st = pos + kg;
           uint32_t pp = po;
           while (st >= S2) { st -= S2; pp ^= 1; }
@@ -173,7 +174,7 @@ tiles_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
         early = 0;
         if (ns < T) early = ld_acquire_gpu(&p.flags[(size_t)(T - 1 - ns) * p.nbt + tile_of(nj)]);
       }
-      if (__any_sync(0xffffffffu, !ok)) break;
+      if (!__shfl_sync(0xffffffffu, ok, 0)) break;
       pos += n_kg;
       while (pos >= S2) { pos -= S2; po ^= 1; }
       if (x) { gs[1] = pos; ph[1] = po; } else { gs[0] = pos; ph[0] = po; }

@@ -380,3 +380,82 @@ def test_wavefront_where_it_measured_faster():
             x = type("OnGpu", (), dict(is_cuda=True, shape=(T, B, H), dtype=bf))
             m = FastLSTM(H, H, num_layers=2, device="meta", dtype=bf)
             assert bool(m._wavefront(x, None, None, grad)) == want
+
+
+def _ring_faults(lanes, start, step, S2, n_kg, items=3):
+    """Walks every interleaving of the producer's lanes, the copies' landing, the issuer and the MMAs' completion over one ring of
+    S2 stages whose fills are told by the parities of `full` and `empty`; returns what goes wrong first, or None.  An item is n_kg
+    groups, the lanes meet behind each; lane l issues groups start(l, pos), start + step, ..."""
+    total = items * n_kg
+    plan = []                                        # per lane and item: the fills (numbers 0.. in ring order) that it issues
+    for l in lanes:
+        plan.append([[it * n_kg + kg for kg in range(start(l, it * n_kg % S2), n_kg, step)] for it in range(items)])
+    # state: item, each lane's position in it; fills armed / landed per stage; fills the issuer has taken / whose MMAs are done
+    first = (0, (0,) * len(lanes), ((-1, True),) * S2, 0, 0)
+    seen, todo = {first}, [first]
+    while todo:
+        item, at, stages, taken, done = todo.pop()
+        moves = []
+        for i, p in enumerate(plan):
+            if item < items and at[i] < len(p[item]):
+                fill = p[item][at[i]]
+                st, turn = fill % S2, fill // S2
+                consumed = len(range(st, done, S2))  # phases of empty[st] that are over
+                if (consumed & 1) != ((turn & 1) ^ 1):          # the lane's wait for that parity returns
+                    if consumed != turn:
+                        return f"lane {lanes[i]} fills stage {st} for the {turn + 1}. time after {consumed} of its fills were consumed"
+                    if not stages[st][1]:
+                        return f"stage {st} armed twice"
+                    moves.append((item, at[:i] + (at[i] + 1,) + at[i + 1:], stages[:st] + ((fill, False),) + stages[st + 1:], taken, done))
+        if item < items and all(a == len(p[item]) for a, p in zip(at, plan)):
+            moves.append((item + 1, (0,) * len(lanes), stages, taken, done))
+        for st, (fill, landed) in enumerate(stages):
+            if not landed:
+                moves.append((item, at, stages[:st] + ((fill, True),) + stages[st + 1:], taken, done))
+        if taken < total:
+            st, turn = taken % S2, taken // S2
+            fill, landed = stages[st]
+            full = (fill // S2 if not landed else fill // S2 + 1) if fill >= 0 else 0      # phases of full[st] that are over
+            if (full & 1) != (turn & 1):
+                if fill != taken or not landed:
+                    return f"the issuer takes fill {fill} of stage {st} for fill {taken}"
+                moves.append((item, at, stages, taken + 1, done))
+        if done < taken:
+            moves.append((item, at, stages, taken, done + 1))
+        if not moves and done < total:
+            return f"nothing moves after {done} of {total} fills"
+        for m in moves:
+            if m not in seen:
+                seen.add(m)
+                todo.append(m)
+    return None
+
+
+def test_the_stages_of_the_backward_ring_are_filled_in_turn():
+    # Which lanes fill the ring of `tiles_kernel`, and with which groups of K chunks, is read from the source; how many stages and
+    # groups there are comes from every plan that batches of a few hundred to some thousand rows get.
+    import fastlstm_b200
+    from fastlstm_b200 import plan_detail
+    with open(os.path.join(os.path.dirname(fastlstm_b200.__file__), "csrc", "sm100_resident_tiles.cu")) as f:
+        code = re.sub(r"//.*", "", f.read())
+    guard, n, first, by = re.search(r"if \(lane (==|<) (\d+)\) \{\s*for \(int kg = ([^;]+); kg < n_kg; (?:kg \+= (\d+)|\+\+kg)\)", code).groups()
+    lanes = [int(n)] if guard == "==" else list(range(int(n)))
+    rings = set()
+    for H in range(256, 1025, 64):
+        for B in range(64, 8193, 32):
+            for half in (False, True):
+                s = plan_detail(torch.bfloat16, 8, B, H, H, "bwd", half)
+                m = re.search(r"tiles=(\d+) .* chunks=(\d+) .*stages=(\d+) chunks_per_stage=(\d+)", s)
+                if m:
+                    rings.add((int(m.group(3)) // 2, -(-int(m.group(2)) // int(m.group(4)))))
+    assert len(rings) >= 4 and any(S2 == 1 and n_kg > 1 for S2, n_kg in rings), rings
+    for S2, n_kg in sorted(rings):
+        fault = _ring_faults(lanes, lambda lane, pos: eval(first, {}, {"lane": lane, "pos": pos}), int(by or 1), S2, n_kg)
+        assert fault is None, (S2, n_kg, fault)
+
+
+def test_two_lanes_cannot_share_a_stage():
+    # (what the walk above has to find: two lanes dealt the groups of a one-stage ring in turn tell their fills by one parity)
+    deal = lambda lane, pos: (lane + pos) & 1
+    assert _ring_faults([0, 1], deal, 2, 1, 2) is not None
+    assert _ring_faults([0, 1], deal, 2, 2, 4) is None and _ring_faults([0], lambda lane, pos: 0, 1, 1, 2) is None
