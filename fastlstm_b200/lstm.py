@@ -295,9 +295,14 @@ def _wavefront_pays(dtype, T, B, H, grad):
     four chunks in turn, from H = 384 on three, and half of the device would have resident weights, 32 rows to a group of H / 32 CTAs at
     most, these win (T=256: B=200, H=320 1.50 / 1.30; B=130, H=448 1.50 / 1.37; B=150, H=384 1.33 / 1.33, T=512 2.57 / 2.41; but
     B=400, H=256, 48 rows, 1.32 / 1.59; B=100, H=512, two chunks, 1.26 / 1.37).
-    Resident weights gain from 128 steps on where half of the device has
-    them too (T=128 and 256: B=128, H=512 0.91 / 0.81 and 1.73 / 1.40; B=440, H=320 0.98 / 0.98 and 1.87 / 1.75), the kernels
-    with several 128-row tiles always (T=128, B=1000, H=192: 1.31 / 1.05).
+    Resident weights gain from 128 steps on where half of the device holds them with two tiles of rows, 64 to a group of H / 32 CTAs at most
+    (T=128 and 256: B=128, H=512 0.91 / 0.81 and 1.73 / 1.40; B=440, H=320 0.98 / 0.98 and 1.87 / 1.75), the kernels
+    with several 128-row tiles always (T=128, B=1000, H=192: 1.31 / 1.05).  With three or four tiles a group on half of the device the
+    layers stay one after the other, where the cell state is held in 32 bits over the whole sequence: as a wavefront the error of the
+    output against 64 bits grows by 0.06 to 0.3 % (bf16 and fp16, T=512 and T=128).  It would gain at some of these sizes and lose at
+    others (T=128 and 256: B=704, H=256 1.10 / 0.90 and 2.14 / 1.65; B=512, H=512 1.25 / 1.20 and 2.45 / 2.23; B=256, H=768
+    1.27 / 1.18 and 2.48 / 2.19; but B=288, H=512 0.93 / 0.97 and 1.80 / 1.80; B=256, H=832 1.33 / 1.37 and 2.60 / 2.56; B=130, H=896
+    1.03 / 1.16 and 1.98 / 2.14; B=256, H=1024 1.51 / 1.70 and 3.01 / 3.19).
 
     A training step's launches for every chunk cost more, so not where both directions stay on the chip (T=256, B=512, H=512
     6.4 / 6.8; T=256, B=32, H=256 1.25 / 1.8) nor for few steps (T=64, B=712, H=320: 1.78 / 1.95, T=128: 3.27 / 3.3, T=256:
@@ -311,7 +316,7 @@ def _wavefront_pays(dtype, T, B, H, grad):
         return True
     half = _family(dtype, T, B, H, H, "fwd", True)
     if fwd == _lib.FAMILY_RESIDENT:
-        return T >= 128 and half in on_chip
+        return T >= 128 and half in on_chip and B <= 64 * (74 // (H // 32))
     lib, whole, part = _lib.load(), _desc(dtype, T, B, H, H), _desc(dtype, T, B, H, H, _lib.FLAG_HALF_DEVICE)
     turns = lib.blstm_plan_turns(whole, _lib.PHASE_FWD)
     if half == _lib.FAMILY_SMALL_BATCH:

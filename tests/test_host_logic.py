@@ -459,3 +459,19 @@ def test_two_lanes_cannot_share_a_stage():
     deal = lambda lane, pos: (lane + pos) & 1
     assert _ring_faults([0, 1], deal, 2, 1, 2) is not None
     assert _ring_faults([0, 1], deal, 2, 2, 4) is None and _ring_faults([0], lambda lane, pos: 0, 1, 1, 2) is None
+
+
+def test_no_wavefront_where_half_of_the_device_takes_several_tiles_in_turn():
+    # without gradients, resident weights: two tiles of rows a group of CTAs on half of the device, or the layers stay one after the
+    # other with their cell states in 32 bits throughout
+    from fastlstm_b200 import lstm, plan_detail
+    bf = torch.bfloat16
+    for H in range(256, 1025, 64):
+        most = 64 * (74 // (H // 32))
+        for B in (most, most + 1, min(most + 97, 1024 if H <= 256 else 768 if H <= 384 else 512 if H <= 576 else 256)):
+            two = B <= most
+            assert ("rows_per_tile" in plan_detail(bf, 64, B, H, H, "fwd", True)) == two, (H, B)
+            for T in (128, 256, 1024):
+                assert lstm._wavefront_pays(bf, T, B, H, False) == two, (T, B, H)
+    for B, H in ((704, 256), (512, 512), (257, 512), (224, 768), (256, 832), (130, 896), (256, 1024)):
+        assert not lstm._wavefront_pays(bf, 256, B, H, False)
