@@ -152,10 +152,11 @@ tiles_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
       bool ok = true;
       int pos = gs[0], po = ph[0];
       if (x) { pos = gs[1]; po = ph[1]; }
-      if (lane == 0) {
-        // One lane fills the stages in the order in which they are consumed: a wait for a parity cannot tell a stage's next turn from the
-        // one after it, so two lanes that met in a stage - a ring of one has no other - could overtake one another.
-        for (int kg = 0; kg < n_kg; ++kg) {
+      // Lane l fills the stages == l (mod nl), in the order in which they are consumed: a wait for a parity cannot tell a stage's next turn
+      // from the one after it, so two lanes must not meet in a stage, and where there is an odd number of them one lane fills all.
+      const int nl = S2 % 2 ? 1 : 2;
+      if (lane < nl) {
+        for (int kg = (lane + pos) % nl; kg < n_kg; kg += nl) {
           int st = pos + kg;
           uint32_t pp = po;
           while (st >= S2) { st -= S2; pp ^= 1; }
@@ -164,17 +165,13 @@ tiles_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
           const int kc = kg * KG, m = min(KG, KC - kc);
           uint8_t* dst = ring + (size_t)(x * S2 + st) * SG;
           mbar_expect_tx(f, m * SLOT);
-          if (m == KG) {
-            tma_load_4d(dst, &tmX, f, 0, tile * N, kc0 + kc, t);
-          } else {
-            for (int i = 0; i < m; ++i) tma_load_4d(dst + i * SLOT, &tmX1, f, 0, tile * N, kc0 + kc + i, t);
-          }
+          tma_load_4d(dst, m == KG ? &tmX : &tmX1, f, 0, tile * N, kc0 + kc, t);
         }
       } else if (lane == 31) {
         early = 0;
         if (ns < T) early = ld_acquire_gpu(&p.flags[(size_t)(T - 1 - ns) * p.nbt + tile_of(nj)]);
       }
-      if (!__shfl_sync(0xffffffffu, ok, 0)) break;
+      if (__any_sync(0xffffffffu, !ok)) break;
       pos += n_kg;
       while (pos >= S2) { pos -= S2; po ^= 1; }
       if (x) { gs[1] = pos; ph[1] = po; } else { gs[0] = pos; ph[0] = po; }
@@ -529,8 +526,12 @@ TilesPlan tiles_plan(const blstm_desc& d, int phase) {
   const int slot = p.N * 128, blk = p.N / 4 * 128;
   const size_t rest = 1024 + (size_t)(p.kc - p.nt) * 16384 + 2 * (16 * blk + 12 * blk + p.N / 4 * 1024) + 512;
   if (rest > 232448) return p;
-  if (p.N == 64) {                       // (B = 4096 in stages of 1, 2 and 4 chunks 25.3, 22.1 and 21.1 us a step, B = 2048 13.5, 11.8 and 12.8)
-    p.group = most > 5 ? 4 : 2;
+  if (p.N == 64) {
+    // Two stages of two chunks, or one of four.  us a step, two / one, four to eight tiles a group: H = 512 12.4 / 13.8, 14.6 / 13.8, 17.1 / 16.1,
+    // 19.7 / 18.6, 22.5 / 21.2; H = 448 13.0 / 13.4, 15.9 / 13.9, 18.1 / 16.0, 19.8 / 18.4, 22.4 / 20.9; H = 384 11.1 / 13.1, 13.0 / 14.0, 15.4 / 15.8,
+    // 17.9 / 18.1, 20.4 / 20.7; H = 320 11.1 / 13.0, 13.0 / 14.2, 15.3 / 16.1, 17.7 / 18.6, 20.2 / 20.6; H = 256, where four chunks are all, 11.2 / 10.1,
+    // 12.4 / 12.3, 14.5 / 14.6, 17.9 / 17.6, 20.5 / 20.0.
+    p.group = p.kc == 4 || (p.kc >= 7 && most > 4) ? 4 : 2;
     p.s2 = 4 / p.group;
   } else {
     // two stages an issuer, in as few and as equal groups as that allows; with fewer than four chunks a stage they do not pay (H = 1024, 16
@@ -574,12 +575,12 @@ int tiles_bwd_recurrence(const blstm_desc& d, const TilesPlan& pl, const void* d
     rc = encode_tensor_map(&tw, Wh, 2, dims, str, box);
     if (rc) return rc;
   }
-  {  // d_ifgo as {k of a chunk, batch row, chunk, step}: a stage's chunks, or one
+  {  // d_ifgo as {k of a chunk, batch row, chunk, step}: a stage's chunks, or those of an item's last stage
     uint64_t dims[4] = {64, (uint64_t)B, (uint64_t)H / 16, (uint64_t)T}, str[3] = {(uint64_t)4 * H * 2, 128, (uint64_t)B * 4 * H * 2};
     uint32_t box[4] = {64, (uint32_t)pl.N, (uint32_t)pl.group, 1};
     rc = encode_tensor_map(&tx, d_ifgo, 4, dims, str, box);
     if (rc) return rc;
-    box[2] = 1;
+    box[2] = pl.kc - (cdiv(pl.kc, pl.group) - 1) * pl.group;
     rc = encode_tensor_map(&tx1, d_ifgo, 4, dims, str, box);
     if (rc) return rc;
   }

@@ -438,8 +438,8 @@ def test_the_stages_of_the_backward_ring_are_filled_in_turn():
     from fastlstm_b200 import plan_detail
     with open(os.path.join(os.path.dirname(fastlstm_b200.__file__), "csrc", "sm100_resident_tiles.cu")) as f:
         code = re.sub(r"//.*", "", f.read())
-    guard, n, first, by = re.search(r"if \(lane (==|<) (\d+)\) \{\s*for \(int kg = ([^;]+); kg < n_kg; (?:kg \+= (\d+)|\+\+kg)\)", code).groups()
-    lanes = [int(n)] if guard == "==" else list(range(int(n)))
+    count, first = re.search(r"const int nl = ([^;]+);\s*if \(lane < nl\) \{\s*for \(int kg = ([^;]+); kg < n_kg; kg \+= nl\)", code).groups()
+    count = re.sub(r"(.+) \? (\d+) : (\d+)", r"\2 if \1 else \3", count)
     rings = set()
     for H in range(256, 1025, 64):
         for B in range(64, 8193, 32):
@@ -450,7 +450,8 @@ def test_the_stages_of_the_backward_ring_are_filled_in_turn():
                     rings.add((int(m.group(3)) // 2, -(-int(m.group(2)) // int(m.group(4)))))
     assert len(rings) >= 4 and any(S2 == 1 and n_kg > 1 for S2, n_kg in rings), rings
     for S2, n_kg in sorted(rings):
-        fault = _ring_faults(lanes, lambda lane, pos: eval(first, {}, {"lane": lane, "pos": pos}), int(by or 1), S2, n_kg)
+        nl = eval(count, {}, {"S2": S2})
+        fault = _ring_faults(list(range(nl)), lambda lane, pos: eval(first, {}, {"lane": lane, "pos": pos, "nl": nl}), nl, S2, n_kg)
         assert fault is None, (S2, n_kg, fault)
 
 
@@ -459,6 +460,16 @@ def test_two_lanes_cannot_share_a_stage():
     deal = lambda lane, pos: (lane + pos) & 1
     assert _ring_faults([0, 1], deal, 2, 1, 2) is not None
     assert _ring_faults([0, 1], deal, 2, 2, 4) is None and _ring_faults([0], lambda lane, pos: 0, 1, 1, 2) is None
+
+
+def test_stages_of_the_backward_ring_where_they_measured_faster():
+    # 64-row tiles: eight groups of CTAs at H = 448 and 512, eleven at 320 and 384, sixteen at 256
+    from fastlstm_b200 import plan_detail
+    for H, groups, long_from in ((256, 16, 4), (320, 11, 9), (384, 11, 9), (448, 8, 5), (512, 8, 5)):
+        for tiles in range(4, 9):
+            s = plan_detail(torch.bfloat16, 8, 64 * groups * tiles, H, H, "bwd")
+            want = "stages=2 chunks_per_stage=4 " if tiles >= long_from else "stages=4 chunks_per_stage=2 "
+            assert f"tiles={tiles} " in s and "n=64 " in s and want in s, (H, tiles, s)
 
 
 def test_no_wavefront_where_half_of_the_device_takes_several_tiles_in_turn():
