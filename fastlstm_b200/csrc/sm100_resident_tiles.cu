@@ -519,6 +519,9 @@ TilesPlan tiles_plan(const blstm_desc& d, int phase) {
   p.nbt = cdiv(d.batch, p.N);
   const int most = cdiv(p.nbt, p.ng);
   if (p.N == 64 ? most > 8 : H >= 768 ? most < (H > 768 ? 3 : 4) || most > 16 : H < 384 || H > 512 || most != 4) return p;
+  // a group of two tiles is two hand-off chains long: H = 832, that kernel / this, B = 289 (groups of three and two) 10.9 / 11.2, B = 384 (three each)
+  // 11.1 / 10.3; from H = 896 on this wins all the same, B = 289 12.8 / 12.0
+  if (H <= 832 && p.N == 32 && p.nbt < 3 * p.ng) return p;
   p.kc = H / 64;
   p.w_col = 2 * p.N + most * p.N / 4;
   p.nt = std::min(p.kc, (512 - p.w_col) / 32);

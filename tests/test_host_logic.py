@@ -486,3 +486,11 @@ def test_no_wavefront_where_half_of_the_device_takes_several_tiles_in_turn():
                 assert lstm._wavefront_pays(bf, T, B, H, False) == two, (T, B, H)
     for B, H in ((704, 256), (512, 512), (257, 512), (224, 768), (256, 832), (130, 896), (256, 1024)):
         assert not lstm._wavefront_pays(bf, 256, B, H, False)
+
+
+def test_backward_of_832_units_leaves_groups_of_two_tiles_to_the_other_kernel():
+    from fastlstm_b200 import _lib, lstm
+    for H, B, family in ((832, 257, _lib.FAMILY_BATCH_TILES), (832, 352, _lib.FAMILY_BATCH_TILES), (832, 353, _lib.FAMILY_RESIDENT),
+                         (832, 512, _lib.FAMILY_RESIDENT), (896, 289, _lib.FAMILY_RESIDENT), (768, 481, _lib.FAMILY_RESIDENT),
+                         (448, 800, _lib.FAMILY_RESIDENT)):
+        assert lstm._family(torch.bfloat16, 64, B, H, H, "bwd") == family, (H, B)
