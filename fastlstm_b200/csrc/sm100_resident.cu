@@ -536,7 +536,10 @@ ResPlan resident_plan(const blstm_desc& d, int phase) {
     p.ng = cap / p.mt;
     if (p.ng < 1) continue;
     // (tiles of eight rows do not pay: B = 64, H = 1024 backward 3.64 us a step as one tile, 3.89 as two, B = 16, H = 2048 4.21 / 4.89)
-    p.ti = cdiv(B, p.ng) > 16 ? 2 : 1;
+    // Backward up to H = 448 one tile of 32 rows beats two of 16: H = 320, 308 and 352 rows 4.37 / 4.40 and 4.36 / 4.55, H = 384, 264, 308 and 352 rows
+    // 4.31 / 4.41, 4.42 / 4.60 and 4.44 / 4.64, H = 448, 256 rows 4.54 / 4.72; from H = 576 on two win (120 rows 4.36 / 4.09, 168 4.65 / 4.66).
+    const int group_rows = cdiv(B, p.ng);
+    p.ti = group_rows <= 16 || (bwd && H <= 448 && group_rows <= 32) ? 1 : 2;
     p.rows = (int)round_up((size_t)cdiv(B, p.ng * p.ti), 8);
     p.ng = cdiv(B, p.rows * p.ti);
     p.own = bwd ? 4 : p.ks;
@@ -608,7 +611,7 @@ static int launch(const blstm_desc& d, const ResPlan& pl, bool bwd, void* x, Res
     return p.fmt ? launch_t<BW, TT, NN, OO, II, __nv_bfloat16>(pl, tw, tx, tx1, p, st) : launch_t<BW, TT, NN, OO, II, __half>(pl, tw, tx, tx1, p, st);
   BLSTM_RES(false, 1, 16, 1, 2) BLSTM_RES(false, 1, 16, 2, 2) BLSTM_RES(false, 2, 16, 1, 2) BLSTM_RES(false, 2, 16, 2, 2)
   BLSTM_RES(false, 2, 32, 1, 2) BLSTM_RES(false, 2, 32, 2, 2)
-  BLSTM_RES(true, 1, 16, 4, 2) BLSTM_RES(true, 2, 16, 4, 2) BLSTM_RES(true, 2, 16, 4, 1) BLSTM_RES(true, 2, 32, 4, 2)
+  BLSTM_RES(true, 1, 16, 4, 2) BLSTM_RES(true, 1, 32, 4, 2) BLSTM_RES(true, 2, 16, 4, 2) BLSTM_RES(true, 2, 16, 4, 1) BLSTM_RES(true, 2, 32, 4, 2)
 #undef BLSTM_RES
   return BLSTM_E_UNSUPPORTED;
 }

@@ -1,4 +1,6 @@
 """Recurrences whose weights stay on the chip (large hidden sizes) against the fp32 step-by-step evaluation."""
+import ctypes
+
 import pytest
 import torch
 
@@ -46,6 +48,17 @@ def test_resident_recurrences_against_fp32_maths(dtype, shape):
 # issuer and with two, of 32 rows, K in two parts forward, enough steps for the tiles to take turns
 @pytest.mark.parametrize("shape", [(9, 64, 1024), (9, 65, 1024), (9, 17, 2048), (9, 32, 2048), (9, 100, 768), (9, 257, 512), (9, 250, 768)])
 def test_tiles_that_take_turns(shape):
+    test_resident_recurrences_against_fp32_maths("bf16", shape)
+    test_resident_recurrences_against_fp32_maths("fp16", shape)
+
+
+# One tile of up to 32 rows a group, backward up to H = 448: a full group, ragged ones, 24 rows, half an M tile, an odd number of K chunks
+@pytest.mark.parametrize("shape", [(9, 352, 320), (5, 289, 320), (9, 350, 384), (4, 264, 384), (9, 255, 448)])
+def test_one_tile_of_32_rows_backward(shape):
+    lib = _lib.load()
+    buf = ctypes.create_string_buffer(512)
+    _lib.check(lib.blstm_plan_detail(_desc("bf16", *shape), _lib.PHASE_BWD, buf, 512))
+    assert b"tiles=1 " in buf.value and b"n=32 " in buf.value, buf.value
     test_resident_recurrences_against_fp32_maths("bf16", shape)
     test_resident_recurrences_against_fp32_maths("fp16", shape)
 
