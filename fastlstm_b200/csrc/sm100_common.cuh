@@ -180,7 +180,7 @@ __device__ __forceinline__ bool mbar_wait_spin(uint64_t* bar, uint32_t parity, c
   return mbar_wait_slow(bar, parity, w);
 }
 
-// Every lane waits for a barrier of its own; the answer is the warp's.
+// All lanes of the warp wait for the same barrier and go on together; the answer is the warp's.
 __device__ __forceinline__ bool warp_wait_all(uint64_t* bar, uint32_t parity, const WaitCtx& w) {
 #pragma unroll 1
   for (int i = 0; i < 4096; ++i)

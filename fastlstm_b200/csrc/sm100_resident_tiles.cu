@@ -58,7 +58,7 @@ tiles_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
   constexpr int KS = 4, UT = 128, RO = N / KS, UP = UT * RO / 256, W = UP / 2, TPR = UT / UP;
   constexpr int SLOT = N * 128;                                     // a K chunk of a tile
   constexpr int STATE = 2 * N;                                      // tensor memory columns: two accumulators, states, weights
-  constexpr int BLK = RO * 128, XB = KS * 4 * BLK;                  // exchanged block; one set of receive slots (32 KB)
+  constexpr int BLK = RO * 128, XB = KS * 4 * BLK;                  // exchanged block; one set of receive slots
   constexpr int SB = 3 * 4 * BLK;                                   // one set of staging slots (own slices stay here)
   constexpr int BOX = RO * 128 * 2 * 4;                             // the CTA's rows on their way out
   constexpr int EW = 8;
@@ -253,7 +253,7 @@ tiles_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
     const size_t H4 = 4 * (size_t)H;
     const T16* ifgo = reinterpret_cast<const T16*>(p.ifgo);
     const T16* cell = reinterpret_cast<const T16*>(p.cell);
-    // on its way out: [4 gates][16 rows][128 units]
+    // on its way out: [4 gates][RO rows][128 units]
     constexpr int GS = RO * 256;
     uint8_t* mine = boxes + lr * (UT * 2) + u * 2;
     // (pieces of 16 bytes at places xor'ed with row and M quarter: see sm100_resident.cu)
@@ -261,7 +261,7 @@ tiles_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
     const float* rd = reinterpret_cast<const float*>(recv) + lr * 32 + (u >> 5) * (BLK / 4);
     const uint32_t d_addr = tmem_base + (uint32_t(q * 32) << 16) + g * (N / 2);
     const uint32_t s_addr = tmem_base + STATE + (uint32_t(q * 32) << 16) + g * UP;
-    // where this warp's half of an accumulator's columns goes: 16 rows each for two owners
+    // where this warp's half of an accumulator's columns goes: RO rows each for two owners
     constexpr int NB = 2;
     uint8_t* put[NB];
     int put_step[NB];                     // distance of the second buffer

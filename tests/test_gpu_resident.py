@@ -9,11 +9,11 @@ from test_gpu_recurrence import TD, _bwd, _cmp, _desc, _fwd, _torch_bwd, _torch_
 
 pytestmark = pytest.mark.gpu
 
-# N = 16, 32, 64; one row, ragged rows and groups; half an M tile in backward (H % 128 == 64); K split over 1 and 2 (forward),
+# N = 16 and 32; one row, ragged rows and groups; half an M tile in backward (H % 128 == 64); K split over 1 and 2 (forward),
 # 4 (one issuer too), 5 and 6 (the same) CTAs backward; weights that fit tensor memory and weights that do not
 SHAPES = [(4, 1, 768), (3, 65, 704), (5, 100, 768), (3, 250, 768), (4, 256, 1024), (2, 130, 960), (3, 33, 1088), (3, 64, 1536),
           (4, 32, 2048), (3, 17, 1984), (2, 9, 2048), (3, 29, 1728), (3, 61, 1408), (3, 90, 1408),
-          # several tiles a group in backward: four, five and eight, a partial last tile, half an M tile, odd numbers of K chunks
+          # several tiles of 64 rows a group in backward: four, five and eight, a partial last tile, half an M tile, odd numbers of K chunks
           (3, 1600, 512), (3, 4096, 512), (5, 2300, 448), (3, 3210, 320), (3, 4000, 256), (1, 2047, 512)]
 
 
@@ -82,10 +82,10 @@ def test_resident_recurrences_give_up_with_a_status_when_nothing_arrives(phase, 
     assert lib.blstm_read_status(ws.data_ptr(), None, s) == _lib.E_WAIT_TIMEOUT
 
 
-# Several 32-row tiles per group, forward: three, four, six, eight (all of tensor memory and of shared memory taken) and sixteen, groups
-# with one tile less, a last tile of one row, weights past tensor memory, an odd number of K chunks
+# Several 32-row tiles per group, forward: three, four, six, eight (all of tensor memory and of shared memory taken), fifteen and
+# sixteen, groups with one tile less, a last tile of one row, weights past tensor memory, an odd number of K chunks
 @pytest.mark.parametrize("dtype", ["fp16", "bf16"])
-@pytest.mark.parametrize("shape", [(9, 289, 1024), (6, 1023, 1024), (3, 1700, 512), (4, 2300, 256), (3, 2849, 768), (5, 400, 832), (1, 600, 960)])
+@pytest.mark.parametrize("shape", [(9, 289, 1024), (6, 1023, 1024), (3, 1700, 512), (4, 2300, 256), (3, 2849, 768), (3, 2913, 768), (5, 400, 832), (1, 600, 960)])
 def test_forward_tiles_against_fp32_maths(dtype, shape):
     lib = _lib.load()
     T, B, H = shape
@@ -126,6 +126,16 @@ def test_backward_tiles_against_fp32_maths(dtype, shape):
     for name, a, b in zip(("d_ifgo", "dh0", "dc0", "db"), got, _torch_bwd(dout, dh, dc, ifgo, cell, Wh)):
         _cmp(name, a, b, (1e-2 if dtype == "bf16" else 3e-3) * float(b.abs().max()))          # as above
     assert all(torch.equal(a, b) for a, b in zip(got, _bwd(lib, d, dout, dh, dc, ifgo, cell, Wh)))
+
+
+# 64-row tiles through every ring that the plans give, enough steps for each stage to be filled many times: two stages of two chunks (H = 320
+# and 384; four tiles at 512), one of four with a shorter last one (448) and without (512), one that holds an item's chunks (256)
+@pytest.mark.parametrize("shape", [(30, 4200, 320), (30, 5632, 384), (30, 3000, 448), (30, 4096, 448), (30, 2048, 512), (30, 3072, 512),
+                                   (30, 4096, 512), (30, 8192, 256)])
+def test_backward_ring_over_many_steps(shape):
+    # (errors do not add up over the steps: what a step carries on in dh shrinks with the gates' derivatives, and dc is held in fp32)
+    test_backward_tiles_against_fp32_maths("bf16", shape)
+    test_backward_tiles_against_fp32_maths("fp16", shape)
 
 
 def test_backward_tiles_give_up_with_a_status_when_nothing_arrives():

@@ -494,3 +494,16 @@ def test_backward_of_832_units_leaves_groups_of_two_tiles_to_the_other_kernel():
                          (832, 512, _lib.FAMILY_RESIDENT), (896, 289, _lib.FAMILY_RESIDENT), (768, 481, _lib.FAMILY_RESIDENT),
                          (448, 800, _lib.FAMILY_RESIDENT)):
         assert lstm._family(torch.bfloat16, 64, B, H, H, "bwd") == family, (H, B)
+
+
+def test_plans_behind_the_tests_of_several_tiles():
+    # what tests/test_gpu_resident.py means to run: tiles of the fullest group, rows of a tile
+    from fastlstm_b200 import plan_detail
+    for phase, cases in (("fwd", ((289, 1024, 3, 32), (1023, 1024, 8, 32), (1700, 512, 6, 32), (2300, 256, 4, 32), (2849, 768, 15, 32), (2913, 768, 16, 32),
+                                  (400, 832, 3, 32), (600, 960, 5, 32))),
+                         ("bwd", ((300, 1024, 3, 32), (1023, 1024, 8, 32), (1024, 512, 4, 32), (1990, 896, 16, 32), (521, 832, 5, 32), (600, 768, 4, 32),
+                                  (700, 960, 6, 32), (1400, 384, 4, 32), (4200, 320, 6, 64), (5632, 384, 8, 64), (3000, 448, 6, 64), (4096, 448, 8, 64),
+                                  (2048, 512, 4, 64), (3072, 512, 6, 64), (4096, 512, 8, 64), (8192, 256, 8, 64)))):
+        for B, H, tiles, rows in cases:
+            s = plan_detail(torch.bfloat16, 8, B, H, H, phase)
+            assert f" tiles={tiles} " in s and f" n={rows} " in s, (phase, B, H, s)
