@@ -134,6 +134,11 @@ tiles_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
         tma_load_2d(dst + 8192, &tmW, w_full, mt * 128 + 64, (kc0 + kc) * 64);
       }
     }
+    // A stage has one lane that fills it, in the order in which it is consumed: a wait for a parity cannot tell a stage's next turn from the one
+    // after it, so two lanes must not meet in a stage.  Lanes 0 and 1 take the even and the odd stages of an even ring; lane 0 takes all of an
+    // odd one, and of a ring of 32-row tiles with four groups an item, where that is faster (us a step, two lanes / one: H = 1024, B = 1024 21.4 / 20.3,
+    // H = 960, B = 2048 41.0 / 39.3; but 64-row tiles H = 512, B = 2048 12.7 / 13.7).
+    const int two = S2 % 2 == 0 && (N == 64 || n_kg < 4);
     int early = 0, s = 0, j = 0;
     int gs[2] = {0, 0};                   // ring position of each issuer's next item
     uint32_t ph[2] = {0, 0};
@@ -152,11 +157,8 @@ tiles_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
       bool ok = true;
       int pos = gs[0], po = ph[0];
       if (x) { pos = gs[1]; po = ph[1]; }
-      // Lane l fills the stages == l (mod nl), in the order in which they are consumed: a wait for a parity cannot tell a stage's next turn
-      // from the one after it, so two lanes must not meet in a stage, and where there is an odd number of them one lane fills all.
-      const int nl = S2 % 2 ? 1 : 2;
-      if (lane < nl) {
-        for (int kg = (lane + pos) % nl; kg < n_kg; kg += nl) {
+      if (lane <= two) {
+        for (int kg = (lane + pos) & two; kg < n_kg; kg += 1 + two) {
           int st = pos + kg;
           uint32_t pp = po;
           while (st >= S2) { st -= S2; pp ^= 1; }

@@ -438,20 +438,20 @@ def test_the_stages_of_the_backward_ring_are_filled_in_turn():
     from fastlstm_b200 import plan_detail
     with open(os.path.join(os.path.dirname(fastlstm_b200.__file__), "csrc", "sm100_resident_tiles.cu")) as f:
         code = re.sub(r"//.*", "", f.read())
-    count, first = re.search(r"const int nl = ([^;]+);\s*if \(lane < nl\) \{\s*for \(int kg = ([^;]+); kg < n_kg; kg \+= nl\)", code).groups()
-    count = re.sub(r"(.+) \? (\d+) : (\d+)", r"\2 if \1 else \3", count)
+    two, first = re.search(r"const int two = ([^;]+);.*?if \(lane <= two\) \{\s*for \(int kg = ([^;]+); kg < n_kg; kg \+= 1 \+ two\)", code, re.S).groups()
+    two = two.replace("&&", "and").replace("||", "or")
     rings = set()
     for H in range(256, 1025, 64):
         for B in range(64, 8193, 32):
             for half in (False, True):
                 s = plan_detail(torch.bfloat16, 8, B, H, H, "bwd", half)
-                m = re.search(r"tiles=(\d+) .* chunks=(\d+) .*stages=(\d+) chunks_per_stage=(\d+)", s)
-                if m:
-                    rings.add((int(m.group(3)) // 2, -(-int(m.group(2)) // int(m.group(4)))))
-    assert len(rings) >= 4 and any(S2 == 1 and n_kg > 1 for S2, n_kg in rings), rings
-    for S2, n_kg in sorted(rings):
-        nl = eval(count, {}, {"S2": S2})
-        fault = _ring_faults(list(range(nl)), lambda lane, pos: eval(first, {}, {"lane": lane, "pos": pos, "nl": nl}), nl, S2, n_kg)
+                m = re.search(r" n=(\d+) .* chunks=(\d+) .*stages=(\d+) chunks_per_stage=(\d+)", s)
+                if m and "tiles=" in s and "rows_per_tile" not in s:
+                    rings.add((int(m.group(3)) // 2, -(-int(m.group(2)) // int(m.group(4))), int(m.group(1))))
+    assert len(rings) >= 6 and any(S2 == 1 and n_kg > 1 for S2, n_kg, _ in rings), rings
+    for S2, n_kg, N in sorted(rings):
+        of = int(eval(two, {}, {"S2": S2, "N": N, "n_kg": n_kg}))
+        fault = _ring_faults(list(range(1 + of)), lambda lane, pos: eval(first, {}, {"lane": lane, "pos": pos, "two": of}), 1 + of, S2, n_kg)
         assert fault is None, (S2, n_kg, fault)
 
 
