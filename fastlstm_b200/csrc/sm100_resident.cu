@@ -18,9 +18,9 @@
 // rows are handed on, the other's products are formed.  Both tiles at half of N cost the tensor cores no more (an MMA of
 // N = 32 takes 18 clocks, of N = 64 34; N = 16 11).
 //
-// us per step, one tile and MMAs issued behind a wait for each chunk -> now (B200): forward B=32 H=2048 4.3 -> 3.7, B=256 H=1024
-// 5.7 -> 4.5, B=128 H=1024 4.2 -> 3.5, B=256 H=768 4.7 -> 3.6, B=512 H=512 4.4 -> 3.6; backward B=32 H=2048 6.8 -> 5.0,
-// B=256 H=1024 6.1 -> 5.2, B=256 H=768 5.6 -> 4.8, B=512 H=512 5.2 -> 4.6, B=32 H=1536 4.5 -> 4.1.
+// us per step, one tile and MMAs issued behind a wait for each chunk -> now (B200, gates saved, inputs out of HBM, launch included):
+// forward B=32 H=2048 4.4 -> 3.9, B=256 H=1024 5.8 -> 4.6, B=128 H=1024 4.3 -> 3.6, B=256 H=768 4.8 -> 4.3, B=512 H=512 4.5 -> 4.3; backward
+// B=32 H=2048 6.9 -> 5.3, B=256 H=1024 6.3 -> 5.4, B=256 H=768 5.7 -> 4.9, B=512 H=512 5.4 -> 4.7, B=32 H=1536 4.6 -> 4.2.
 // Bound by a tile's chain (some 7 to 9 k clocks a step), with K in four parts and 64 rows by the epilogue warps.
 #include <algorithm>
 #include <cstdio>
@@ -75,7 +75,8 @@ resident_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
   constexpr int EW = 8;
   // Who counts the CTA in: the last of its eight warps whose rows are stored, or a warp of its own, which keeps the 1.1 k clocks of
   // the release off the eight but comes some 200 later.  us a step, last warp / own warp: backward, two tiles of 32 rows,
-  // B=512 H=512 5.28 / 4.59, B=256 H=768 5.41 / 4.77; B=32 H=2048 5.00 / 5.91; forward B=512 H=512 3.58 / 3.67, B=256 H=768 3.61 / 3.81.
+  // B=512 H=512 5.28 / 4.59, B=256 H=768 5.41 / 4.77; B=32 H=2048 5.00 / 5.91.  Forward, where the last warp does it, two tiles of 32 rows: B=512
+  // H=512 4.24 / 3.80, B=256 H=768 4.32 / 3.95, B=400 H=384 4.16 / 3.52, but H=1024 B=256 4.60 / 4.64 and, without gradients, 4.34 / 4.45.
   constexpr bool PUBLISHER = BWD && TI == 2 && N == 32;
   static_assert(UP <= 4, "");
   extern __shared__ uint8_t smem_raw[];

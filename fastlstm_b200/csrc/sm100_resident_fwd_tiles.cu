@@ -324,7 +324,8 @@ FwdTilesPlan fwd_tiles_plan(const blstm_desc& d, int phase) {
   p.nbt = cdiv(d.batch, RF_N);
   const int most = cdiv(p.nbt, p.ng);
   // us a step, the kernel with the batch on the M side / this: H = 512, 6 and 7 tiles 9.3 / 8.1 and 9.3 / 9.3; H = 448, 6 and 8 9.2 / 7.9
-  // and 9.4 / 10.5; H = 256, 4 and 6 6.0 / 5.3 and 7.4 / 7.8; from H = 576 on all that fit: 8 tiles 12.3 / 10.6, H = 1024 19.9 / 14.3
+  // and 9.4 / 10.5; H = 256, 4 and 6 6.0 / 5.3 and 7.4 / 7.8; from H = 576 on all that fit: every count of three to sixteen takes 0.43 to 0.89 of
+  // that kernel's time, H = 832, 7 tiles 24.2 / 10.4, H = 576, 8 and 16 12.3 / 10.9 and 24.3 / 21.4, H = 1024, 8 20.0 / 14.6
   if (most < 3 || most > (H > 512 ? RF_TILES : H > 320 ? 6 : 4)) return p;
   p.kc = H / 64;
   p.w_col = RF_STATE + 8 * most;

@@ -10,10 +10,10 @@
 // accumulators leave.  Two issuers take every other tile, each with its own accumulator and its own half of the ring, which
 // is what weights and exchange leave of shared memory, in stages of up to eight K chunks.  A CTA has 128 units where the
 // kernel with the batch on the M side had 64 a cluster, which halves what a step reads of d_ifgo (67 MB at B = 4096, H = 512).
-// us per step, that kernel -> this, launched alone: B = 4096, H = 512: 25.5 -> 21.1 (it runs into the power cap; 24.5 inside a
-// training step); B = 2048: 12.9 -> 11.7; B = 4096, H = 256: 12.5 -> 9.4; B = 3000, H = 384: 19.1 -> 11.8.  Tiles of 32 rows: B = 1024,
-// H = 1024 27.8 -> 20.6, B = 600 20.5 -> 13.3; B = 1500, H = 768 25.7 -> 19.5, B = 600 12.6 -> 8.2;
-// B = 1024, H = 512 8.4 -> 7.6; B = 1400, H = 384 9.5 -> 7.5.
+// us per step, that kernel -> this, launched alone: B = 4096, H = 512: 25.5 -> 20.2 (25.6 inside a training step, under the power cap);
+// B = 2048: 12.9 -> 11.0; B = 4096, H = 256: 12.5 -> 9.1; B = 3000, H = 384: 19.1 -> 11.7.  Tiles of 32 rows: B = 1024,
+// H = 1024 27.8 -> 19.3, B = 600 20.5 -> 12.4; B = 1500, H = 768 25.7 -> 18.9, B = 600 12.6 -> 8.3; B = 700, H = 896 16.1 -> 11.4;
+// B = 1024, H = 512 8.4 -> 7.6; B = 1400, H = 384 9.5 -> 7.6.
 // The epilogue warps set the pace (a 64-row tile takes them 4.4 k clocks: read-out and shipping 1.2, gate maths 1.1, bias gradient
 // 0.9, fetching 0.5); sixteen of them with half the cells each were no faster (22.4).
 #include <algorithm>
@@ -506,9 +506,10 @@ tiles_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CU
 
 // Tiles of 64 rows up to H = 512 where there are four to eight.  Tiles of 32 rows from H = 768 on, where the kernel with the batch on the
 // M side works with narrow slices or a short ring, and four of them from H = 384 to 512.  us a step, that kernel / this: H = 1024, 3, 4, 5
-// and 8 tiles 13.3 / 11.7, 13.9 / 10.4, 20.5 / 13.3, 27.8 / 20.6; H = 896, 6 and 16 16.0 / 11.7, 41.9 / 35.5; H = 768, 3, 4 and 10 9.6 / 10.2,
-// 12.6 / 8.2, 25.7 / 19.5; but H = 704, 7 and 10 12.9 / 14.4, 16.5 / 20.9, H = 640, 8 15.2 / 15.5, H = 576, 8 13.3 / 15.9; H = 512, 4 and 6
-// 8.4 / 7.6, 9.7 / 11.2; H = 384 and 448, 4 9.5 / 7.5, 8.2 / 7.7; H = 320, 6 9.6 / 11.1.
+// and 8 tiles 14.3 / 10.3, 14.6 / 10.3, 21.2 / 13.6, 28.2 / 20.4; H = 896, 6 and 16 16.6 / 12.7, 42.6 / 32.5; H = 768, 4, 10 and 16 13.4 / 9.2,
+// 29.4 / 20.1, 42.8 / 31.4; H = 512, 448 and 384, 4 9.0 / 8.5, 8.9 / 8.6, 10.2 / 8.4.  Not taken, measured while a shorter last stage took a load for each
+// of its chunks: H = 768, 3 9.6 / 10.2; H = 704, 7 and 10 12.9 / 14.4, 16.5 / 20.9, H = 640, 8 15.2 / 15.5, H = 576, 8 13.3 / 15.9; H = 512, 6 9.7 / 11.2;
+// H = 320, 6 9.6 / 11.1.
 TilesPlan tiles_plan(const blstm_desc& d, int phase) {
   TilesPlan p{};
   const int H = d.hidden_size;
@@ -522,7 +523,7 @@ TilesPlan tiles_plan(const blstm_desc& d, int phase) {
   const int most = cdiv(p.nbt, p.ng);
   if (p.N == 64 ? most > 8 : H >= 768 ? most < (H > 768 ? 3 : 4) || most > 16 : H < 384 || H > 512 || most != 4) return p;
   // a group of two tiles is two hand-off chains long: H = 832, that kernel / this, B = 289 (groups of three and two) 10.9 / 11.2, B = 384 (three each)
-  // 11.1 / 10.3; from H = 896 on this wins all the same, B = 289 12.8 / 12.0
+  // 11.1 / 9.2; from H = 896 on this wins all the same, B = 289 12.8 / 12.0
   if (H <= 832 && p.N == 32 && p.nbt < 3 * p.ng) return p;
   p.kc = H / 64;
   p.w_col = 2 * p.N + most * p.N / 4;
@@ -532,10 +533,10 @@ TilesPlan tiles_plan(const blstm_desc& d, int phase) {
   const size_t rest = 1024 + (size_t)(p.kc - p.nt) * 16384 + 2 * (16 * blk + 12 * blk + p.N / 4 * 1024) + 512;
   if (rest > 232448) return p;
   if (p.N == 64) {
-    // Two stages of two chunks, or one of four.  us a step, two / one, four to eight tiles a group: H = 512 12.4 / 13.8, 14.6 / 13.8, 17.1 / 16.1,
-    // 19.7 / 18.6, 22.5 / 21.2; H = 448 13.0 / 13.4, 15.9 / 13.9, 18.1 / 16.0, 19.8 / 18.4, 22.4 / 20.9; H = 384 11.1 / 13.1, 13.0 / 14.0, 15.4 / 15.8,
-    // 17.9 / 18.1, 20.4 / 20.7; H = 320 11.1 / 13.0, 13.0 / 14.2, 15.3 / 16.1, 17.7 / 18.6, 20.2 / 20.6; H = 256, where four chunks are all, 11.2 / 10.1,
-    // 12.4 / 12.3, 14.5 / 14.6, 17.9 / 17.6, 20.5 / 20.0.
+    // Two stages of two chunks, or one of four.  us a step, two / one, four to eight tiles a group: H = 512 12.0 / 13.4, 14.1 / 13.5, 16.6 / 15.8,
+    // 19.2 / 18.3, 22.0 / 20.9; H = 448 12.2 / 13.0, 14.1 / 13.6, 16.4 / 15.5, 18.8 / 17.6, 21.3 / 20.0; H = 384 10.9 / 12.9, 12.7 / 13.7, 15.0 / 15.7,
+    // 17.4 / 17.9, 19.7 / 20.6; H = 320 10.9 / 12.7, 12.7 / 14.1, 14.9 / 16.0, 17.2 / 18.0, 19.5 / 20.5; H = 256, where four chunks are all, 10.0 / 10.0,
+    // 12.3 / 12.1, 14.4 / 14.4, 17.7 / 17.4, 20.2 / 19.7.
     p.group = p.kc == 4 || (p.kc >= 7 && most > 4) ? 4 : 2;
     p.s2 = 4 / p.group;
   } else {

@@ -296,7 +296,7 @@ def _wavefront_pays(dtype, T, B, H, grad):
     most, these win (T=256: B=200, H=320 1.50 / 1.30; B=130, H=448 1.50 / 1.37; B=150, H=384 1.33 / 1.33, T=512 2.57 / 2.41; but
     B=400, H=256, 48 rows, 1.32 / 1.59; B=100, H=512, two chunks, 1.26 / 1.37).
     Resident weights gain from 128 steps on where half of the device holds them with two tiles of rows, 64 to a group of H / 32 CTAs at most
-    (T=128 and 256: B=128, H=512 0.91 / 0.81 and 1.73 / 1.40; B=440, H=320 0.98 / 0.98 and 1.87 / 1.75), the kernels
+    (T=128 and 256: B=128, H=512 0.81 / 0.65 and 1.56 / 1.17; B=448, H=320 0.90 / 0.82 and 1.75 / 1.53; B=128, H=1024 1.09 / 1.05 and 2.13 / 1.91), the kernels
     with several 128-row tiles always (T=128, B=1000, H=192: 1.31 / 1.05).  With three or four tiles a group on half of the device the
     layers stay one after the other, where the cell state is held in 32 bits over the whole sequence: as a wavefront the error of the
     output against 64 bits grows by 0.06 to 0.3 % (bf16 and fp16, T=512 and T=128).  It would gain at some of these sizes and lose at
